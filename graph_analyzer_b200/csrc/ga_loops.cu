@@ -26,14 +26,13 @@
 // back after each (the reference's host loop with its one sync per round).
 //
 // Small core rounds: most of the thousands of core rounds of a power-law graph are small (R-MAT scale 22: 9,543
-// rounds, two thirds with at most 32K alive vertices, the median destroying some 20K incidence entries), and a grid
-// round of three dependent kernels costs tens of microseconds of launch and drain latency whatever its size. In graph
-// mode the core round's body therefore starts with k_core_small_rounds, ONE thread block cluster (16 CTAs of 1,024
-// threads, 8 where 16 cannot be co-scheduled) that runs consecutive rounds itself - minimum, frontier, update, close -
-// with cluster barriers between the phases instead of kernel boundaries, for as long as the alive list holds at most
-// 8 vertices per cluster thread and the next round destroys at most kSmallWork incidence entries. The first round that does not fit
-// is left untouched for the grid kernels that follow in the same body; the loop decisions and every result are the
-// grid round's, so the output is unchanged.
+// rounds, nine in ten with at most 131,072 alive vertices, the median removing three), and a grid round of three
+// dependent kernels costs tens of microseconds of launch and drain latency whatever its size. In graph mode the core
+// round's body therefore starts with k_core_small_rounds, ONE thread block cluster (16 CTAs of 1,024 threads, 8 where
+// 16 cannot be co-scheduled) that keeps the whole loop state in its shared memory and runs consecutive rounds itself
+// with cluster barriers between the phases, for as long as the alive list fits its slots and the next round reads at
+// most kSmallWork incidence entries. The first round that does not fit is left untouched for the grid kernels that
+// follow in the same body; the loop decisions and every result are the grid round's, so the output is unchanged.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -103,6 +102,7 @@ struct ga_loops {
     uint32_t* out = nullptr;          // n: removed_round (peel) or core (core)
     uint32_t* alive[2] = {nullptr, nullptr};
     uint32_t* frontier[2] = {nullptr, nullptr};   // n each: the frontier of even / odd rounds
+    uint32_t* loc = nullptr;          // n, core loops: local ids of the cluster rounds (all ones outside them)
     uint32_t* item_x = nullptr;       // item capacity
     uint32_t* item_c = nullptr;
     uint64_t item_cap = 0;
@@ -126,11 +126,12 @@ struct ga_loops {
 namespace ga {
 
 __global__ void k_loop_init(uint8_t* __restrict__ state, uint32_t* __restrict__ out, uint32_t* __restrict__ alive0,
-                            uint32_t n) {
+                            uint32_t* __restrict__ loc, uint32_t n) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         state[v] = 1;
         out[v] = 0xFFFFFFFFu;
         alive0[v] = v;
+        if (loc) loc[v] = GA_EMPTY;
     }
 }
 
@@ -588,239 +589,367 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
     close_round_if_last(sc, kind, handle, use_handle, sg);
 }
 
-// ---- small core rounds in one thread block cluster ----------------------------------------------------------------
+// ---- core rounds of at most 131,072 alive vertices, in one thread block cluster ------------------------------------
+// R-MAT scale 22 runs 9,300 such rounds one after the other, each reading some 20-35K incidence entries of two to four
+// frontier vertices, so a round is bound by latency and by what 16 SMs can do with scattered accesses. It is kept to
+// two cluster barriers and one chain of global loads (incidence entry -> local id), the rest in shared memory:
+//   * alive vertex i of the list the cluster takes over gets local id i, held by CTA i % C in slot i / C: its triangle
+//     count, the start and the length of its incidence list. loc[v] maps a vertex to its local id (~0: not alive).
+//   * every CTA keeps a copy of all local vertices' states (2 bits each: alive, frontier, removed). The copies stay
+//     equal without communication, because every CTA sees the whole frontier.
+//   * level: a CTA finds the minimum of its own counts and its candidates (counts at or below max(level, own minimum))
+//     and writes both into an inbox of every CTA. After one cluster barrier every CTA has all minima and candidate
+//     lists, so all compute the same level, frontier and size of the round, and mark it in their own copy.
+//   * update: warps read slices of the frontier's lists. A round's decrements fall on about a thousand vertices, some
+//     forty each, and a decrement of another CTA's count costs an SM 3.3 cycles a lane, against 0.3 for one in its own
+//     shared memory (1.4 for one in L2), so a CTA first sums its decrements by vertex in a small hash table and then
+//     sends each sum once (red.shared::cluster); they are complete at the second barrier. The local ids are read
+//     through L1: a round's entries name each vertex many times.
+// R-MAT 22 cores: 147 ms with every decrement sent on its own, 235 ms with the round's state in global memory.
 constexpr uint32_t kSmallThreads = 1024;     // threads per CTA of the cluster
-constexpr uint32_t kSmallAlive = 1u << 16;   // alive vertices up to which a round may run in an 8-CTA cluster
-constexpr uint32_t kSmallWork = 1u << 17;    // incidence entries a round may destroy in the cluster
-constexpr uint32_t kSmallChunk = 64;         // incidence entries per update item of the cluster
+constexpr uint32_t kSmallSlots = 8192;       // local vertices per CTA (8 per thread): 131,072 with 16 CTAs
+constexpr uint32_t kSmallInbox = 128;        // candidates a CTA can publish per round
+constexpr uint32_t kSmallWork = 1u << 20;    // incidence entries a round may read in the cluster
+constexpr uint32_t kSmallMaxCtas = 16;
+constexpr uint32_t kSmallFront = kSmallMaxCtas * kSmallInbox;
+constexpr uint32_t kSmallSums = 4096;        // slots of a CTA's table of decrements (4 per thread at the flush)
+constexpr uint32_t kSmallSumsBits = 12, kSmallSumsTries = 8;
+constexpr uint32_t kSmallDead = 0xFFFFFFFFu; // count of a removed (or unused) slot
 
-// Alive entries per thread: a round runs in the cluster while its alive list fits 8 entries per thread, 65,536
-// vertices in an 8-CTA cluster and 131,072 in a 16-CTA one (R-MAT 22 cores: 233-236 ms against 245-248 ms with the
-// 65,536 limit for both sizes).
-constexpr uint32_t kSmallPer = kSmallAlive / (8 * kSmallThreads);
-static_assert(kSmallPer * 8 * kSmallThreads == kSmallAlive, "alive entries must split evenly over the threads");
-
-// The round's level and size in one reduction: the minimum triangle count over the alive list, the incidence entries
-// of the vertices at that minimum, and the incidence entries of the vertices at or below the current level.
-struct MinWork {
-    uint32_t mn;
-    unsigned long long at_min, at_level;
+// A frontier candidate: local id, incidence list (start: 34 bits, the upper two beside the length, which is capped -
+// a round with a capped list is over kSmallWork and never read here).
+struct alignas(16) SmallEntry {
+    uint32_t lid, len_hi, beg_lo, pad;
 };
+constexpr uint32_t kSmallLenMask = 0x3FFFFFFFu;
+struct SmallHead {    // a CTA's minimum count and number of candidates
+    uint32_t mn, count;
+};
+struct SmallShared {
+    uint32_t tri[kSmallSlots];
+    uint32_t beg_lo[kSmallSlots];
+    uint32_t len_hi[kSmallSlots];
+    uint32_t st[kSmallSlots * kSmallMaxCtas / 16];   // 2 bits per local vertex: 1 alive, 2 frontier, 0 removed
+    uint32_t sum_key[kSmallSums];                    // local id (GA_EMPTY: free) ...
+    uint32_t sum_cnt[kSmallSums];                    // ... and its decrements in this round
+    SmallEntry inbox[kSmallFront];
+    SmallHead head[kSmallMaxCtas];
+    uint16_t front[kSmallFront];                     // inbox positions of the round's frontier
+    uint32_t flid[2][kSmallFront];                   // its local ids, by round parity (retired in the next round)
+    uint32_t wmin[kSmallThreads / 32], wwork[kSmallThreads / 32];
+    unsigned long long destroyed;                    // triangles this CTA destroyed since the kernel started
+    uint32_t count, survivors;
+};
+static_assert(sizeof(SmallShared) <= 227 * 1024, "must fit an SM's shared memory");
 
-__device__ __forceinline__ MinWork combine(const MinWork& a, const MinWork& b) {
-    MinWork r;
-    r.mn = min(a.mn, b.mn);
-    r.at_min = (a.mn == r.mn ? a.at_min : 0ull) + (b.mn == r.mn ? b.at_min : 0ull);
-    r.at_level = a.at_level + b.at_level;
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t remote_addr(uint32_t addr, uint32_t cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
     return r;
 }
-
-__device__ __forceinline__ MinWork shfl_xor(const MinWork& a, int o) {
-    MinWork r;
-    r.mn = __shfl_xor_sync(GA_FULL_MASK, a.mn, o);
-    r.at_min = __shfl_xor_sync(GA_FULL_MASK, a.at_min, o);
-    r.at_level = __shfl_xor_sync(GA_FULL_MASK, a.at_level, o);
-    return r;
+__device__ __forceinline__ void remote_sub(uint32_t addr, uint32_t v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(0u - v) : "memory");
 }
 
-__device__ __forceinline__ MinWork warp_combine(MinWork x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = combine(x, shfl_xor(x, o));
-    return x;
-}
-
-// Cluster-wide MinWork: warps -> the CTA's slot (warp 0 combines the warps' parts), then after the cluster barrier
-// every warp combines the CTAs' slots, one distributed shared memory load per lane.
-__device__ __forceinline__ MinWork cluster_combine(cooperative_groups::cluster_group& cluster, MinWork x,
-                                                   MinWork* part, MinWork* slot) {
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const MinWork none = {0xFFFFFFFFu, 0ull, 0ull};
-    x = warp_combine(x);
-    if (lane == 0) part[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        x = warp_combine(lane < blockDim.x / 32 ? part[lane] : none);
-        if (lane == 0) *slot = x;
+// One decrement of local vertex `lid`: summed in the CTA's table, or sent at once when its bucket run is full.
+__device__ __forceinline__ void small_dec(SmallShared& s, uint32_t tri0, uint32_t lid, uint32_t C, uint32_t cbits) {
+    uint32_t h = hash_slot(lid, kSmallSumsBits);
+    for (uint32_t t = 0; t < kSmallSumsTries; t++) {
+        uint32_t key = *(volatile uint32_t*)&s.sum_key[h];
+        if (key == GA_EMPTY) key = atomicCAS(&s.sum_key[h], GA_EMPTY, lid);
+        if (key == GA_EMPTY || key == lid) {
+            atomicAdd(&s.sum_cnt[h], 1u);
+            return;
+        }
+        h = (h + 1) & (kSmallSums - 1);
     }
-    cluster.sync();
-    x = lane < cluster.num_blocks() ? *cluster.map_shared_rank(slot, lane) : none;
-    return warp_combine(x);
+    remote_sub(remote_addr(tri0 + 4 * (lid >> cbits), lid & (C - 1)), 1u);
 }
-
-// Counters of one cluster round, in rank 0's shared memory (two sets, alternating by round).
-struct SmallCounters {
-    uint32_t frontier, items, survivors, pad;
-    unsigned long long destroyed;
-};
 
 // Runs consecutive core rounds (the work of k_core_min, k_core_mark, k_frontier_update_list and close_round_if_last
-// for LOOP_CORE) inside one cluster while the alive list has at most kSmallPer vertices per thread and a round destroys at
-// most kSmallWork incidence entries; returns at the first round that is larger (untouched, for the grid kernels),
-// when the loop ends (the WHILE condition is set to 0) or at a status other than LS_OK.
-//
-// A round is one pass over the alive list, whose entries (vertex, triangle count, incidence length) each thread
-// keeps in registers from the level's reduction to the mark, and three cluster barriers: after the level reduction,
-// after the mark, after the update. Every thread carries the loop state (level, parity, alive and triangle totals,
-// status) in registers and computes the close itself from the same counters, so every decision to stay or leave is
-// the same in all CTAs; thread 0 of rank 0 writes the state back for the grid kernels. The round's counters live in
-// rank 0's shared memory in two sets by round parity; the set a round uses was last read before the round's first
-// barrier, after which rank 0 clears the other one. Arrays that other CTAs write between phases are read with
-// ld.global.cg (L2).
+// for LOOP_CORE) inside one cluster of C CTAs while the alive list fits the CTAs' slots, a round reads at most
+// kSmallWork incidence entries and no CTA has more than kSmallInbox candidates; returns at the first round that is
+// larger (untouched, for the grid kernels, which find tri[], state[] and the alive list as if they had run the rounds
+// before), when the loop ends (the WHILE condition is set to 0) or at a status other than LS_OK. Every decision is
+// computed by every thread from values all CTAs hold identically, so all CTAs leave in the same round.
 __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
     LoopScalars* sc, uint32_t* __restrict__ tri, uint8_t* __restrict__ state, uint32_t* __restrict__ core,
-    uint32_t* alive0, uint32_t* alive1, uint32_t* fr0, uint32_t* fr1, uint32_t* __restrict__ item_x,
-    uint32_t* __restrict__ item_c, const uint2* __restrict__ inc, const unsigned long long* __restrict__ inc_ptr,
+    uint32_t* alive0, uint32_t* alive1, const uint32_t* fr0, const uint32_t* fr1, uint32_t* loc,
+    const uint2* __restrict__ inc, const unsigned long long* __restrict__ inc_ptr,
     cudaGraphConditionalHandle handle) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    __shared__ MinWork s_part[kSmallThreads / 32];
-    __shared__ MinWork s_slot;
-    __shared__ SmallCounters s_cnt[2];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t tid = cluster.block_rank() * blockDim.x + threadIdx.x;
-    const uint32_t nthr = cluster.num_blocks() * blockDim.x;
-    const uint32_t gwarp = tid >> 5, nwarps = nthr >> 5;
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    SmallShared& s = *reinterpret_cast<SmallShared*>(small_raw);
+    const uint32_t C = cluster.num_blocks(), rank = cluster.block_rank(), cbits = 31 - __clz(C);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t tid = rank * kSmallThreads + threadIdx.x, nthr = C * kSmallThreads;
+    const uint32_t gwarp = warp * C + rank, nwarps = nthr >> 5;   // consecutive slices go to different CTAs
     const bool writer = tid == 0;
-    if (threadIdx.x < 2) s_cnt[threadIdx.x] = SmallCounters{0, 0, 0, 0, 0ull};
-    // the state the grid kernels (or the loop's set-up) left; nothing writes it until the first close
-    volatile LoopScalars* vs = sc;
-    uint32_t cont = vs->cont, p = vs->parity, round = vs->round, fprev = vs->fprev, kcur = vs->kcur;
-    uint32_t na = vs->alive_count[vs->parity], status = vs->status, iters = vs->iters;
-    const uint32_t max_rounds = vs->max_rounds;
-    unsigned long long nalive = vs->nalive, T = vs->T;
-    cluster.sync();
-    SmallCounters* cnt0 = cluster.map_shared_rank(s_cnt, 0);
-    for (;;) {
-        if (!cont) {   // the loop is over: the WHILE node must stop whoever cleared `cont`
-            if (writer) cudaGraphSetConditional(handle, 0);
-            break;
-        }
-        if (na > kSmallPer * nthr) break;   // kSmallAlive with 8 CTAs, twice that with 16
-        uint32_t* in = p ? alive1 : alive0;
-        uint32_t* outl = p ? alive0 : alive1;
-        uint32_t* frontier = (round & 1) ? fr1 : fr0;
+    // the state the grid kernels (or the loop's set-up) left; nothing writes it until the cluster leaves
+    const uint32_t p = sc->parity, na0 = sc->alive_count[p];
+    const uint32_t max_rounds = sc->max_rounds;
+    uint32_t cont = sc->cont, round = sc->round, kcur = sc->kcur, status = sc->status, iters = sc->iters;
+    unsigned long long nalive = sc->nalive;
+    if (!cont) {   // the loop is over: the WHILE node must stop whoever cleared `cont`
+        if (writer) cudaGraphSetConditional(handle, 0);
+        return;
+    }
+    if (na0 > kSmallSlots * C) return;
+    uint32_t* in = p ? alive1 : alive0;
+    uint32_t* outl = p ? alive0 : alive1;
+    {   // the previous grid round's frontier leaves for good (the grid kernels do it again: idempotent)
         const uint32_t* prev = (round & 1) ? fr0 : fr1;
-        SmallCounters* cnt = cnt0 + (round & 1);
-        // retire the previous round's frontier (the grid kernels do it again if they take this round: idempotent)
-        for (uint32_t i = tid; i < fprev; i += nthr) state[__ldcg(prev + i)] = 0;
-        // this thread's alive entries, all loads in flight together
-        uint32_t v[kSmallPer], t[kSmallPer], d[kSmallPer];
-#pragma unroll
-        for (uint32_t j = 0; j < kSmallPer; j++) {
-            const uint32_t i = tid + j * nthr;
-            v[j] = i < na ? __ldcg(in + i) : 0u;
+        const uint32_t fprev = sc->fprev;
+        for (uint32_t i = tid; i < fprev; i += nthr) state[prev[i]] = 0;
+    }
+    if (threadIdx.x == 0) {
+        s.destroyed = 0;
+        s.survivors = 0;
+        s.count = 0;
+    }
+    for (uint32_t h = threadIdx.x; h < kSmallSums; h += kSmallThreads) {
+        s.sum_key[h] = GA_EMPTY;
+        s.sum_cnt[h] = 0;
+    }
+    for (uint32_t w = threadIdx.x; w < kSmallSlots * C / 16; w += kSmallThreads) {
+        const uint32_t left = na0 > 16 * w ? na0 - 16 * w : 0;   // local vertices of this word: all alive
+        s.st[w] = left >= 16 ? 0x55555555u : 0x55555555u & ((1u << (2 * left)) - 1);
+    }
+    for (uint32_t slot = threadIdx.x; slot < kSmallSlots; slot += kSmallThreads) {
+        const uint32_t i = slot * C + rank;
+        uint32_t t = kSmallDead, lh = 0;
+        unsigned long long b = 0;
+        if (i < na0) {
+            const uint32_t v = in[i];
+            t = tri[v];
+            b = inc_ptr[v];
+            lh = (uint32_t)min(inc_ptr[v + 1] - b, (unsigned long long)kSmallLenMask) | (uint32_t)(b >> 32) << 30;
+            loc[v] = i;
         }
-#pragma unroll
-        for (uint32_t j = 0; j < kSmallPer; j++) {
-            const bool valid = tid + j * nthr < na;
-            t[j] = valid ? __ldcg(tri + v[j]) : 0xFFFFFFFFu;
-            d[j] = valid ? (uint32_t)(inc_ptr[v[j] + 1] - inc_ptr[v[j]]) : 0u;
+        s.tri[slot] = t;
+        s.beg_lo[slot] = (uint32_t)b;
+        s.len_hi[slot] = lh;
+    }
+    __threadfence();
+    cluster.sync();   // loc[] is complete, and every CTA runs before its shared memory is written from others
+    const uint32_t tri0 = smem_addr(s.tri);
+    uint32_t done = 0, fprev = 0;   // rounds run here, the last one's frontier
+    while (cont) {
+        // the last round's frontier leaves the states
+        for (uint32_t f = threadIdx.x; f < fprev; f += kSmallThreads) {
+            const uint32_t lid = s.flid[(done & 1) ^ 1][f];
+            atomicAnd(&s.st[lid >> 4], ~(3u << (2 * (lid & 15))));
         }
-        // k = max(k, min over alive of tri); the round's size = incidence entries of {alive v : tri[v] <= k}
-        MinWork mw = {0xFFFFFFFFu, 0ull, 0ull};
+        // this CTA's minimum (scan of 8 slots per thread) and candidates, published to every CTA
+        const uint4 t0 = reinterpret_cast<const uint4*>(s.tri)[threadIdx.x];
+        const uint4 t1 = reinterpret_cast<const uint4*>(s.tri)[threadIdx.x + kSmallThreads];
+        const uint32_t mine = min(min(min(t0.x, t0.y), min(t0.z, t0.w)), min(min(t1.x, t1.y), min(t1.z, t1.w)));
+        const uint32_t wm = __reduce_min_sync(GA_FULL_MASK, mine);
+        if (lane == 0) s.wmin[warp] = wm;
+        __syncthreads();
+        const uint32_t bmin = __reduce_min_sync(GA_FULL_MASK, s.wmin[lane]);
+        const uint32_t thr = max(kcur, bmin);
+        if (bmin != kSmallDead && mine <= thr) {
+            const uint32_t ts[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
-        for (uint32_t j = 0; j < kSmallPer; j++) {
-            mw = combine(mw, MinWork{t[j], d[j], t[j] <= kcur ? d[j] : 0u});
-        }
-        mw = cluster_combine(cluster, mw, s_part, &s_slot);
-        const uint32_t k = max(kcur, mw.mn);
-        const unsigned long long work = mw.mn >= kcur ? mw.at_min : mw.at_level;
-        if (work > kSmallWork) break;   // the grid kernels take this round
-        if (writer) cnt0[(round & 1) ^ 1] = SmallCounters{0, 0, 0, 0, 0ull};   // the next round's set
-        // frontier and survivors (k_core_mark), with update items of kSmallChunk entries
-#pragma unroll
-        for (uint32_t j = 0; j < kSmallPer; j++) {
-            if (tid - lane + j * nthr >= na) break;   // the warp's entries of this slice are all past the list
-            const bool valid = tid + j * nthr < na;
-            const bool rem = valid && t[j] <= k;
-            if (rem) {
-                state[v[j]] = 2;
-                core[v[j]] = k;
+            for (int j = 0; j < 8; j++) {
+                if (ts[j] > thr) continue;
+                const uint32_t slot = 4 * threadIdx.x + (j & 3) + (j >> 2) * 4 * kSmallThreads;
+                const uint32_t at = atomicAdd(&s.count, 1u);
+                if (at >= kSmallInbox) continue;   // counted: the round goes to the grid kernels
+                const uint32_t a = smem_addr(&s.inbox[rank * kSmallInbox + at]);
+                const uint32_t lid = slot * C + rank, lh = s.len_hi[slot], bl = s.beg_lo[slot];
+                for (uint32_t c = 0; c < C; c++)
+                    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(remote_addr(a, c)),
+                                 "r"(lid), "r"(lh), "r"(bl), "r"(0u)
+                                 : "memory");
             }
-            uint32_t bal = __ballot_sync(GA_FULL_MASK, rem);
-            if (bal) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&cnt->frontier, (uint32_t)__popc(bal));
-                base = __shfl_sync(GA_FULL_MASK, base, 0);
-                const uint32_t nc = rem ? (uint32_t)(((unsigned long long)d[j] + kSmallChunk - 1) / kSmallChunk) : 0u;
-                if (rem) frontier[base + __popc(bal & ((1u << lane) - 1))] = v[j];
-                const uint32_t incl = warp_incl_scan(nc, lane);
-                const uint32_t tot = __shfl_sync(GA_FULL_MASK, incl, 31);
-                uint32_t ib = 0;
-                if (lane == 31 && tot) ib = atomicAdd(&cnt->items, tot);
-                ib = __shfl_sync(GA_FULL_MASK, ib, 31);
-                for (uint32_t c = 0; c < nc; c++) {
-                    item_x[ib + incl - nc + c] = v[j];
-                    item_c[ib + incl - nc + c] = c;
+        }
+        __syncthreads();
+        if (threadIdx.x < C)
+            asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(
+                             remote_addr(smem_addr(&s.head[rank]), threadIdx.x)),
+                         "r"(bmin), "r"(s.count)
+                         : "memory");
+        cluster.sync();
+        // level, frontier and size of the round: the same in every warp of the cluster
+        if (threadIdx.x == 0) s.count = 0;
+        const SmallHead h = lane < C ? s.head[lane] : SmallHead{kSmallDead, 0};
+        const uint32_t gmin = __reduce_min_sync(GA_FULL_MASK, h.mn);
+        const uint32_t k = max(kcur, gmin);
+        // every count <= k is a candidate of its CTA exactly when the CTA's minimum is <= k
+        const uint32_t cnt = h.mn <= k && h.mn != kSmallDead ? h.count : 0u;
+        if (__any_sync(GA_FULL_MASK, cnt > kSmallInbox)) break;   // the grid kernels take this round
+        const uint32_t incl = warp_incl_scan(cnt, lane);
+        const uint32_t F = __shfl_sync(GA_FULL_MASK, incl, 31);
+        uint32_t* flid = s.flid[done & 1];
+        // the frontier's inbox positions, in order. Up to 32 vertices (almost every round) every warp finds them for
+        // itself; more are spread over the block.
+        const bool wide = F > 32;
+        SmallEntry e = {0, 0, 0, 0};
+        uint32_t work = 0;   // capped lengths: a sum over at most 2,048 lists fits 32 bits
+        for (uint32_t f0 = wide ? 32 * warp : 0; f0 < F; f0 += kSmallThreads) {   // warp-uniform
+            const uint32_t f = f0 + lane;
+            uint32_t c = 0, before = 0;
+            for (uint32_t q = 0; q < C; q++) {
+                const uint32_t end = __shfl_sync(GA_FULL_MASK, incl, q);
+                if (end <= f) { c = q + 1; before = end; }
+            }
+            if (f < F) {
+                const uint32_t at = c * kSmallInbox + (f - before);
+                e = s.inbox[at];
+                work += min(e.len_hi & kSmallLenMask, kSmallWork + 1);
+                if (wide || warp == 0) {
+                    s.front[f] = (uint16_t)at;
+                    flid[f] = e.lid;
                 }
             }
-            const bool keep = valid && !rem;
-            bal = __ballot_sync(GA_FULL_MASK, keep);
-            if (bal) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&cnt->survivors, (uint32_t)__popc(bal));
-                base = __shfl_sync(GA_FULL_MASK, base, 0);
-                if (keep) outl[base + __popc(bal & ((1u << lane) - 1))] = v[j];
+        }
+        work = __reduce_add_sync(GA_FULL_MASK, work);
+        if (wide) {
+            if (lane == 0) s.wwork[warp] = work;
+            __syncthreads();
+            work = __reduce_add_sync(GA_FULL_MASK, min(s.wwork[lane], kSmallWork + 1));
+        }
+        if (work > kSmallWork) break;    // the grid kernels take this round
+        const bool last = F == nalive;   // nothing survives: no count is left to update
+        // mark the frontier in this CTA's copy; its owner also takes it out of the counts and writes its core number
+        for (uint32_t f = threadIdx.x; f < F; f += kSmallThreads) {
+            const uint32_t lid = wide ? flid[f] : e.lid;
+            atomicXor(&s.st[lid >> 4], 3u << (2 * (lid & 15)));   // 1 -> 2
+            if ((lid & (C - 1)) == rank) {
+                s.tri[lid >> cbits] = kSmallDead;
+                const uint32_t v = in[lid];
+                core[v] = k;
+                state[v] = 0;
             }
         }
-        __threadfence();
-        cluster.sync();
-        const uint32_t F = cnt->frontier, nitems = cnt->items;
-        // update (k_frontier_update_list): each destroyed triangle once, by its smallest-id frontier corner
-        unsigned long long destroyed = 0;
-        for (uint32_t it = gwarp; it < nitems; it += nwarps) {
-            const uint32_t x = __ldcg(item_x + it);
-            const unsigned long long b = inc_ptr[x] + (unsigned long long)__ldcg(item_c + it) * kSmallChunk;
-            const unsigned long long e = min(inc_ptr[x + 1], b + kSmallChunk);
-            for (unsigned long long i = b + lane; i < e; i += 32) {
-                const uint2 yw = inc[i];
-                const uint8_t sy = __ldcg(state + yw.x), sw = __ldcg(state + yw.y);
-                if (!sy || !sw) continue;
-                if ((sy == 2 && yw.x < x) || (sw == 2 && yw.y < x)) continue;
-                destroyed++;
-                if (sy == 1) atomicSub(&tri[yw.x], 1u);
-                if (sw == 1) atomicSub(&tri[yw.y], 1u);
+        __syncthreads();
+        // update (k_frontier_update_list): each destroyed triangle once, by its smallest frontier corner
+        if (!last) {
+            const uint32_t per = (work + nthr - 1) / nthr;   // entries per lane
+            const uint32_t chunk = 32 * min(max(per, 1u), 8u);
+            uint32_t destroyed = 0, base = 0;
+            for (uint32_t f0 = 0; f0 < F; f0 += 32) {
+                if (wide) {
+                    e = SmallEntry{0, 0, 0, 0};
+                    if (f0 + lane < F) e = s.inbox[s.front[f0 + lane]];
+                }
+                const uint32_t len = e.len_hi & kSmallLenMask;
+                const uint32_t nc = (len + chunk - 1) / chunk;
+                const uint32_t ci = warp_incl_scan(nc, lane);
+                const uint32_t tot = __shfl_sync(GA_FULL_MASK, ci, 31);
+                // this warp's slices j (numbered over the whole frontier): j = gwarp mod nwarps
+                for (uint32_t j = (gwarp - base) & (nwarps - 1); j < tot; j += nwarps) {
+                    const uint32_t o = __ffs(__ballot_sync(GA_FULL_MASK, ci > j)) - 1;
+                    const uint32_t x = __shfl_sync(GA_FULL_MASK, e.lid, o);
+                    const uint32_t xl = __shfl_sync(GA_FULL_MASK, len, o);
+                    const uint32_t first = (j - __shfl_sync(GA_FULL_MASK, ci - nc, o)) * chunk;
+                    const unsigned long long b = (unsigned long long)(__shfl_sync(GA_FULL_MASK, e.len_hi, o) >> 30) << 32 |
+                                                 __shfl_sync(GA_FULL_MASK, e.beg_lo, o);
+                    const uint2* list = inc + b;
+                    const uint32_t end = min(xl, first + chunk);
+                    for (uint32_t i = first + lane; i < end; i += 128) {
+                        uint2 yw[4];
+                        uint32_t ly[4], lw[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            if (i + 32 * q < end) yw[q] = __ldcs(list + i + 32 * q);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const bool in_list = i + 32 * q < end;
+                            ly[q] = in_list ? __ldca(loc + yw[q].x) : GA_EMPTY;
+                            lw[q] = in_list ? __ldca(loc + yw[q].y) : GA_EMPTY;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (ly[q] == GA_EMPTY || lw[q] == GA_EMPTY) continue;   // removed before the cluster began
+                            const uint32_t sy = (s.st[ly[q] >> 4] >> (2 * (ly[q] & 15))) & 3;
+                            const uint32_t sw = (s.st[lw[q] >> 4] >> (2 * (lw[q] & 15))) & 3;
+                            if (!sy || !sw) continue;
+                            if ((sy == 2 && ly[q] < x) || (sw == 2 && lw[q] < x)) continue;
+                            destroyed++;
+                            if (sy == 1) small_dec(s, tri0, ly[q], C, cbits);
+                            if (sw == 1) small_dec(s, tri0, lw[q], C, cbits);
+                        }
+                    }
+                }
+                base += tot;
+            }
+            destroyed = __reduce_add_sync(GA_FULL_MASK, destroyed);
+            if (lane == 0 && destroyed) atomicAdd(&s.destroyed, (unsigned long long)destroyed);
+            __syncthreads();
+            // send the sums and clear the table
+            uint4* keys = reinterpret_cast<uint4*>(s.sum_key) + threadIdx.x;
+            const uint4 kq = *keys;
+            if ((kq.x & kq.y & kq.z & kq.w) != GA_EMPTY) {
+                uint4* cnts = reinterpret_cast<uint4*>(s.sum_cnt) + threadIdx.x;
+                const uint4 cq = *cnts;
+                const uint32_t ks[4] = {kq.x, kq.y, kq.z, kq.w}, cs[4] = {cq.x, cq.y, cq.z, cq.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (ks[q] != GA_EMPTY)
+                        remote_sub(remote_addr(tri0 + 4 * (ks[q] >> cbits), ks[q] & (C - 1)), cs[q]);
+                *keys = make_uint4(GA_EMPTY, GA_EMPTY, GA_EMPTY, GA_EMPTY);
+                *cnts = make_uint4(0, 0, 0, 0);
             }
         }
-        destroyed = warp_sum_u64(destroyed);
-        if (lane == 0 && destroyed) atomicAdd(&cnt->destroyed, destroyed);
-        __threadfence();
         cluster.sync();
         // close (close_round_if_last for LOOP_CORE), the same in every thread
-        const unsigned long long des = cnt->destroyed;
-        const uint32_t survivors = cnt->survivors;
         if (F == 0 && nalive > 0) status = LS_NO_PROGRESS;
         if (F > nalive) status = LS_OVER_REMOVED;
-        if (des > T) status = LS_OVER_REMOVED;
-        if (k < kcur) status = LS_LEVEL_DOWN;
         nalive -= min((unsigned long long)F, nalive);
-        T -= min(des, T);
         iters++;
         if (iters > max_rounds + 1) status = LS_ROUND_LIMIT;   // count_iteration's bound
         if (status == LS_OK && nalive > 0 && round + 1 >= max_rounds) status = LS_ROUND_LIMIT;
         cont = (status == LS_OK && nalive > 0 && iters <= max_rounds) ? 1u : 0u;
-        if (writer) {   // the state the grid kernels read (their counters are untouched by the cluster: zero)
-            vs->nalive = nalive;
-            vs->T = T;
-            vs->kcur = k;
-            vs->kround = k;
-            vs->round = round + 1;
-            vs->parity = p ^ 1;
-            vs->alive_count[p] = 0;
-            vs->alive_count[p ^ 1] = survivors;
-            vs->fprev = F;
-            vs->iters = iters;
-            vs->status = status;
-            vs->cont = cont;
-            if (!cont) cudaGraphSetConditional(handle, 0);
-        }
         kcur = k;
         round++;
-        p ^= 1;
+        done++;
         fprev = F;
-        na = survivors;
     }
-    cluster.sync();   // no CTA leaves while another may still read its shared memory
+    // leave: local ids end; with rounds run, the survivors' counts, list and the loop state go back to global memory
+    uint32_t* survivors = cluster.map_shared_rank(&s.survivors, 0);
+    for (uint32_t s0 = 32 * warp; s0 * C < na0; s0 += kSmallThreads) {   // warp-uniform
+        const uint32_t slot = s0 + lane;
+        const bool used = slot * C + rank < na0;
+        const uint32_t v = used ? in[slot * C + rank] : 0u, t = used ? s.tri[slot] : kSmallDead;
+        if (used) loc[v] = GA_EMPTY;
+        const bool keep = done && t != kSmallDead;
+        const uint32_t bal = __ballot_sync(GA_FULL_MASK, keep);
+        uint32_t at = 0;
+        if (lane == 0 && bal) at = atomicAdd(survivors, (uint32_t)__popc(bal));
+        at = __shfl_sync(GA_FULL_MASK, at, 0);
+        if (keep) {
+            tri[v] = t;
+            outl[at + __popc(bal & ((1u << lane) - 1))] = v;
+        }
+    }
+    __syncthreads();
+    if (done && threadIdx.x == 0 && rank != 0 && s.destroyed)
+        atomicAdd(cluster.map_shared_rank(&s.destroyed, 0), s.destroyed);
+    cluster.sync();   // the sums are complete; no CTA leaves while another may still write its shared memory
+    if (writer && done) {
+        const unsigned long long T = sc->T, des = s.destroyed;
+        if (des > T) status = LS_OVER_REMOVED;
+        if (status == LS_OK && s.survivors != (uint32_t)nalive) status = LS_OVER_REMOVED;
+        if (status != LS_OK) cont = 0;
+        sc->nalive = nalive;
+        sc->T = nalive == 0 ? 0ull : T - min(des, T);   // the last round takes what is left
+        sc->kcur = kcur;
+        sc->kround = kcur;
+        sc->round = round;
+        sc->parity = p ^ 1;
+        sc->alive_count[p] = 0;
+        sc->alive_count[p ^ 1] = s.survivors;
+        sc->fprev = 0;   // every frontier of these rounds is retired
+        sc->iters = iters;
+        sc->status = status;
+        sc->cont = cont;
+        if (!cont) cudaGraphSetConditional(handle, 0);
+    }
 }
 
 // Cluster size for k_core_small_rounds: 16 CTAs where 16 can be co-scheduled, else 8 (0: neither).
@@ -832,6 +961,7 @@ static int small_round_cluster(int device) {
     if (cached[device]) return cached[device] > 0 ? cached[device] : 0;
     int best = -1;
     cudaFuncSetAttribute(k_core_small_rounds, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_core_small_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared));
     for (int c : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -841,6 +971,7 @@ static int small_round_cluster(int device) {
         attr[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3(c);
         cfg.blockDim = dim3(kSmallThreads);
+        cfg.dynamicSmemBytes = sizeof(SmallShared);
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
@@ -961,8 +1092,8 @@ void reset_loops(ga_graph* g) {
     ga_loops* L = g->loops;
     if (!L) return;
     cudaStreamSynchronize(g->stream);
-    void* bufs[] = {L->tri, L->state, L->out, L->alive[0], L->alive[1], L->frontier[0], L->frontier[1], L->item_x,
-                    L->item_c, L->sc,
+    void* bufs[] = {L->tri, L->state, L->out, L->alive[0], L->alive[1], L->frontier[0], L->frontier[1], L->loc,
+                    L->item_x, L->item_c, L->sc,
                     L->inc, L->inc_ptr, L->segs.T, L->segs.nalive, L->segs.removed, L->segs.destroyed,
                     L->segs.best_num, L->segs.best_den, L->segs.T0, L->segs.best_round, L->segs.rounds,
                     L->segs.status};
@@ -992,8 +1123,7 @@ static ga_status build_lists(ga_graph* g, uint64_t T0) {
     cudaStream_t st = g->stream;
     const uint32_t n = g->n;
     const uint64_t entries = 3 * T0;
-    // the grid rounds' items (kListChunk entries) and a cluster round's (kSmallChunk entries, at most kSmallWork)
-    const uint64_t need_items = (uint64_t)n + std::max<uint64_t>(entries / kListChunk, kSmallWork / kSmallChunk) + 1;
+    const uint64_t need_items = (uint64_t)n + entries / kListChunk + 1;
     ga_status s = dalloc(g, &L->inc_ptr, (size_t)n + 1);
     if (s == GA_OK) s = dalloc(g, &L->inc, entries ? entries : 1);
     uint32_t *ix = nullptr, *ic = nullptr;
@@ -1064,12 +1194,14 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
             attr[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3(csize);
             cfg.blockDim = dim3(kSmallThreads);
+            cfg.dynamicSmemBytes = sizeof(SmallShared);
             cfg.stream = st;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             GA_CUDA(cudaLaunchKernelEx(&cfg, k_core_small_rounds, L->sc, L->tri, L->state, L->out, L->alive[0],
-                                       L->alive[1], L->frontier[0], L->frontier[1], L->item_x, L->item_c,
-                                       (const uint2*)L->inc, (const unsigned long long*)L->inc_ptr, h));
+                                       L->alive[1], (const uint32_t*)L->frontier[0],
+                                       (const uint32_t*)L->frontier[1], L->loc, (const uint2*)L->inc,
+                                       (const unsigned long long*)L->inc_ptr, h));
         }
         k_core_min<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->alive[0], L->alive[1], L->state, L->frontier[0],
                                                  L->frontier[1], h, use_h);
@@ -1137,6 +1269,7 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     cudaStream_t st = g->stream;
     L->cores_in_out = false;   // out[] is rewritten below
     const uint32_t n = g->n;
+    if (KIND == LOOP_CORE && !L->loc) GA_TRY(dalloc(g, &L->loc, n));
     // tri[] = triangles per vertex on the whole graph (uint32 counters; T < 2^32 is checked below): the list lengths
     // when the incidence lists exist, else one per-vertex triangle pass
     if (L->lists == 1) {
@@ -1149,7 +1282,8 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
         GA_TRY((run_tc<TC_VSUP, false, unsigned int>(g, a, true)));
     }
     if (n) {
-        k_loop_init<<<grid_for(n, 256), 256, 0, st>>>(L->state, L->out, L->alive[0], n);
+        k_loop_init<<<grid_for(n, 256), 256, 0, st>>>(L->state, L->out, L->alive[0],
+                                                      KIND == LOOP_CORE ? L->loc : nullptr, n);
         GA_CUDA(cudaGetLastError());
     }
     GA_CUDA(cudaMemcpyAsync(g->h_scalars, g->d_scalars, 8, cudaMemcpyDeviceToHost, st));

@@ -231,3 +231,28 @@ def test_core_level_density_every_level(ga, oracle, golden, cuda_ok, kernel):
             d.set_option(ga.OPT_TC_KERNEL, kernel)
             for k in sorted(set(core.tolist()) | {0, kmax + 1}):
                 assert d.core_level_density(core, k) == oracle.core_level_density(g, core, k), k
+
+
+@pytest.mark.parametrize("shape", ["hk-131060", "hk-131072", "hk-131090", "rmat-15", "cliques-2046", "cliques-2049",
+                                   "cliques-40000"])
+def test_core_rounds_at_cluster_limits(ga, oracle, cuda_ok, shape):
+    """Core rounds around the limits of the cluster kernel: alive lists at its 131,072 slots, rounds whose frontier
+    is at and just above the 2,048 candidates its CTAs can publish, rounds that alternate with grid rounds."""
+    kind, k = shape.split("-")
+    k = int(k)
+    if kind == "hk":
+        g = ga.graph_from_pairs(k, ga.gen_holme_kim(k, 4, 7, 0.5, 0.6, seed=11))
+    elif kind == "rmat":
+        g = ga.graph_from_pairs(1 << k, ga.gen_rmat(k, 12 << k, seed=3))
+    else:   # k vertices in triangles (one round of k at level 1), then cliques of 4 to 40 vertices (a round each)
+        e = [(3 * t + a, 3 * t + b) for t in range(k // 3) for a, b in ((0, 1), (0, 2), (1, 2))]
+        at = 3 * (k // 3)
+        for size in range(4, 41):
+            e += [(at + a, at + b) for a in range(size) for b in range(a + 1, size)]
+            at += size
+        g = ga.build_graph_from_edges(at, np.array(e, np.uint32))
+    core, kmax, rounds = oracle.core_levels_inc(g)
+    with ga.DeviceGraph(g) as d:
+        for _ in range(2):       # again, on the state the first run left
+            r = d.core_decomposition()
+            assert (r.kmax, r.rounds) == (kmax, rounds) and np.array_equal(r.core, core)
