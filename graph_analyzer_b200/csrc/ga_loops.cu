@@ -622,6 +622,7 @@ struct alignas(16) SmallEntry {
     uint32_t lid, len_hi, beg_lo, pad;
 };
 constexpr uint32_t kSmallLenMask = 0x3FFFFFFFu;
+constexpr uint32_t kSmallPrefetch = 1u << 15;   // entries of a candidate's list brought to L2
 struct SmallHead {    // a CTA's minimum count and number of candidates
     uint32_t mn, count;
 };
@@ -632,7 +633,8 @@ struct SmallShared {
     uint32_t st[kSmallSlots * kSmallMaxCtas / 16];   // 2 bits per local vertex: 1 alive, 2 frontier, 0 removed
     uint32_t sum_key[kSmallSums];                    // local id (GA_EMPTY: free) ...
     uint32_t sum_cnt[kSmallSums];                    // ... and its decrements in this round
-    SmallEntry inbox[kSmallFront];
+    SmallEntry own[kSmallInbox];                     // this CTA's candidates
+    SmallEntry inbox[kSmallFront];                   // every CTA's
     SmallHead head[kSmallMaxCtas];
     uint16_t front[kSmallFront];                     // inbox positions of the round's frontier
     uint32_t flid[2][kSmallFront];                   // its local ids, by round parity (retired in the next round)
@@ -736,12 +738,19 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
     cluster.sync();   // loc[] is complete, and every CTA runs before its shared memory is written from others
     const uint32_t tri0 = smem_addr(s.tri);
     uint32_t done = 0, fprev = 0;   // rounds run here, the last one's frontier
-    while (cont) {
-        // the last round's frontier leaves the states
-        for (uint32_t f = threadIdx.x; f < fprev; f += kSmallThreads) {
+    // the last round's frontier (F vertices at level k): out of the states, core numbers written by the owners
+    auto retire = [&](uint32_t F, uint32_t k) {
+        for (uint32_t f = threadIdx.x; f < F; f += kSmallThreads) {
             const uint32_t lid = s.flid[(done & 1) ^ 1][f];
             atomicAnd(&s.st[lid >> 4], ~(3u << (2 * (lid & 15))));
+            if ((lid & (C - 1)) == rank) {
+                const uint32_t v = in[lid];
+                core[v] = k;
+                state[v] = 0;
+            }
         }
+    };
+    while (cont) {
         // this CTA's minimum (scan of 8 slots per thread) and candidates, published to every CTA
         const uint4 t0 = reinterpret_cast<const uint4*>(s.tri)[threadIdx.x];
         const uint4 t1 = reinterpret_cast<const uint4*>(s.tri)[threadIdx.x + kSmallThreads];
@@ -759,21 +768,35 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
                 const uint32_t slot = 4 * threadIdx.x + (j & 3) + (j >> 2) * 4 * kSmallThreads;
                 const uint32_t at = atomicAdd(&s.count, 1u);
                 if (at >= kSmallInbox) continue;   // counted: the round goes to the grid kernels
-                const uint32_t a = smem_addr(&s.inbox[rank * kSmallInbox + at]);
-                const uint32_t lid = slot * C + rank, lh = s.len_hi[slot], bl = s.beg_lo[slot];
-                for (uint32_t c = 0; c < C; c++)
-                    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(remote_addr(a, c)),
-                                 "r"(lid), "r"(lh), "r"(bl), "r"(0u)
+                const uint32_t lh = s.len_hi[slot], bl = s.beg_lo[slot];
+                s.own[at] = SmallEntry{slot * C + rank, lh, bl, 0};
+                // its list is wanted in this round or in one soon after: from DRAM to L2 while the level is agreed on
+                const uint32_t bytes = min(lh & kSmallLenMask, kSmallPrefetch) * 8u & ~15u;
+                const char* list = (const char*)(inc + ((unsigned long long)(lh >> 30) << 32 | bl));
+                if (bytes)
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((uint64_t)list & ~15ull), "r"(bytes)
                                  : "memory");
             }
         }
         __syncthreads();
+        const uint32_t mycount = s.count;
+        for (uint32_t i = threadIdx.x; i < min(mycount, kSmallInbox) * C; i += kSmallThreads) {   // (candidate, CTA)
+            const uint32_t at = i >> cbits;
+            const SmallEntry e = s.own[at];
+            asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
+                             remote_addr(smem_addr(&s.inbox[rank * kSmallInbox + at]), i & (C - 1))),
+                         "r"(e.lid), "r"(e.len_hi), "r"(e.beg_lo), "r"(0u)
+                         : "memory");
+        }
         if (threadIdx.x < C)
             asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(
                              remote_addr(smem_addr(&s.head[rank]), threadIdx.x)),
-                         "r"(bmin), "r"(s.count)
+                         "r"(bmin), "r"(mycount)
                          : "memory");
-        cluster.sync();
+        cluster.barrier_arrive();
+        retire(fprev, kcur);   // while the others arrive
+        fprev = 0;
+        cluster.barrier_wait();
         // level, frontier and size of the round: the same in every warp of the cluster
         if (threadIdx.x == 0) s.count = 0;
         const SmallHead h = lane < C ? s.head[lane] : SmallHead{kSmallDead, 0};
@@ -784,6 +807,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         if (__any_sync(GA_FULL_MASK, cnt > kSmallInbox)) break;   // the grid kernels take this round
         const uint32_t incl = warp_incl_scan(cnt, lane);
         const uint32_t F = __shfl_sync(GA_FULL_MASK, incl, 31);
+        const uint32_t taking = __ballot_sync(GA_FULL_MASK, cnt != 0);
         uint32_t* flid = s.flid[done & 1];
         // the frontier's inbox positions, in order. Up to 32 vertices (almost every round) every warp finds them for
         // itself; more are spread over the block.
@@ -792,10 +816,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         uint32_t work = 0;   // capped lengths: a sum over at most 2,048 lists fits 32 bits
         for (uint32_t f0 = wide ? 32 * warp : 0; f0 < F; f0 += kSmallThreads) {   // warp-uniform
             const uint32_t f = f0 + lane;
-            uint32_t c = 0, before = 0;
-            for (uint32_t q = 0; q < C; q++) {
-                const uint32_t end = __shfl_sync(GA_FULL_MASK, incl, q);
-                if (end <= f) { c = q + 1; before = end; }
+            uint32_t c = 0, before = 0;   // the CTA of candidate f: the last taking one whose range starts at or below f
+            for (uint32_t left = taking; left; left &= left - 1) {
+                const uint32_t q = __ffs(left) - 1, start = __shfl_sync(GA_FULL_MASK, incl - cnt, q);
+                if (start <= f) { c = q; before = start; }
             }
             if (f < F) {
                 const uint32_t at = c * kSmallInbox + (f - before);
@@ -815,16 +839,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         }
         if (work > kSmallWork) break;    // the grid kernels take this round
         const bool last = F == nalive;   // nothing survives: no count is left to update
-        // mark the frontier in this CTA's copy; its owner also takes it out of the counts and writes its core number
+        // mark the frontier in this CTA's copy; its owner also takes it out of the counts
         for (uint32_t f = threadIdx.x; f < F; f += kSmallThreads) {
             const uint32_t lid = wide ? flid[f] : e.lid;
             atomicXor(&s.st[lid >> 4], 3u << (2 * (lid & 15)));   // 1 -> 2
-            if ((lid & (C - 1)) == rank) {
-                s.tri[lid >> cbits] = kSmallDead;
-                const uint32_t v = in[lid];
-                core[v] = k;
-                state[v] = 0;
-            }
+            if ((lid & (C - 1)) == rank) s.tri[lid >> cbits] = kSmallDead;
         }
         __syncthreads();
         // update (k_frontier_update_list): each destroyed triangle once, by its smallest frontier corner
@@ -910,6 +929,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         done++;
         fprev = F;
     }
+    retire(fprev, kcur);
     // leave: local ids end; with rounds run, the survivors' counts, list and the loop state go back to global memory
     uint32_t* survivors = cluster.map_shared_rank(&s.survivors, 0);
     for (uint32_t s0 = 32 * warp; s0 * C < na0; s0 += kSmallThreads) {   // warp-uniform
