@@ -61,6 +61,27 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
     return lo;
 }
 
+// ---- the index's formats --------------------------------------------------------------------------------------------
+constexpr uint32_t kPad = 0xFFFFFFFFu;   // padding of the last oct of a row in colr: above every place
+
+// in_rng: the padded position of the edge's entry in its source's row plus one (35 bits: up to 2^32 octs of 8) and the
+// octs from there to the row's end that hold entries after it (29 bits: a row has fewer than 2^32 entries).
+__host__ __device__ __forceinline__ unsigned long long pack_rng(unsigned long long at, uint32_t octs) {
+    return (unsigned long long)octs << 35 | (at + 1);
+}
+__device__ __forceinline__ unsigned long long rng_at(unsigned long long r) { return (r & ((1ull << 35) - 1)) - 1; }
+__device__ __forceinline__ uint32_t rng_oct(unsigned long long r) {   // the first oct of the suffix
+    return (uint32_t)((r & ((1ull << 35) - 1)) >> 3);
+}
+__device__ __forceinline__ uint32_t rng_octs(unsigned long long r) { return (uint32_t)(r >> 35); }
+
+// The tiny bin: anchors of so few out-neighbours (two octs) that an in-edge is one lane's work, without hubs among
+// their in-lists (a warp takes 32 such anchors at once).
+constexpr uint32_t kTinyDeg = 16, kTinyIn = 32, kTinyWork = 256, kTinyGroups = 4;
+__device__ __forceinline__ uint32_t is_tiny(uint32_t d, uint32_t in, uint32_t work, uint32_t light_max_deg) {
+    return d && work && d <= kTinyDeg && in <= kTinyIn && work <= kTinyWork && d <= light_max_deg;
+}
+
 // ---- grid sizing ------------------------------------------------------------------------------------------------
 inline unsigned grid_for(uint64_t threads, int block, unsigned cap = 148u * 64u) {
     uint64_t b = (threads + block - 1) / block;
@@ -73,13 +94,11 @@ inline unsigned grid_for(uint64_t threads, int block, unsigned cap = 148u * 64u)
 
 struct ga_loops;   // round-loop state (ga_loops.cu)
 
-// Work list of one kernel bin: item i covers in-edges [k0[i], k1[i]) of anchor v[i].
+// Work items of the triangle kernels, heavy then light then tiny, each bin by ascending anchor: item i covers in-edges
+// [k0[i], k1[i]) of anchor (place) v[i]. The bins' sizes are on the device (info[0..2]).
 struct ga_items {
-    uint32_t count = 0;
-    uint32_t* v = nullptr;
-    uint32_t* k0 = nullptr;
-    uint32_t* k1 = nullptr;
-    uint32_t max_dv = 0;      // largest anchor out-degree in the bin
+    uint32_t *v = nullptr, *k0 = nullptr, *k1 = nullptr, *info = nullptr;
+    uint64_t capacity = 0, bound = 0;   // entries allocated; at least the number of items
 };
 
 struct ga_graph {
@@ -94,29 +113,26 @@ struct ga_graph {
     uint32_t* col = nullptr;      // m
     uint32_t* src = nullptr;      // m (built on the device)
 
-    // transpose of the oriented CSR: in-edges of v are in_src/in_eid[in_ptr[v] .. in_ptr[v+1])
-    uint32_t* in_ptr = nullptr;   // n+1
-    uint32_t* in_src = nullptr;   // m: source u of the in-edge
-    uint32_t* in_eid = nullptr;   // m: index of the edge u->v in col
+    uint32_t* deg = nullptr;      // n: degree, out + in (built on the device with the upload checks)
+    uint32_t max_degree = 0, isolated = 0;   // largest degree, vertices of degree 0 (the first places)
+    uint64_t octs = 0;            // octs of all rows: sum of ceil(d+ / 8)
+    uint64_t row_work = 0;        // sum of d+ * ceil(d+ / 8): bounds the probe work
+    uint64_t row_hist[33] = {};   // edges by 1 + floor(log2) of their row's length
+    bool misoriented = false;     // an edge is not oriented by (degree, id): every use that needs it refuses
 
-    // the oriented CSR again with every row ordered by (degree, id) - the orientation order - instead of by id: for
-    // an in-edge u->v, only the out-neighbours of u after v in this order can close a triangle u->v->x, so the count
-    // kernels probe that suffix of u's row alone
-    uint32_t* colk = nullptr;     // m (+4 zero padding, 16-byte aligned like col)
-    uint32_t* origk = nullptr;    // m: position in col of colk[e]
-    // every vertex's place in the (degree, id) order, and colk with each entry replaced by that place: an anchor's
-    // out-neighbours then lie in a short range of places just above the anchor's own (R-MAT 22: within 65,536 for
-    // every anchor of more than 128 out-neighbours), which the count kernel covers with a bitmap
-    uint32_t* vrank = nullptr;    // n
-    uint32_t* colr = nullptr;     // m (+4 zero padding, 16-byte aligned like colk)
-    // m: in-edge k's probe list in colk, [the place of its edge u->v in u's reordered row + 1, end of u's row);
-    // read by the count kernels in one 64-bit load instead of the source and then its row end (R-MAT 22 count:
-    // 2.58 vs 2.69 ms)
-    uint2* in_rng = nullptr;
+    // the index (ga_graph.cu): vertices numbered by (degree, id), rows and in-lists in these numbers (places)
+    uint32_t* vrank = nullptr;    // n: place of every id
+    uint32_t* order = nullptr;    // n: id of every place
+    uint32_t* dout = nullptr;     // n: out-degree, by place
+    uint32_t* work = nullptr;     // n: octs to probe for an anchor, by place
+    uint2* pos = nullptr;         // n+1, by place: start of its in-edges in in_rng (x), of its row in colr (y, octs)
+    uint32_t* colr = nullptr;     // 8 * octs: rows as ascending places, padded with kPad
+    uint32_t* osrc = nullptr;     // octs: place of the row an oct belongs to
+    unsigned long long* in_rng = nullptr;   // m: in-edge u->v as pack_rng(padded position of v in u's row, suffix octs)
 
-    unsigned long long* anchor_work = nullptr;   // n+1: probe work of the anchors below v (cuts shards)
-    ga_items light, heavy;        // degree-binned work lists of the hash-probe kernel
-    bool index_ready = false;     // src, in-lists, colk / origk / in_rng / vrank / colr built
+    unsigned long long* anchor_work = nullptr;   // n+1: probe work of the anchors below a place (cuts shards; lazy)
+    ga_items items;               // work lists of the triangle kernels
+    bool index_ready = false;     // vrank .. in_rng built
     bool prepared = false;        // ... and the work items for the current light_max_deg / item_work
     ga_loops* loops = nullptr;    // peeling / core loop state, allocated on first use
     // a batch: the graph is the disjoint union of seg_count graphs, graph s owning vertices [seg_off[s], seg_off[s+1])
@@ -187,8 +203,10 @@ ga_status use_device(const ga_graph* g);
 // Frees the loop state (CUDA graphs, pinned buffers) of g.
 void destroy_loops(ga_graph* g);
 
-// Builds src, in-lists, the (degree, id)-ordered rows (once) and the work lists for the current options (idempotent).
+// Builds the index (once) and the work lists for the current options (idempotent).
 ga_status prepare(ga_graph* g);
+// prepare, and the work prefix that cuts shards.
+ga_status prepare_shards(ga_graph* g);
 
 // Picks the count kernel for GA_OPT_TC_KERNEL = 0 from the graph's degree-distribution signature (cached per
 // signature; times both kernels once for a new one). Called by ga_graph_prepare.
@@ -196,8 +214,6 @@ ga_status autotune(ga_graph* g);
 // prepare + autotune (GA_OPT_TC_KERNEL = 0): what every synchronous entry point does first.
 ga_status ready(ga_graph* g);
 
-// Device-wide exclusive scan of n uint32 values (in place allowed) on g's stream.
-ga_status exclusive_scan_u32(ga_graph* g, const uint32_t* in, uint32_t* out, uint32_t n, bool write_total);
 // In-place exclusive scan of n uint64 values on g's stream.
 ga_status scan_u64(ga_graph* g, unsigned long long* data, uint64_t n);
 

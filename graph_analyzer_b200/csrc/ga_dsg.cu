@@ -47,14 +47,14 @@ __global__ void k_level_entries(const uint2* __restrict__ inc, const unsigned lo
 // corner c, whose entry is (middle, highest); c is the lowest exactly when it precedes the entry's first vertex.
 // Positions come from one atomic per warp and chunk; entries past `cap` are counted but not written.
 __global__ void k_list_triangles(const uint2* __restrict__ inc, const unsigned long long* __restrict__ inc_ptr,
-                                 const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ in_ptr, uint32_t n,
+                                 const uint32_t* __restrict__ vrank, uint32_t n,
                                  uint32_t* __restrict__ tris, unsigned long long cap,
                                  unsigned long long* __restrict__ count) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const uint32_t c = (uint32_t)v;
-        const uint32_t dc = rowptr[c + 1] - rowptr[c] + in_ptr[c + 1] - in_ptr[c];
+        const uint32_t rc = vrank[c];
         const unsigned long long b = inc_ptr[c], e = inc_ptr[c + 1];
         for (unsigned long long i = b; i < e; i += 32) {
             const unsigned long long j = i + lane;
@@ -62,8 +62,7 @@ __global__ void k_list_triangles(const uint2* __restrict__ inc, const unsigned l
             uint2 t = make_uint2(0, 0);
             if (j < e) {
                 t = inc[j];
-                const uint32_t dp = rowptr[t.x + 1] - rowptr[t.x] + in_ptr[t.x + 1] - in_ptr[t.x];
-                lowest = dc != dp ? dc < dp : c < t.x;
+                lowest = rc < vrank[t.x];
             }
             const uint32_t mask = __ballot_sync(GA_FULL_MASK, lowest);
             unsigned long long base = 0;
@@ -122,7 +121,7 @@ ga_status graph_triangles(ga_graph* g, std::vector<uint32_t>* tris, std::vector<
     GA_TRY(s_cnt.alloc(&d_cnt, 1));
     GA_CUDA(cudaMemsetAsync(d_cnt, 0, 8, st));
     if (n) {
-        k_list_triangles<<<grid_for((uint64_t)n * 32, 256), 256, 0, st>>>(inc, inc_ptr, g->rowptr, g->in_ptr, n,
+        k_list_triangles<<<grid_for((uint64_t)n * 32, 256), 256, 0, st>>>(inc, inc_ptr, g->vrank, n,
                                                                           d_tris, T, d_cnt);
         GA_CUDA(cudaGetLastError());
     }

@@ -1,14 +1,19 @@
 // ga_graph.cu - device-resident graph handle: upload, validation, and the derived structures every query shares.
 //
-// Derived structures (built once per handle, on the device, kept resident):
-//   src[m]                 row owner of every edge (the reference builds it on the host, graph.h:64)
-//   in_ptr/in_src/in_eid   transpose of the oriented CSR: for every vertex v the edges u->v (source, edge index)
-//   colk/origk/in_rng      every row again in (degree, id) order, where each entry sits in it, and for each
-//                          in-edge u->v the part of u's reordered row after v (its probe suffix)
-//   vrank/colr             every vertex's place in the (degree, id) order, and colk with entries as places
-//   light / heavy items    degree-binned work lists of the hash-probe kernels: one item = a slice of v's in-edges
-//                          whose probe work (sum of out-degrees of the sources) is bounded; anchors with a large
-//                          out-degree go to the block-wide "heavy" bin, the rest to the per-warp "light" bin.
+// Derived structures (built on the device, kept resident). The orientation order (degree, id) numbers the vertices; a
+// vertex's number is its PLACE, and everything the triangle kernels read is kept in places:
+//   src[m], deg[n]         row owner and degree of every edge / vertex, by id (made with the checks at upload)
+//   vrank[n] / order[n]    place of every id and id of every place
+//   pos[n+1]               by place: where its in-edges start (x) and where its row starts in colr (y, in octs)
+//   colr                   every row as ascending places, padded to whole octs (8 entries, one 32-byte sector) with
+//                          kPad, which no place reaches: a probe loop reads whole octs and tests no ends
+//   osrc                   place of the row every oct belongs to
+//   in_rng[m]              for every in-edge u->v, laid out anchor by anchor (v): where v sits in u's row and how many
+//                          octs of that row hold entries after v (its probe suffix)
+//   dout[n], work[n]       by place: out-degree, and octs its in-edges have to probe
+//   items                  work lists of the triangle kernels: one item = a slice of an anchor's in-edges whose probe
+//                          work is bounded; anchors of a large out-degree are "heavy" (a block each), others "light"
+//                          (a warp each), the smallest "tiny" (counts take 32 of them at a time)
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -17,46 +22,60 @@
 
 namespace ga {
 
-// ---- scan (reduce-then-scan over tiles of 256 threads x 16 elements) --------------------------------------------
-constexpr int kScanThreads = 256, kScanItems = 16, kScanTile = kScanThreads * kScanItems;
+// ---- exclusive scan: tiles of 512 threads x 8 elements, two launches -------------------------------------------------
+// k_scan_sums writes every tile's sum; k_scan_tiles adds up the sums of the tiles before its own itself (a few KB from
+// L2 for the sizes here) and scans its tile from registers, so there is no third launch for the sums. Above
+// kScanDirect tiles the sums are scanned first.
+constexpr int kScanThreads = 512, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
+constexpr uint64_t kScanDirect = 8192;
 constexpr unsigned long long kHeavyItemFactor = 64;   // heavy items carry 64x the probe work of light items
 
+// Sum over the block (every thread gets it). s_w: kScanThreads / 32 slots.
 template <class T>
-__global__ void k_tile_reduce(const T* __restrict__ in, uint64_t n, T* __restrict__ sums) {
-    __shared__ T s_w[kScanThreads / 32];
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-    T acc = 0;
-    for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {
-        const uint64_t k = base + i;
-        if (k < n) acc += in[k];
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(GA_FULL_MASK, acc, o);
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = acc;
+__device__ __forceinline__ T block_sum(T x, T* s_w) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(GA_FULL_MASK, x, o);
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = x;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        T t = 0;
-        for (int w = 0; w < kScanThreads / 32; w++) t += s_w[w];
-        sums[blockIdx.x] = t;
-    }
+    T t = 0;
+    for (int w = 0; w < kScanThreads / 32; w++) t += s_w[w];
+    __syncthreads();
+    return t;
 }
 
-// Scans one tile; `offsets` (may be null) holds the exclusive prefix of every tile.
 template <class T>
-__global__ void k_tile_scan(const T* __restrict__ in, T* __restrict__ out, uint64_t n, const T* __restrict__ offsets,
-                            int inclusive) {
-    __shared__ T s_tile[kScanTile];
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const T* __restrict__ in, uint64_t n, T* __restrict__ sums) {
     __shared__ T s_w[kScanThreads / 32];
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-    for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {   // coalesced load through shared memory
-        const uint64_t k = base + i;
-        s_tile[i] = k < n ? in[k] : (T)0;
-    }
-    __syncthreads();
-    T v[kScanItems];
-    T run = 0;
+    const uint64_t base = (uint64_t)blockIdx.x * kScanTile + threadIdx.x;
+    T acc = 0;
 #pragma unroll
-    for (int j = 0; j < kScanItems; j++) { v[j] = s_tile[threadIdx.x * kScanItems + j]; run += v[j]; }
-    // exclusive prefix of the thread totals across the block
+    for (int j = 0; j < kScanItems; j++) {
+        const uint64_t k = base + (uint64_t)j * kScanThreads;
+        if (k < n) acc += in[k];
+    }
+    acc = block_sum(acc, s_w);
+    if (threadIdx.x == 0) sums[blockIdx.x] = acc;
+}
+
+// sums: the tiles' sums (scanned = false) or their exclusive prefix (true); null for a single tile. In place allowed.
+template <class T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T* in, T* out, uint64_t n, const T* __restrict__ sums,
+                                                             bool scanned) {
+    __shared__ T s_w[kScanThreads / 32];
+    T before = 0;
+    if (sums && scanned) before = sums[blockIdx.x];
+    else if (sums) {
+        T acc = 0;
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) acc += sums[b];
+        before = block_sum(acc, s_w);
+    }
+    // thread t scans elements 8t .. 8t + 7 of the tile
+    const uint64_t k0 = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    T v[kScanItems], run = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; j++) {
+        v[j] = k0 + j < n ? in[k0 + j] : (T)0;
+        run += v[j];
+    }
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     T x = run;
     for (int o = 1; o < 32; o <<= 1) {
@@ -65,241 +84,321 @@ __global__ void k_tile_scan(const T* __restrict__ in, T* __restrict__ out, uint6
     }
     if (lane == 31) s_w[w] = x;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        T acc = 0;
-        for (int i = 0; i < kScanThreads / 32; i++) { const T t = s_w[i]; s_w[i] = acc; acc += t; }
-    }
-    __syncthreads();
-    T pre = x - run + s_w[w] + (offsets ? offsets[blockIdx.x] : (T)0);
+    T pre = before + x - run;
+    for (uint32_t q = 0; q < w; q++) pre += s_w[q];
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
-        const T val = v[j];
-        s_tile[threadIdx.x * kScanItems + j] = inclusive ? pre + val : pre;
-        pre += val;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {
-        const uint64_t k = base + i;
-        if (k < n) out[k] = s_tile[i];
+        if (k0 + j < n) out[k0 + j] = pre;
+        pre += v[j];
     }
 }
 
 template <class T>
-static ga_status scan_impl(cudaStream_t st, const T* in, T* out, uint64_t n, bool inclusive) {
+static ga_status scan_impl(cudaStream_t st, const T* in, T* out, uint64_t n) {
     if (n == 0) return GA_OK;
     const uint64_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 1) {
-        k_tile_scan<T><<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, inclusive);
+        k_scan_tiles<T><<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, false);
         GA_CUDA(cudaGetLastError());
         return GA_OK;
     }
     T* sums = nullptr;
     GA_CUDA(pool_malloc((void**)&sums, nb * sizeof(T), st));
-    k_tile_reduce<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, sums);
+    k_scan_sums<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, sums);
     ga_status s = GA_OK;
-    if (cudaGetLastError() != cudaSuccess) s = fail(GA_ERR_CUDA, "scan reduce launch failed");
-    if (s == GA_OK) s = scan_impl<T>(st, sums, sums, nb, false);
+    if (cudaGetLastError() != cudaSuccess) s = fail(GA_ERR_CUDA, "scan sums launch failed");
+    const bool scanned = nb > kScanDirect;
+    if (s == GA_OK && scanned) s = scan_impl<T>(st, sums, sums, nb);
     if (s == GA_OK) {
-        k_tile_scan<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, sums, inclusive);
+        k_scan_tiles<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, sums, scanned);
         if (cudaGetLastError() != cudaSuccess) s = fail(GA_ERR_CUDA, "scan launch failed");
     }
     cudaFreeAsync(sums, st);
     return s;
 }
 
-ga_status exclusive_scan_u32(ga_graph* g, const uint32_t* in, uint32_t* out, uint32_t n, bool write_total) {
-    GA_TRY(scan_impl<uint32_t>(g->stream, in, out, n, false));
-    (void)write_total;
-    return GA_OK;
-}
-
 ga_status scan_u64(ga_graph* g, unsigned long long* data, uint64_t n) {
-    return scan_impl<unsigned long long>(g->stream, data, data, n, false);
+    return scan_impl<unsigned long long>(g->stream, data, data, n);
 }
 
 // ---- validation and derived structures -------------------------------------------------------------------------
 
-// Flags in *err: 1 rowptr not monotone / beyond m, 2 endpoint >= n, 4 self loop, 8 row not strictly ascending.
-__global__ void k_validate(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t n,
-                           uint32_t m, unsigned long long* err) {
-    uint32_t bad = 0;
-    uint32_t maxdeg = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t b = rowptr[v], e = rowptr[v + 1];
-        if (b > e || e > m) { bad |= 1; continue; }
-        maxdeg = max(maxdeg, e - b);
-        for (uint32_t i = b; i < e; i++) {
-            const uint32_t x = col[i];
-            if (x >= n) bad |= 2;
-            if (x == v) bad |= 4;
-            if (i > b && col[i - 1] >= x) bad |= 8;
+// d_scalars slots of the upload checks.
+enum : int { SC_HIST = 8, SC_ISOLATED = 55, SC_ORIENT = 56, SC_MAXDEG = 57, SC_WORK = 58, SC_OCTS = 59, SC_MAXOUT = 60,
+             SC_ERR = 61 };
+
+// One pass over the rows: the checks, src[], the in-degrees (indeg[] zeroed before) and the sums that size the index.
+// A warp takes 32 consecutive rows, whose entries are consecutive: lanes read them coalesced and find their row among
+// the 32 starts. Rows of a warp whose starts are not ascending within [0, m] are flagged and not read.
+// Flags in sc[SC_ERR]: 1 rowptr not monotone / beyond m, 2 endpoint >= n, 4 self loop, 8 row not strictly ascending.
+__global__ void __launch_bounds__(256) k_rows(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
+                                              uint32_t n, uint32_t m, uint32_t* __restrict__ src,
+                                              uint32_t* __restrict__ indeg, unsigned long long* __restrict__ sc) {
+    __shared__ unsigned long long s_hist[33];
+    if (threadIdx.x < 33) s_hist[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t bad = 0, maxout = 0;
+    unsigned long long octs = 0, work = 0;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < n; v0 += stride) {
+        const uint32_t v = (uint32_t)v0 + lane;
+        const bool row = v0 + lane < n;
+        const uint32_t b = row ? rowptr[v] : 0u;
+        const uint32_t e = row ? rowptr[v + 1] : 0u;
+        const bool wrong = row && (b > e || e > m);
+        if (__any_sync(GA_FULL_MASK, wrong)) {
+            bad |= wrong;
+            continue;
+        }
+        const uint32_t d = e - b;
+        maxout = max(maxout, d);
+        octs += (d + 7) >> 3;
+        work += (unsigned long long)d * ((d + 7) >> 3);
+        {   // edges by log2 of the row's length (the autotuner's signature), one add per bucket and warp
+            const uint32_t bucket = d ? 32 - __clz(d) : 0u;
+            const uint32_t peers = __match_any_sync(GA_FULL_MASK, bucket);
+            const uint32_t sum = __reduce_add_sync(peers, d);
+            if (bucket && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&s_hist[bucket], (unsigned long long)sum);
+        }
+        const uint32_t nrows = (uint32_t)min((uint64_t)32, n - v0);
+        const uint32_t first = __shfl_sync(GA_FULL_MASK, b, 0), last = __shfl_sync(GA_FULL_MASK, e, nrows - 1);
+        const uint32_t start = row ? b : last;   // lanes past the last row start at the end: never found below it
+        for (uint32_t i0 = first; i0 < last; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const bool in = i >= i0 && i < last;   // i >= i0: no wrap past 2^32
+            // row of entry i: the last lane whose start is <= i (empty rows share their start with the next)
+            uint32_t r = 0;
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1) {
+                const uint32_t at = __shfl_sync(GA_FULL_MASK, start, r + step);
+                if (in && at <= i) r += step;
+            }
+            const uint32_t rb = __shfl_sync(GA_FULL_MASK, b, r);
+            const uint32_t x = in ? col[i] : 0u;
+            uint32_t prev = __shfl_up_sync(GA_FULL_MASK, x, 1);
+            if (lane == 0 && in && i > rb) prev = col[i - 1];
+            if (in) {
+                const uint32_t u = (uint32_t)v0 + r;
+                src[i] = u;
+                if (x >= n) bad |= 2;
+                else atomicAdd(&indeg[x], 1u);
+                if (x == u) bad |= 4;
+                if (i > rb && prev >= x) bad |= 8;
+            }
+            if (last - i0 <= 32) break;   // no wrap of i0
         }
     }
-    if (bad) atomicOr(err, (unsigned long long)bad);
-    maxdeg = __reduce_max_sync(GA_FULL_MASK, maxdeg);
-    if ((threadIdx.x & 31) == 0 && maxdeg) atomicMax(err - 1, (unsigned long long)maxdeg);   // max out-degree
+    bad = __reduce_or_sync(GA_FULL_MASK, bad);
+    maxout = __reduce_max_sync(GA_FULL_MASK, maxout);
+    octs = warp_sum_u64(octs);
+    work = warp_sum_u64(work);
+    if (lane == 0) {
+        if (bad) atomicOr(&sc[SC_ERR], (unsigned long long)bad);
+        if (maxout) atomicMax(&sc[SC_MAXOUT], (unsigned long long)maxout);
+        if (octs) atomicAdd(&sc[SC_OCTS], octs);
+        if (work) atomicAdd(&sc[SC_WORK], work);
+    }
+    __syncthreads();
+    if (threadIdx.x < 33 && s_hist[threadIdx.x]) atomicAdd(&sc[SC_HIST + threadIdx.x], s_hist[threadIdx.x]);
 }
 
-// src[e] = owner row; in-degree histogram.
-__global__ void k_src_and_indeg(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t n,
-                                uint32_t* __restrict__ src, uint32_t* __restrict__ indeg) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t b = rowptr[v], e = rowptr[v + 1];
-        for (uint32_t i = b; i < e; i++) {
-            src[i] = v;
-            atomicAdd(&indeg[col[i]], 1u);
+// deg[v] += out-degree (deg holds the in-degrees): total degrees, their maximum and the number of isolated vertices.
+__global__ void __launch_bounds__(256) k_degrees(const uint32_t* __restrict__ rowptr, uint32_t n,
+                                                 uint32_t* __restrict__ deg, unsigned long long* __restrict__ sc) {
+    uint32_t mx = 0, isolated = 0;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t d = deg[v] + rowptr[v + 1] - rowptr[v];
+        deg[v] = d;
+        mx = max(mx, d);
+        isolated += d == 0;
+    }
+    mx = __reduce_max_sync(GA_FULL_MASK, mx);
+    isolated = __reduce_add_sync(GA_FULL_MASK, isolated);
+    if ((threadIdx.x & 31) == 0) {
+        if (mx) atomicMax(&sc[SC_MAXDEG], (unsigned long long)mx);
+        if (isolated) atomicAdd(&sc[SC_ISOLATED], (unsigned long long)isolated);
+    }
+}
+
+// The orientation rule of graph.h:43-45 for every edge: from the smaller to the larger endpoint by (degree, id).
+// sc[SC_ORIENT] != 0: an edge points the wrong way. (Endpoints >= n are skipped: k_rows has refused the graph.)
+__global__ void __launch_bounds__(256) k_orient(const uint32_t* __restrict__ src, const uint32_t* __restrict__ col,
+                                                const uint32_t* __restrict__ deg, uint32_t n, uint32_t m,
+                                                unsigned long long* __restrict__ sc) {
+    bool bad = false;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t u = src[e], x = col[e];
+        if (x >= n || u >= n) continue;
+        const uint32_t du = deg[u], dx = deg[x];
+        bad |= !(du != dx ? du < dx : u < x);
+    }
+    if (__any_sync(GA_FULL_MASK, bad) && (threadIdx.x & 31) == 0) atomicOr(&sc[SC_ORIENT], 1ull);
+}
+
+// ---- rows in places ----------------------------------------------------------------------------------------------
+// Every row's entries become places (one gather of vrank), are sorted (places alone: the sort carries nothing else) and
+// written as whole octs; in the same pass the edge's entry of its anchor's in-list is filled in. A row is sorted by a
+// bitonic network over E keys per lane, element l * E + i in register i of lane l: strides below E stay inside a
+// thread (min / max), larger ones are one shuffle. (64-bit (degree, id) keys counted against each other in shared
+// memory with the entries' positions carried along, then a scatter and a gather of their own, took 4.0 ms of R-MAT 22's
+// 5.4 ms of build kernels.)
+template <int E, int LANES>
+__device__ __forceinline__ void sort_keys(uint32_t (&k)[E], uint32_t l) {
+#pragma unroll
+    for (int size = 2; size <= E * LANES; size <<= 1) {
+#pragma unroll
+        for (int st = size >> 1; st > 0; st >>= 1) {
+            if (st >= E) {
+                const uint32_t xl = st / E;
+                const bool lower = (l & xl) == 0;
+                const bool up = size >= E * LANES || (l & (size / E)) == 0;
+#pragma unroll
+                for (int i = 0; i < E; i++) {
+                    const uint32_t o = __shfl_xor_sync(GA_FULL_MASK, k[i], xl);
+                    k[i] = lower == up ? min(k[i], o) : max(k[i], o);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < E; i++) {
+                    if ((i & st) == 0) {
+                        const bool up = size < E ? (i & size) == 0 : size >= E * LANES || (l & (size / E)) == 0;
+                        const uint32_t a = k[i], b = k[i | st];
+                        k[i] = up ? min(a, b) : max(a, b);
+                        k[i | st] = up ? max(a, b) : min(a, b);
+                    }
+                }
+            }
         }
     }
 }
 
-// Scatter every edge u->v into v's in-list.
-__global__ void k_in_scatter(const uint32_t* __restrict__ col, const uint32_t* __restrict__ src,
-                             const uint32_t* __restrict__ in_ptr, uint32_t m, uint32_t* __restrict__ fill,
-                             uint32_t* __restrict__ in_src, uint32_t* __restrict__ in_eid) {
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-        const uint32_t u = src[e], v = col[e];
-        const uint32_t p = in_ptr[v] + atomicAdd(&fill[v], 1u);
-        in_src[p] = u;
-        in_eid[p] = e;
-    }
+// Entry j (place x) of place a's row of d entries, starting at oct o0: its record in x's in-list and x's probe work.
+__device__ __forceinline__ void emit_in_edge(uint32_t x, uint32_t j, uint32_t d, uint32_t o0,
+                                             const uint2* __restrict__ pos, uint32_t* __restrict__ fill,
+                                             uint32_t* __restrict__ work, unsigned long long* __restrict__ in_rng) {
+    const unsigned long long at = (unsigned long long)o0 * 8 + j;   // padded position of the entry
+    const uint32_t octs = j + 1 < d ? ((d + 7) >> 3) - ((j + 1) >> 3) : 0u;
+    const uint32_t k = pos[x].x + atomicAdd(&fill[x], 1u);
+    in_rng[k] = pack_rng(at, octs);
+    if (octs) atomicAdd(&work[x], octs);
 }
 
-// key[e] = (degree << 32) | id of the endpoint col[e], degree = out + in: the orientation order of graph.h:43-45.
-// Also checks that rule for the edge src[e] -> col[e] (flag 16 in *err when it points the wrong way); the owner's
-// degree is the same for a row's consecutive edges.
-__global__ void k_edge_keys(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
-                            const uint32_t* __restrict__ src, const uint32_t* __restrict__ in_ptr, uint32_t m,
-                            unsigned long long* __restrict__ key, unsigned long long* err) {
-    uint32_t bad = 0;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-        const uint32_t x = col[e], u = src[e];
-        const uint32_t deg = rowptr[x + 1] - rowptr[x] + in_ptr[x + 1] - in_ptr[x];
-        const uint32_t du = rowptr[u + 1] - rowptr[u] + in_ptr[u + 1] - in_ptr[u];
-        if (!(du != deg ? du < deg : u < x)) bad |= 16;
-        key[e] = ((unsigned long long)deg << 32) | x;
-    }
-    if (bad) atomicOr(err, (unsigned long long)bad);
-}
-
-constexpr int kOrderWarps = 4, kOrderStage = 1024;   // rows up to kOrderStage entries stage their keys in smem
-
-// Sorting the rows' keys (degree << 32 | id: distinct, the id is the low word) with the entry positions alongside,
-// in two kernels. Each writes colk/origk in sorted order and posk[e] = where entry e went.
-//
-// k_order_rows_small: rows of at most 8 entries (most rows of a power-law graph), four rows per warp, one per 8-lane
-// group: a bitonic network across the group's registers (xor partners below 8 stay inside the group). Longer rows are
-// appended to `listed` (one atomic per warp) for k_order_rows_listed.
-__global__ void __launch_bounds__(256) k_order_rows_small(const uint32_t* __restrict__ rowptr,
-                                                          const unsigned long long* __restrict__ key, uint32_t n,
-                                                          uint32_t* __restrict__ colk, uint32_t* __restrict__ origk,
-                                                          uint32_t* __restrict__ posk, uint32_t* __restrict__ listed,
+// Rows of at most 8 entries, four rows per warp, one per 8-lane group. Longer rows are appended to `listed`.
+__global__ void __launch_bounds__(256) k_place_rows_small(const uint32_t* __restrict__ rowptr,
+                                                          const uint32_t* __restrict__ col,
+                                                          const uint32_t* __restrict__ vrank,
+                                                          const uint32_t* __restrict__ order,
+                                                          const uint2* __restrict__ pos, uint32_t first, uint32_t n,
+                                                          uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
+                                                          uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
+                                                          unsigned long long* __restrict__ in_rng,
+                                                          uint32_t* __restrict__ listed,
                                                           uint32_t* __restrict__ nlisted) {
     const uint32_t lane = threadIdx.x & 31, sub = lane & 7;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < (uint64_t)n * 8; t0 += stride) {
-        const uint64_t t = t0 + lane;
-        const uint32_t u = (uint32_t)(t >> 3);
+    for (uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < (uint64_t)(n - first) * 8;
+         t0 += stride) {
+        const uint64_t row = first + ((t0 + lane) >> 3);
+        const bool valid = row < n;
+        const uint32_t a = (uint32_t)row;
         uint32_t b = 0, d = 0;
-        if (u < n) {
+        if (valid) {
+            const uint32_t u = order[a];
             b = rowptr[u];
             d = rowptr[u + 1] - b;
         }
         const bool mine = d >= 1 && d <= 8;   // the whole group agrees (same row)
-        unsigned long long k = mine && sub < d ? key[b + sub] : ~0ull;
-        uint32_t idx = sub;
-#pragma unroll
-        for (uint32_t size = 2; size <= 8; size <<= 1) {
-#pragma unroll
-            for (uint32_t st = size >> 1; st > 0; st >>= 1) {
-                const unsigned long long ok = __shfl_xor_sync(GA_FULL_MASK, k, st);
-                const uint32_t oi = __shfl_xor_sync(GA_FULL_MASK, idx, st);
-                const bool up = (sub & size) == 0, lower = (sub & st) == 0;
-                if (lower == up ? ok < k : ok > k) { k = ok; idx = oi; }
-            }
+        uint32_t k[1] = {mine && sub < d ? vrank[col[b + sub]] : kPad};
+        sort_keys<1, 8>(k, sub);
+        if (mine) {
+            const uint32_t o0 = pos[a].y;
+            colr[(size_t)o0 * 8 + sub] = k[0];
+            if (sub == 0) osrc[o0] = a;
+            if (sub < d) emit_in_edge(k[0], sub, d, o0, pos, fill, work, in_rng);
         }
-        if (mine && sub < d) {
-            colk[b + sub] = (uint32_t)k;
-            origk[b + sub] = b + idx;
-            posk[b + idx] = b + sub;
-        }
-        const bool longer = u < n && d > 8 && sub == 0;
+        const bool longer = valid && d > 8 && sub == 0;
         const uint32_t bal = __ballot_sync(GA_FULL_MASK, longer);
         if (bal) {
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(nlisted, (uint32_t)__popc(bal));
             base = __shfl_sync(GA_FULL_MASK, base, 0);
-            if (longer) listed[base + __popc(bal & ((1u << lane) - 1))] = u;
+            if (longer) listed[base + __popc(bal & ((1u << lane) - 1))] = a;
         }
     }
 }
 
-// k_order_rows_listed: the rows k_order_rows_small listed, one warp per row. Up to 32 entries: a bitonic network
-// across the warp's registers. Longer: every entry's place is the number of entries with a smaller key, counted
-// against the row's keys staged in the warp's shared memory (read by all lanes at once; rows longer than
-// kOrderStage, rare since d+ is at most sqrt(2m) in this orientation, read them from global memory), four entries
-// per lane per pass over the row.
-__global__ void __launch_bounds__(kOrderWarps * 32) k_order_rows_listed(const uint32_t* __restrict__ rowptr,
-                                                                        const unsigned long long* __restrict__ key,
-                                                                        const uint32_t* __restrict__ listed,
-                                                                        const uint32_t* __restrict__ nlisted,
-                                                                        uint32_t* __restrict__ colk,
-                                                                        uint32_t* __restrict__ origk,
-                                                                        uint32_t* __restrict__ posk) {
-    __shared__ unsigned long long s_key[kOrderWarps][kOrderStage];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+template <int E>
+__device__ __forceinline__ void place_row(const uint32_t* __restrict__ row, uint32_t d, uint32_t a, uint32_t lane,
+                                          const uint32_t* __restrict__ vrank, const uint2* __restrict__ pos,
+                                          uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
+                                          uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
+                                          unsigned long long* __restrict__ in_rng) {
+    uint32_t k[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) k[i] = lane + 32 * i < d ? vrank[row[lane + 32 * i]] : kPad;   // any start order
+    sort_keys<E, 32>(k, lane);
+    const uint32_t o0 = pos[a].y, end = (d + 7) & ~7u;
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        const uint32_t j = lane * E + i;
+        if (E < 4 && j < end) colr[(size_t)o0 * 8 + j] = k[i];
+        if (E >= 4 && (i & 3) == 0 && j < end)
+            *reinterpret_cast<uint4*>(colr + (size_t)o0 * 8 + j) =
+                make_uint4(k[i], k[E >= 4 ? i + 1 : 0], k[E >= 4 ? i + 2 : 0], k[E >= 4 ? i + 3 : 0]);
+        if (j < end && (j & 7) == 0) osrc[o0 + (j >> 3)] = a;
+        if (j < d) emit_in_edge(k[i], j, d, o0, pos, fill, work, in_rng);
+    }
+}
+
+// The listed rows, one warp per row, the last (largest places, mostly the longest rows) first. Up to 512 entries: the
+// register network; longer rows (rare: out-degrees are at most sqrt(2m) in this orientation) count smaller places.
+__global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __restrict__ rowptr,
+                                                           const uint32_t* __restrict__ col,
+                                                           const uint32_t* __restrict__ vrank,
+                                                           const uint32_t* __restrict__ order,
+                                                           const uint2* __restrict__ pos,
+                                                           uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
+                                                           uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
+                                                           unsigned long long* __restrict__ in_rng,
+                                                           const uint32_t* __restrict__ listed,
+                                                           const uint32_t* __restrict__ nlisted) {
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = *nlisted;
-    unsigned long long* sk = s_key[w];
     for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < count; r += nwarps) {
-        const uint32_t u = listed[r];
+        const uint32_t a = listed[count - 1 - r], u = order[a];
         const uint32_t b = rowptr[u], d = rowptr[u + 1] - b;
-        if (d <= 32) {
-            unsigned long long k = lane < d ? key[b + lane] : ~0ull;
-            uint32_t idx = lane;
+        const uint32_t* row = col + b;
+        if (d <= 32) place_row<1>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        else if (d <= 64) place_row<2>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        else if (d <= 128) place_row<4>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        else if (d <= 256) place_row<8>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        else if (d <= 512) place_row<16>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        else {
+            const uint32_t o0 = pos[a].y, end = (d + 7) & ~7u;
+            for (uint32_t i0 = lane; i0 < d; i0 += 256) {   // eight entries per lane per pass over the row
+                uint32_t kq[8], rk[8];
 #pragma unroll
-            for (uint32_t size = 2; size <= 32; size <<= 1) {
+                for (int q = 0; q < 8; q++) {
+                    kq[q] = i0 + 32 * q < d ? vrank[row[i0 + 32 * q]] : 0u;
+                    rk[q] = 0;
+                }
+                for (uint32_t j = 0; j < d; j++) {
+                    const uint32_t kj = vrank[row[j]];
 #pragma unroll
-                for (uint32_t st = size >> 1; st > 0; st >>= 1) {
-                    const unsigned long long ok = __shfl_xor_sync(GA_FULL_MASK, k, st);
-                    const uint32_t oi = __shfl_xor_sync(GA_FULL_MASK, idx, st);
-                    const bool up = (lane & size) == 0, lower = (lane & st) == 0;
-                    if (lower == up ? ok < k : ok > k) { k = ok; idx = oi; }
+                    for (int q = 0; q < 8; q++) rk[q] += kj < kq[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    if (i0 + 32 * q >= d) continue;
+                    colr[(size_t)o0 * 8 + rk[q]] = kq[q];
+                    emit_in_edge(kq[q], rk[q], d, o0, pos, fill, work, in_rng);
                 }
             }
-            if (lane < d) {
-                colk[b + lane] = (uint32_t)k;
-                origk[b + lane] = b + idx;
-                posk[b + idx] = b + lane;
-            }
-            continue;
+            for (uint32_t j = d + lane; j < end; j += 32) colr[(size_t)o0 * 8 + j] = kPad;
+            for (uint32_t j = lane; j < end >> 3; j += 32) osrc[o0 + j] = a;
         }
-        const bool staged = d <= kOrderStage;
-        if (staged) {
-            for (uint32_t i = lane; i < d; i += 32) sk[i] = key[b + i];
-            __syncwarp();
-        }
-        const unsigned long long* kr = staged ? sk : key + b;
-        for (uint32_t i0 = lane; i0 < d; i0 += 128) {
-            unsigned long long kq[4];
-            uint32_t rk[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int q = 0; q < 4; q++) kq[q] = i0 + 32 * q < d ? kr[i0 + 32 * q] : ~0ull;
-            for (uint32_t j = 0; j < d; j++) {
-                const unsigned long long kj = kr[j];
-#pragma unroll
-                for (int q = 0; q < 4; q++) rk[q] += kj < kq[q];
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const uint32_t i = i0 + 32 * q;
-                if (i < d) {
-                    colk[b + rk[q]] = (uint32_t)kq[q];
-                    origk[b + rk[q]] = b + i;
-                    posk[b + i] = b + rk[q];
-                }
-            }
-        }
-        __syncwarp();
     }
 }
 
@@ -310,18 +409,6 @@ __global__ void __launch_bounds__(kOrderWarps * 32) k_order_rows_listed(const ui
 // every chunk its start in each digit's range, and k_rank_scatter writes the chunk's entries in order (lanes with the
 // same digit ranked by __match_any_sync, a per-digit running count per warp in shared memory).
 constexpr uint32_t kRankBits = 9, kRankDigits = 1u << kRankBits, kRankChunk = 512, kRankWarps = 8;
-
-__global__ void k_vertex_degree(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ in_ptr, uint32_t n,
-                                uint32_t* __restrict__ deg, unsigned long long* maxdeg) {
-    uint32_t mx = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t d = rowptr[v + 1] - rowptr[v] + in_ptr[v + 1] - in_ptr[v];
-        deg[v] = d;
-        mx = max(mx, d);
-    }
-    mx = __reduce_max_sync(GA_FULL_MASK, mx);
-    if ((threadIdx.x & 31) == 0 && mx) atomicMax(maxdeg, (unsigned long long)mx);
-}
 
 // counts[d * nchunks + c] = entries of chunk c whose digit is d (cur == nullptr: the identity order).
 __global__ void __launch_bounds__(kRankWarps * 32) k_rank_count(const uint32_t* __restrict__ cur,
@@ -376,103 +463,80 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rank_scatter(const uint32_t
     }
 }
 
-// vrank[order[i]] = i.
-__global__ void k_rank_invert(const uint32_t* __restrict__ order, uint32_t n, uint32_t* __restrict__ vrank) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) vrank[order[i]] = i;
-}
-
-// in_rng[k] = [posk[in_eid[k]] + 1, rowptr[in_src[k] + 1]): where the probe list of in-edge k (u->v) starts and ends
-// in colk, i.e. the part of u's (degree, id)-ordered row after v.
-__global__ void k_in_rng(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ in_src,
-                         const uint32_t* __restrict__ in_eid, const uint32_t* __restrict__ posk, uint32_t m,
-                         uint2* __restrict__ in_rng) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x)
-        in_rng[k] = make_uint2(posk[in_eid[k]] + 1, rowptr[in_src[k] + 1]);
-}
-
-// colr[e] = vrank[colk[e]].
-__global__ void k_colr(const uint32_t* __restrict__ colk, const uint32_t* __restrict__ vrank, uint32_t m,
-                       uint32_t* __restrict__ colr) {
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x)
-        colr[e] = vrank[colk[e]];
-}
-
-// anchor_work[v] = probe work of the anchors below v (prefix = inclusive scan of the work over in-edges, which are
-// laid out anchor by anchor); anchor_work[n] = the whole work.
-__global__ void k_anchor_work(const uint32_t* __restrict__ in_ptr, const unsigned long long* __restrict__ prefix,
-                              uint32_t n, unsigned long long* __restrict__ anchor_work) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
-        anchor_work[v] = in_ptr[v] ? prefix[in_ptr[v] - 1] : 0ull;
-}
-
-// work[k] = probe length of in-edge k (u->v): the entries of u's (degree, id)-ordered row after v.
-__global__ void k_in_work(const uint2* __restrict__ in_rng, uint32_t m, unsigned long long* __restrict__ work) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-        const uint2 r = in_rng[k];
-        work[k] = r.y - r.x;
+// By place: vrank[order[a]] = a, dout, and what pos[] is the scan of (in-degree in the low word, octs of the row in the
+// high word: neither sum reaches 2^32, so one 64-bit scan gives both).
+__global__ void k_places(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ deg,
+                         const uint32_t* __restrict__ order, uint32_t n, uint32_t* __restrict__ vrank,
+                         uint32_t* __restrict__ dout, unsigned long long* __restrict__ pos) {
+    for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a <= n; a += (uint64_t)gridDim.x * blockDim.x) {
+        if (a == n) { pos[n] = 0; continue; }
+        const uint32_t u = order[a], d = rowptr[u + 1] - rowptr[u];
+        vrank[u] = (uint32_t)a;
+        dout[a] = d;
+        pos[a] = (unsigned long long)((d + 7) >> 3) << 32 | (deg[u] - d);
     }
 }
 
-// Items per anchor. prefix = inclusive scan of work over in-edges. An anchor with out-degree 0, no in-edge or no
-// probe work has no item; otherwise ceil(work / target) items (at most one per in-edge), light or heavy by its
-// out-degree
-// (heavy items are `heavy_factor` times larger: the block-wide table is built once per item).
-__global__ void k_count_items(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ in_ptr,
-                              const unsigned long long* __restrict__ prefix, uint32_t n, uint32_t light_max_deg,
-                              unsigned long long target, unsigned long long heavy_target,
-                              uint32_t* __restrict__ cnt_light, uint32_t* __restrict__ cnt_heavy,
-                              unsigned* max_dv_heavy) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t dv = rowptr[v + 1] - rowptr[v];
-        const uint32_t b = in_ptr[v], e = in_ptr[v + 1];
-        const bool heavy = dv > light_max_deg;
-        uint32_t c = 0;
-        if (dv > 0 && e > b) {
-            const unsigned long long w = prefix[e - 1] - (b ? prefix[b - 1] : 0ull);
-            const unsigned long long t = heavy ? heavy_target : target;
-            c = (uint32_t)((w + t - 1) / t);   // no item when no in-edge has anything to probe
-            if (c > e - b) c = e - b;
+__global__ void k_widen(const uint32_t* __restrict__ in, uint32_t n, unsigned long long* __restrict__ out) {
+    for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a <= n; a += (uint64_t)gridDim.x * blockDim.x)
+        out[a] = a < n ? in[a] : 0ull;
+}
+
+// Items of anchor a: none without out-neighbours or probe work, else ceil(work / target) (at most one per in-edge;
+// heavy anchors have kHeavyItemFactor times the target, since the block-wide set is built once per item).
+// cnt[a] = light items | heavy items << 32, tiny[a] = 1 for an anchor of the tiny bin (one item).
+__global__ void k_count_items(const uint2* __restrict__ pos, const uint32_t* __restrict__ dout,
+                              const uint32_t* __restrict__ work, uint32_t n, uint32_t light_max_deg,
+                              unsigned long long target, unsigned long long* __restrict__ cnt,
+                              uint32_t* __restrict__ tiny) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (uint64_t)gridDim.x * blockDim.x) {
+        unsigned long long c = 0;
+        uint32_t t = 0;
+        if (i < n) {
+            const uint32_t a = (uint32_t)i, d = dout[a], in = pos[a + 1].x - pos[a].x;
+            const unsigned long long w = (unsigned long long)work[a] * 8;
+            if (d && w) {
+                const bool heavy = d > light_max_deg;
+                const unsigned long long tg = heavy ? target * kHeavyItemFactor : target;
+                const unsigned long long want = min((w + tg - 1) / tg, (unsigned long long)in);
+                t = is_tiny(d, in, work[a], light_max_deg);
+                c = t ? 0ull : heavy ? want << 32 : want;
+            }
         }
-        cnt_light[v] = heavy ? 0 : c;
-        cnt_heavy[v] = heavy ? c : 0;
-        if (heavy && c) atomicMax(max_dv_heavy, dv);
+        cnt[i] = c;
+        tiny[i] = t;
     }
 }
 
-// One thread per item: finds its anchor by binary search over the item offsets, then the item's in-edge range:
-// chunk j of c covers the in-edges whose local inclusive work prefix lies in (j*w/c, (j+1)*w/c] (chunks can be
-// empty; together they cover the anchor's in-edges exactly once).
-__global__ void k_emit_items(const uint32_t* __restrict__ in_ptr, const unsigned long long* __restrict__ prefix,
-                             const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ off, uint32_t n,
-                             uint32_t total, uint32_t* __restrict__ it_v, uint32_t* __restrict__ it_k0,
-                             uint32_t* __restrict__ it_k1) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        // anchor = last v with off[v] <= i and cnt[v] > 0  (off is the exclusive scan of cnt)
-        uint32_t lo = 0, hi = n;
+// One thread per item, in the order heavy, light, tiny (each by ascending anchor): finds its anchor by binary search
+// over the bin's offsets, then its part of the anchor's in-edges (equal numbers: the in-lists are in no order of work).
+// Thread 0 leaves the bins' sizes in info[0..2].
+__global__ void k_emit_items(const uint2* __restrict__ pos, const unsigned long long* __restrict__ off,
+                             const uint32_t* __restrict__ toff, uint32_t n, uint32_t* __restrict__ it_v,
+                             uint32_t* __restrict__ it_k0, uint32_t* __restrict__ it_k1, uint32_t* __restrict__ info) {
+    const uint32_t H = (uint32_t)(off[n] >> 32), L = (uint32_t)off[n], T = toff[n];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        info[0] = H;
+        info[1] = L;
+        info[2] = T;
+    }
+    const uint64_t total = (uint64_t)H + L + T;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const int bin = i < H ? 0 : i < (uint64_t)H + L ? 1 : 2;
+        const uint32_t q = (uint32_t)(bin == 0 ? i : bin == 1 ? i - H : i - H - L);
+        auto at = [&](uint32_t a) -> uint32_t {
+            return bin == 2 ? toff[a] : bin == 1 ? (uint32_t)off[a] : (uint32_t)(off[a] >> 32);
+        };
+        uint32_t lo = 0, hi = n;   // anchor = last a with at(a) <= q (one without items shares its offset with the next)
         while (lo < hi) {
             const uint32_t mid = lo + ((hi - lo) >> 1);
-            if (off[mid] <= i) lo = mid + 1; else hi = mid;
+            if (at(mid) <= q) lo = mid + 1; else hi = mid;
         }
-        const uint32_t v = lo - 1;   // an anchor without items shares its offset with the next, so the last match has items
-        const uint32_t c = cnt[v], j = i - off[v];
-        const uint32_t b = in_ptr[v], e = in_ptr[v + 1];
-        const unsigned long long base = b ? prefix[b - 1] : 0ull, w = prefix[e - 1] - base;
-        uint32_t bound[2];
-        for (int q = 0; q < 2; q++) {
-            const uint32_t jj = j + q;
-            if (jj == 0) { bound[q] = b; continue; }
-            if (jj == c) { bound[q] = e; continue; }
-            const unsigned long long goal = base + (w * jj) / c;
-            uint32_t l2 = b, h2 = e;                   // first k with prefix[k] > goal
-            while (l2 < h2) {
-                const uint32_t mid = l2 + ((h2 - l2) >> 1);
-                if (prefix[mid] <= goal) l2 = mid + 1; else h2 = mid;
-            }
-            bound[q] = l2;
-        }
-        it_v[i] = v;
-        it_k0[i] = bound[0];
-        it_k1[i] = bound[1];
+        const uint32_t a = lo - 1, o = at(a), c = at(a + 1) - o, j = q - o;
+        const uint32_t b = pos[a].x, len = pos[a + 1].x - b;
+        it_v[i] = a;
+        it_k0[i] = b + (uint32_t)((uint64_t)len * j / c);
+        it_k1[i] = b + (uint32_t)((uint64_t)len * (j + 1) / c);
     }
 }
 
@@ -541,192 +605,114 @@ cudaMemPool_t pool_of_current() {
     return device >= 0 && device < 64 ? g_pools[device] : nullptr;
 }
 
-static ga_status build_items(ga_graph* g, const unsigned long long* prefix, uint32_t* cnt_l, uint32_t* cnt_h,
-                             uint32_t* off_l, uint32_t* off_h, unsigned* d_maxdv) {
-    cudaStream_t st = g->stream;
-    const uint32_t n = g->n;
-    const unsigned grid = grid_for(n, 256);
-    const unsigned long long target = g->item_work;   // probes per item (bounds the tail of the dynamic queue)
-    GA_CUDA(cudaMemsetAsync(d_maxdv, 0, sizeof(unsigned), st));
-    k_count_items<<<grid, 256, 0, st>>>(g->rowptr, g->in_ptr, prefix, n, g->light_max_deg, target,
-                                        target * kHeavyItemFactor, cnt_l, cnt_h, d_maxdv);
-    GA_CUDA(cudaGetLastError());
-    GA_TRY(scan_impl<uint32_t>(st, cnt_l, off_l, n, false));
-    GA_TRY(scan_impl<uint32_t>(st, cnt_h, off_h, n, false));
-    uint32_t h[5] = {0, 0, 0, 0, 0};
-    GA_CUDA(cudaMemcpyAsync(&h[0], off_l + n - 1, 4, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaMemcpyAsync(&h[1], cnt_l + n - 1, 4, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaMemcpyAsync(&h[2], off_h + n - 1, 4, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaMemcpyAsync(&h[3], cnt_h + n - 1, 4, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaMemcpyAsync(&h[4], d_maxdv, 4, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaStreamSynchronize(st));
-    ga_items* bins[2] = {&g->light, &g->heavy};
-    const uint32_t totals[2] = {h[0] + h[1], h[2] + h[3]};
-    uint32_t* cnts[2] = {cnt_l, cnt_h};
-    uint32_t* offs[2] = {off_l, off_h};
-    for (int b = 0; b < 2; b++) {
-        ga_items* it = bins[b];
-        dfree(g, it->v); dfree(g, it->k0); dfree(g, it->k1);
-        *it = ga_items{};
-        it->count = totals[b];
-        GA_TRY(dalloc(g, &it->v, totals[b]));
-        GA_TRY(dalloc(g, &it->k0, totals[b]));
-        GA_TRY(dalloc(g, &it->k1, totals[b]));
-        if (totals[b]) {
-            k_emit_items<<<grid_for(totals[b], 256), 256, 0, st>>>(g->in_ptr, prefix, cnts[b], offs[b], n,
-                                                                    totals[b], it->v, it->k0, it->k1);
-            GA_CUDA(cudaGetLastError());
-        }
-    }
-    g->light.max_dv = std::min<uint32_t>(g->light_max_deg, g->max_out_degree);
-    g->heavy.max_dv = h[4];
-    return GA_OK;
-}
-
-// The derived index (built once per handle): src, the in-lists, the (degree, id)-ordered rows and their in-edge
-// positions; checks the orientation on the way.
+// The derived index (built once per handle, on the stream, without a synchronisation: the upload checks left every size
+// it needs on the host).
 static ga_status prepare_index(ga_graph* g) {
     if (g->index_ready) return GA_OK;
-    cudaStream_t st = g->stream;
-    const uint32_t n = g->n, m = g->m;
-    GA_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t** p : {&g->src, &g->in_ptr, &g->in_src, &g->in_eid, &g->colk, &g->origk, &g->vrank, &g->colr}) {
-        dfree(g, *p);
-        *p = nullptr;
-    }
-    GA_TRY(dalloc(g, &g->src, m));
-    GA_TRY(dalloc(g, &g->in_ptr, (size_t)n + 1));
-    GA_TRY(dalloc(g, &g->in_src, m));
-    GA_TRY(dalloc(g, &g->in_eid, m));
-    GA_TRY(dalloc(g, &g->colk, (size_t)m + 4));   // padded like col: quad loads of the last row stay inside
-    GA_TRY(dalloc(g, &g->origk, m));
-    GA_CUDA(cudaMemsetAsync(g->colk + m, 0, 16, st));
-    uint32_t *indeg = nullptr, *fill = nullptr;
-    GA_CUDA(pool_malloc((void**)&indeg, ((size_t)n + 1) * 4, st));
-    GA_CUDA(pool_malloc((void**)&fill, ((size_t)n + 1) * 4, st));
-    unsigned long long* err = g->d_scalars + 63;
-    GA_CUDA(cudaMemsetAsync(err, 0, 8, st));
-    GA_CUDA(cudaMemsetAsync(indeg, 0, ((size_t)n + 1) * 4, st));
-    GA_CUDA(cudaMemsetAsync(fill, 0, ((size_t)n + 1) * 4, st));
-    const unsigned gv = grid_for(n, 256), ge = grid_for(m, 256);
-    if (n) {
-        k_src_and_indeg<<<gv, 256, 0, st>>>(g->rowptr, g->col, n, g->src, indeg);
-        GA_CUDA(cudaGetLastError());
-    }
-    GA_TRY(scan_impl<uint32_t>(st, indeg, g->in_ptr, (uint64_t)n + 1, false));   // indeg[n] = 0 -> in_ptr[n] = m
-    if (m) {
-        k_in_scatter<<<ge, 256, 0, st>>>(g->col, g->src, g->in_ptr, m, fill, g->in_src, g->in_eid);
-        GA_CUDA(cudaGetLastError());
-        // rows in (degree, id) order, from one 64-bit key per edge
-        unsigned long long* key = nullptr;
-        uint32_t* posk = nullptr;
-        GA_CUDA(pool_malloc((void**)&key, (size_t)m * 8, st));
-        GA_CUDA(pool_malloc((void**)&posk, (size_t)m * 4, st));
-        k_edge_keys<<<ge, 256, 0, st>>>(g->rowptr, g->col, g->src, g->in_ptr, m, key, err);
-        uint32_t* listed = nullptr;   // rows longer than 8, then their count
-        GA_CUDA(pool_malloc((void**)&listed, ((size_t)n + 1) * 4, st));
-        GA_CUDA(cudaMemsetAsync(listed + n, 0, 4, st));
-        k_order_rows_small<<<grid_for((uint64_t)n * 8, 256), 256, 0, st>>>(g->rowptr, key, n, g->colk, g->origk,
-                                                                            posk, listed, listed + n);
-        if (g->max_out_degree > 8)
-            k_order_rows_listed<<<(unsigned)g->sm_count * 6, kOrderWarps * 32, 0, st>>>(
-                g->rowptr, key, listed, listed + n, g->colk, g->origk, posk);
-        cudaFreeAsync(listed, st);
-        dfree(g, g->in_rng);
-        g->in_rng = nullptr;
-        GA_TRY(dalloc(g, &g->in_rng, m));
-        k_in_rng<<<ge, 256, 0, st>>>(g->rowptr, g->in_src, g->in_eid, posk, m, g->in_rng);
-        GA_CUDA(cudaGetLastError());
-        cudaFreeAsync(key, st);
-        cudaFreeAsync(posk, st);
-    }
-    cudaFreeAsync(indeg, st);
-    cudaFreeAsync(fill, st);
-    // every vertex's degree (out + in) and the largest, which sets the number of radix passes below
-    uint32_t* deg = nullptr;
-    unsigned long long* maxdeg = g->d_scalars + 61;
-    GA_CUDA(cudaMemsetAsync(maxdeg, 0, 8, st));
-    if (n) {
-        GA_CUDA(pool_malloc((void**)&deg, (size_t)n * 4, st));
-        k_vertex_degree<<<gv, 256, 0, st>>>(g->rowptr, g->in_ptr, n, deg, maxdeg);
-        GA_CUDA(cudaGetLastError());
-    }
-    unsigned long long herr = 0, hmax = 0;
-    GA_CUDA(cudaMemcpyAsync(&herr, err, 8, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaMemcpyAsync(&hmax, maxdeg, 8, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaStreamSynchronize(st));
-    if (herr & 16) {
-        cudaFreeAsync(deg, st);
+    if (g->misoriented)
         return fail(GA_ERR_INVALID_GRAPH, "CSR is not oriented by (degree, id) (graph.h:43-45): an edge points from "
                                           "the larger to the smaller endpoint, or an undirected edge is stored twice");
-    }
-    if (n) {   // vertex places in the (degree, id) order, and colk as places
-        GA_TRY(dalloc(g, &g->vrank, n));
-        GA_TRY(dalloc(g, &g->colr, (size_t)m + 4));
-        GA_CUDA(cudaMemsetAsync(g->colr + m, 0, 16, st));
+    cudaStream_t st = g->stream;
+    const uint32_t n = g->n, m = g->m;
+    auto drop = [&](auto*& p) {   // left by a build that failed half way
+        dfree(g, p);
+        p = nullptr;
+    };
+    drop(g->vrank); drop(g->order); drop(g->dout); drop(g->work);
+    drop(g->pos); drop(g->colr); drop(g->osrc); drop(g->in_rng);
+    GA_TRY(dalloc(g, &g->vrank, n));
+    GA_TRY(dalloc(g, &g->order, n));
+    GA_TRY(dalloc(g, &g->dout, n));
+    GA_TRY(dalloc(g, &g->work, n));
+    GA_TRY(dalloc(g, &g->pos, (size_t)n + 1));
+    GA_TRY(dalloc(g, &g->colr, (size_t)g->octs * 8));
+    GA_TRY(dalloc(g, &g->osrc, g->octs));
+    GA_TRY(dalloc(g, &g->in_rng, m));
+    if (n) {
+        // the vertices in (degree, id) order
+        const unsigned gv = grid_for((uint64_t)n + 1, 256);
         const uint32_t nchunks = (uint32_t)(((uint64_t)n + kRankChunk - 1) / kRankChunk);
         const uint64_t ncounts = (uint64_t)kRankDigits * nchunks;
-        uint32_t *ord0 = nullptr, *ord1 = nullptr, *counts = nullptr;
-        GA_CUDA(pool_malloc((void**)&ord0, (size_t)n * 4, st));
-        GA_CUDA(pool_malloc((void**)&ord1, (size_t)n * 4, st));
+        uint32_t passes = 1;
+        while (passes * kRankBits < 32 && (g->max_degree >> (passes * kRankBits)) != 0) passes++;
+        uint32_t *other = nullptr, *counts = nullptr;
+        GA_CUDA(pool_malloc((void**)&other, (size_t)n * 4, st));
         GA_CUDA(pool_malloc((void**)&counts, ncounts * 4, st));
         const unsigned gr = (nchunks + kRankWarps - 1) / kRankWarps;
         const uint32_t* cur = nullptr;   // the identity (id order) before the first pass
-        uint32_t* next = ord0;
-        uint32_t shift = 0;
-        do {
-            k_rank_count<<<gr, kRankWarps * 32, 0, st>>>(cur, deg, n, shift, nchunks, counts);
+        for (uint32_t ps = 0; ps < passes; ps++) {
+            uint32_t* next = ((passes - ps) & 1) ? g->order : other;   // the last pass ends in order
+            k_rank_count<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, counts);
             GA_CUDA(cudaGetLastError());
-            GA_TRY(scan_impl<uint32_t>(st, counts, counts, ncounts, false));
-            k_rank_scatter<<<gr, kRankWarps * 32, 0, st>>>(cur, deg, n, shift, nchunks, counts, next);
+            GA_TRY(scan_impl<uint32_t>(st, counts, counts, ncounts));
+            k_rank_scatter<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, counts, next);
             GA_CUDA(cudaGetLastError());
             cur = next;
-            next = next == ord0 ? ord1 : ord0;
-            shift += kRankBits;
-        } while (shift < 32 && (hmax >> shift) != 0);
-        k_rank_invert<<<gv, 256, 0, st>>>(cur, n, g->vrank);
-        GA_CUDA(cudaGetLastError());
-        if (m) {
-            k_colr<<<ge, 256, 0, st>>>(g->colk, g->vrank, m, g->colr);
-            GA_CUDA(cudaGetLastError());
         }
-        cudaFreeAsync(ord0, st);
-        cudaFreeAsync(ord1, st);
+        k_places<<<gv, 256, 0, st>>>(g->rowptr, g->deg, g->order, n, g->vrank, g->dout, (unsigned long long*)g->pos);
+        GA_CUDA(cudaGetLastError());
+        GA_TRY(scan_impl<unsigned long long>(st, (unsigned long long*)g->pos, (unsigned long long*)g->pos,
+                                             (uint64_t)n + 1));
+        GA_CUDA(cudaMemsetAsync(g->work, 0, (size_t)n * 4, st));
+        if (m) {
+            uint32_t *fill = nullptr, *listed = nullptr;   // cursors; rows longer than 8, then their count
+            GA_CUDA(pool_malloc((void**)&fill, (size_t)n * 4, st));
+            GA_CUDA(pool_malloc((void**)&listed, ((size_t)n + 1) * 4, st));
+            GA_CUDA(cudaMemsetAsync(fill, 0, (size_t)n * 4, st));
+            GA_CUDA(cudaMemsetAsync(listed + n, 0, 4, st));
+            k_place_rows_small<<<grid_for((uint64_t)(n - g->isolated) * 8, 256), 256, 0, st>>>(
+                g->rowptr, g->col, g->vrank, g->order, g->pos, g->isolated, n, g->colr, g->osrc, fill, g->work,
+                g->in_rng, listed, listed + n);
+            GA_CUDA(cudaGetLastError());
+            if (g->max_out_degree > 8)
+                k_place_rows_listed<<<(unsigned)g->sm_count * 8, 128, 0, st>>>(
+                    g->rowptr, g->col, g->vrank, g->order, g->pos, g->colr, g->osrc, fill, g->work, g->in_rng, listed,
+                    listed + n);
+            GA_CUDA(cudaGetLastError());
+            cudaFreeAsync(fill, st);
+            cudaFreeAsync(listed, st);
+        }
+        cudaFreeAsync(other, st);
         cudaFreeAsync(counts, st);
-        cudaFreeAsync(deg, st);
     }
     g->index_ready = true;
     return GA_OK;
 }
 
-// The work items of the hash kernel for the current light_max_deg / item_work (rebuilt when those change, e.g. by
-// the autotuner trying candidates): the probe work of every in-edge, its prefix, the items cut from it.
+// The work items for the current light_max_deg / item_work (rebuilt when those change, e.g. by the autotuner trying
+// candidates). Their number stays on the device (it_info); the arrays are sized by a bound: one item per anchor plus
+// one per `item_work` probes, at most one per in-edge.
 static ga_status prepare_items(ga_graph* g) {
     cudaStream_t st = g->stream;
     const uint32_t n = g->n, m = g->m;
-    unsigned long long* prefix = nullptr;
-    GA_CUDA(pool_malloc((void**)&prefix, ((size_t)m + 1) * 8, st));
-    if (m) {   // work prefix over in-edges (64-bit: the total probe count can exceed 2^32)
-        k_in_work<<<grid_for(m, 256), 256, 0, st>>>(g->in_rng, m, prefix);
-        GA_CUDA(cudaGetLastError());
-        GA_TRY(scan_impl<unsigned long long>(st, prefix, prefix, m, true));
+    if (!n || !m) return GA_OK;
+    const uint64_t bound = std::min<uint64_t>(m, (uint64_t)std::min(n, m) + g->row_work * 8 / g->item_work + 1);
+    if (bound > g->items.capacity) {
+        dfree(g, g->items.v); dfree(g, g->items.k0); dfree(g, g->items.k1);
+        g->items.v = g->items.k0 = g->items.k1 = nullptr;
+        g->items.capacity = 0;
+        GA_TRY(dalloc(g, &g->items.v, bound));
+        GA_TRY(dalloc(g, &g->items.k0, bound));
+        GA_TRY(dalloc(g, &g->items.k1, bound));
+        g->items.capacity = bound;
     }
-    if (!g->anchor_work) GA_TRY(dalloc(g, &g->anchor_work, (size_t)n + 1));
-    k_anchor_work<<<grid_for((uint64_t)n + 1, 256), 256, 0, st>>>(g->in_ptr, prefix, n, g->anchor_work);
+    if (!g->items.info) GA_TRY(dalloc(g, &g->items.info, 3));
+    g->items.bound = bound;
+    unsigned long long* cnt = nullptr;
+    uint32_t* tiny = nullptr;
+    GA_CUDA(pool_malloc((void**)&cnt, ((size_t)n + 1) * 8, st));
+    GA_CUDA(pool_malloc((void**)&tiny, ((size_t)n + 1) * 4, st));
+    k_count_items<<<grid_for((uint64_t)n + 1, 256), 256, 0, st>>>(g->pos, g->dout, g->work, n, g->light_max_deg,
+                                                                  g->item_work, cnt, tiny);
     GA_CUDA(cudaGetLastError());
-    uint32_t *cnt_l = nullptr, *cnt_h = nullptr, *off_l = nullptr, *off_h = nullptr;
-    GA_CUDA(pool_malloc((void**)&cnt_l, ((size_t)n + 1) * 4, st));
-    GA_CUDA(pool_malloc((void**)&cnt_h, ((size_t)n + 1) * 4, st));
-    GA_CUDA(pool_malloc((void**)&off_l, ((size_t)n + 1) * 4, st));
-    GA_CUDA(pool_malloc((void**)&off_h, ((size_t)n + 1) * 4, st));
-    ga_status s = GA_OK;
-    if (n) s = build_items(g, prefix, cnt_l, cnt_h, off_l, off_h, (unsigned*)(g->d_scalars + 62));
-    cudaFreeAsync(prefix, st);
-    cudaFreeAsync(cnt_l, st);
-    cudaFreeAsync(cnt_h, st);
-    cudaFreeAsync(off_l, st);
-    cudaFreeAsync(off_h, st);
-    return s;
+    GA_TRY(scan_impl<unsigned long long>(st, cnt, cnt, (uint64_t)n + 1));
+    GA_TRY(scan_impl<uint32_t>(st, tiny, tiny, (uint64_t)n + 1));
+    k_emit_items<<<grid_for(bound, 256), 256, 0, st>>>(g->pos, cnt, tiny, n, g->items.v, g->items.k0, g->items.k1,
+                                                       g->items.info);
+    GA_CUDA(cudaGetLastError());
+    cudaFreeAsync(cnt, st);
+    cudaFreeAsync(tiny, st);
+    return GA_OK;
 }
 
 ga_status prepare(ga_graph* g) {
@@ -736,6 +722,17 @@ ga_status prepare(ga_graph* g) {
     GA_TRY(prepare_items(g));
     g->prepared = true;
     return GA_OK;
+}
+
+ga_status prepare_shards(ga_graph* g) {
+    GA_TRY(prepare(g));
+    if (g->anchor_work) return GA_OK;
+    unsigned long long* w = nullptr;
+    GA_TRY(dalloc(g, &w, (size_t)g->n + 1));
+    g->anchor_work = w;
+    k_widen<<<grid_for((uint64_t)g->n + 1, 256), 256, 0, g->stream>>>(g->work, g->n, w);
+    GA_CUDA(cudaGetLastError());
+    return scan_u64(g, w, (uint64_t)g->n + 1);
 }
 
 static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint32_t n, uint32_t m, int device,
@@ -774,17 +771,23 @@ static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint
     if (cudaMemsetAsync(g->col + m, 0, 16, g->stream) != cudaSuccess)
         return bail(fail(GA_ERR_CUDA, "cudaMemsetAsync failed"));
     if ((s = dalloc(g, &g->d_scalars, 64)) != GA_OK) return bail(s);
-    if ((s = dalloc(g, &g->d_queue, 8)) != GA_OK) return bail(s);
+    if ((s = dalloc(g, &g->d_queue, 16)) != GA_OK) return bail(s);
     const cudaMemcpyKind kind = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (cudaMemcpyAsync(g->rowptr, rowptr, ((size_t)n + 1) * 4, kind, g->stream) != cudaSuccess ||
         (m && cudaMemcpyAsync(g->col, col, (size_t)m * 4, kind, g->stream) != cudaSuccess))
         return bail(fail(GA_ERR_CUDA, "CSR copy to the device failed"));
-    // validation flags in d_scalars[63], max out-degree in d_scalars[62]
-    unsigned long long* err = g->d_scalars + 63;
-    cudaMemsetAsync(g->d_scalars + 62, 0, 16, g->stream);
-    if (n) k_validate<<<grid_for(n, 256), 256, 0, g->stream>>>(g->rowptr, g->col, n, m, err);
+    // the checks, with everything the index will be sized by, in one pass (results: d_scalars, SC_*)
+    if ((s = dalloc(g, &g->src, m)) != GA_OK) return bail(s);
+    if ((s = dalloc(g, &g->deg, n)) != GA_OK) return bail(s);
+    cudaMemsetAsync(g->d_scalars, 0, 64 * 8, g->stream);
+    if (n) {
+        cudaMemsetAsync(g->deg, 0, (size_t)n * 4, g->stream);
+        k_rows<<<grid_for(n, 256), 256, 0, g->stream>>>(g->rowptr, g->col, n, m, g->src, g->deg, g->d_scalars);
+        k_degrees<<<grid_for(n, 256), 256, 0, g->stream>>>(g->rowptr, n, g->deg, g->d_scalars);
+        if (m) k_orient<<<grid_for(m, 256), 256, 0, g->stream>>>(g->src, g->col, g->deg, n, m, g->d_scalars);
+    }
     uint32_t ends[2] = {0, 0};
-    cudaMemcpyAsync(g->h_scalars + 62, g->d_scalars + 62, 16, cudaMemcpyDeviceToHost, g->stream);
+    cudaMemcpyAsync(g->h_scalars, g->d_scalars, 64 * 8, cudaMemcpyDeviceToHost, g->stream);
     if (from_device) {
         cudaMemcpyAsync(&ends[0], g->rowptr, 4, cudaMemcpyDeviceToHost, g->stream);
         cudaMemcpyAsync(&ends[1], g->rowptr + n, 4, cudaMemcpyDeviceToHost, g->stream);
@@ -795,10 +798,16 @@ static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint
     }
     if (from_device && (ends[0] != 0 || ends[1] != m))
         return bail(fail(GA_ERR_INVALID_GRAPH, "rowptr[0] must be 0 and rowptr[n] must equal m"));
-    if (g->h_scalars[63])
+    if (g->h_scalars[SC_ERR])
         return bail(fail(GA_ERR_INVALID_GRAPH, "invalid CSR (flags 0x%llx: 1 rowptr, 2 endpoint >= n, 4 self loop, "
-                                               "8 row not strictly ascending)", g->h_scalars[63]));
-    g->max_out_degree = (uint32_t)g->h_scalars[62];
+                                               "8 row not strictly ascending)", g->h_scalars[SC_ERR]));
+    g->max_out_degree = (uint32_t)g->h_scalars[SC_MAXOUT];
+    g->max_degree = (uint32_t)g->h_scalars[SC_MAXDEG];
+    g->isolated = (uint32_t)g->h_scalars[SC_ISOLATED];
+    g->octs = g->h_scalars[SC_OCTS];
+    g->row_work = g->h_scalars[SC_WORK];
+    g->misoriented = g->h_scalars[SC_ORIENT] != 0;
+    for (int b = 0; b < 33; b++) g->row_hist[b] = g->h_scalars[SC_HIST + b];
     *out = g;
     return GA_OK;
 }

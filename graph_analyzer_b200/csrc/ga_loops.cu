@@ -152,8 +152,7 @@ __global__ void k_loop_scalars(LoopScalars* sc, const unsigned long long* total,
 // Appends the frontier vertex v (mark kernels): its id to frontier[], and ceil(deg(v) / kChunk) update items.
 // All 32 lanes call it; `take` marks the lanes that append. One atomic per warp for each list.
 // With incidence lists (inc_ptr != null) the items are ceil(|Tri(v)| / kListChunk) slices of v's list instead.
-__device__ __forceinline__ void append_frontier(bool take, uint32_t v, const uint32_t* __restrict__ rowptr,
-                                                const uint32_t* __restrict__ in_ptr,
+__device__ __forceinline__ void append_frontier(bool take, uint32_t v, const uint32_t* __restrict__ degree,
                                                 const unsigned long long* __restrict__ inc_ptr, LoopScalars* sc,
                                                 uint32_t* __restrict__ frontier, uint32_t* __restrict__ item_x,
                                                 uint32_t* __restrict__ item_c, uint32_t lane) {
@@ -168,8 +167,7 @@ __device__ __forceinline__ void append_frontier(bool take, uint32_t v, const uin
         if (inc_ptr) {
             nc = (uint32_t)((inc_ptr[v + 1] - inc_ptr[v] + kListChunk - 1) / kListChunk);
         } else {
-            const uint32_t deg = rowptr[v + 1] - rowptr[v] + in_ptr[v + 1] - in_ptr[v];
-            nc = (deg + kChunk - 1) / kChunk;
+            nc = (uint32_t)(((uint64_t)degree[v] + kChunk - 1) / kChunk);
         }
     }
     const uint32_t incl = warp_incl_scan(nc, lane);
@@ -210,8 +208,7 @@ __global__ void __launch_bounds__(256) k_peel_mark(LoopScalars* sc, const uint32
                                                    uint8_t* __restrict__ state, uint32_t* __restrict__ removed_round,
                                                    uint32_t* alive0, uint32_t* alive1, uint32_t* fr0, uint32_t* fr1,
                                                    uint32_t* __restrict__ item_x,
-                                                   uint32_t* __restrict__ item_c, const uint32_t* __restrict__ rowptr,
-                                                   const uint32_t* __restrict__ in_ptr,
+                                                   uint32_t* __restrict__ item_c, const uint32_t* __restrict__ degree,
                                                    const unsigned long long* __restrict__ inc_ptr, Segs sg) {
     const uint32_t p = sc->parity;
     uint32_t* frontier = (sc->round & 1) ? fr1 : fr0;
@@ -263,7 +260,7 @@ __global__ void __launch_bounds__(256) k_peel_mark(LoopScalars* sc, const uint32
                     atomicAdd(&sg.removed[s], (unsigned long long)__popc(peers));
             }
         }
-        append_frontier(rem, v, rowptr, in_ptr, inc_ptr, sc, frontier, item_x, item_c, lane);
+        append_frontier(rem, v, degree, inc_ptr, sc, frontier, item_x, item_c, lane);
         append_survivor(valid && !rem && !drop, v, outl, &sc->alive_count[p ^ 1], lane);
     }
 }
@@ -295,8 +292,7 @@ __global__ void __launch_bounds__(256) k_core_mark(LoopScalars* sc, const uint32
                                                    uint8_t* __restrict__ state, uint32_t* __restrict__ core,
                                                    uint32_t* alive0, uint32_t* alive1, uint32_t* fr0, uint32_t* fr1,
                                                    uint32_t* __restrict__ item_x,
-                                                   uint32_t* __restrict__ item_c, const uint32_t* __restrict__ rowptr,
-                                                   const uint32_t* __restrict__ in_ptr,
+                                                   uint32_t* __restrict__ item_c, const uint32_t* __restrict__ degree,
                                                    const unsigned long long* __restrict__ inc_ptr) {
     if (!sc->cont) return;
     const uint32_t p = sc->parity;
@@ -320,7 +316,7 @@ __global__ void __launch_bounds__(256) k_core_mark(LoopScalars* sc, const uint32
                 core[v] = k;
             }
         }
-        append_frontier(rem, v, rowptr, in_ptr, inc_ptr, sc, frontier, item_x, item_c, lane);
+        append_frontier(rem, v, degree, inc_ptr, sc, frontier, item_x, item_c, lane);
         append_survivor(valid && !rem, v, outl, &sc->alive_count[p ^ 1], lane);
     }
 }
@@ -432,7 +428,7 @@ __device__ __forceinline__ bool last_round(const LoopScalars* sc, const Segs& sg
 // rows N+(x) and N+(w).
 __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
     LoopScalars* sc, const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
-    const uint32_t* __restrict__ in_ptr, const uint32_t* __restrict__ in_src, const uint32_t* __restrict__ item_x,
+    const uint32_t* __restrict__ degree, TcIndex ix, const uint32_t* __restrict__ item_x,
     const uint32_t* __restrict__ item_c, const uint8_t* __restrict__ state, uint32_t* __restrict__ tri, Segs sg,
     int kind, cudaGraphConditionalHandle handle, int use_handle) {
     constexpr uint32_t kSlots = 2 * kChunk;   // 512 slots, load <= 1/2
@@ -454,14 +450,17 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
         if (sg.count && sg.removed[seg] == sg.nalive[seg]) continue;   // its graph's last round
         const unsigned long long d0 = destroyed;
         const uint32_t xb = rowptr[x], dout = rowptr[x + 1] - xb;
-        const uint32_t ib = in_ptr[x], din = in_ptr[x + 1] - ib;
-        const uint32_t deg = dout + din;
+        const uint32_t ib = ix.pos[ix.vrank[x]].x;   // in-edges of x: their sources through the index
+        const uint32_t deg = degree[x];
+        auto neighbour = [&](uint32_t q) {
+            return q < dout ? col[xb + q] : ix.order[ix.osrc[rng_at(ix.in_rng[ib + q - dout]) >> 3]];
+        };
         const bool local = deg <= kChunk;
         if (local) {
             for (uint32_t s = lane; s < kSlots; s += 32) key[s] = GA_EMPTY;
             __syncwarp();
             for (uint32_t q = lane; q < deg; q += 32) {
-                const uint32_t y = q < dout ? col[xb + q] : in_src[ib + q - dout];
+                const uint32_t y = neighbour(q);
                 if (state[y] == 0) continue;
                 uint32_t h = hash_slot(y, kBits);
                 while (atomicCAS(&key[h], GA_EMPTY, y) != GA_EMPTY) h = (h + 1) & (kSlots - 1);
@@ -474,7 +473,7 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
             uint32_t d = 0, rb = 0, y = 0;
             uint8_t sy = 0;
             if (q < q1) {
-                y = q < dout ? col[xb + q] : in_src[ib + q - dout];
+                y = neighbour(q);
                 sy = state[y];
                 if (sy) {
                     rb = rowptr[y];
@@ -1201,8 +1200,8 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
     const Segs sg = KIND == LOOP_PEEL ? L->segs : Segs{};
     if (KIND == LOOP_PEEL) {
         k_peel_mark<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
-                                                  L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->rowptr,
-                                                  g->in_ptr, inc_ptr, sg);
+                                                  L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->deg,
+                                                  inc_ptr, sg);
     } else {
         const int csize = use_h && L->lists == 1 ? small_round_cluster(g->device) : 0;
         if (csize) {   // the small rounds first, in one cluster; the grid kernels below take the first large one
@@ -1226,15 +1225,15 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
         k_core_min<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->alive[0], L->alive[1], L->state, L->frontier[0],
                                                  L->frontier[1], h, use_h);
         k_core_mark<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
-                                                  L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->rowptr,
-                                                  g->in_ptr, inc_ptr);
+                                                  L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->deg,
+                                                  inc_ptr);
     }
     // the update kernel's last block closes the round and sets the loop condition
     if (L->lists == 1)
         k_frontier_update_list<<<L->grid_update, 256, 0, st>>>(L->sc, L->inc, L->inc_ptr, L->item_x, L->item_c,
                                                                L->state, L->tri, sg, KIND, h, use_h);
     else
-        k_frontier_update<<<L->grid_update, kUpdWarps * 32, 0, st>>>(L->sc, g->rowptr, g->col, g->in_ptr, g->in_src,
+        k_frontier_update<<<L->grid_update, kUpdWarps * 32, 0, st>>>(L->sc, g->rowptr, g->col, g->deg, tc_index(g),
                                                                 L->item_x, L->item_c, L->state, L->tri, sg, KIND,
                                                                 h, use_h);
     GA_CUDA(cudaGetLastError());

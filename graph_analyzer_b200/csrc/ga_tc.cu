@@ -7,30 +7,36 @@
 //
 //     T = sum over anchors v of sum over in-edges u->v of |N+(u) ∩ N+(v)|
 //
-// N+(v) is loaded ONCE into a shared-memory hash set and the in-neighbours' lists are streamed past it (probe). A
-// common neighbour x of u and v has v->x, so it comes after v in the orientation order; with every row also kept in
-// (degree, id) order (colk, built by ga_graph.cu), the probe list of in-edge u->v is just the part of u's row after
-// v. Probe work is sum_u d+(u)(d+(u)-1)/2, half of sum_u d+(u)^2 and a quarter or less of the merge sum's
+// N+(v) is loaded ONCE into a shared-memory set and the in-neighbours' lists are streamed past it (probe). A common
+// neighbour x of u and v has v->x, so it comes after v in the orientation order; the index (ga_graph.cu) numbers the
+// vertices in that order (places) and keeps every row ascending, so the probe list of in-edge u->v is just the part of
+// u's row after v. Probe work is sum_u d+(u)(d+(u)-1)/2, half of sum_u d+(u)^2 and a quarter or less of the merge sum's
 // sum_{u->v} (d+(u) + d+(v)) on power-law graphs, and each probe is one shared-memory load instead of a merge step
-// or a binary search in global memory.
+// or a binary search in global memory. Rows are padded to octs (8 places, one 32-byte sector) with a value that is in
+// no set: a lane reads one oct and does eight probes without testing where the list starts or ends, so the search for
+// the list an oct belongs to and the loop around it are paid once per eight probes (once per four, with two range tests
+// a probe, when rows were unpadded ids: R-MAT 22 count 2.56 ms against 2.23, R-MAT 20 0.79 against 0.49).
 //
 // Scheduler (degree-binned, one persistent launch):
 //   * work items = slices of an anchor's in-edge list with bounded probe work (built in ga_graph.cu);
-//   * HEAVY bin: anchors with out-degree > light_max_deg. The whole block (8 warps) shares one hash set of N+(v) in
-//     dynamic shared memory and splits the in-edges; anchors whose set does not fit fall back to binary search in
-//     the sorted global row;
+//   * HEAVY bin: anchors with out-degree > light_max_deg. The whole block (8 warps) shares one set of N+(v) in dynamic
+//     shared memory - for counts a bitmap over places, else a hash set - and splits the in-edges; anchors whose set
+//     does not fit fall back to binary search in their row;
 //   * LIGHT bin: every warp owns a 512-slot hash set and takes items on its own;
-//   * blocks drain the heavy queue first, then the light queue (one atomic per item fetch).
-// Inside an item a warp processes 32 in-edges at a time: lane l loads the l-th source, a warp scan of the list
-// lengths flattens the 32 lists into one probe sequence, and lane p takes probes p, p+32, ... so lanes stay busy
+//   * TINY bin: anchors of at most 16 out-neighbours and 32 in-edges; a count takes 32 consecutive ones at a time, one
+//     lane per in-edge, without any set (other passes run them like light ones);
+//   * blocks drain the heavy queue first, then the light queue, then the tiny one (one atomic per fetch).
+// Inside an item a warp processes 32 in-edges at a time: lane l loads the l-th record, a warp scan of the list
+// lengths flattens the 32 lists into one sequence of octs, and lane p takes octs p, p+32, ... so lanes stay busy
 // whatever the list lengths are (load-balanced search: each lane advances its owner index monotonically).
 //
 // Results per triangle (u->v in-edge, x common, x at position e of N+(u) and j of N+(v)):
 //   COUNT: T only, one 64-bit atomic per block at the end.
 //   VSUP : per-vertex counts: x through a per-slot shared counter (flushed once per item), u through a per-in-edge
 //          shared counter (flushed once per 32 in-edges), v through a warp reduction (once per item).
-//   ESUP : per-edge counts indexed like col (for_each_triangle's (e_uv, e_ux, e_vx), dsg.h:67-79): e_uv and e_vx
-//          through shared counters as above, e_ux with one global atomic per triangle.
+//   ESUP : per-edge counts (for_each_triangle's (e_uv, e_ux, e_vx), dsg.h:67-79): e_uv and e_vx through shared
+//          counters as above, e_ux with one global atomic per triangle, all at the entries' positions in colr; moved
+//          to col order after the pass.
 //   ALIVE: restricts everything to the subgraph induced by alive[] (tc_per_vertex_alive, kernels.cuh:399-425).
 #include <algorithm>
 #include <cstdio>
@@ -44,7 +50,8 @@
 namespace ga {
 
 #ifndef GA_TC_MIN_BLOCKS
-#define GA_TC_MIN_BLOCKS 8                // resident blocks per SM the hash kernel is compiled for (full occupancy)
+#define GA_TC_MIN_BLOCKS 8                // resident blocks per SM the hash kernel is compiled for (R-MAT 22 count:
+                                          // 2.23 ms; 6: 2.24, 5: 2.36, 4: 2.62)
 #endif
 
 constexpr int kWarps = 8;                 // warps per block of the hash kernel
@@ -65,8 +72,8 @@ struct SlotLayout {   // 32-bit words per hash slot: key, +count (VSUP/ESUP), +p
     static constexpr int words = 1 + (counters(MODE) ? 1 : 0) + (MODE == TC_ESUP ? 1 : 0);
 };
 
-// Per-warp batch area: incl[32], rb[32], re[32], ecnt[32], u[32].
-constexpr int kBatchWords = 160;
+// Per-warp batch area: incl[32], base[32], ecnt[32], u[32].
+constexpr int kBatchWords = 128;
 
 // Shared memory of the light phase per warp: slots * words + the batch area.
 template <int MODE>
@@ -107,8 +114,8 @@ __device__ __forceinline__ uint32_t bucket_match(const uint32_t* key, uint32_t b
     }
 }
 
-// Writes the triangle (u lowest, v middle, x highest) into the incidence list of each corner. A list is sized by the
-// counting pass; an entry that would land past its list's end is dropped and counted in *overflow instead.
+// Writes the triangle (u lowest, v middle, x highest; ids) into the incidence list of each corner. A list is sized by
+// the counting pass; an entry that would land past its list's end is dropped and counted in *overflow instead.
 template <class CT>
 __device__ __forceinline__ void list_one(const TcArgs<CT>& a, uint32_t c, uint32_t p, uint32_t q) {
     const unsigned long long pos = a.inc_ptr[c] + atomicAdd(&a.fill[c], 1u);
@@ -122,117 +129,115 @@ __device__ __forceinline__ void list_triangle(const TcArgs<CT>& a, uint32_t u, u
     list_one(a, v, u, x);
 }
 
-template <int MODE, bool ALIVE, class CT>
-__device__ __forceinline__ void on_hit(const TcArgs<CT>& a, uint32_t* cnt, uint32_t h, uint32_t* ecnt,
-                                       uint32_t owner, uint32_t e, uint32_t anchor, uint32_t x, const uint32_t* s_u) {
-    if (counters(MODE)) {
-        atomicAdd(&cnt[h], 1u);
-        atomicAdd(&ecnt[owner], 1u);
-    }
-    if (MODE == TC_ESUP) atomicAdd(&a.esupk[e], 1u);   // u->x at its probe position; folded into col order after
-    if (MODE == TC_LIST) list_triangle(a, s_u[owner], anchor, x);
+// An anchor as the probe loops see it: its row (octs of colr), its members in a table (bits > 0) or only in the row.
+struct Anchor {
+    uint32_t v, id, row, dv;   // place, id (LIST), first oct of the row, out-degree
+    uint32_t bits;             // table size; 0: binary search in the row
+};
+
+template <int MODE, class CT>
+__device__ __forceinline__ void on_hit(const TcArgs<CT>& a, uint32_t* s_ecnt, uint32_t owner, size_t e,
+                                       const Anchor& an, uint32_t x, const uint32_t* s_u) {
+    if (counters(MODE)) atomicAdd(&s_ecnt[owner], 1u);
+    if (MODE == TC_ESUP) atomicAdd(&a.esupk[e], 1u);   // u->x at its place in u's row; moved to col order after the pass
+    if (MODE == TC_LIST) list_triangle(a, s_u[owner], an.id, a.ix.order[x]);
 }
 
-// Looks x (at colk position e, probe list of in-edge `owner`) up in the hash set or, when `global`, by binary search
-// in the id-sorted row N+(v) = col[vb, vb + dv). Returns 1 on a hit and books the supports of the found triangle.
+// Looks place x (entry e of colr, probe list of in-edge `owner`) up in the hash set or, without one, by binary search
+// in the row of the anchor. Returns 1 on a hit and books the supports of the found triangle. The padding of a row is
+// above every place, so it is never found.
 template <int MODE, bool ALIVE, class CT>
-__device__ __forceinline__ uint32_t probe_one(const uint32_t* __restrict__ col, const TcArgs<CT>& a, uint32_t x,
-                                              uint32_t e, uint32_t owner, const uint32_t* key, uint32_t* cnt,
-                                              uint32_t bits, bool global, uint32_t vb, uint32_t dv,
-                                              uint32_t* s_ecnt, uint32_t anchor, const uint32_t* s_u) {
-    if (!global) {
+__device__ __forceinline__ uint32_t probe_one(const TcArgs<CT>& a, uint32_t x, size_t e, uint32_t owner,
+                                              const uint32_t* key, uint32_t* cnt, const Anchor& an,
+                                              uint32_t* s_ecnt, const uint32_t* s_u) {
+    if (an.bits) {
         // bucketed set (bucket_slots<MODE>() slots per bucket); a bucket fills its slots in order, so an empty last
         // slot ends the search. One shared load resolves almost every lookup.
-        const uint32_t nb = bits + bucket_shift<MODE>(), mask = (1u << nb) - 1;
+        const uint32_t nb = an.bits + bucket_shift<MODE>(), mask = (1u << nb) - 1;
         uint32_t b = hash_slot(x, nb);
         for (;;) {
             bool open;
             const uint32_t m = bucket_match<MODE>(key, b, x, &open);
             if (m) {
-                on_hit<MODE, ALIVE, CT>(a, cnt, bucket_slots<MODE>() * b + (__ffs(m) - 1), s_ecnt, owner, e, anchor,
-                                        x, s_u);
+                if (counters(MODE)) atomicAdd(&cnt[bucket_slots<MODE>() * b + (__ffs(m) - 1)], 1u);
+                on_hit<MODE, CT>(a, s_ecnt, owner, e, an, x, s_u);
                 return 1;
             }
             if (open) return 0;
             b = (b + 1) & mask;
         }
     }
-    const uint32_t j = lower_bound_u32(col, vb, vb + dv, x);
-    if (j < vb + dv && col[j] == x && (!ALIVE || a.alive[x])) {
-        if (counters(MODE)) atomicAdd(&s_ecnt[owner], 1u);
+    const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
+    const uint32_t j = lower_bound_u32(row, 0, an.dv, x);
+    if (j < an.dv && row[j] == x && (!ALIVE || a.alive[x])) {
         if (MODE == TC_VSUP) atomicAdd(&a.vsup[x], (CT)1);
-        if (MODE == TC_ESUP) {
-            atomicAdd(&a.esupk[e], 1u);
-            atomicAdd(&a.esup[j], 1u);
-        }
-        if (MODE == TC_LIST) list_triangle(a, s_u[owner], anchor, x);
+        if (MODE == TC_ESUP) atomicAdd(&a.esupk[(size_t)an.row * 8 + j], 1u);
+        on_hit<MODE, CT>(a, s_ecnt, owner, e, an, x, s_u);
         return 1;
     }
     return 0;
 }
 
-// Probes one batch of up to 32 in-edges [kb, kend) of anchor v (one warp). Lane l loads the l-th in-edge's probe
-// list, the part of its source u's (degree, id)-ordered row after v, colk[rb, re), from in_rng in one 64-bit load
-// (sources are read only where the mode needs them). The list is cut into 16-byte quads (colk is 16-byte aligned and
-// padded, so a quad never leaves the allocation), a warp scan of the quad counts flattens the 32 lists into one
-// sequence, and lane p takes quads p, p+32, ...: one 128-bit load, then up to 4 probes of the elements inside
-// [rb, re). Each lane advances its owner index monotonically. Returns this lane's hits.
-template <int MODE, bool ALIVE, class CT>
-__device__ __forceinline__ unsigned long long probe_batch(
-    const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col, const uint32_t* __restrict__ colk,
-    const uint32_t* __restrict__ in_src, const uint32_t* __restrict__ in_eid,
-    const TcArgs<CT>& a, uint32_t kb, uint32_t kend, const uint32_t* key, uint32_t* cnt, uint32_t bits, bool global,
-    uint32_t vb, uint32_t dv, uint32_t* s_incl, uint32_t* s_rb, uint32_t* s_ecnt, uint32_t lane, uint32_t anchor) {
-    unsigned long long hits = 0;
-    uint32_t* s_re = s_rb + 32;   // the caller's batch area: incl[32], rb[32], re[32], ecnt[32], u[32]
-    uint32_t* s_u = s_rb + 96;
+// The probe lists of a batch of up to 32 in-edges [kb, kend) (one warp): lane l takes the l-th in-edge's suffix of its
+// source's row, a run of whole octs, from in_rng. A warp scan of the oct counts flattens the lists into one sequence:
+// oct p of it is oct s_base[owner] + p of colr, owner the first with s_incl[owner] > p. Entries of the first oct before
+// the suffix are at or below the anchor's place and the last oct's padding is above every place, so neither is a member
+// of N+(anchor) and the probes test no ends. Returns the octs of the batch; *r this lane's record (0: none).
+template <bool ALIVE, class IX>
+__device__ __forceinline__ uint32_t open_batch(const IX& ix, const uint8_t* alive, uint32_t kb, uint32_t kend,
+                                               uint32_t lane, uint32_t* s_incl, uint32_t* s_base,
+                                               unsigned long long* rec) {
     const uint32_t k = kb + lane;
-    uint32_t nq = 0, rb = 0, re = 0, u = 0;
-    if (k < kend) {
-        if (ALIVE || MODE == TC_LIST || MODE == TC_VSUP) u = in_src[k];   // the source's mask, list entry, count
-        if (!ALIVE || a.alive[u]) {
-            const uint2 r = a.in_rng[k];
-            rb = r.x;
-            re = r.y;
-            if (re > rb) nq = ((re + 3) >> 2) - (rb >> 2);
-        }
-    }
+    unsigned long long r = k < kend ? ix.in_rng[k] : 0ull;
+    uint32_t nq = rng_octs(r);
+    if (ALIVE && nq && !alive[ix.osrc[rng_at(r) >> 3]]) nq = 0;
     const uint32_t incl = warp_incl_scan(nq, lane);
-    const uint32_t tot = __shfl_sync(GA_FULL_MASK, incl, 31);
     s_incl[lane] = incl;
-    s_rb[lane] = rb;
-    s_re[lane] = re;
-    if (MODE == TC_LIST) s_u[lane] = u;
+    s_base[lane] = rng_oct(r) - (incl - nq);
+    *rec = nq ? r : 0ull;
     __syncwarp();
-    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(colk);
-    uint32_t owner = 0;
-    if (MODE == TC_COUNT && !global) {
-        // counts in a table: the four lookups of a quad are issued without branches (elements outside the list
-        // still read a bucket, their result is masked), so they overlap; a bucket that is full without a match
-        // (rare at a load of at most 1/4 per bucket) continues in the next buckets afterwards
-        const uint32_t nb = bits + bucket_shift<MODE>(), bmask = (1u << nb) - 1;
+    return __shfl_sync(GA_FULL_MASK, incl, 31);
+}
+
+// Probes one batch of anchor `an` and books what MODE asks for. Returns this lane's hits.
+template <int MODE, bool ALIVE, class CT>
+__device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb, uint32_t kend, const uint32_t* key,
+                                                uint32_t* cnt, const Anchor& an, uint32_t* s_incl, uint32_t* s_base,
+                                                uint32_t lane) {
+    uint32_t hits = 0;
+    uint32_t *s_ecnt = s_base + 32, *s_u = s_base + 64;   // the caller's batch area: incl, base, ecnt, u
+    unsigned long long rec;
+    const uint32_t tot = open_batch<ALIVE>(a.ix, a.alive, kb, kend, lane, s_incl, s_base, &rec);
+    uint32_t u = 0;
+    if ((MODE == TC_LIST || MODE == TC_VSUP) && rec) u = a.ix.osrc[rng_at(rec) >> 3];   // the source's place
+    if (MODE == TC_LIST) {
+        s_u[lane] = rec ? a.ix.order[u] : 0u;
+        __syncwarp();
+    }
+    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
+    uint32_t owner = 0, end = s_incl[0];
+    if (MODE == TC_COUNT && an.bits) {
+        // counts in a table: the eight lookups of an oct are issued without branches, so they overlap; a bucket that
+        // is full without a match (rare) continues in the next buckets afterwards
+        const uint32_t nb = an.bits + bucket_shift<MODE>(), bmask = (1u << nb) - 1;
         for (uint32_t p = lane; p < tot; p += 32) {
-            while (s_incl[owner] <= p) owner++;
-            const uint32_t lo = s_rb[owner], span = s_re[owner] - lo;
-            const uint32_t q = (lo >> 2) + (p - (owner ? s_incl[owner - 1] : 0u));
-            const uint4 v = __ldg(col4 + q);
-            const uint32_t off = (q << 2) - lo;   // element i of the quad is in the list iff off + i < span
-            const uint32_t xs[4] = {v.x, v.y, v.z, v.w};
-            uint32_t found = 0, more = 0;
+            while (end <= p) end = s_incl[++owner];
+            const size_t q = s_base[owner] + p;
+            const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
+            const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            uint32_t more = 0;
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
+            for (int i = 0; i < 8; i++) {
                 const uint32_t x = xs[i];
                 bool open;
                 const bool m = bucket_match<MODE>(key, hash_slot(x, nb), x, &open) != 0;
-                const bool in = off + i < span;
-                found |= (uint32_t)(in & m) << i;
-                more |= (uint32_t)(in & !m & !open) << i;
+                hits += m;
+                more |= (uint32_t)(!m & !open) << i;
             }
-            hits += __popc(found);
             while (more) {
                 const int i = __ffs(more) - 1;
                 more &= more - 1;
-                const uint32_t x = xs[i];
+                const uint32_t x = __ldg(a.ix.colr + 8 * q + i);
                 uint32_t b = hash_slot(x, nb);
                 for (;;) {
                     b = (b + 1) & bmask;
@@ -246,30 +251,20 @@ __device__ __forceinline__ unsigned long long probe_batch(
         return hits;
     }
     for (uint32_t p = lane; p < tot; p += 32) {
-        while (s_incl[owner] <= p) owner++;
-        const uint32_t lo = s_rb[owner], hi = s_re[owner];
-        const uint32_t q = (lo >> 2) + (p - (owner ? s_incl[owner - 1] : 0u));
-        const uint4 v = __ldg(col4 + q);
-        const uint32_t e0 = q << 2;
-        if (e0 >= lo && e0 < hi)
-            hits += probe_one<MODE, ALIVE, CT>(col, a, v.x, e0, owner, key, cnt, bits, global, vb, dv, s_ecnt,
-                                               anchor, s_u);
-        if (e0 + 1 >= lo && e0 + 1 < hi)
-            hits += probe_one<MODE, ALIVE, CT>(col, a, v.y, e0 + 1, owner, key, cnt, bits, global, vb, dv, s_ecnt,
-                                               anchor, s_u);
-        if (e0 + 2 >= lo && e0 + 2 < hi)
-            hits += probe_one<MODE, ALIVE, CT>(col, a, v.z, e0 + 2, owner, key, cnt, bits, global, vb, dv, s_ecnt,
-                                               anchor, s_u);
-        if (e0 + 3 >= lo && e0 + 3 < hi)
-            hits += probe_one<MODE, ALIVE, CT>(col, a, v.w, e0 + 3, owner, key, cnt, bits, global, vb, dv, s_ecnt,
-                                               anchor, s_u);
+        while (end <= p) end = s_incl[++owner];
+        const size_t q = s_base[owner] + p;
+        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
+        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            hits += probe_one<MODE, ALIVE, CT>(a, xs[i], 8 * q + i, owner, key, cnt, an, s_ecnt, s_u);
     }
     __syncwarp();
     if (counters(MODE)) {
         const uint32_t c = s_ecnt[lane];
         if (c) {
             if (MODE == TC_VSUP) atomicAdd(&a.vsup[u], (CT)c);
-            else atomicAdd(&a.esup[in_eid[k]], c);
+            else atomicAdd(&a.esupk[rng_at(rec)], c);
             s_ecnt[lane] = 0;
         }
     }
@@ -291,18 +286,18 @@ __device__ __forceinline__ uint32_t table_bits(uint32_t dv, uint32_t cap) {
 // bucket, or moves on to the next bucket when all of them are taken, flagging the full one where the mode keeps spill
 // flags (kTabSpill in its last slot, which holds a key by then). tid/nthr cover the cooperating threads.
 template <int MODE, bool ALIVE, class CT>
-__device__ __forceinline__ void build_table(const uint32_t* __restrict__ col, const TcArgs<CT>& a, uint32_t vb,
-                                            uint32_t dv, uint32_t* key, uint32_t* cnt, uint32_t* pos, uint32_t bits,
-                                            uint32_t tid, uint32_t nthr, bool sync_block) {
+__device__ __forceinline__ void build_table(const TcArgs<CT>& a, const Anchor& an, uint32_t* key, uint32_t* cnt,
+                                            uint32_t* pos, uint32_t tid, uint32_t nthr, bool sync_block) {
     constexpr uint32_t B = bucket_slots<MODE>();
-    const uint32_t S = 4u << bits, nb = bits + bucket_shift<MODE>(), mask = (1u << nb) - 1;
-    for (uint32_t s = tid; s < S; s += nthr) {
-        key[s] = kTabEmpty;
-        if (counters(MODE)) cnt[s] = 0;
+    const uint32_t S = 4u << an.bits, nb = an.bits + bucket_shift<MODE>(), mask = (1u << nb) - 1;
+    for (uint32_t s = tid; s < S / 4; s += nthr) {
+        reinterpret_cast<uint4*>(key)[s] = make_uint4(kTabEmpty, kTabEmpty, kTabEmpty, kTabEmpty);
+        if (counters(MODE)) reinterpret_cast<uint4*>(cnt)[s] = make_uint4(0, 0, 0, 0);
     }
     if (sync_block) __syncthreads(); else __syncwarp();
-    for (uint32_t i = tid; i < dv; i += nthr) {
-        const uint32_t x = col[vb + i];
+    const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
+    for (uint32_t i = tid; i < an.dv; i += nthr) {
+        const uint32_t x = row[i];
         if (ALIVE && !a.alive[x]) continue;
         uint32_t b = hash_slot(x, nb), slot = B * b;
         while (atomicCAS(&key[slot], kTabEmpty, x) != kTabEmpty) {
@@ -318,66 +313,45 @@ __device__ __forceinline__ void build_table(const uint32_t* __restrict__ col, co
     if (sync_block) __syncthreads(); else __syncwarp();
 }
 
-// Heavy anchors of a count use a bitmap of N+(v) instead of a hash set when it fits the table's shared memory: in the
-// (degree, id) order every out-neighbour of v comes after v, and for the anchors of many out-neighbours (high degree)
-// they lie in a short range of places above v's own (R-MAT 22: under 65,536 places for every anchor of more than 128
-// out-neighbours, against 4.2M vertices). Bit o of the bitmap is set iff the vertex at place base + o is an (alive)
-// out-neighbour of v, base = v's place + 1; span = the largest out-neighbour's place - v's place bounds o. A probe is
-// then one shared 32-bit load and a bit test, with no collisions and nothing to continue.
+// Heavy anchors of a count use a bitmap of N+(v) instead of a hash set when it fits the table's shared memory: every
+// out-neighbour's place is above v's own, and for the anchors of many out-neighbours (high degree) they lie in a short
+// range (R-MAT 22: under 65,536 places for every anchor of more than 128 out-neighbours, against 4.2M vertices). Bit o
+// of the bitmap is set iff place base + o is an (alive) out-neighbour of v, base = v + 1; span = the largest
+// out-neighbour - v bounds o. A probe is then one shared 32-bit load and a bit test, with no collisions and nothing to
+// continue; the entries before the suffix and the padding fall outside [0, span).
 template <bool ALIVE, class CT>
-__device__ __forceinline__ void build_bitmap(const uint32_t* __restrict__ colk, const TcArgs<CT>& a, uint32_t vb,
-                                             uint32_t dv, uint32_t base, uint32_t span, uint32_t* bm) {
-    const uint32_t words = (span + 31) >> 5;
-    for (uint32_t w = threadIdx.x; w < words; w += kThreads) bm[w] = 0;
+__device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& an, uint32_t span, uint32_t* bm) {
+    const uint32_t quads = (span + 127) >> 7;
+    for (uint32_t w = threadIdx.x; w < quads; w += kThreads) reinterpret_cast<uint4*>(bm)[w] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < dv; i += kThreads) {
-        if (ALIVE && !a.alive[colk[vb + i]]) continue;
-        const uint32_t o = a.colr[vb + i] - base;
-        if (o < span) atomicOr(&bm[o >> 5], 1u << (o & 31));
+    const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
+    for (uint32_t i = threadIdx.x; i < an.dv; i += kThreads) {
+        const uint32_t x = row[i];
+        if (ALIVE && !a.alive[x]) continue;
+        const uint32_t o = x - an.v - 1;
+        atomicOr(&bm[o >> 5], 1u << (o & 31));
     }
     __syncthreads();
 }
 
-// probe_batch for a count against the bitmap of a heavy anchor: the probe lists are read as quads of places (colr)
-// instead of ids; a place outside [base, base + span) is not an out-neighbour of v. Returns this lane's hits.
+// probe_batch for a count against the bitmap of a heavy anchor. Returns this lane's hits.
 template <bool ALIVE, class CT>
-__device__ __forceinline__ uint32_t probe_batch_bitmap(const uint32_t* __restrict__ rowptr,
-                                                       const uint32_t* __restrict__ in_src,
-                                                       const TcArgs<CT>& a,
-                                                       uint32_t kb, uint32_t kend, const uint32_t* bm, uint32_t base,
-                                                       uint32_t span, uint32_t* s_incl, uint32_t* s_rb,
-                                                       uint32_t lane) {
-    uint32_t* s_re = s_rb + 32;
-    const uint32_t k = kb + lane;
-    uint32_t nq = 0, rb = 0, re = 0;
-    if (k < kend) {
-        if (!ALIVE || a.alive[in_src[k]]) {
-            const uint2 r = a.in_rng[k];
-            rb = r.x;
-            re = r.y;
-            if (re > rb) nq = ((re + 3) >> 2) - (rb >> 2);
-        }
-    }
-    const uint32_t incl = warp_incl_scan(nq, lane);
-    const uint32_t tot = __shfl_sync(GA_FULL_MASK, incl, 31);
-    s_incl[lane] = incl;
-    s_rb[lane] = rb;
-    s_re[lane] = re;
-    __syncwarp();
-    const uint4* __restrict__ colr4 = reinterpret_cast<const uint4*>(a.colr);
-    uint32_t owner = 0, hits = 0;
+__device__ __forceinline__ uint32_t probe_batch_bitmap(const TcArgs<CT>& a, uint32_t kb, uint32_t kend,
+                                                       const uint32_t* bm, uint32_t base, uint32_t span,
+                                                       uint32_t* s_incl, uint32_t* s_base, uint32_t lane) {
+    unsigned long long rec;
+    const uint32_t tot = open_batch<ALIVE>(a.ix, a.alive, kb, kend, lane, s_incl, s_base, &rec);
+    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
+    uint32_t owner = 0, end = s_incl[0], hits = 0;
     for (uint32_t p = lane; p < tot; p += 32) {
-        while (s_incl[owner] <= p) owner++;
-        const uint32_t lo = s_rb[owner], len = s_re[owner] - lo;
-        const uint32_t q = (lo >> 2) + (p - (owner ? s_incl[owner - 1] : 0u));
-        const uint4 r4 = __ldg(colr4 + q);
-        const uint32_t off = (q << 2) - lo;   // element i of the quad is in the list iff off + i < len
-        const uint32_t rs[4] = {r4.x, r4.y, r4.z, r4.w};
+        while (end <= p) end = s_incl[++owner];
+        const size_t q = s_base[owner] + p;
+        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
+        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t o = rs[i] - base;
-            const bool look = (off + i < len) & (o < span);
-            const uint32_t w = look ? bm[o >> 5] : 0u;
+        for (int i = 0; i < 8; i++) {
+            const uint32_t o = xs[i] - base;
+            const uint32_t w = o < span ? bm[o >> 5] : 0u;
             hits += (w >> (o & 31)) & 1u;
         }
     }
@@ -385,87 +359,187 @@ __device__ __forceinline__ uint32_t probe_batch_bitmap(const uint32_t* __restric
     return hits;
 }
 
-// Adds the per-slot counters of an item to the outputs (x's vertex count or edge v->x's count).
-template <int MODE, class CT>
-__device__ __forceinline__ void flush_table(const TcArgs<CT>& a, uint32_t vb, const uint32_t* key,
-                                            const uint32_t* cnt, const uint32_t* pos, uint32_t bits, uint32_t tid,
-                                            uint32_t nthr) {
-    if (!counters(MODE)) return;
-    const uint32_t S = 4u << bits;
-    for (uint32_t s = tid; s < S; s += nthr) {
-        const uint32_t c = cnt[s];
-        if (c) {
-            if (MODE == TC_VSUP) atomicAdd(&a.vsup[key[s]], (CT)c);   // 4-slot buckets: no spill flags
-            else atomicAdd(&a.esup[vb + pos[s]], c);
+__device__ __forceinline__ void load_oct(const uint32_t* __restrict__ colr, size_t q, uint32_t (&x)[8]) {
+    const uint4* p = reinterpret_cast<const uint4*>(colr) + 2 * q;
+    const uint4 a = __ldg(p), b = __ldg(p + 1);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+
+// Common entries of octs x and y of ascending rows, calling hit(place) for each when the caller books them.
+// Padding must not match padding: y's is replaced by its first entry, which a row's every oct has.
+template <bool BOOK, class F>
+__device__ __forceinline__ uint32_t oct_common(const uint32_t (&x)[8], const uint32_t (&y)[8], F hit) {
+    uint32_t z[8], c = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) z[j] = y[j] == kPad ? y[0] : y[j];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        bool f = false;
+#pragma unroll
+        for (int j = 0; j < 8; j++) f |= x[i] == z[j];
+        c += f;
+        if (BOOK && f) hit(x[i]);
+    }
+    return c;
+}
+
+// Common places of an in-edge's suffix (octs q.. of colr, `octs` of them) and its anchor's row (octs r.. up to rend):
+// both ascend, so the oct with the smaller last entry is done after one comparison of all pairs.
+template <bool BOOK, class F>
+__device__ __forceinline__ uint32_t suffix_common(const uint32_t* __restrict__ colr, size_t q, uint32_t octs, size_t r,
+                                                  size_t rend, F hit) {
+    const size_t qend = q + octs;
+    uint32_t x[8], y[8], c = 0;
+    load_oct(colr, q, x);
+    load_oct(colr, r, y);
+    for (;;) {
+        if (x[7] >= y[0])   // else the whole oct is below the row (padding counts as above)
+            c += oct_common<BOOK>(x, y, hit);
+        if (x[7] <= y[7]) {
+            if (++q >= qend) return c;
+            load_oct(colr, q, x);
+        } else {
+            if (++r >= rend) return c;
+            load_oct(colr, r, y);
         }
     }
 }
 
-// esup[origk[e]] += esupk[e]: supports booked at colk positions moved to the caller's col order (origk is a
-// permutation within each row, so every target is written by one thread).
-__global__ void k_esup_fold(const uint32_t* __restrict__ esupk, const uint32_t* __restrict__ origk, uint32_t m,
-                            uint32_t* __restrict__ esup) {
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-        const uint32_t c = esupk[e];
-        if (c) esup[origk[e]] += c;
+// The tiny bin of a count: one warp takes 32 consecutive places, flattens the in-edges of the tiny anchors among them,
+// and every lane intersects one in-edge's suffix with its anchor's row, oct against oct in registers. An anchor of the
+// light bin costs a warp some thousand cycles of item, table and batch set-up whatever its size; Holme-Kim graphs and
+// the tails of R-MAT graphs are mostly anchors with a handful of probes. Rows are whole 32-byte sectors, so an in-edge
+// of a short row is one sector.
+template <class CT>
+__device__ __forceinline__ uint32_t tiny_group(const TcArgs<CT>& a, uint32_t p0, uint32_t pend, uint32_t light_max_deg,
+                                               uint32_t* s_incl, uint32_t* s_base, uint32_t* s_row, uint32_t* s_deg,
+                                               uint32_t lane) {
+    const uint32_t v = p0 + lane;
+    uint32_t in = 0, k0 = 0, row = 0, d = 0;
+    if (v < pend) {
+        const uint32_t w = a.ix.work[v];
+        d = a.ix.dout[v];
+        if (w && d && d <= kTinyDeg) {
+            const uint2 b = a.ix.pos[v];
+            k0 = b.x;
+            row = b.y;
+            in = a.ix.pos[v + 1].x - k0;
+            if (!is_tiny(d, in, w, light_max_deg)) in = 0;
+        }
+    }
+    const uint32_t incl = warp_incl_scan(in, lane);
+    const uint32_t tot = __shfl_sync(GA_FULL_MASK, incl, 31);
+    if (!tot) return 0;
+    s_incl[lane] = incl;
+    s_base[lane] = k0 - (incl - in);
+    s_row[lane] = row;
+    s_deg[lane] = d;
+    __syncwarp();
+    uint32_t owner = 0, end = s_incl[0], hits = 0;
+    for (uint32_t p = lane; p < tot; p += 32) {
+        while (end <= p) end = s_incl[++owner];
+        const unsigned long long r = a.ix.in_rng[s_base[owner] + p];
+        if (rng_octs(r))
+            hits += suffix_common<false>(a.ix.colr, rng_oct(r), rng_octs(r), s_row[owner],
+                                         s_row[owner] + ((s_deg[owner] + 7) >> 3), [](uint32_t) {});
+    }
+    __syncwarp();
+    return hits;
+}
+
+// Adds the per-slot counters of an item to the outputs (x's vertex count or edge v->x's count).
+template <int MODE, class CT>
+__device__ __forceinline__ void flush_table(const TcArgs<CT>& a, const Anchor& an, const uint32_t* key,
+                                            const uint32_t* cnt, const uint32_t* pos, uint32_t tid, uint32_t nthr) {
+    if (!counters(MODE)) return;
+    const uint32_t S = 4u << an.bits;
+    for (uint32_t s = tid; s < S; s += nthr) {
+        const uint32_t c = cnt[s];
+        if (c) {
+            if (MODE == TC_VSUP) atomicAdd(&a.vsup[key[s]], (CT)c);   // 4-slot buckets: no spill flags
+            else atomicAdd(&a.esupk[(size_t)an.row * 8 + pos[s]], c);
+        }
     }
 }
 
-// bounds (optional, device): this launch's item ranges [bounds[0], bounds[1]) of the heavy and [bounds[2], bounds[3])
-// of the light bin (a shard); null means every item.
+// esup[e] = esupk at the padded position of edge e's entry in its row: the place of col[e], found in the (short, sorted)
+// row. Every edge is written, so esup needs no clearing.
+__global__ void k_esup_fold(TcIndex ix, const uint32_t* __restrict__ src, const uint32_t* __restrict__ col, uint32_t m,
+                            const uint32_t* __restrict__ esupk, uint32_t* __restrict__ esup) {
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t a = ix.vrank[src[e]], x = ix.vrank[col[e]];
+        const size_t b = (size_t)ix.pos[a].y * 8;
+        const uint32_t j = lower_bound_u32(ix.colr + b, 0, ix.dout[a], x);
+        esup[e] = esupk[b + j];
+    }
+}
+
+// alive mask by id -> by place; counts by place -> by id.
+__global__ void k_alive_places(const uint8_t* __restrict__ alive, const uint32_t* __restrict__ order, uint32_t n,
+                               uint8_t* __restrict__ out) {
+    for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (uint64_t)gridDim.x * blockDim.x)
+        out[a] = alive[order[a]];
+}
+template <class CT>
+__global__ void k_counts_by_id(const CT* __restrict__ by_place, const uint32_t* __restrict__ vrank, uint32_t n,
+                               CT* __restrict__ out) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        out[v] = by_place[vrank[v]];
+}
+
+// bounds (optional, device): this launch's item ranges (a shard), [bounds[2b], bounds[2b + 1]) of the items of bin b
+// (heavy, light, tiny); null means every item. tiny_groups: counts of the whole graph take the tiny bin in groups of 32
+// places from tiny_first on; otherwise its items are run like light ones.
 template <int MODE, bool ALIVE, class CT>
-__global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(const uint32_t* __restrict__ rowptr,
-                                                      const uint32_t* __restrict__ col,
-                                                      const uint32_t* __restrict__ colk,
-                                                      const uint32_t* __restrict__ in_src,
-                                                      const uint32_t* __restrict__ in_eid,
-                                                      ga_items heavy,
-                                                      ga_items light, const uint32_t* __restrict__ bounds,
+__global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds,
                                                       uint32_t heavy_bits_max, uint32_t* __restrict__ queue,
+                                                      uint32_t tiny_first, uint32_t tiny_end, uint32_t light_max_deg,
                                                       TcArgs<CT> a) {
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t s_item, s_next;
     __shared__ unsigned long long s_red[kWarps];
     constexpr int W = SlotLayout<MODE>::words;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long hits = 0;
-    const uint32_t h0 = bounds ? bounds[0] : 0u, h1 = bounds ? bounds[1] : heavy.count;
-    const uint32_t l0 = bounds ? bounds[2] : 0u, l1 = bounds ? bounds[3] : light.count;
+    const uint32_t H = items.info[0], L = items.info[1], T = items.info[2];
+    const uint32_t h0 = bounds ? bounds[0] : 0u, h1 = bounds ? bounds[1] : H;
+    const uint32_t l0 = bounds ? bounds[2] : H, l1 = bounds ? bounds[3] : H + L;
+    const uint32_t t0 = bounds ? bounds[4] : H + L, t1 = bounds ? bounds[5] : H + L + T;
+    const bool groups = MODE == TC_COUNT && !ALIVE && tiny_first < tiny_end;
 
-    // ---- heavy bin: the block shares one hash set of N+(v) per item; its warps pull 32-in-edge batches from a
-    //      shared counter, so no warp waits for another until the item is exhausted ----
+    // ---- heavy bin: the block shares one set of N+(v) per item; its warps pull 32-in-edge batches from a shared
+    //      counter, so no warp waits for another until the item is exhausted ----
     {
         const uint32_t Smax = 4u << heavy_bits_max;
         uint32_t* key = smem;
         uint32_t* cnt = key + Smax;
         uint32_t* pos = cnt + (counters(MODE) ? Smax : 0);
         uint32_t* wbase = smem + (size_t)Smax * W + warp * kBatchWords;
-        uint32_t *s_incl = wbase, *s_rb = wbase + 32, *s_ecnt = wbase + 96;
-        s_ecnt[lane] = 0;
+        uint32_t *s_incl = wbase, *s_base = wbase + 32;
+        wbase[64 + lane] = 0;   // ecnt
         for (;;) {
             if (threadIdx.x == 0) s_item = h0 + atomicAdd(&queue[0], 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= h1) break;
-            const uint32_t v = heavy.v[item];
-            if (ALIVE && !a.alive[v]) {
+            Anchor an;
+            an.v = items.v[item];
+            if (ALIVE && !a.alive[an.v]) {
                 __syncthreads();          // everyone has read s_item before thread 0 overwrites it
                 continue;
             }
-            const uint32_t vb = rowptr[v], dv = rowptr[v + 1] - vb;
-            const uint32_t k0 = heavy.k0[item], k1 = heavy.k1[item];
-            uint32_t base = 0, span = 0;
-            if (MODE == TC_COUNT && a.vrank && dv) {
-                const uint32_t rv = a.vrank[v];
-                base = rv + 1;
-                span = a.colr[vb + dv - 1] - rv;   // the last entry of the ordered row has the largest place
-            }
-            const bool bitmap = MODE == TC_COUNT && a.vrank && dv && span <= (Smax << 5);
-            const uint32_t bits = bitmap ? 0u : table_bits(dv, heavy_bits_max);
-            const bool global = !bitmap && bits == 0;
+            an.row = a.ix.pos[an.v].y;
+            an.dv = a.ix.dout[an.v];
+            an.id = MODE == TC_LIST ? a.ix.order[an.v] : 0u;
+            const uint32_t k0 = items.k0[item], k1 = items.k1[item];
+            // the last entry of the row has the largest place
+            const uint32_t span = MODE == TC_COUNT ? a.ix.colr[(size_t)an.row * 8 + an.dv - 1] - an.v : 0u;
+            const bool bitmap = MODE == TC_COUNT && a.bitmaps && span <= (Smax << 5);
+            an.bits = bitmap ? 0u : table_bits(an.dv, heavy_bits_max);
             if (threadIdx.x == 0) s_next = k0;
-            if (bitmap) build_bitmap<ALIVE, CT>(colk, a, vb, dv, base, span, key);
-            else if (!global) build_table<MODE, ALIVE, CT>(col, a, vb, dv, key, cnt, pos, bits, threadIdx.x, kThreads, true);
+            if (bitmap) build_bitmap<ALIVE, CT>(a, an, span, key);
+            else if (an.bits) build_table<MODE, ALIVE, CT>(a, an, key, cnt, pos, threadIdx.x, kThreads, true);
             else __syncthreads();
             unsigned long long h = 0;
             for (;;) {
@@ -474,60 +548,76 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(const ui
                 kb = __shfl_sync(GA_FULL_MASK, kb, 0);
                 if (kb >= k1) break;
                 if (MODE == TC_COUNT && bitmap)
-                    h += probe_batch_bitmap<ALIVE, CT>(rowptr, in_src, a, kb, min(kb + 32, k1), key, base, span,
-                                                       s_incl, s_rb, lane);
+                    h += probe_batch_bitmap<ALIVE, CT>(a, kb, min(kb + 32, k1), key, an.v + 1, span, s_incl, s_base,
+                                                       lane);
                 else
-                    h += probe_batch<MODE, ALIVE, CT>(rowptr, col, colk, in_src, in_eid, a, kb,
-                                                      min(kb + 32, k1), key, cnt, bits, global, vb, dv, s_incl, s_rb,
-                                                      s_ecnt, lane, v);
+                    h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, cnt, an, s_incl, s_base, lane);
             }
             hits += h;
             if (MODE == TC_VSUP) {
                 const unsigned long long t = warp_sum_u64(h);
-                if (lane == 0 && t) atomicAdd(&a.vsup[v], (CT)t);
+                if (lane == 0 && t) atomicAdd(&a.vsup[an.v], (CT)t);
             }
             __syncthreads();
-            if (!global && !bitmap) flush_table<MODE, CT>(a, vb, key, cnt, pos, bits, threadIdx.x, kThreads);
+            if (an.bits) flush_table<MODE, CT>(a, an, key, cnt, pos, threadIdx.x, kThreads);
             __syncthreads();
         }
     }
-    // ---- light bin: one warp per item, private hash set of light_slots<MODE>() slots ----
-    {
-        constexpr int PW = light_warp_words<MODE>();
-        constexpr int LS = light_slots<MODE>();
-        uint32_t* key = smem + warp * PW;
-        uint32_t* cnt = key + LS;
-        uint32_t* pos = cnt + (counters(MODE) ? LS : 0);
-        uint32_t* s_incl = key + LS * W;
-        uint32_t *s_rb = s_incl + 32, *s_ecnt = s_incl + 96;
-        s_ecnt[lane] = 0;
+    // ---- light bin (and the tiny one, unless it is taken in groups): one warp per item, private hash set of
+    //      light_slots<MODE>() slots ----
+    constexpr int PW = light_warp_words<MODE>();
+    constexpr int LS = light_slots<MODE>();
+    uint32_t* key = smem + warp * PW;
+    uint32_t* cnt = key + LS;
+    uint32_t* pos = cnt + (counters(MODE) ? LS : 0);
+    uint32_t* s_incl = key + LS * W;
+    uint32_t* s_base = s_incl + 32;
+    s_incl[64 + lane] = 0;   // ecnt
+    __syncwarp();
+    const uint32_t nl = l1 - l0, total = nl + (groups ? 0u : t1 - t0);
+    for (;;) {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(&queue[1], 1u);
+        i = __shfl_sync(GA_FULL_MASK, i, 0);
+        if (i >= total) break;
+        const uint32_t item = i < nl ? l0 + i : t0 + (i - nl);
+        Anchor an;
+        an.v = items.v[item];
+        if (ALIVE && !a.alive[an.v]) continue;
+        an.row = a.ix.pos[an.v].y;
+        an.dv = a.ix.dout[an.v];
+        an.id = MODE == TC_LIST ? a.ix.order[an.v] : 0u;
+        // a table unless the anchor is too large for this mode's set (GA_OPT_LIGHT_MAX_DEG above 128 in the
+        // support modes): then binary search in the row
+        an.bits = table_bits(an.dv, light_bits<MODE>());
+        if (an.bits) build_table<MODE, ALIVE, CT>(a, an, key, cnt, pos, lane, 32, false);
+        unsigned long long h = 0;
+        const uint32_t k1 = items.k1[item];
+        for (uint32_t kb = items.k0[item]; kb < k1; kb += 32)
+            h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, cnt, an, s_incl, s_base, lane);
+        hits += h;
+        if (MODE == TC_VSUP) {
+            const unsigned long long t = warp_sum_u64(h);
+            if (lane == 0 && t) atomicAdd(&a.vsup[an.v], (CT)t);
+        }
         __syncwarp();
-        for (;;) {
-            uint32_t item = 0;
-            if (lane == 0) item = l0 + atomicAdd(&queue[1], 1u);
-            item = __shfl_sync(GA_FULL_MASK, item, 0);
-            if (item >= l1) break;
-            const uint32_t v = light.v[item];
-            if (ALIVE && !a.alive[v]) continue;
-            const uint32_t vb = rowptr[v], dv = rowptr[v + 1] - vb;
-            // a table unless the anchor is too large for this mode's set (GA_OPT_LIGHT_MAX_DEG above 128 in the
-            // support modes): then binary search in the global row
-            const uint32_t bits = table_bits(dv, light_bits<MODE>());
-            const bool global = bits == 0;
-            if (!global) build_table<MODE, ALIVE, CT>(col, a, vb, dv, key, cnt, pos, bits, lane, 32, false);
-            unsigned long long h = 0;
-            const uint32_t k1 = light.k1[item];
-            for (uint32_t kb = light.k0[item]; kb < k1; kb += 32)
-                h += probe_batch<MODE, ALIVE, CT>(rowptr, col, colk, in_src, in_eid, a, kb, min(kb + 32, k1),
-                                                  key, cnt, bits, global, vb, dv, s_incl, s_rb, s_ecnt, lane, v);
-            hits += h;
-            if (MODE == TC_VSUP) {
-                const unsigned long long t = warp_sum_u64(h);
-                if (lane == 0 && t) atomicAdd(&a.vsup[v], (CT)t);
+        if (an.bits) flush_table<MODE, CT>(a, an, key, cnt, pos, lane, 32);
+        __syncwarp();
+    }
+    // ---- tiny bin of a whole count: groups of 32 places ----
+    if constexpr (MODE == TC_COUNT && !ALIVE) {
+        if (groups) {
+            const uint32_t ngroups = (uint32_t)(((uint64_t)tiny_end - tiny_first + 31) / 32);
+            for (;;) {
+                uint32_t g0 = 0;
+                if (lane == 0) g0 = atomicAdd(&queue[2], kTinyGroups);
+                g0 = __shfl_sync(GA_FULL_MASK, g0, 0);
+                if (g0 >= ngroups) break;
+                const uint32_t g1 = min(g0 + kTinyGroups, ngroups);
+                for (uint32_t g = g0; g < g1; g++)
+                    hits += tiny_group<CT>(a, tiny_first + 32 * g, tiny_end, light_max_deg, s_incl, s_base, s_incl + 64,
+                                           s_incl + 96, lane);
             }
-            __syncwarp();
-            if (!global) flush_table<MODE, CT>(a, vb, key, cnt, pos, bits, lane, 32);
-            __syncwarp();
         }
     }
     // ---- one 64-bit atomic per block ----
@@ -539,6 +629,48 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(const ui
         for (int w = 0; w < kWarps; w++) t += s_red[w];
         if (t) atomicAdd(a.total, t);
     }
+}
+
+// The one-thread-per-edge form on the index: thread k takes in-edge k, whose record names its suffix and, one entry
+// before it, its anchor; suffix and anchor's row are intersected oct against oct in registers. For graphs of short rows
+// (Holme-Kim), where an anchor's set costs more than its probes: there an in-edge is two 32-byte sectors and some 70
+// compares, against two unaligned rows merged entry by entry, each step waiting for the last, in k_tc_plain.
+// VSUP: consecutive in-edges share their anchor, so a warp adds up its lanes' triangles by anchor before the atomic.
+template <int MODE, bool ALIVE, class CT>
+__global__ void __launch_bounds__(256) k_tc_octs(uint32_t m, TcArgs<CT> a) {
+    static_assert(MODE == TC_COUNT || MODE == TC_VSUP, "the modes this form serves");
+    const uint32_t lane = threadIdx.x & 31;
+    unsigned long long local = 0;
+    for (uint64_t k0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < m;
+         k0 += (uint64_t)gridDim.x * blockDim.x) {   // warp-uniform
+        const unsigned long long r = k0 + lane < m ? a.ix.in_rng[k0 + lane] : 0ull;
+        const uint32_t octs = rng_octs(r);
+        uint32_t c = 0, v = 0, u = 0;
+        if (octs) {
+            const size_t at = rng_at(r);
+            v = __ldg(a.ix.colr + at);
+            const uint32_t row = a.ix.pos[v].y, rend = a.ix.pos[v + 1].y;
+            if (ALIVE || MODE == TC_VSUP) u = a.ix.osrc[at >> 3];
+            if (row != rend && (!ALIVE || (a.alive[u] && a.alive[v]))) {
+                const uint32_t all = suffix_common<(ALIVE || MODE != TC_COUNT)>(
+                    a.ix.colr, rng_oct(r), octs, row, rend, [&](uint32_t x) {
+                        if (ALIVE && !a.alive[x]) return;
+                        c++;
+                        if (MODE == TC_VSUP) atomicAdd(&a.vsup[x], (CT)1);
+                    });
+                if (MODE == TC_COUNT && !ALIVE) c = all;
+            }
+        }
+        local += c;
+        if (MODE == TC_VSUP && __any_sync(GA_FULL_MASK, c != 0)) {
+            if (c) atomicAdd(&a.vsup[u], (CT)c);
+            const uint32_t peers = __match_any_sync(GA_FULL_MASK, c ? v : kPad);
+            const uint32_t sum = __reduce_add_sync(peers, c);
+            if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[v], (CT)sum);
+        }
+    }
+    local = warp_sum_u64(local);
+    if (lane == 0 && local) atomicAdd(a.total, local);
 }
 
 // Plain form (GA_OPT_TC_KERNEL = 1): one thread per oriented edge, two-pointer merge of N+(u) and N+(v), one
@@ -602,22 +734,22 @@ static uint32_t heavy_bits_for(const ga_graph* g, int mode) {
     // shared memory stays near the light bin's and 7-8 blocks stay resident per SM
     if (mode == TC_VSUP || mode == TC_ESUP) cap = std::min(cap, 9u);
     uint32_t need = 3;
-    while ((1u << need) < g->heavy.max_dv) need++;
+    const uint32_t largest = g->max_out_degree > g->light_max_deg ? g->max_out_degree : 0u;   // of the heavy bin
+    while (need < cap && (1u << need) < largest) need++;
     return std::min(need, cap);
 }
 
-// Item ranges of shard `shard` of `nshards` in both bins (heavy then light, [lo, hi) each, into out[4]). A shard is a
-// range of anchors cut by their cumulative probe work (anchor_work[v] = work of the anchors below v): anchor v goes
-// to the shard its work starts in. Per-anchor work depends only on the graph - not on the bin cutoff or item work the
-// autotuner picked for this copy, nor on the order a build left an in-list in - so copies of a graph prepared
-// independently on several GPUs cut the same anchors, and the shards partition the triangles (each is counted at its
-// middle vertex). The items of an anchor range are found by binary search (items are in ascending anchor order).
-__global__ void k_shard_bounds(const unsigned long long* __restrict__ anchor_work, uint32_t n,
-                               const uint32_t* __restrict__ hv, uint32_t hcount, const uint32_t* __restrict__ lv,
-                               uint32_t lcount, uint32_t shard, uint32_t nshards, uint32_t* __restrict__ out) {
-    const uint32_t t = threadIdx.x;   // 4 threads: heavy lo, heavy hi, light lo, light hi
-    if (t >= 4) return;
-    const uint32_t part = shard + (t & 1);
+// Item ranges of shard `shard` of `nshards` in the three bins ([lo, hi) each, into out[6], as indexes of the whole item
+// array). A shard is a range of anchors cut by their cumulative probe work (anchor_work[a] = work of the anchors below
+// place a): an anchor goes to the shard its work starts in. Per-anchor work depends only on the graph - not on the bin
+// cutoff or item work the autotuner picked for this copy, nor on the order a build left an in-list in - so copies of a
+// graph prepared independently on several GPUs cut the same anchors, and the shards partition the triangles (each is
+// counted at its middle vertex). The items of an anchor range are found by binary search (each bin ascends).
+__global__ void k_shard_bounds(const unsigned long long* __restrict__ anchor_work, uint32_t n, ga_items items,
+                               uint32_t shard, uint32_t nshards, uint32_t* __restrict__ out) {
+    const uint32_t t = threadIdx.x;   // 6 threads: lo and hi of each bin
+    if (t >= 6) return;
+    const uint32_t part = shard + (t & 1), bin = t >> 1;
     uint32_t first = n;               // first anchor of shard `part` (n for the end)
     if (part < nshards) {
         const unsigned long long W = anchor_work[n];
@@ -629,18 +761,19 @@ __global__ void k_shard_bounds(const unsigned long long* __restrict__ anchor_wor
         }
         first = part == 0 ? 0u : lo;
     }
-    const uint32_t* v = t < 2 ? hv : lv;
-    const uint32_t count = t < 2 ? hcount : lcount;
-    uint32_t lo = 0, hi = count;      // first item whose anchor is >= first
-    while (lo < hi) {
+    uint32_t lo = 0;
+    for (uint32_t b = 0; b < bin; b++) lo += items.info[b];
+    uint32_t hi = lo + items.info[bin];
+    while (lo < hi) {                 // first item of the bin whose anchor is >= first
         const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (v[mid] < first) lo = mid + 1; else hi = mid;
+        if (items.v[mid] < first) lo = mid + 1; else hi = mid;
     }
     out[t] = lo;
 }
 
 template <int MODE, bool ALIVE, class CT>
-static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a0) {
+static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
+    cudaStream_t st = g->stream;
     const uint32_t hb = heavy_bits_for(g, MODE);
     const size_t smem = hash_smem_bytes<MODE>(hb);
     auto kern = k_tc_hash<MODE, ALIVE, CT>;
@@ -648,35 +781,62 @@ static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a0) {
     int occ = 0;
     GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
     occ = std::max(occ, 1);
-    TcArgs<CT> a = a0;
-    a.origk = g->origk;
-    a.colr = g->colr;
-    a.in_rng = g->in_rng;
-    a.vrank = g->opt_count_bitmap ? nullptr : g->vrank;   // no place array: hash sets for every anchor
     const uint32_t* bounds = nullptr;
-    uint64_t want = std::max<uint64_t>(g->heavy.count, (g->light.count + kWarps - 1) / kWarps);
-    if (a.nshards > 1) {   // this shard's anchors (cut on the device; the queue counters sit in d_queue[0..1])
-        uint32_t* b = g->d_queue + 4;
-        k_shard_bounds<<<1, 32, 0, g->stream>>>(g->anchor_work, g->n, g->heavy.v, g->heavy.count, g->light.v,
-                                                g->light.count, a.shard, a.nshards, b);
+    uint64_t want = (g->items.bound + kWarps - 1) / kWarps;
+    uint32_t tiny_first = g->isolated, tiny_end = g->n;
+    if (a.nshards > 1) {   // this shard's anchors (cut on the device; the queue counters sit in d_queue[0..3])
+        uint32_t* b = g->d_queue + 8;
+        k_shard_bounds<<<1, 32, 0, st>>>(g->anchor_work, g->n, g->items, a.shard, a.nshards, b);
         GA_CUDA(cudaGetLastError());
         bounds = b;
         want = (want + a.nshards - 1) / a.nshards + 1;
+        tiny_end = tiny_first;
     }
+    want = std::max<uint64_t>(want, (uint64_t)g->max_out_degree > g->light_max_deg ? (uint64_t)g->sm_count * occ : 1);
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g->sm_count * occ, want));
-    GA_CUDA(cudaMemsetAsync(g->d_queue, 0, 4 * sizeof(uint32_t), g->stream));
-    if (MODE == TC_ESUP && g->m) {   // u->x supports by probe position (nearby addresses along a probe list)
-        GA_CUDA(pool_malloc((void**)&a.esupk, (size_t)g->m * 4, g->stream));
-        GA_CUDA(cudaMemsetAsync(a.esupk, 0, (size_t)g->m * 4, g->stream));
-    }
-    kern<<<grid, kThreads, smem, g->stream>>>(g->rowptr, g->col, g->colk, g->in_src, g->in_eid, g->heavy,
-                                              g->light, bounds, hb, g->d_queue, a);
+    GA_CUDA(cudaMemsetAsync(g->d_queue, 0, 4 * sizeof(uint32_t), st));
+    kern<<<grid, kThreads, smem, st>>>(g->items, bounds, hb, g->d_queue, tiny_first, tiny_end, g->light_max_deg, a);
     GA_CUDA(cudaGetLastError());
-    if (MODE == TC_ESUP && g->m) {
-        k_esup_fold<<<grid_for(g->m, 256), 256, 0, g->stream>>>(a.esupk, g->origk, g->m, a.esup);
-        GA_CUDA(cudaGetLastError());
-        cudaFreeAsync(a.esupk, g->stream);
+    return GA_OK;
+}
+
+// One pass on the index (octs: one thread per in-edge, else the hash kernel). The caller's arrays are by id (and by col
+// position); the kernels' by place.
+template <int MODE, bool ALIVE, class CT>
+static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
+    cudaStream_t st = g->stream;
+    TcArgs<CT> a = a0;
+    a.ix = tc_index(g);
+    a.bitmaps = !g->opt_count_bitmap;
+    void* tmp = nullptr;   // outputs (and the mask) by place
+    const size_t osize = MODE == TC_ESUP ? (size_t)g->octs * 8 * 4 : MODE == TC_VSUP ? (size_t)g->n * sizeof(CT) : 0;
+    if (osize + (ALIVE ? g->n : 0)) {
+        GA_CUDA(pool_malloc(&tmp, osize + (ALIVE ? g->n : 0), st));
+        if (osize) GA_CUDA(cudaMemsetAsync(tmp, 0, osize, st));
+        if (MODE == TC_ESUP) a.esupk = (uint32_t*)tmp;
+        if (MODE == TC_VSUP) a.vsup = (CT*)tmp;
+        if (ALIVE) {
+            uint8_t* al = (uint8_t*)tmp + osize;
+            k_alive_places<<<grid_for(g->n, 256), 256, 0, st>>>(a0.alive, g->order, g->n, al);
+            GA_CUDA(cudaGetLastError());
+            a.alive = al;
+        }
     }
+    if constexpr (MODE == TC_COUNT || MODE == TC_VSUP) {
+        if (octs) {
+            k_tc_octs<MODE, ALIVE, CT><<<grid_for(g->m, 256, (unsigned)g->sm_count * 64), 256, 0, st>>>(g->m, a);
+            GA_CUDA(cudaGetLastError());
+        }
+    }
+    ga_status s = GA_OK;
+    if (!octs) s = launch_hash<MODE, ALIVE, CT>(g, a);
+    if (s == GA_OK && MODE == TC_ESUP)
+        k_esup_fold<<<grid_for(g->m, 256), 256, 0, st>>>(a.ix, g->src, g->col, g->m, a.esupk, a0.esup);
+    if (s == GA_OK && MODE == TC_VSUP)
+        k_counts_by_id<CT><<<grid_for(g->n, 256), 256, 0, st>>>(a.vsup, g->vrank, g->n, a0.vsup);
+    if (tmp) cudaFreeAsync(tmp, st);
+    GA_TRY(s);
+    GA_CUDA(cudaGetLastError());
     return GA_OK;
 }
 
@@ -699,24 +859,33 @@ static ga_status launch_plain(ga_graph* g, const TcArgs<CT>& a) {
 
 template <int MODE, bool ALIVE, class CT>
 ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
-    GA_TRY(prepare(g));
-    cudaStream_t st = g->stream;
-    if (zero_outputs) {
-        GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
-        if (MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
-        if (MODE == TC_ESUP && g->m) GA_CUDA(cudaMemsetAsync(a.esup, 0, (size_t)g->m * sizeof(uint32_t), st));
-    }
-    // automatic choice: the autotuned kernel for counts; the hash kernel for supports and incidence lists, whose
-    // per-triangle appends and increments contend on hub vertices in the one-thread-per-edge form (lists of the
-    // Holme-Kim 1.7M graph: 154 ms plain vs 4 ms hash; first peel of the 4,096-graph batch: 3.2 s vs 1.1 s)
+    // Automatic choice: the autotuned kernel for counts. Supports take the one-thread-per-edge form too when it counts
+    // faster and rows are short (row_work / m, the octs of an edge's row on average, at most 2.5: Holme-Kim graphs have
+    // 1 to 2.1; edge supports of the 1.7M one take 400 us against 2,010 us, vertex supports of a 200,003-vertex one 380
+    // against 510), else the hash kernel: with longer rows there are more triangles an edge, whose increments contend
+    // on hub vertices (R-MAT 14, 4.3 octs: vertex supports 334 us against 139). Incidence lists always take the hash
+    // kernel (Holme-Kim 1.7M: 154 ms plain vs 4 ms hash).
     // A sharded count always uses the hash kernel unless one is forced: every GPU must cut the same partition, and
     // an autotuned choice could differ between GPUs.
+    GA_TRY(a.nshards > 1 ? prepare_shards(g) : prepare(g));
     int64_t kernel = g->opt_tc_kernel ? g->opt_tc_kernel
-                                      : (MODE == TC_COUNT && a.nshards <= 1 ? g->tuned_kernel : 2);
+                                      : (MODE == TC_COUNT || (MODE != TC_LIST && g->row_work * 2 <= 5ull * g->m)) &&
+                                                a.nshards <= 1
+                                            ? g->tuned_kernel
+                                            : 2;
     if (g->n > kTabEmpty) kernel = 1;   // ids of kTabEmpty and above do not fit the hash kernel's table slots
-    if (kernel == 1) return launch_plain<MODE, ALIVE, CT>(g, a);
-    if (g->heavy.count == 0 && g->light.count == 0) return GA_OK;
-    return launch_hash<MODE, ALIVE, CT>(g, a);
+    // the one-thread-per-edge form on the index for counts of any kind (per-edge supports are written in col's own order
+    // by the plain form, without a pass to move them: 400 us vs 590); shards cut the edges themselves
+    const bool octs = kernel == 1 && (MODE == TC_COUNT || MODE == TC_VSUP) && a.nshards <= 1 && g->n <= kTabEmpty;
+    const bool index = (kernel != 1 || octs) && g->m;
+    cudaStream_t st = g->stream;
+    if (zero_outputs) {   // on the index, supports are written whole from the kernels' own arrays
+        GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
+        if (!index && MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
+        if (!index && MODE == TC_ESUP && g->m) GA_CUDA(cudaMemsetAsync(a.esup, 0, (size_t)g->m * sizeof(uint32_t), st));
+    }
+    if (!g->m) return GA_OK;
+    return index ? launch_index<MODE, ALIVE, CT>(g, a, octs) : launch_plain<MODE, ALIVE, CT>(g, a);
 }
 
 // ---- autotuner ----------------------------------------------------------------------------------------------------
@@ -730,18 +899,6 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
 // new one is decided by timing candidates on the graph: the hash kernel and the plain kernel at the current options,
 // then the cutoffs {32, 64, 128, 256} and the item works {1024, 4096, 16384} (coordinate-wise; options the caller
 // set explicitly stay as set). Every candidate gives the same count.
-
-__global__ void k_degree_hist(const uint32_t* __restrict__ rowptr, uint32_t n, unsigned long long* hist) {
-    __shared__ unsigned long long s_h[33];
-    if (threadIdx.x < 33) s_h[threadIdx.x] = 0;
-    __syncthreads();
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t d = rowptr[v + 1] - rowptr[v];
-        if (d) atomicAdd(&s_h[32 - __clz(d)], (unsigned long long)d);
-    }
-    __syncthreads();
-    if (threadIdx.x < 33 && s_h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], s_h[threadIdx.x]);
-}
 
 struct TuneChoice {
     int kernel = 2;
@@ -777,32 +934,20 @@ static void tune_cache_store_locked(uint64_t key, const TuneChoice& c) {
     std::fclose(f);
 }
 
-// Degree-distribution signature of g (one small kernel and a sync).
-static ga_status tune_key(ga_graph* g, uint64_t* out) {
-    cudaStream_t st = g->stream;
-    const uint32_t n = g->n;
-    unsigned long long* d_hist = nullptr;
-    GA_CUDA(pool_malloc((void**)&d_hist, 33 * 8, st));
-    unsigned long long hist[33] = {};
-    cudaMemsetAsync(d_hist, 0, 33 * 8, st);
-    k_degree_hist<<<grid_for(n, 256, (unsigned)g->sm_count * 8), 256, 0, st>>>(g->rowptr, n, d_hist);
-    cudaMemcpyAsync(hist, d_hist, 33 * 8, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(d_hist, st);
-    GA_CUDA(cudaStreamSynchronize(st));
-    uint64_t key = mix64(32 - __builtin_clz(n | 1)) ^ mix64(0x100 + 32 - __builtin_clz(g->m)) ^ mix64(0x5e2);
+// Degree-distribution signature of g (from the histogram the upload checks made).
+static uint64_t tune_key(const ga_graph* g) {
+    uint64_t key = mix64(32 - __builtin_clz(g->n | 1)) ^ mix64(0x100 + 32 - __builtin_clz(g->m)) ^ mix64(0x5e2);
     for (int b = 0; b < 33; b++) {
-        const uint64_t q = (hist[b] * 16 + g->m / 2) / g->m;   // sixteenths of the edges
+        const uint64_t q = (g->row_hist[b] * 16 + g->m / 2) / g->m;   // sixteenths of the edges
         key = mix64(key ^ (q << 8) ^ (uint64_t)b);
     }
-    *out = key;
-    return GA_OK;
+    return key;
 }
 
 ga_status ready(ga_graph* g) {
     // a signature seen before sets the options before the work items are built, so they are built once
     if (g->opt_tc_kernel == 0 && !g->tuned_kernel && !g->prepared && g->m) {
-        uint64_t key = 0;
-        GA_TRY(tune_key(g, &key));
+        const uint64_t key = tune_key(g);
         std::lock_guard<std::mutex> lock(g_tune_mu);
         tune_cache_load_locked();
         auto it = g_tune_cache.find(key);
@@ -834,11 +979,9 @@ static ga_status apply_choice(ga_graph* g, const TuneChoice& c) {
 ga_status autotune(ga_graph* g) {
     if (g->tuned_kernel) return GA_OK;
     cudaStream_t st = g->stream;
-    const uint32_t n = g->n;
     if (g->m == 0) { g->tuned_kernel = 2; return GA_OK; }
-    if (n > kTabEmpty) { g->tuned_kernel = 1; return GA_OK; }   // beyond the hash kernel's ids
-    uint64_t key = 0;
-    GA_TRY(tune_key(g, &key));
+    if (g->n > kTabEmpty) { g->tuned_kernel = 1; return GA_OK; }   // beyond the hash kernel's ids
+    const uint64_t key = tune_key(g);
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         tune_cache_load_locked();
@@ -1085,8 +1228,14 @@ ga_status ga_graph_tuning(ga_graph* g, ga_tuning* out) {
     out->item_work = g->item_work;
     out->signature = g->tune_key;
     out->measured_ms = g->opt_tc_kernel ? 0.0 : (double)g->tune_ms;
-    out->heavy_items = g->heavy.count;
-    out->light_items = g->light.count;
+    out->heavy_items = out->light_items = 0;
+    if (g->items.info && g->prepared) {
+        uint32_t info[3];
+        GA_CUDA(cudaMemcpyAsync(info, g->items.info, sizeof info, cudaMemcpyDeviceToHost, g->stream));
+        GA_CUDA(cudaStreamSynchronize(g->stream));
+        out->heavy_items = info[0];
+        out->light_items = (uint64_t)info[1] + info[2];
+    }
     return GA_OK;
 }
 

@@ -8,6 +8,18 @@ namespace ga {
 // incidence lists of its three corners (the other two corners of each triangle through v, in inc[inc_ptr[v] ..]).
 enum TcMode { TC_COUNT = 0, TC_VSUP = 1, TC_ESUP = 2, TC_LIST = 3 };
 
+// The index the hash kernel reads (ga_graph.cu; everything by place).
+struct TcIndex {
+    const uint32_t *vrank, *order, *dout, *work;
+    const uint2* pos;
+    const uint32_t *colr, *osrc;
+    const unsigned long long* in_rng;
+};
+
+inline TcIndex tc_index(const ga_graph* g) {
+    return TcIndex{g->vrank, g->order, g->dout, g->work, g->pos, g->colr, g->osrc, g->in_rng};
+}
+
 // Outputs of one triangle pass. `total` (device) receives T; `vsup` (n counters of type CT) the per-vertex counts;
 // `esup` (m) the per-edge counts; `alive` (n bytes, optional) restricts the pass to the induced subgraph;
 // `inc`/`inc_ptr`/`fill` the incidence lists of TC_LIST (fill: n zeroed cursors).
@@ -21,12 +33,11 @@ struct TcArgs {
     const unsigned long long* inc_ptr = nullptr;
     uint32_t* fill = nullptr;
     uint32_t* overflow = nullptr;   // TC_LIST: entries that found their list full (must stay 0)
-    const uint32_t* origk = nullptr;  // set by the launcher: position in col of each (degree, id)-ordered entry
-    const uint32_t* colr = nullptr;   // set by the launcher: the (degree, id)-ordered rows as vertex places
-    const uint32_t* vrank = nullptr;  // set by the launcher: every vertex's place in the (degree, id) order
-    const uint2* in_rng = nullptr;    // set by the launcher: in-edge k's probe list [start, end) in colk / colr
-    uint32_t* esupk = nullptr;        // set by the launcher (ESUP, hash kernel): supports by colk position, m zeroed
-    // shard `shard` of `nshards` (0 = the whole graph): equal parts of the work items (hash kernel) or of the edges
+    // set by the launcher of the hash kernel (whose vsup and alive are by place)
+    TcIndex ix = {};
+    uint32_t* esupk = nullptr;      // ESUP: supports by padded position in colr, zeroed
+    bool bitmaps = false;           // COUNT: heavy anchors may use bitmaps
+    // shard `shard` of `nshards` (0 = the whole graph): equal parts of the probe work (hash kernel) or of the edges
     // (plain kernel); the shards of a graph partition its triangles
     uint32_t shard = 0, nshards = 0;
 };
