@@ -134,8 +134,10 @@ enum : int { SC_HIST = 8, SC_ISOLATED = 55, SC_ORIENT = 56, SC_MAXDEG = 57, SC_W
 __global__ void __launch_bounds__(256) k_rows(const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
                                               uint32_t n, uint32_t m, uint32_t* __restrict__ src,
                                               uint32_t* __restrict__ indeg, unsigned long long* __restrict__ sc) {
-    __shared__ unsigned long long s_hist[33];
+    // the block's sums: histogram, then SC_WORK .. SC_ERR (one atomic each per block: a per-warp one serialises)
+    __shared__ unsigned long long s_hist[33], s_sum[4];
     if (threadIdx.x < 33) s_hist[threadIdx.x] = 0;
+    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -194,18 +196,27 @@ __global__ void __launch_bounds__(256) k_rows(const uint32_t* __restrict__ rowpt
     octs = warp_sum_u64(octs);
     work = warp_sum_u64(work);
     if (lane == 0) {
-        if (bad) atomicOr(&sc[SC_ERR], (unsigned long long)bad);
-        if (maxout) atomicMax(&sc[SC_MAXOUT], (unsigned long long)maxout);
-        if (octs) atomicAdd(&sc[SC_OCTS], octs);
-        if (work) atomicAdd(&sc[SC_WORK], work);
+        if (bad) atomicOr(&s_sum[SC_ERR - SC_WORK], (unsigned long long)bad);
+        if (maxout) atomicMax(&s_sum[SC_MAXOUT - SC_WORK], (unsigned long long)maxout);
+        if (octs) atomicAdd(&s_sum[SC_OCTS - SC_WORK], octs);
+        if (work) atomicAdd(&s_sum[0], work);
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_sum[SC_ERR - SC_WORK]) atomicOr(&sc[SC_ERR], s_sum[SC_ERR - SC_WORK]);
+        atomicMax(&sc[SC_MAXOUT], s_sum[SC_MAXOUT - SC_WORK]);
+        atomicAdd(&sc[SC_OCTS], s_sum[SC_OCTS - SC_WORK]);
+        atomicAdd(&sc[SC_WORK], s_sum[0]);
+    }
     if (threadIdx.x < 33 && s_hist[threadIdx.x]) atomicAdd(&sc[SC_HIST + threadIdx.x], s_hist[threadIdx.x]);
 }
 
 // deg[v] += out-degree (deg holds the in-degrees): total degrees, their maximum and the number of isolated vertices.
 __global__ void __launch_bounds__(256) k_degrees(const uint32_t* __restrict__ rowptr, uint32_t n,
                                                  uint32_t* __restrict__ deg, unsigned long long* __restrict__ sc) {
+    __shared__ uint32_t s_mx, s_isolated;
+    if (threadIdx.x == 0) s_mx = s_isolated = 0;
+    __syncthreads();
     uint32_t mx = 0, isolated = 0;
     for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t d = deg[v] + rowptr[v + 1] - rowptr[v];
@@ -216,8 +227,13 @@ __global__ void __launch_bounds__(256) k_degrees(const uint32_t* __restrict__ ro
     mx = __reduce_max_sync(GA_FULL_MASK, mx);
     isolated = __reduce_add_sync(GA_FULL_MASK, isolated);
     if ((threadIdx.x & 31) == 0) {
-        if (mx) atomicMax(&sc[SC_MAXDEG], (unsigned long long)mx);
-        if (isolated) atomicAdd(&sc[SC_ISOLATED], (unsigned long long)isolated);
+        if (mx) atomicMax(&s_mx, mx);
+        if (isolated) atomicAdd(&s_isolated, isolated);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_mx) atomicMax(&sc[SC_MAXDEG], (unsigned long long)s_mx);
+        if (s_isolated) atomicAdd(&sc[SC_ISOLATED], (unsigned long long)s_isolated);
     }
 }
 
@@ -238,11 +254,13 @@ __global__ void __launch_bounds__(256) k_orient(const uint32_t* __restrict__ src
 
 // ---- rows in places ----------------------------------------------------------------------------------------------
 // Every row's entries become places (one gather of vrank), are sorted (places alone: the sort carries nothing else) and
-// written as whole octs; in the same pass the edge's entry of its anchor's in-list is filled in. A row is sorted by a
-// bitonic network over E keys per lane, element l * E + i in register i of lane l: strides below E stay inside a
-// thread (min / max), larger ones are one shuffle. (64-bit (degree, id) keys counted against each other in shared
-// memory with the entries' positions carried along, then a scatter and a gather of their own, took 4.0 ms of R-MAT 22's
-// 5.4 ms of build kernels.)
+// written as whole octs. A row is sorted by a bitonic network over E keys per lane, element l * E + i in register i of
+// lane l: strides below E stay inside a thread (min / max), larger ones are one shuffle. k_in_lists then reads the
+// octs once, in order, and writes every entry's in-list record; it is a kernel of its own because it only waits (an
+// atomic with a result and a scattered write per entry) and wants all the warps an SM holds, which the sort's registers
+// do not leave (both in one kernel: 2.64 ms for R-MAT 22's rows of more than 8 entries). (64-bit (degree, id) keys
+// counted against each other in shared memory with the entries' positions carried along, then a scatter and a gather of
+// their own, took 4.0 ms of R-MAT 22's 5.4 ms of build kernels.)
 template <int E, int LANES>
 __device__ __forceinline__ void sort_keys(uint32_t (&k)[E], uint32_t l) {
 #pragma unroll
@@ -273,17 +291,6 @@ __device__ __forceinline__ void sort_keys(uint32_t (&k)[E], uint32_t l) {
     }
 }
 
-// Entry j (place x) of place a's row of d entries, starting at oct o0: its record in x's in-list and x's probe work.
-__device__ __forceinline__ void emit_in_edge(uint32_t x, uint32_t j, uint32_t d, uint32_t o0,
-                                             const uint2* __restrict__ pos, uint32_t* __restrict__ fill,
-                                             uint32_t* __restrict__ work, unsigned long long* __restrict__ in_rng) {
-    const unsigned long long at = (unsigned long long)o0 * 8 + j;   // padded position of the entry
-    const uint32_t octs = j + 1 < d ? ((d + 7) >> 3) - ((j + 1) >> 3) : 0u;
-    const uint32_t k = pos[x].x + atomicAdd(&fill[x], 1u);
-    in_rng[k] = pack_rng(at, octs);
-    if (octs) atomicAdd(&work[x], octs);
-}
-
 // Rows of at most 8 entries, four rows per warp, one per 8-lane group. Longer rows are appended to `listed`.
 __global__ void __launch_bounds__(256) k_place_rows_small(const uint32_t* __restrict__ rowptr,
                                                           const uint32_t* __restrict__ col,
@@ -291,8 +298,6 @@ __global__ void __launch_bounds__(256) k_place_rows_small(const uint32_t* __rest
                                                           const uint32_t* __restrict__ order,
                                                           const uint2* __restrict__ pos, uint32_t first, uint32_t n,
                                                           uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
-                                                          uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
-                                                          unsigned long long* __restrict__ in_rng,
                                                           uint32_t* __restrict__ listed,
                                                           uint32_t* __restrict__ nlisted) {
     const uint32_t lane = threadIdx.x & 31, sub = lane & 7;
@@ -315,7 +320,6 @@ __global__ void __launch_bounds__(256) k_place_rows_small(const uint32_t* __rest
             const uint32_t o0 = pos[a].y;
             colr[(size_t)o0 * 8 + sub] = k[0];
             if (sub == 0) osrc[o0] = a;
-            if (sub < d) emit_in_edge(k[0], sub, d, o0, pos, fill, work, in_rng);
         }
         const bool longer = valid && d > 8 && sub == 0;
         const uint32_t bal = __ballot_sync(GA_FULL_MASK, longer);
@@ -331,9 +335,7 @@ __global__ void __launch_bounds__(256) k_place_rows_small(const uint32_t* __rest
 template <int E>
 __device__ __forceinline__ void place_row(const uint32_t* __restrict__ row, uint32_t d, uint32_t a, uint32_t lane,
                                           const uint32_t* __restrict__ vrank, const uint2* __restrict__ pos,
-                                          uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
-                                          uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
-                                          unsigned long long* __restrict__ in_rng) {
+                                          uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc) {
     uint32_t k[E];
 #pragma unroll
     for (int i = 0; i < E; i++) k[i] = lane + 32 * i < d ? vrank[row[lane + 32 * i]] : kPad;   // any start order
@@ -347,7 +349,6 @@ __device__ __forceinline__ void place_row(const uint32_t* __restrict__ row, uint
             *reinterpret_cast<uint4*>(colr + (size_t)o0 * 8 + j) =
                 make_uint4(k[i], k[E >= 4 ? i + 1 : 0], k[E >= 4 ? i + 2 : 0], k[E >= 4 ? i + 3 : 0]);
         if (j < end && (j & 7) == 0) osrc[o0 + (j >> 3)] = a;
-        if (j < d) emit_in_edge(k[i], j, d, o0, pos, fill, work, in_rng);
     }
 }
 
@@ -359,8 +360,6 @@ __global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __res
                                                            const uint32_t* __restrict__ order,
                                                            const uint2* __restrict__ pos,
                                                            uint32_t* __restrict__ colr, uint32_t* __restrict__ osrc,
-                                                           uint32_t* __restrict__ fill, uint32_t* __restrict__ work,
-                                                           unsigned long long* __restrict__ in_rng,
                                                            const uint32_t* __restrict__ listed,
                                                            const uint32_t* __restrict__ nlisted) {
     const uint32_t lane = threadIdx.x & 31;
@@ -370,11 +369,11 @@ __global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __res
         const uint32_t a = listed[count - 1 - r], u = order[a];
         const uint32_t b = rowptr[u], d = rowptr[u + 1] - b;
         const uint32_t* row = col + b;
-        if (d <= 32) place_row<1>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
-        else if (d <= 64) place_row<2>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
-        else if (d <= 128) place_row<4>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
-        else if (d <= 256) place_row<8>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
-        else if (d <= 512) place_row<16>(row, d, a, lane, vrank, pos, colr, osrc, fill, work, in_rng);
+        if (d <= 32) place_row<1>(row, d, a, lane, vrank, pos, colr, osrc);
+        else if (d <= 64) place_row<2>(row, d, a, lane, vrank, pos, colr, osrc);
+        else if (d <= 128) place_row<4>(row, d, a, lane, vrank, pos, colr, osrc);
+        else if (d <= 256) place_row<8>(row, d, a, lane, vrank, pos, colr, osrc);
+        else if (d <= 512) place_row<16>(row, d, a, lane, vrank, pos, colr, osrc);
         else {
             const uint32_t o0 = pos[a].y, end = (d + 7) & ~7u;
             for (uint32_t i0 = lane; i0 < d; i0 += 256) {   // eight entries per lane per pass over the row
@@ -393,7 +392,6 @@ __global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __res
                 for (int q = 0; q < 8; q++) {
                     if (i0 + 32 * q >= d) continue;
                     colr[(size_t)o0 * 8 + rk[q]] = kq[q];
-                    emit_in_edge(kq[q], rk[q], d, o0, pos, fill, work, in_rng);
                 }
             }
             for (uint32_t j = d + lane; j < end; j += 32) colr[(size_t)o0 * 8 + j] = kPad;
@@ -402,18 +400,44 @@ __global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __res
     }
 }
 
+// One lane per entry of colr: the entry x of place a's row is the in-edge a->x, whose record goes to the next free place
+// of x's in-list. cur[x] holds that place in its low word and the octs x's in-edges have to probe in its high word, so
+// one 64-bit atomic serves both (neither reaches 2^32: an in-edge with a suffix of s octs needs a row of 8(s-1) others).
+__global__ void __launch_bounds__(256) k_in_lists(const uint32_t* __restrict__ colr, const uint32_t* __restrict__ osrc,
+                                                  const uint2* __restrict__ pos, uint64_t entries,
+                                                  unsigned long long* __restrict__ cur,
+                                                  unsigned long long* __restrict__ in_rng) {
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < entries;
+         e += (uint64_t)gridDim.x * blockDim.x) {   // entries is a multiple of 8: an oct's lanes are here together
+        const uint32_t x = colr[e];
+        if (x == kPad) continue;
+        uint32_t octs = pos[osrc[e >> 3] + 1].y - (uint32_t)((e + 1) >> 3);
+        if (((e + 1) & 7) && colr[e + 1] == kPad) octs = 0;   // the row's last entry: nothing to probe after it
+        const unsigned long long at = atomicAdd(&cur[x], (unsigned long long)octs << 32 | 1u);
+        in_rng[(uint32_t)at] = pack_rng(e, octs);
+    }
+}
+
+// cur[a] = start of a's in-list.
+__global__ void k_in_cursors(const uint2* __restrict__ pos, uint32_t n, unsigned long long* __restrict__ cur) {
+    for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (uint64_t)gridDim.x * blockDim.x)
+        cur[a] = pos[a].x;
+}
+
 // ---- vertex places in the (degree, id) order ---------------------------------------------------------------------
 // A stable LSD radix sort of the vertices by degree (out + in), 9 bits per pass, starting from id order, so that
 // equal degrees stay in id order: the result is the (degree, id) order of graph.h:43-45. Each warp owns a chunk of
-// kRankChunk consecutive entries: k_rank_count counts the chunk's digits, an exclusive scan over (digit, chunk) gives
+// `chunk` consecutive entries: k_rank_count counts the chunk's digits, an exclusive scan over (digit, chunk) gives
 // every chunk its start in each digit's range, and k_rank_scatter writes the chunk's entries in order (lanes with the
 // same digit ranked by __match_any_sync, a per-digit running count per warp in shared memory).
-constexpr uint32_t kRankBits = 9, kRankDigits = 1u << kRankBits, kRankChunk = 512, kRankWarps = 8;
+constexpr uint32_t kRankBits = 9, kRankDigits = 1u << kRankBits, kRankWarps = 8;
+// entries per chunk: a warp walks its chunk serially (16 dependent steps), so small inputs take shorter ones
+static uint32_t rank_chunk(uint32_t n) { return n <= 1u << 16 ? 128 : 512; }
 
 // counts[d * nchunks + c] = entries of chunk c whose digit is d (cur == nullptr: the identity order).
 __global__ void __launch_bounds__(kRankWarps * 32) k_rank_count(const uint32_t* __restrict__ cur,
                                                                 const uint32_t* __restrict__ deg, uint32_t n,
-                                                                uint32_t shift, uint32_t nchunks,
+                                                                uint32_t shift, uint32_t nchunks, uint32_t chunk,
                                                                 uint32_t* __restrict__ counts) {
     __shared__ uint32_t s_h[kRankWarps][kRankDigits];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -422,7 +446,7 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rank_count(const uint32_t* 
     uint32_t* h = s_h[w];
     for (uint32_t d = lane; d < kRankDigits; d += 32) h[d] = 0;
     __syncwarp();
-    const uint32_t b = c * kRankChunk, e = min(n, b + kRankChunk);
+    const uint32_t b = c * chunk, e = (uint32_t)min((uint64_t)n, (uint64_t)b + chunk);
     for (uint32_t i = b + lane; i < e; i += 32) {
         const uint32_t x = cur ? cur[i] : i;
         atomicAdd(&h[(deg[x] >> shift) & (kRankDigits - 1)], 1u);
@@ -434,7 +458,7 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rank_count(const uint32_t* 
 // Writes the chunk's entries to next[] at their digit's place (offs = exclusive scan of counts), in chunk order.
 __global__ void __launch_bounds__(kRankWarps * 32) k_rank_scatter(const uint32_t* __restrict__ cur,
                                                                   const uint32_t* __restrict__ deg, uint32_t n,
-                                                                  uint32_t shift, uint32_t nchunks,
+                                                                  uint32_t shift, uint32_t nchunks, uint32_t chunk,
                                                                   const uint32_t* __restrict__ offs,
                                                                   uint32_t* __restrict__ next) {
     __shared__ uint32_t s_run[kRankWarps][kRankDigits];
@@ -444,7 +468,7 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rank_scatter(const uint32_t
     uint32_t* run = s_run[w];
     for (uint32_t d = lane; d < kRankDigits; d += 32) run[d] = 0;
     __syncwarp();
-    const uint32_t b = c * kRankChunk, e = min(n, b + kRankChunk);
+    const uint32_t b = c * chunk, e = (uint32_t)min((uint64_t)n, (uint64_t)b + chunk);
     for (uint32_t i0 = b; i0 < e; i0 += 32) {
         const uint32_t i = i0 + lane;
         const bool valid = i < e;
@@ -475,6 +499,12 @@ __global__ void k_places(const uint32_t* __restrict__ rowptr, const uint32_t* __
         dout[a] = d;
         pos[a] = (unsigned long long)((d + 7) >> 3) << 32 | (deg[u] - d);
     }
+}
+
+// work[a] = octs to probe for anchor a, from the cursors.
+__global__ void k_work(const unsigned long long* __restrict__ cur, uint32_t n, uint32_t* __restrict__ work) {
+    for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (uint64_t)gridDim.x * blockDim.x)
+        work[a] = (uint32_t)(cur[a] >> 32);
 }
 
 __global__ void k_widen(const uint32_t* __restrict__ in, uint32_t n, unsigned long long* __restrict__ out) {
@@ -631,7 +661,8 @@ static ga_status prepare_index(ga_graph* g) {
     if (n) {
         // the vertices in (degree, id) order
         const unsigned gv = grid_for((uint64_t)n + 1, 256);
-        const uint32_t nchunks = (uint32_t)(((uint64_t)n + kRankChunk - 1) / kRankChunk);
+        const uint32_t chunk = rank_chunk(n);
+        const uint32_t nchunks = (uint32_t)(((uint64_t)n + chunk - 1) / chunk);
         const uint64_t ncounts = (uint64_t)kRankDigits * nchunks;
         uint32_t passes = 1;
         while (passes * kRankBits < 32 && (g->max_degree >> (passes * kRankBits)) != 0) passes++;
@@ -642,10 +673,10 @@ static ga_status prepare_index(ga_graph* g) {
         const uint32_t* cur = nullptr;   // the identity (id order) before the first pass
         for (uint32_t ps = 0; ps < passes; ps++) {
             uint32_t* next = ((passes - ps) & 1) ? g->order : other;   // the last pass ends in order
-            k_rank_count<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, counts);
+            k_rank_count<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, chunk, counts);
             GA_CUDA(cudaGetLastError());
             GA_TRY(scan_impl<uint32_t>(st, counts, counts, ncounts));
-            k_rank_scatter<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, counts, next);
+            k_rank_scatter<<<gr, kRankWarps * 32, 0, st>>>(cur, g->deg, n, ps * kRankBits, nchunks, chunk, counts, next);
             GA_CUDA(cudaGetLastError());
             cur = next;
         }
@@ -653,24 +684,30 @@ static ga_status prepare_index(ga_graph* g) {
         GA_CUDA(cudaGetLastError());
         GA_TRY(scan_impl<unsigned long long>(st, (unsigned long long*)g->pos, (unsigned long long*)g->pos,
                                              (uint64_t)n + 1));
-        GA_CUDA(cudaMemsetAsync(g->work, 0, (size_t)n * 4, st));
         if (m) {
-            uint32_t *fill = nullptr, *listed = nullptr;   // cursors; rows longer than 8, then their count
-            GA_CUDA(pool_malloc((void**)&fill, (size_t)n * 4, st));
+            unsigned long long* cur = nullptr;
+            uint32_t* listed = nullptr;   // rows longer than 8, then their count
+            GA_CUDA(pool_malloc((void**)&cur, (size_t)n * 8, st));
             GA_CUDA(pool_malloc((void**)&listed, ((size_t)n + 1) * 4, st));
-            GA_CUDA(cudaMemsetAsync(fill, 0, (size_t)n * 4, st));
             GA_CUDA(cudaMemsetAsync(listed + n, 0, 4, st));
+            k_in_cursors<<<gv, 256, 0, st>>>(g->pos, n, cur);
+            GA_CUDA(cudaGetLastError());
             k_place_rows_small<<<grid_for((uint64_t)(n - g->isolated) * 8, 256), 256, 0, st>>>(
-                g->rowptr, g->col, g->vrank, g->order, g->pos, g->isolated, n, g->colr, g->osrc, fill, g->work,
-                g->in_rng, listed, listed + n);
+                g->rowptr, g->col, g->vrank, g->order, g->pos, g->isolated, n, g->colr, g->osrc, listed, listed + n);
             GA_CUDA(cudaGetLastError());
             if (g->max_out_degree > 8)
                 k_place_rows_listed<<<(unsigned)g->sm_count * 8, 128, 0, st>>>(
-                    g->rowptr, g->col, g->vrank, g->order, g->pos, g->colr, g->osrc, fill, g->work, g->in_rng, listed,
-                    listed + n);
+                    g->rowptr, g->col, g->vrank, g->order, g->pos, g->colr, g->osrc, listed, listed + n);
             GA_CUDA(cudaGetLastError());
-            cudaFreeAsync(fill, st);
+            k_in_lists<<<grid_for(g->octs * 8, 256, (unsigned)g->sm_count * 64), 256, 0, st>>>(
+                g->colr, g->osrc, g->pos, g->octs * 8, cur, g->in_rng);
+            GA_CUDA(cudaGetLastError());
+            k_work<<<gv, 256, 0, st>>>(cur, n, g->work);
+            GA_CUDA(cudaGetLastError());
+            cudaFreeAsync(cur, st);
             cudaFreeAsync(listed, st);
+        } else {
+            GA_CUDA(cudaMemsetAsync(g->work, 0, (size_t)n * 4, st));
         }
         cudaFreeAsync(other, st);
         cudaFreeAsync(counts, st);
@@ -782,8 +819,9 @@ static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint
     cudaMemsetAsync(g->d_scalars, 0, 64 * 8, g->stream);
     if (n) {
         cudaMemsetAsync(g->deg, 0, (size_t)n * 4, g->stream);
-        k_rows<<<grid_for(n, 256), 256, 0, g->stream>>>(g->rowptr, g->col, n, m, g->src, g->deg, g->d_scalars);
-        k_degrees<<<grid_for(n, 256), 256, 0, g->stream>>>(g->rowptr, n, g->deg, g->d_scalars);
+        const unsigned few = (unsigned)g->sm_count * 8;   // one wave: the kernels end in per-block sums
+        k_rows<<<grid_for(n, 256, few), 256, 0, g->stream>>>(g->rowptr, g->col, n, m, g->src, g->deg, g->d_scalars);
+        k_degrees<<<grid_for(n, 256, few), 256, 0, g->stream>>>(g->rowptr, n, g->deg, g->d_scalars);
         if (m) k_orient<<<grid_for(m, 256), 256, 0, g->stream>>>(g->src, g->col, g->deg, n, m, g->d_scalars);
     }
     uint32_t ends[2] = {0, 0};

@@ -631,6 +631,19 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
     }
 }
 
+// One atomic per block of 256 threads (all of them call it).
+__device__ __forceinline__ void add_total(unsigned long long local, unsigned long long* total) {
+    __shared__ unsigned long long s_red[8];
+    local = warp_sum_u64(local);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long t = 0;
+        for (int w = 0; w < 8; w++) t += s_red[w];
+        if (t) atomicAdd(total, t);
+    }
+}
+
 // The one-thread-per-edge form on the index: thread k takes in-edge k, whose record names its suffix and, one entry
 // before it, its anchor; suffix and anchor's row are intersected oct against oct in registers. For graphs of short rows
 // (Holme-Kim), where an anchor's set costs more than its probes: there an in-edge is two 32-byte sectors and some 70
@@ -669,8 +682,7 @@ __global__ void __launch_bounds__(256) k_tc_octs(uint32_t m, TcArgs<CT> a) {
             if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[v], (CT)sum);
         }
     }
-    local = warp_sum_u64(local);
-    if (lane == 0 && local) atomicAdd(a.total, local);
+    add_total(local, a.total);
 }
 
 // Plain form (GA_OPT_TC_KERNEL = 1): one thread per oriented edge, two-pointer merge of N+(u) and N+(v), one
@@ -710,8 +722,7 @@ __global__ void __launch_bounds__(256) k_tc_plain(const uint32_t* __restrict__ r
             }
         }
     }
-    local = warp_sum_u64(local);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(a.total, local);
+    add_total(local, a.total);
 }
 
 // ---- host launchers ---------------------------------------------------------------------------------------------
@@ -824,7 +835,7 @@ static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
     }
     if constexpr (MODE == TC_COUNT || MODE == TC_VSUP) {
         if (octs) {
-            k_tc_octs<MODE, ALIVE, CT><<<grid_for(g->m, 256, (unsigned)g->sm_count * 64), 256, 0, st>>>(g->m, a);
+            k_tc_octs<MODE, ALIVE, CT><<<grid_for(g->m, 256, (unsigned)g->sm_count * 16), 256, 0, st>>>(g->m, a);
             GA_CUDA(cudaGetLastError());
         }
     }
