@@ -50,8 +50,8 @@
 namespace ga {
 
 #ifndef GA_TC_MIN_BLOCKS
-#define GA_TC_MIN_BLOCKS 8                // resident blocks per SM the hash kernel is compiled for (R-MAT 22 count:
-                                          // 2.23 ms; 6: 2.24, 5: 2.36, 4: 2.62)
+#define GA_TC_MIN_BLOCKS 6                // resident blocks per SM the hash kernel is compiled for (8, 7, 6: R-MAT 22
+                                          // count 2.28, 2.28, 2.28 ms, R-MAT 16 edge supports 174, 136, 130 us; 5: 2.36 ms)
 #endif
 
 constexpr int kWarps = 8;                 // warps per block of the hash kernel
@@ -98,7 +98,7 @@ constexpr uint32_t kTabEmpty = 0x7FFFFFFFu, kTabSpill = 0x80000000u;
 
 template <int MODE>
 constexpr bool spill_flags() { return bucket_slots<MODE>() == 2; }
-static_assert(!spill_flags<TC_VSUP>() && !spill_flags<TC_ESUP>(), "flush_table reads the support modes' keys as ids");
+static_assert(!spill_flags<TC_VSUP>() && !spill_flags<TC_ESUP>(), "flush_counts reads the support modes' keys as ids");
 
 // Slots of bucket b that hold x (bit i = slot i); *open when the search for x ends at this bucket.
 template <int MODE>
@@ -117,10 +117,14 @@ __device__ __forceinline__ uint32_t bucket_match(const uint32_t* key, uint32_t b
 // Writes the triangle (u lowest, v middle, x highest; ids) into the incidence list of each corner. A list is sized by
 // the counting pass; an entry that would land past its list's end is dropped and counted in *overflow instead.
 template <class CT>
-__device__ __forceinline__ void list_one(const TcArgs<CT>& a, uint32_t c, uint32_t p, uint32_t q) {
-    const unsigned long long pos = a.inc_ptr[c] + atomicAdd(&a.fill[c], 1u);
+__device__ __forceinline__ void list_at(const TcArgs<CT>& a, uint32_t c, uint32_t at, uint32_t p, uint32_t q) {
+    const unsigned long long pos = a.inc_ptr[c] + at;
     if (pos < a.inc_ptr[c + 1]) a.inc[pos] = make_uint2(p, q);
     else atomicAdd(a.overflow, 1u);
+}
+template <class CT>
+__device__ __forceinline__ void list_one(const TcArgs<CT>& a, uint32_t c, uint32_t p, uint32_t q) {
+    list_at(a, c, atomicAdd(&a.fill[c], 1u), p, q);
 }
 template <class CT>
 __device__ __forceinline__ void list_triangle(const TcArgs<CT>& a, uint32_t u, uint32_t v, uint32_t x) {
@@ -129,27 +133,27 @@ __device__ __forceinline__ void list_triangle(const TcArgs<CT>& a, uint32_t u, u
     list_one(a, v, u, x);
 }
 
-// An anchor as the probe loops see it: its row (octs of colr), its members in a table (bits > 0) or only in the row.
+// An anchor and the set of its members as the probe loops see them: a bitmap (counts and, with ranks, supports), a hash
+// table (bits > 0), or nothing but its row (bits 0: binary search).
 struct Anchor {
-    uint32_t v, id, row, dv;   // place, id (LIST), first oct of the row, out-degree
-    uint32_t bits;             // table size; 0: binary search in the row
+    uint32_t v, id, row, dv;   // place, id (LIST, VSUP), first oct of the row, out-degree
+    uint32_t bits;             // table size
+    uint32_t span;             // bitmap: places above v it covers (0: no bitmap)
 };
 
-template <int MODE, class CT>
-__device__ __forceinline__ void on_hit(const TcArgs<CT>& a, uint32_t* s_ecnt, uint32_t owner, size_t e,
-                                       const Anchor& an, uint32_t x, const uint32_t* s_u) {
-    if (counters(MODE)) atomicAdd(&s_ecnt[owner], 1u);
-    if (MODE == TC_ESUP) atomicAdd(&a.esupk[e], 1u);   // u->x at its place in u's row; moved to col order after the pass
-    if (MODE == TC_LIST) list_triangle(a, s_u[owner], an.id, a.ix.order[x]);
-}
-
-// Looks place x (entry e of colr, probe list of in-edge `owner`) up in the hash set or, without one, by binary search
-// in the row of the anchor. Returns 1 on a hit and books the supports of the found triangle. The padding of a row is
-// above every place, so it is never found.
+// Finds place x among the members of anchor `an`: its counter's index - rank in the row (bitmap, row) or table slot -
+// or GA_EMPTY. A row's padding is above every place, so it is never found. key: table or bitmap; pre: the bitmap's
+// ranks (members below every word).
 template <int MODE, bool ALIVE, class CT>
-__device__ __forceinline__ uint32_t probe_one(const TcArgs<CT>& a, uint32_t x, size_t e, uint32_t owner,
-                                              const uint32_t* key, uint32_t* cnt, const Anchor& an,
-                                              uint32_t* s_ecnt, const uint32_t* s_u) {
+__device__ __forceinline__ uint32_t find_member(const TcArgs<CT>& a, const Anchor& an, uint32_t x,
+                                                const uint32_t* key, const uint16_t* pre) {
+    if (an.span) {
+        const uint32_t o = x - an.v - 1;
+        if (o >= an.span) return GA_EMPTY;
+        const uint32_t w = key[o >> 5], bit = 1u << (o & 31);
+        if (!(w & bit)) return GA_EMPTY;
+        return counters(MODE) ? pre[o >> 5] + __popc(w & (bit - 1)) : 0u;
+    }
     if (an.bits) {
         // bucketed set (bucket_slots<MODE>() slots per bucket); a bucket fills its slots in order, so an empty last
         // slot ends the search. One shared load resolves almost every lookup.
@@ -158,24 +162,14 @@ __device__ __forceinline__ uint32_t probe_one(const TcArgs<CT>& a, uint32_t x, s
         for (;;) {
             bool open;
             const uint32_t m = bucket_match<MODE>(key, b, x, &open);
-            if (m) {
-                if (counters(MODE)) atomicAdd(&cnt[bucket_slots<MODE>() * b + (__ffs(m) - 1)], 1u);
-                on_hit<MODE, CT>(a, s_ecnt, owner, e, an, x, s_u);
-                return 1;
-            }
-            if (open) return 0;
+            if (m) return bucket_slots<MODE>() * b + (__ffs(m) - 1);
+            if (open) return GA_EMPTY;
             b = (b + 1) & mask;
         }
     }
     const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
     const uint32_t j = lower_bound_u32(row, 0, an.dv, x);
-    if (j < an.dv && row[j] == x && (!ALIVE || a.alive[x])) {
-        if (MODE == TC_VSUP) atomicAdd(&a.vsup[x], (CT)1);
-        if (MODE == TC_ESUP) atomicAdd(&a.esupk[(size_t)an.row * 8 + j], 1u);
-        on_hit<MODE, CT>(a, s_ecnt, owner, e, an, x, s_u);
-        return 1;
-    }
-    return 0;
+    return j < an.dv && row[j] == x && (!ALIVE || a.alive[x]) ? j : GA_EMPTY;
 }
 
 // The probe lists of a batch of up to 32 in-edges [kb, kend) (one warp): lane l takes the l-th in-edge's suffix of its
@@ -199,65 +193,129 @@ __device__ __forceinline__ uint32_t open_batch(const IX& ix, const uint8_t* aliv
     return __shfl_sync(GA_FULL_MASK, incl, 31);
 }
 
-// Probes one batch of anchor `an` and books what MODE asks for. Returns this lane's hits.
+// The members of the anchor among the eight entries of oct q: their number, and their positions in the oct three bits
+// each in *list. Without branches for a bitmap or a table; buckets that are full without a match (rare) are followed
+// afterwards.
+template <int MODE, bool ALIVE, class CT>
+__device__ __forceinline__ uint32_t oct_members(const TcArgs<CT>& a, const Anchor& an, uint32_t q, const uint32_t* key,
+                                                uint32_t* list) {
+    const uint4* p = reinterpret_cast<const uint4*>(a.ix.colr) + 2 * (size_t)q;
+    const uint4 v0 = __ldg(p), v1 = __ldg(p + 1);
+    const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    uint32_t l = 0, c3 = 0;   // c3: three times the number found
+    if (an.span) {
+        const uint32_t base = an.v + 1;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t o = xs[i] - base;
+            const uint32_t w = o < an.span ? key[o >> 5] : 0u;
+            const bool m = (w >> (o & 31)) & 1u;
+            l |= m ? i << c3 : 0;
+            c3 += m ? 3 : 0;
+        }
+    } else if (an.bits) {
+        const uint32_t nb = an.bits + bucket_shift<MODE>();
+        uint32_t more = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            bool open;
+            const bool m = bucket_match<MODE>(key, hash_slot(xs[i], nb), xs[i], &open) != 0;
+            l |= m ? i << c3 : 0;
+            c3 += m ? 3 : 0;
+            more |= (uint32_t)(!m & !open) << i;
+        }
+        while (more) {
+            const uint32_t i = __ffs(more) - 1;
+            more &= more - 1;
+            if (find_member<MODE, ALIVE, CT>(a, an, __ldg(a.ix.colr + 8 * (size_t)q + i), key, nullptr) != GA_EMPTY) {
+                l |= i << c3;
+                c3 += 3;
+            }
+        }
+    } else {
+        for (uint32_t i = 0; i < 8; i++)
+            if (find_member<MODE, ALIVE, CT>(a, an, a.ix.colr[8 * (size_t)q + i], key, nullptr) != GA_EMPTY) {
+                l |= i << c3;
+                c3 += 3;
+            }
+    }
+    *list = l;
+    return c3 / 3;
+}
+
+// Probes one batch of anchor `an` and books what MODE (supports, lists) asks for. A lane takes an oct and finds all its
+// members; the hits of the 32 octs, a fifth to a quarter of the entries and unevenly spread, are then dealt out to the
+// lanes 32 at a time, so the booking runs with full warps, and neighbouring lanes hold hits of one oct (their increments
+// of the edges u->x share a sector; the entries of the anchor's list are consecutive). What an oct's triangles have in
+// common (the edge u->v, u's list) is booked once per oct. Returns this lane's hits. (R-MAT 22 edge supports: booking
+// inside the probe of each entry 7.4 ms; a loop over a lane's own hits 7.8 ms, 290 instructions a hit, most lanes idle.)
 template <int MODE, bool ALIVE, class CT>
 __device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb, uint32_t kend, const uint32_t* key,
-                                                uint32_t* cnt, const Anchor& an, uint32_t* s_incl, uint32_t* s_base,
-                                                uint32_t lane) {
-    uint32_t hits = 0;
+                                                const uint16_t* pre, uint32_t* cnt, const Anchor& an, uint32_t* s_incl,
+                                                uint32_t* s_base, uint32_t lane) {
     uint32_t *s_ecnt = s_base + 32, *s_u = s_base + 64;   // the caller's batch area: incl, base, ecnt, u
     unsigned long long rec;
     const uint32_t tot = open_batch<ALIVE>(a.ix, a.alive, kb, kend, lane, s_incl, s_base, &rec);
     uint32_t u = 0;
-    if ((MODE == TC_LIST || MODE == TC_VSUP) && rec) u = a.ix.osrc[rng_at(rec) >> 3];   // the source's place
+    if ((MODE == TC_LIST || MODE == TC_VSUP) && rec) u = a.ix.order[a.ix.osrc[rng_at(rec) >> 3]];   // the source's id
     if (MODE == TC_LIST) {
-        s_u[lane] = rec ? a.ix.order[u] : 0u;
+        s_u[lane] = u;
         __syncwarp();
     }
-    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
-    uint32_t owner = 0, end = s_incl[0];
-    if (MODE == TC_COUNT && an.bits) {
-        // counts in a table: the eight lookups of an oct are issued without branches, so they overlap; a bucket that
-        // is full without a match (rare) continues in the next buckets afterwards
-        const uint32_t nb = an.bits + bucket_shift<MODE>(), bmask = (1u << nb) - 1;
-        for (uint32_t p = lane; p < tot; p += 32) {
+    uint32_t owner = 0, end = s_incl[0], hits = 0;
+    for (uint32_t p0 = 0; p0 < tot; p0 += 32) {   // warp-uniform
+        const uint32_t p = p0 + lane;
+        uint32_t list = 0, c = 0, q = 0;
+        if (p < tot) {
             while (end <= p) end = s_incl[++owner];
-            const size_t q = s_base[owner] + p;
-            const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
-            const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            uint32_t more = 0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t x = xs[i];
-                bool open;
-                const bool m = bucket_match<MODE>(key, hash_slot(x, nb), x, &open) != 0;
-                hits += m;
-                more |= (uint32_t)(!m & !open) << i;
+            q = s_base[owner] + p;
+            c = oct_members<MODE, ALIVE, CT>(a, an, q, key, &list);
+        }
+        __syncwarp();
+        const uint32_t incl = warp_incl_scan(c, lane), excl = incl - c, all = __shfl_sync(GA_FULL_MASK, incl, 31);
+        if (!all) continue;
+        hits += c;
+        uint32_t bv = 0, bu = 0, uid = 0;
+        if (MODE == TC_LIST) {
+            if (lane == 0) bv = atomicAdd(&a.fill[an.id], all);
+            bv = __shfl_sync(GA_FULL_MASK, bv, 0);
+            if (c) {
+                uid = s_u[owner];
+                bu = atomicAdd(&a.fill[uid], c);
             }
-            while (more) {
-                const int i = __ffs(more) - 1;
-                more &= more - 1;
-                const uint32_t x = __ldg(a.ix.colr + 8 * q + i);
-                uint32_t b = hash_slot(x, nb);
-                for (;;) {
-                    b = (b + 1) & bmask;
-                    bool open;
-                    if (bucket_match<MODE>(key, b, x, &open)) { hits++; break; }
-                    if (open) break;
-                }
+        } else if (c) {
+            atomicAdd(&s_ecnt[owner], c);
+        }
+        for (uint32_t h0 = 0; h0 < all; h0 += 32) {   // hit h0 + lane: the k-th of lane `from`
+            const uint32_t h = h0 + lane;
+            uint32_t from = 0;
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(GA_FULL_MASK, excl, from + step) <= h) from += step;
+            const uint32_t k = h - __shfl_sync(GA_FULL_MASK, excl, from);
+            const uint32_t i = (__shfl_sync(GA_FULL_MASK, list, from) >> (3 * (k & 7))) & 7;
+            const size_t e = (size_t)__shfl_sync(GA_FULL_MASK, q, from) * 8 + i;
+            uint32_t hu = 0, hb = 0;
+            if (MODE == TC_LIST) {
+                hu = __shfl_sync(GA_FULL_MASK, uid, from);
+                hb = __shfl_sync(GA_FULL_MASK, bu, from) + k;
+            }
+            if (h >= all) continue;
+            const uint32_t x = __ldg(a.ix.colr + e);
+            if (MODE == TC_LIST) {   // (u, v, x), lowest to highest
+                const uint32_t xid = a.ix.order[x];
+                list_at(a, an.id, bv + h, hu, xid);
+                list_at(a, hu, hb, an.id, xid);
+                list_at(a, xid, atomicAdd(&a.fill[xid], 1u), hu, an.id);
+            } else {
+                const uint32_t slot = find_member<MODE, ALIVE, CT>(a, an, x, key, pre);
+                if (an.span || an.bits) atomicAdd(&cnt[slot], 1u);
+                else if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)1);
+                else atomicAdd(&a.esupk[(size_t)an.row * 8 + slot], 1u);
+                if (MODE == TC_ESUP) atomicAdd(&a.esupk[e], 1u);   // u->x at its place in u's row
             }
         }
         __syncwarp();
-        return hits;
-    }
-    for (uint32_t p = lane; p < tot; p += 32) {
-        while (end <= p) end = s_incl[++owner];
-        const size_t q = s_base[owner] + p;
-        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
-        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            hits += probe_one<MODE, ALIVE, CT>(a, xs[i], 8 * q + i, owner, key, cnt, an, s_ecnt, s_u);
     }
     __syncwarp();
     if (counters(MODE)) {
@@ -266,6 +324,63 @@ __device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb
             if (MODE == TC_VSUP) atomicAdd(&a.vsup[u], (CT)c);
             else atomicAdd(&a.esupk[rng_at(rec)], c);
             s_ecnt[lane] = 0;
+        }
+    }
+    __syncwarp();
+    return hits;
+}
+
+// Probes one batch of anchor `an` for a count, one lane per oct, in the anchor's table (or, without one, by binary
+// search in its row). Returns this lane's hits.
+template <bool ALIVE, class CT>
+__device__ __forceinline__ uint32_t count_batch(const TcArgs<CT>& a, uint32_t kb, uint32_t kend, const uint32_t* key,
+                                                const Anchor& an, uint32_t* s_incl, uint32_t* s_base, uint32_t lane) {
+    unsigned long long rec;
+    const uint32_t tot = open_batch<ALIVE>(a.ix, a.alive, kb, kend, lane, s_incl, s_base, &rec);
+    uint32_t owner = 0, end = s_incl[0], hits = 0;
+    if (!an.bits) {
+        const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
+        for (uint32_t p = lane; p < tot; p += 32) {
+            while (end <= p) end = s_incl[++owner];
+            const uint32_t q = s_base[owner] + p;
+#pragma unroll 1
+            for (int i = 0; i < 8; i++) {
+                const uint32_t x = a.ix.colr[8 * (size_t)q + i], j = lower_bound_u32(row, 0, an.dv, x);
+                hits += j < an.dv && row[j] == x && (!ALIVE || a.alive[x]);
+            }
+        }
+        __syncwarp();
+        return hits;
+    }
+    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
+    // the eight lookups of an oct are issued without branches, so they overlap; a bucket that is full without a match
+    // (rare) continues in the next buckets afterwards
+    const uint32_t nb = an.bits + bucket_shift<TC_COUNT>(), bmask = (1u << nb) - 1;
+    for (uint32_t p = lane; p < tot; p += 32) {
+        while (end <= p) end = s_incl[++owner];
+        const size_t q = s_base[owner] + p;
+        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
+        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        uint32_t more = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t x = xs[i];
+            bool open;
+            const bool m = bucket_match<TC_COUNT>(key, hash_slot(x, nb), x, &open) != 0;
+            hits += m;
+            more |= (uint32_t)(!m & !open) << i;
+        }
+        while (more) {
+            const int i = __ffs(more) - 1;
+            more &= more - 1;
+            const uint32_t x = __ldg(a.ix.colr + 8 * q + i);
+            uint32_t b = hash_slot(x, nb);
+            for (;;) {
+                b = (b + 1) & bmask;
+                bool open;
+                if (bucket_match<TC_COUNT>(key, b, x, &open)) { hits++; break; }
+                if (open) break;
+            }
         }
     }
     __syncwarp();
@@ -313,16 +428,20 @@ __device__ __forceinline__ void build_table(const TcArgs<CT>& a, const Anchor& a
     if (sync_block) __syncthreads(); else __syncwarp();
 }
 
-// Heavy anchors of a count use a bitmap of N+(v) instead of a hash set when it fits the table's shared memory: every
+// Heavy anchors use a bitmap of N+(v) instead of a hash set when it fits the table's shared memory: every
 // out-neighbour's place is above v's own, and for the anchors of many out-neighbours (high degree) they lie in a short
 // range (R-MAT 22: under 65,536 places for every anchor of more than 128 out-neighbours, against 4.2M vertices). Bit o
-// of the bitmap is set iff place base + o is an (alive) out-neighbour of v, base = v + 1; span = the largest
-// out-neighbour - v bounds o. A probe is then one shared 32-bit load and a bit test, with no collisions and nothing to
-// continue; the entries before the suffix and the padding fall outside [0, span).
-template <bool ALIVE, class CT>
-__device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& an, uint32_t span, uint32_t* bm) {
-    const uint32_t quads = (span + 127) >> 7;
+// of the bitmap is set iff place v + 1 + o is an (alive) out-neighbour of v; span = the largest out-neighbour - v bounds
+// o. A probe is then one shared 32-bit load and a bit test, with no collisions and nothing to continue; the entries
+// before the suffix and the padding fall outside [0, span). Supports also need which member it is: pre[w], the members
+// below word w, plus a population count: the rank among the row's (alive) members, which the flush goes through again.
+template <int MODE, bool ALIVE, class CT>
+__device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& an, uint32_t* bm, uint16_t* pre,
+                                             uint32_t* cnt) {
+    const uint32_t quads = (an.span + 127) >> 7;
     for (uint32_t w = threadIdx.x; w < quads; w += kThreads) reinterpret_cast<uint4*>(bm)[w] = make_uint4(0, 0, 0, 0);
+    if (counters(MODE))
+        for (uint32_t i = threadIdx.x; i < an.dv; i += kThreads) cnt[i] = 0;
     __syncthreads();
     const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
     for (uint32_t i = threadIdx.x; i < an.dv; i += kThreads) {
@@ -332,11 +451,30 @@ __device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& 
         atomicOr(&bm[o >> 5], 1u << (o & 31));
     }
     __syncthreads();
+    if (counters(MODE)) {
+        // exclusive scan of the words' population counts: every warp scans a stretch, then adds the stretches before
+        __shared__ uint32_t s_part[kWarps];
+        const uint32_t words = (an.span + 31) >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const uint32_t per = ((words + kWarps - 1) / kWarps + 31) & ~31u, w0 = warp * per, w1 = min(words, w0 + per);
+        uint32_t run = 0;
+        for (uint32_t w = w0; w < w1; w += 32) run += __reduce_add_sync(GA_FULL_MASK, w + lane < w1 ? __popc(bm[w + lane]) : 0);
+        if (lane == 0) s_part[warp] = run;
+        __syncthreads();
+        run = 0;
+        for (uint32_t q = 0; q < warp; q++) run += s_part[q];
+        for (uint32_t w = w0; w < w1; w += 32) {
+            const uint32_t c = w + lane < w1 ? __popc(bm[w + lane]) : 0u;
+            const uint32_t incl = warp_incl_scan(c, lane);
+            if (w + lane < w1) pre[w + lane] = (uint16_t)(run + incl - c);
+            run += __shfl_sync(GA_FULL_MASK, incl, 31);
+        }
+        __syncthreads();
+    }
 }
 
-// probe_batch for a count against the bitmap of a heavy anchor. Returns this lane's hits.
+// A batch of a count against the bitmap of a heavy anchor. Returns this lane's hits.
 template <bool ALIVE, class CT>
-__device__ __forceinline__ uint32_t probe_batch_bitmap(const TcArgs<CT>& a, uint32_t kb, uint32_t kend,
+__device__ __forceinline__ uint32_t count_batch_bitmap(const TcArgs<CT>& a, uint32_t kb, uint32_t kend,
                                                        const uint32_t* bm, uint32_t base, uint32_t span,
                                                        uint32_t* s_incl, uint32_t* s_base, uint32_t lane) {
     unsigned long long rec;
@@ -448,16 +586,31 @@ __device__ __forceinline__ uint32_t tiny_group(const TcArgs<CT>& a, uint32_t p0,
     return hits;
 }
 
-// Adds the per-slot counters of an item to the outputs (x's vertex count or edge v->x's count).
-template <int MODE, class CT>
-__device__ __forceinline__ void flush_table(const TcArgs<CT>& a, const Anchor& an, const uint32_t* key,
-                                            const uint32_t* cnt, const uint32_t* pos, uint32_t tid, uint32_t nthr) {
+// Adds an item's counters to the outputs (x's vertex count or edge v->x's count): by table slot, or by rank among the
+// (alive) members of the row for a bitmap.
+template <int MODE, bool ALIVE, class CT>
+__device__ __forceinline__ void flush_counts(const TcArgs<CT>& a, const Anchor& an, const uint32_t* key,
+                                             const uint16_t* pre, const uint32_t* cnt, const uint32_t* pos,
+                                             uint32_t tid, uint32_t nthr) {
     if (!counters(MODE)) return;
+    if (an.span) {
+        const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
+        for (uint32_t j = tid; j < an.dv; j += nthr) {
+            const uint32_t x = row[j];
+            if (ALIVE && !a.alive[x]) continue;
+            const uint32_t o = x - an.v - 1;
+            const uint32_t c = cnt[ALIVE ? pre[o >> 5] + __popc(key[o >> 5] & ((1u << (o & 31)) - 1)) : j];
+            if (!c) continue;
+            if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)c);
+            else atomicAdd(&a.esupk[(size_t)an.row * 8 + j], c);
+        }
+        return;
+    }
     const uint32_t S = 4u << an.bits;
     for (uint32_t s = tid; s < S; s += nthr) {
         const uint32_t c = cnt[s];
         if (c) {
-            if (MODE == TC_VSUP) atomicAdd(&a.vsup[key[s]], (CT)c);   // 4-slot buckets: no spill flags
+            if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[key[s]]], (CT)c);   // 4-slot buckets: no spill flags
             else atomicAdd(&a.esupk[(size_t)an.row * 8 + pos[s]], c);
         }
     }
@@ -475,19 +628,12 @@ __global__ void k_esup_fold(TcIndex ix, const uint32_t* __restrict__ src, const 
     }
 }
 
-// alive mask by id -> by place; counts by place -> by id.
+// alive mask by id -> by place.
 __global__ void k_alive_places(const uint8_t* __restrict__ alive, const uint32_t* __restrict__ order, uint32_t n,
                                uint8_t* __restrict__ out) {
     for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (uint64_t)gridDim.x * blockDim.x)
         out[a] = alive[order[a]];
 }
-template <class CT>
-__global__ void k_counts_by_id(const CT* __restrict__ by_place, const uint32_t* __restrict__ vrank, uint32_t n,
-                               CT* __restrict__ out) {
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-        out[v] = by_place[vrank[v]];
-}
-
 // bounds (optional, device): this launch's item ranges (a shard), [bounds[2b], bounds[2b + 1]) of the items of bin b
 // (heavy, light, tiny); null means every item. tiny_groups: counts of the whole graph take the tiny bin in groups of 32
 // places from tiny_first on; otherwise its items are run like light ones.
@@ -531,14 +677,19 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
             }
             an.row = a.ix.pos[an.v].y;
             an.dv = a.ix.dout[an.v];
-            an.id = MODE == TC_LIST ? a.ix.order[an.v] : 0u;
+            an.id = MODE == TC_LIST || MODE == TC_VSUP ? a.ix.order[an.v] : 0u;
             const uint32_t k0 = items.k0[item], k1 = items.k1[item];
-            // the last entry of the row has the largest place
-            const uint32_t span = MODE == TC_COUNT ? a.ix.colr[(size_t)an.row * 8 + an.dv - 1] - an.v : 0u;
-            const bool bitmap = MODE == TC_COUNT && a.bitmaps && span <= (Smax << 5);
+            // the last entry of the row has the largest place; the bitmap takes the table's place, with the ranks and
+            // counters of the support modes behind it
+            const uint32_t span = a.ix.colr[(size_t)an.row * 8 + an.dv - 1] - an.v;
+            const uint32_t words = (span + 127) >> 7 << 2, ranks = counters(MODE) ? words / 2 : 0;
+            const bool bitmap = a.bitmaps && words + ranks + (counters(MODE) ? an.dv : 0u) <= Smax * W && an.dv <= 0xFFFFu;
+            an.span = bitmap ? span : 0u;
             an.bits = bitmap ? 0u : table_bits(an.dv, heavy_bits_max);
+            uint16_t* pre = reinterpret_cast<uint16_t*>(key + words);
+            uint32_t* cn = bitmap ? key + words + ranks : cnt;
             if (threadIdx.x == 0) s_next = k0;
-            if (bitmap) build_bitmap<ALIVE, CT>(a, an, span, key);
+            if (bitmap) build_bitmap<MODE, ALIVE, CT>(a, an, key, pre, cn);
             else if (an.bits) build_table<MODE, ALIVE, CT>(a, an, key, cnt, pos, threadIdx.x, kThreads, true);
             else __syncthreads();
             unsigned long long h = 0;
@@ -547,19 +698,21 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
                 if (lane == 0) kb = atomicAdd(&s_next, 32u);
                 kb = __shfl_sync(GA_FULL_MASK, kb, 0);
                 if (kb >= k1) break;
-                if (MODE == TC_COUNT && bitmap)
-                    h += probe_batch_bitmap<ALIVE, CT>(a, kb, min(kb + 32, k1), key, an.v + 1, span, s_incl, s_base,
-                                                       lane);
-                else
-                    h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, cnt, an, s_incl, s_base, lane);
+                if constexpr (MODE == TC_COUNT) {
+                    if (bitmap) h += count_batch_bitmap<ALIVE, CT>(a, kb, min(kb + 32, k1), key, an.v + 1, span, s_incl,
+                                                                   s_base, lane);
+                    else h += count_batch<ALIVE, CT>(a, kb, min(kb + 32, k1), key, an, s_incl, s_base, lane);
+                } else {
+                    h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, pre, cn, an, s_incl, s_base, lane);
+                }
             }
             hits += h;
             if (MODE == TC_VSUP) {
                 const unsigned long long t = warp_sum_u64(h);
-                if (lane == 0 && t) atomicAdd(&a.vsup[an.v], (CT)t);
+                if (lane == 0 && t) atomicAdd(&a.vsup[an.id], (CT)t);
             }
             __syncthreads();
-            if (an.bits) flush_table<MODE, CT>(a, an, key, cnt, pos, threadIdx.x, kThreads);
+            if (an.span || an.bits) flush_counts<MODE, ALIVE, CT>(a, an, key, pre, cn, pos, threadIdx.x, kThreads);
             __syncthreads();
         }
     }
@@ -586,22 +739,27 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
         if (ALIVE && !a.alive[an.v]) continue;
         an.row = a.ix.pos[an.v].y;
         an.dv = a.ix.dout[an.v];
-        an.id = MODE == TC_LIST ? a.ix.order[an.v] : 0u;
+        an.id = MODE == TC_LIST || MODE == TC_VSUP ? a.ix.order[an.v] : 0u;
         // a table unless the anchor is too large for this mode's set (GA_OPT_LIGHT_MAX_DEG above 128 in the
         // support modes): then binary search in the row
+        an.span = 0;
         an.bits = table_bits(an.dv, light_bits<MODE>());
         if (an.bits) build_table<MODE, ALIVE, CT>(a, an, key, cnt, pos, lane, 32, false);
         unsigned long long h = 0;
         const uint32_t k1 = items.k1[item];
-        for (uint32_t kb = items.k0[item]; kb < k1; kb += 32)
-            h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, cnt, an, s_incl, s_base, lane);
+        for (uint32_t kb = items.k0[item]; kb < k1; kb += 32) {
+            if constexpr (MODE == TC_COUNT)
+                h += count_batch<ALIVE, CT>(a, kb, min(kb + 32, k1), key, an, s_incl, s_base, lane);
+            else
+                h += probe_batch<MODE, ALIVE, CT>(a, kb, min(kb + 32, k1), key, nullptr, cnt, an, s_incl, s_base, lane);
+        }
         hits += h;
         if (MODE == TC_VSUP) {
             const unsigned long long t = warp_sum_u64(h);
-            if (lane == 0 && t) atomicAdd(&a.vsup[an.v], (CT)t);
+            if (lane == 0 && t) atomicAdd(&a.vsup[an.id], (CT)t);
         }
         __syncwarp();
-        if (an.bits) flush_table<MODE, CT>(a, an, key, cnt, pos, lane, 32);
+        if (an.bits) flush_counts<MODE, ALIVE, CT>(a, an, key, nullptr, cnt, pos, lane, 32);
         __syncwarp();
     }
     // ---- tiny bin of a whole count: groups of 32 places ----
@@ -669,17 +827,17 @@ __global__ void __launch_bounds__(256) k_tc_octs(uint32_t m, TcArgs<CT> a) {
                     a.ix.colr, rng_oct(r), octs, row, rend, [&](uint32_t x) {
                         if (ALIVE && !a.alive[x]) return;
                         c++;
-                        if (MODE == TC_VSUP) atomicAdd(&a.vsup[x], (CT)1);
+                        if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)1);
                     });
                 if (MODE == TC_COUNT && !ALIVE) c = all;
             }
         }
         local += c;
         if (MODE == TC_VSUP && __any_sync(GA_FULL_MASK, c != 0)) {
-            if (c) atomicAdd(&a.vsup[u], (CT)c);
+            if (c) atomicAdd(&a.vsup[a.ix.order[u]], (CT)c);
             const uint32_t peers = __match_any_sync(GA_FULL_MASK, c ? v : kPad);
             const uint32_t sum = __reduce_add_sync(peers, c);
-            if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[v], (CT)sum);
+            if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[a.ix.order[v]], (CT)sum);
         }
     }
     add_total(local, a.total);
@@ -811,21 +969,21 @@ static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
     return GA_OK;
 }
 
-// One pass on the index (octs: one thread per in-edge, else the hash kernel). The caller's arrays are by id (and by col
-// position); the kernels' by place.
+// One pass on the index (octs: one thread per in-edge, else the hash kernel). Per-vertex outputs are the caller's, by id:
+// by place the hubs' counters would be neighbours, and the atomics on them meet in a few L2 sectors (vertex supports of
+// R-MAT 18: 1.06 ms against 0.78). Per-edge outputs are by position in colr and moved to the caller's col order.
 template <int MODE, bool ALIVE, class CT>
 static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
     cudaStream_t st = g->stream;
     TcArgs<CT> a = a0;
     a.ix = tc_index(g);
     a.bitmaps = !g->opt_count_bitmap;
-    void* tmp = nullptr;   // outputs (and the mask) by place
-    const size_t osize = MODE == TC_ESUP ? (size_t)g->octs * 8 * 4 : MODE == TC_VSUP ? (size_t)g->n * sizeof(CT) : 0;
+    void* tmp = nullptr;   // supports by position in colr, the mask by place
+    const size_t osize = MODE == TC_ESUP ? (size_t)g->octs * 8 * 4 : 0;
     if (osize + (ALIVE ? g->n : 0)) {
         GA_CUDA(pool_malloc(&tmp, osize + (ALIVE ? g->n : 0), st));
         if (osize) GA_CUDA(cudaMemsetAsync(tmp, 0, osize, st));
         if (MODE == TC_ESUP) a.esupk = (uint32_t*)tmp;
-        if (MODE == TC_VSUP) a.vsup = (CT*)tmp;
         if (ALIVE) {
             uint8_t* al = (uint8_t*)tmp + osize;
             k_alive_places<<<grid_for(g->n, 256), 256, 0, st>>>(a0.alive, g->order, g->n, al);
@@ -843,8 +1001,6 @@ static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
     if (!octs) s = launch_hash<MODE, ALIVE, CT>(g, a);
     if (s == GA_OK && MODE == TC_ESUP)
         k_esup_fold<<<grid_for(g->m, 256), 256, 0, st>>>(a.ix, g->src, g->col, g->m, a.esupk, a0.esup);
-    if (s == GA_OK && MODE == TC_VSUP)
-        k_counts_by_id<CT><<<grid_for(g->n, 256), 256, 0, st>>>(a.vsup, g->vrank, g->n, a0.vsup);
     if (tmp) cudaFreeAsync(tmp, st);
     GA_TRY(s);
     GA_CUDA(cudaGetLastError());
@@ -890,9 +1046,9 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
     const bool octs = kernel == 1 && (MODE == TC_COUNT || MODE == TC_VSUP) && a.nshards <= 1 && g->n <= kTabEmpty;
     const bool index = (kernel != 1 || octs) && g->m;
     cudaStream_t st = g->stream;
-    if (zero_outputs) {   // on the index, supports are written whole from the kernels' own arrays
+    if (zero_outputs) {   // on the index, edge supports are written whole from the kernels' own array
         GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
-        if (!index && MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
+        if (MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
         if (!index && MODE == TC_ESUP && g->m) GA_CUDA(cudaMemsetAsync(a.esup, 0, (size_t)g->m * sizeof(uint32_t), st));
     }
     if (!g->m) return GA_OK;

@@ -33,10 +33,10 @@ struct TcArgs {
     const unsigned long long* inc_ptr = nullptr;
     uint32_t* fill = nullptr;
     uint32_t* overflow = nullptr;   // TC_LIST: entries that found their list full (must stay 0)
-    // set by the launcher of the hash kernel (whose vsup and alive are by place)
+    // set by the launcher of the kernels on the index (whose alive is by place)
     TcIndex ix = {};
     uint32_t* esupk = nullptr;      // ESUP: supports by padded position in colr, zeroed
-    bool bitmaps = false;           // COUNT: heavy anchors may use bitmaps
+    bool bitmaps = false;           // heavy anchors may use bitmaps
     // shard `shard` of `nshards` (0 = the whole graph): equal parts of the probe work (hash kernel) or of the edges
     // (plain kernel); the shards of a graph partition its triangles
     uint32_t shard = 0, nshards = 0;
