@@ -43,7 +43,7 @@
 namespace ga {
 
 constexpr uint32_t kChunk = 256;     // neighbours of a frontier vertex per update item (enumeration update)
-constexpr uint32_t kListChunk = 1024;   // incidence entries of a frontier vertex per update item (list update)
+constexpr uint32_t kListChunk = 512;    // incidence entries of a frontier vertex per update item (list update)
 constexpr int kUpdWarps = 8;
 
 enum LoopKind { LOOP_PEEL = 0, LOOP_CORE = 1 };
@@ -110,7 +110,7 @@ struct ga_loops {
     ga::LoopScalars h_sc = {};         // host copy of the round state
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     cudaGraph_t graph[2] = {nullptr, nullptr};
-    unsigned grid_scan = 1, grid_update = 1;
+    unsigned grid_scan = 1, grid_update = 1, grid_list = 1;
     // triangle incidence lists (built once per graph when memory allows): for every vertex v the other two corners
     // of each triangle through v, in inc[inc_ptr[v] .. inc_ptr[v+1])
     int lists = -1;                    // -1 undecided, 0 enumeration update, 1 incidence-list update
@@ -149,36 +149,58 @@ __global__ void k_loop_scalars(LoopScalars* sc, const unsigned long long* total,
     *sc = s;
 }
 
-// Appends the frontier vertex v (mark kernels): its id to frontier[], and ceil(deg(v) / kChunk) update items.
-// All 32 lanes call it; `take` marks the lanes that append. One atomic per warp for each list.
-// With incidence lists (inc_ptr != null) the items are ceil(|Tri(v)| / kListChunk) slices of v's list instead.
-__device__ __forceinline__ void append_frontier(bool take, uint32_t v, const uint32_t* __restrict__ degree,
-                                                const unsigned long long* __restrict__ inc_ptr, LoopScalars* sc,
-                                                uint32_t* __restrict__ frontier, uint32_t* __restrict__ item_x,
-                                                uint32_t* __restrict__ item_c, uint32_t lane) {
-    const uint32_t bal = __ballot_sync(GA_FULL_MASK, take);
-    if (!bal) return;
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&sc->fcount, (uint32_t)__popc(bal));
-    base = __shfl_sync(GA_FULL_MASK, base, 0);
+constexpr int kMarkThreads = 256;
+
+// Where the mark kernels' blocks meet: per warp the frontier vertices, survivors and update items, then their bases.
+struct MarkShared {
+    uint32_t n[3][kMarkThreads / 32], base[3];
+};
+
+// Appends this block's vertices (one per thread, every thread calls it): frontier vertices `rem` with their update items
+// - ceil(|Tri(v)| / kListChunk) slices of v's incidence list, or ceil(deg(v) / kChunk) of its neighbours without lists -
+// and survivors `keep` to the next alive list. One atomic per block and list: with one per warp, the first round over
+// eight million vertices waited for 750,000 atomics on three addresses (0.55 ms).
+__device__ __forceinline__ void append_block(bool rem, bool keep, uint32_t v, const uint32_t* __restrict__ degree,
+                                             const unsigned long long* __restrict__ inc_ptr, LoopScalars* sc,
+                                             uint32_t* __restrict__ frontier, uint32_t* __restrict__ item_x,
+                                             uint32_t* __restrict__ item_c, uint32_t* __restrict__ out_list,
+                                             uint32_t* out_count, MarkShared& sh) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t br = __ballot_sync(GA_FULL_MASK, rem), bk = __ballot_sync(GA_FULL_MASK, keep);
     uint32_t nc = 0;
-    if (take) {
-        frontier[base + __popc(bal & ((1u << lane) - 1))] = v;
-        if (inc_ptr) {
-            nc = (uint32_t)((inc_ptr[v + 1] - inc_ptr[v] + kListChunk - 1) / kListChunk);
-        } else {
-            nc = (uint32_t)(((uint64_t)degree[v] + kChunk - 1) / kChunk);
+    if (rem)
+        nc = inc_ptr ? (uint32_t)((inc_ptr[v + 1] - inc_ptr[v] + kListChunk - 1) / kListChunk)
+                     : (uint32_t)(((uint64_t)degree[v] + kChunk - 1) / kChunk);
+    const uint32_t incl = br ? warp_incl_scan(nc, lane) : 0u;   // br is the same in the whole warp
+    if (lane == 31) {
+        sh.n[0][w] = __popc(br);
+        sh.n[1][w] = __popc(bk);
+        sh.n[2][w] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        uint32_t sum = 0;
+        for (int q = 0; q < kMarkThreads / 32; q++) sum += sh.n[threadIdx.x][q];
+        uint32_t* counter = threadIdx.x == 0 ? &sc->fcount : threadIdx.x == 1 ? out_count : &sc->nitems;
+        sh.base[threadIdx.x] = sum ? atomicAdd(counter, sum) : 0u;
+    }
+    __syncthreads();
+    uint32_t at[3] = {sh.base[0], sh.base[1], sh.base[2]};
+    for (uint32_t q = 0; q < w; q++) {
+        at[0] += sh.n[0][q];
+        at[1] += sh.n[1][q];
+        at[2] += sh.n[2][q];
+    }
+    const uint32_t below = (1u << lane) - 1;
+    if (rem) {
+        frontier[at[0] + __popc(br & below)] = v;
+        for (uint32_t c = 0; c < nc; c++) {
+            item_x[at[2] + incl - nc + c] = v;
+            item_c[at[2] + incl - nc + c] = c;
         }
     }
-    const uint32_t incl = warp_incl_scan(nc, lane);
-    const uint32_t tot = __shfl_sync(GA_FULL_MASK, incl, 31);
-    uint32_t ib = 0;
-    if (lane == 31 && tot) ib = atomicAdd(&sc->nitems, tot);
-    ib = __shfl_sync(GA_FULL_MASK, ib, 31);
-    for (uint32_t c = 0; c < nc; c++) {
-        item_x[ib + incl - nc + c] = v;
-        item_c[ib + incl - nc + c] = c;
-    }
+    if (keep) out_list[at[1] + __popc(bk & below)] = v;
+    __syncthreads();   // the counts are read before the next tile's replace them
 }
 
 // The previous round's frontier leaves for good (state 2 -> 0). Run by the first kernel of a round, before any
@@ -189,22 +211,11 @@ __device__ __forceinline__ void retire_previous(const LoopScalars* sc, uint8_t* 
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < F; i += gridDim.x * blockDim.x) state[prev[i]] = 0;
 }
 
-// Survivors go to the next alive list (one atomic per warp).
-__device__ __forceinline__ void append_survivor(bool keep, uint32_t v, uint32_t* __restrict__ out_list,
-                                                uint32_t* out_count, uint32_t lane) {
-    const uint32_t bal = __ballot_sync(GA_FULL_MASK, keep);
-    if (!bal) return;
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(out_count, (uint32_t)__popc(bal));
-    base = __shfl_sync(GA_FULL_MASK, base, 0);
-    if (keep) out_list[base + __popc(bal & ((1u << lane) - 1))] = v;
-}
-
 // Peel round, step 1: best-density bookkeeping (peel_improves, densest.h:297) and the mark_peel rule
 // (kernels.cuh:448-451) over the alive list. With segments each vertex uses its own graph's T and alive count (the
 // per-graph best density is kept by the tail), removals are counted per graph (one atomic per graph per warp), and
 // the vertices of a graph that was refused or failed leave the loop silently.
-__global__ void __launch_bounds__(256) k_peel_mark(LoopScalars* sc, const uint32_t* __restrict__ tri,
+__global__ void __launch_bounds__(kMarkThreads) k_peel_mark(LoopScalars* sc, const uint32_t* __restrict__ tri,
                                                    uint8_t* __restrict__ state, uint32_t* __restrict__ removed_round,
                                                    uint32_t* alive0, uint32_t* alive1, uint32_t* fr0, uint32_t* fr1,
                                                    uint32_t* __restrict__ item_x,
@@ -226,10 +237,11 @@ __global__ void __launch_bounds__(256) k_peel_mark(LoopScalars* sc, const uint32
             sc->best_round = round;
         }
     }
+    __shared__ MarkShared sh;
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < na; i0 += stride) {
-        const uint32_t i = i0 + lane;
+    const uint64_t stride = (uint64_t)gridDim.x * kMarkThreads;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kMarkThreads; i0 < na; i0 += stride) {   // block-uniform
+        const uint64_t i = i0 + threadIdx.x;
         const bool valid = i < na;
         const uint32_t v = valid ? in[i] : 0;
         bool rem = false, drop = false;
@@ -260,8 +272,8 @@ __global__ void __launch_bounds__(256) k_peel_mark(LoopScalars* sc, const uint32
                     atomicAdd(&sg.removed[s], (unsigned long long)__popc(peers));
             }
         }
-        append_frontier(rem, v, degree, inc_ptr, sc, frontier, item_x, item_c, lane);
-        append_survivor(valid && !rem && !drop, v, outl, &sc->alive_count[p ^ 1], lane);
+        append_block(rem, valid && !rem && !drop, v, degree, inc_ptr, sc, frontier, item_x, item_c, outl,
+                     &sc->alive_count[p ^ 1], sh);
     }
 }
 
@@ -288,7 +300,7 @@ __global__ void __launch_bounds__(256) k_core_min(LoopScalars* sc, const uint32_
 
 // Core round, step 2: k = max(k, min); frontier = alive with tri <= k, core = k (core_find_frontier,
 // kernels.cuh:549-562).
-__global__ void __launch_bounds__(256) k_core_mark(LoopScalars* sc, const uint32_t* __restrict__ tri,
+__global__ void __launch_bounds__(kMarkThreads) k_core_mark(LoopScalars* sc, const uint32_t* __restrict__ tri,
                                                    uint8_t* __restrict__ state, uint32_t* __restrict__ core,
                                                    uint32_t* alive0, uint32_t* alive1, uint32_t* fr0, uint32_t* fr1,
                                                    uint32_t* __restrict__ item_x,
@@ -302,10 +314,10 @@ __global__ void __launch_bounds__(256) k_core_mark(LoopScalars* sc, const uint32
     const uint32_t na = sc->alive_count[p];
     const uint32_t k = max(sc->kcur, sc->min_tri);
     if (blockIdx.x == 0 && threadIdx.x == 0) sc->kround = k;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < na; i0 += stride) {
-        const uint32_t i = i0 + lane;
+    __shared__ MarkShared sh;
+    const uint64_t stride = (uint64_t)gridDim.x * kMarkThreads;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kMarkThreads; i0 < na; i0 += stride) {   // block-uniform
+        const uint64_t i = i0 + threadIdx.x;
         const bool valid = i < na;
         const uint32_t v = valid ? in[i] : 0;
         bool rem = false;
@@ -316,8 +328,8 @@ __global__ void __launch_bounds__(256) k_core_mark(LoopScalars* sc, const uint32
                 core[v] = k;
             }
         }
-        append_frontier(rem, v, degree, inc_ptr, sc, frontier, item_x, item_c, lane);
-        append_survivor(valid && !rem, v, outl, &sc->alive_count[p ^ 1], lane);
+        append_block(rem, valid && !rem, v, degree, inc_ptr, sc, frontier, item_x, item_c, outl,
+                     &sc->alive_count[p ^ 1], sh);
     }
 }
 
@@ -538,10 +550,14 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
     close_round_if_last(sc, kind, handle, use_handle, sg);
 }
 
-// Incidence-list update: one warp per item = up to kListChunk entries (y, w) of frontier vertex x's list, read
-// coalesced. The triangle {x, y, w} still exists iff y and w are alive or in the frontier; it is handled by its
-// smallest-id frontier corner (kernels.cuh:607), which subtracts 1 from tri[] of its alive corners and counts it as
-// destroyed. Over a whole run every triangle is read at most three times (once per corner).
+// Incidence-list update over items of up to kListChunk entries (y, w) of frontier vertex x's list, read coalesced. The
+// triangle {x, y, w} still exists iff y and w are alive or in the frontier; it is handled by its smallest-id frontier
+// corner (kernels.cuh:607), which subtracts 1 from tri[] of its alive corners and counts it as destroyed. Over a whole
+// run every triangle is read at most three times (once per corner).
+// A warp takes up to 32 items at a time - one per lane, their entries flattened by a warp scan like the count's probe
+// lists - when there are that many per warp, else fewer: the first rounds of a peeling remove millions of vertices
+// whose lists hold some tens of entries, and one item at a time was a chain of four dependent loads for half-empty
+// warps (batch of 256 Holme-Kim graphs: 3.5 ms of updates a peeling).
 __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, const uint2* __restrict__ inc,
                                                               const unsigned long long* __restrict__ inc_ptr,
                                                               const uint32_t* __restrict__ item_x,
@@ -549,33 +565,59 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
                                                               const uint8_t* __restrict__ state,
                                                               uint32_t* __restrict__ tri, Segs sg, int kind,
                                                               cudaGraphConditionalHandle handle, int use_handle) {
-    __shared__ unsigned long long s_red[8];
+    __shared__ unsigned long long s_red[8], s_beg[8][32];
+    __shared__ uint32_t s_incl[8][32], s_x[8][32], s_des[8][32];
     if (!sc->cont) return;
     count_iteration(sc, handle, use_handle);
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t nitems = last_round(sc, sg) ? 0u : sc->nitems;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t per = min(32u, max(1u, nitems / nwarps));   // items a warp takes at a time
     unsigned long long destroyed = 0;
-    for (uint32_t it = gwarp; it < nitems; it += nwarps) {
-        const uint32_t x = item_x[it];
-        const uint32_t seg = sg.count ? seg_of(sg, x) : 0u;
-        if (sg.count && sg.removed[seg] == sg.nalive[seg]) continue;   // its graph's last round
-        const unsigned long long b = inc_ptr[x] + (unsigned long long)item_c[it] * kListChunk;
-        const unsigned long long e = min(inc_ptr[x + 1], b + kListChunk);
-        const unsigned long long d0 = destroyed;
-        for (unsigned long long i = b + lane; i < e; i += 32) {
-            const uint2 yw = inc[i];
+    for (uint64_t it0 = (uint64_t)gwarp * per; it0 < nitems; it0 += (uint64_t)nwarps * per) {   // warp-uniform
+        uint32_t x = 0, seg = 0, len = 0;
+        unsigned long long b = 0;
+        if (lane < per && it0 + lane < nitems) {
+            x = item_x[it0 + lane];
+            seg = sg.count ? seg_of(sg, x) : 0u;
+            if (!sg.count || sg.removed[seg] != sg.nalive[seg]) {   // not its graph's last round
+                b = inc_ptr[x] + (unsigned long long)item_c[it0 + lane] * kListChunk;
+                len = (uint32_t)min(inc_ptr[x + 1] - b, (unsigned long long)kListChunk);
+            }
+        }
+        const uint32_t incl = warp_incl_scan(len, lane), tot = __shfl_sync(GA_FULL_MASK, incl, 31);
+        s_incl[w][lane] = incl;
+        s_beg[w][lane] = b - (incl - len);
+        s_x[w][lane] = x;
+        s_des[w][lane] = 0;
+        __syncwarp();
+        uint32_t owner = 0, end = s_incl[w][0], mine = 0;
+        for (uint32_t p = lane; p < tot; p += 32) {
+            if (end <= p) {
+                if (sg.count && mine) atomicAdd(&s_des[w][owner], mine);
+                destroyed += mine;
+                mine = 0;
+                while (end <= p) end = s_incl[w][++owner];
+            }
+            const uint2 yw = inc[s_beg[w][owner] + p];
+            const uint32_t xv = s_x[w][owner];
             const uint8_t sy = state[yw.x], sw = state[yw.y];
             if (!sy || !sw) continue;                               // destroyed in an earlier round
-            if ((sy == 2 && yw.x < x) || (sw == 2 && yw.y < x)) continue;   // a smaller frontier corner owns it
-            destroyed++;
+            if ((sy == 2 && yw.x < xv) || (sw == 2 && yw.y < xv)) continue;   // a smaller frontier corner owns it
+            mine++;
             if (sy == 1) atomicSub(&tri[yw.x], 1u);
             if (sw == 1) atomicSub(&tri[yw.y], 1u);
         }
-        if (sg.count) {   // per-graph count of destroyed triangles
-            const unsigned long long t = warp_sum_u64(destroyed - d0);
-            if (lane == 0 && t) atomicAdd(&sg.destroyed[seg], t);
+        destroyed += mine;
+        if (sg.count) {   // per-graph count of destroyed triangles, lanes of one graph combined
+            if (mine) atomicAdd(&s_des[w][owner], mine);
+            __syncwarp();
+            const uint32_t d = s_des[w][lane];
+            const uint32_t peers = __match_any_sync(GA_FULL_MASK, d ? seg : GA_EMPTY);
+            const uint32_t sum = __reduce_add_sync(peers, d);
+            if (d && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&sg.destroyed[seg], (unsigned long long)sum);
         }
+        __syncwarp();
     }
     destroyed = warp_sum_u64(destroyed);
     if (lane == 0) s_red[w] = destroyed;
@@ -1004,22 +1046,11 @@ static int small_round_cluster(int device) {
     return best > 0 ? best : 0;
 }
 
-// Per graph: T0 = (sum of its vertices' triangle counts) / 3. One block per graph.
-__global__ void k_seg_T(const uint32_t* __restrict__ tri, Segs sg) {
-    __shared__ unsigned long long s_w[8];
-    for (uint32_t s = blockIdx.x; s < sg.count; s += gridDim.x) {
-        unsigned long long acc = 0;
-        for (unsigned long long v = sg.off[s] + threadIdx.x; v < sg.off[s + 1]; v += blockDim.x) acc += tri[v];
-        acc = warp_sum_u64(acc);
-        if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_w[w];
-            sg.T0[s] = t / 3;
-        }
-        __syncthreads();
-    }
+// Per graph: T0 = (sum of its vertices' triangle counts) / 3, from the ends of its incidence lists when they exist
+// (sums = inc_ptr), else from the prefix sums of tri[].
+__global__ void k_seg_T(const unsigned long long* __restrict__ sums, Segs sg) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < sg.count; s += gridDim.x * blockDim.x)
+        sg.T0[s] = (sums[sg.off[s + 1]] - sums[sg.off[s]]) / 3;
 }
 
 // Per graph: the state a lone batch_peel_loop starts from (densest.h:284-297): peel_arith_ok refusal, alive = n,
@@ -1078,8 +1109,10 @@ static ga_status ensure_loops(ga_graph* g) {
     // fixed launch shapes (the graph body is captured once): grid-stride scans, persistent update grid
     int occ = 0;
     GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_frontier_update, kUpdWarps * 32, 0));
-    L->grid_scan = (unsigned)g->sm_count * 4;
+    L->grid_scan = (unsigned)g->sm_count * 8;
     L->grid_update = (unsigned)g->sm_count * (unsigned)std::max(occ, 1);
+    GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_frontier_update_list, 256, 0));
+    L->grid_list = (unsigned)g->sm_count * (unsigned)std::max(occ, 1);
     return GA_OK;
 }
 
@@ -1120,6 +1153,8 @@ void reset_loops(ga_graph* g) {
     destroy_loops(g);
 }
 
+static ga_status segment_counts(ga_graph* g);
+
 __global__ void k_widen_counts(const uint32_t* __restrict__ tri, unsigned long long* __restrict__ out, uint32_t n) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
         out[v] = v < n ? tri[v] : 0ull;
@@ -1130,6 +1165,23 @@ __global__ void k_list_lengths(const unsigned long long* __restrict__ inc_ptr, u
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
         tri[v] = (uint32_t)(inc_ptr[v + 1] - inc_ptr[v]);
     if (blockIdx.x == 0 && threadIdx.x == 0) *total = inc_ptr[n] / 3;
+}
+
+// T0 of every graph of a batch (tri[] holds the per-vertex counts).
+static ga_status segment_counts(ga_graph* g) {
+    ga_loops* L = g->loops;
+    cudaStream_t st = g->stream;
+    unsigned long long* sums = nullptr;
+    if (L->lists != 1) {
+        GA_CUDA(pool_malloc((void**)&sums, ((size_t)g->n + 1) * 8, st));
+        k_widen_counts<<<grid_for((uint64_t)g->n + 1, 256), 256, 0, st>>>(L->tri, sums, g->n);
+        GA_CUDA(cudaGetLastError());
+        GA_TRY(scan_u64(g, sums, (uint64_t)g->n + 1));
+    }
+    k_seg_T<<<grid_for(L->segs.count, 256), 256, 0, st>>>(sums ? sums : L->inc_ptr, L->segs);
+    GA_CUDA(cudaGetLastError());
+    if (sums) cudaFreeAsync(sums, st);
+    return GA_OK;
 }
 
 // Decides the update method once per graph. With GA_OPT_UPDATE_MODE 0 (auto) or 2, the incidence lists are built
@@ -1199,7 +1251,7 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
     const unsigned long long* inc_ptr = L->lists == 1 ? L->inc_ptr : nullptr;
     const Segs sg = KIND == LOOP_PEEL ? L->segs : Segs{};
     if (KIND == LOOP_PEEL) {
-        k_peel_mark<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
+        k_peel_mark<<<L->grid_scan, kMarkThreads, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
                                                   L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->deg,
                                                   inc_ptr, sg);
     } else {
@@ -1224,13 +1276,13 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
         }
         k_core_min<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->alive[0], L->alive[1], L->state, L->frontier[0],
                                                  L->frontier[1], h, use_h);
-        k_core_mark<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
+        k_core_mark<<<L->grid_scan, kMarkThreads, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
                                                   L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->deg,
                                                   inc_ptr);
     }
     // the update kernel's last block closes the round and sets the loop condition
     if (L->lists == 1)
-        k_frontier_update_list<<<L->grid_update, 256, 0, st>>>(L->sc, L->inc, L->inc_ptr, L->item_x, L->item_c,
+        k_frontier_update_list<<<L->grid_list, 256, 0, st>>>(L->sc, L->inc, L->inc_ptr, L->item_x, L->item_c,
                                                                L->state, L->tri, sg, KIND, h, use_h);
     else
         k_frontier_update<<<L->grid_update, kUpdWarps * 32, 0, st>>>(L->sc, g->rowptr, g->col, g->deg, tc_index(g),
@@ -1311,7 +1363,7 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     const bool seg = KIND == LOOP_PEEL && L->segs.count > 0;
     if (seg) {
         // a batch: every graph is checked on its own (peel_arith_ok with its own n and T0)
-        k_seg_T<<<std::min<uint32_t>(L->segs.count, 148u * 16u), 256, 0, st>>>(L->tri, L->segs);
+        GA_TRY(segment_counts(g));
         k_seg_init<<<grid_for(L->segs.count, 256), 256, 0, st>>>(L->segs, num, den);
         GA_CUDA(cudaGetLastError());
     } else if (T0 >= (1ull << 32)) {
@@ -1428,8 +1480,7 @@ ga_status count_segments(ga_graph* g, uint64_t* triangles) {
     a.total = g->d_scalars;
     a.vsup = L->tri;
     GA_TRY((run_tc<TC_VSUP, false, unsigned int>(g, a, true)));
-    k_seg_T<<<std::min<uint32_t>(L->segs.count, 148u * 16u), 256, 0, st>>>(L->tri, L->segs);
-    GA_CUDA(cudaGetLastError());
+    GA_TRY(segment_counts(g));
     GA_CUDA(cudaMemcpyAsync(triangles, L->segs.T0, (size_t)L->segs.count * 8, cudaMemcpyDeviceToHost, st));
     GA_CUDA(cudaStreamSynchronize(st));
     return GA_OK;

@@ -69,7 +69,7 @@ uint64_t estimate_bytes(const GraphEntry& e, ga_request_kind kind) {
     b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (n + (2 * e.tri_bound + 8 * m) / 1024 + 1) + 1024;
     if (kind != GA_REQ_TC) {
         const uint64_t T = e.triangles != UINT64_MAX ? e.triangles : e.tri_bound;
-        b += 29 * n + 8 * (n + 3 * T / 1024 + 1) + 24 * T + 8 * (n + 1);
+        b += 29 * n + 8 * (n + 3 * T / 512 + 1) + 24 * T + 8 * (n + 1);
     }
     return b;
 }
