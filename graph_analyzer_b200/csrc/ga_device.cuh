@@ -101,6 +101,14 @@ struct ga_items {
     uint64_t capacity = 0, bound = 0;   // entries allocated; at least the number of items
 };
 
+// Counters of a handle's triangle passes (device): work queues, the blocks that have finished, the triangles so far. All
+// zero between passes (the last block of a pass clears them). bounds: the item ranges of a shard.
+struct ga_sync {
+    uint32_t queue[4], ticket, pad;
+    unsigned long long acc;
+    uint32_t bounds[6];
+};
+
 struct ga_graph {
     int device = 0;
     int sm_count = 148;
@@ -141,8 +149,8 @@ struct ga_graph {
 
     // small device / pinned host scalars
     unsigned long long* d_scalars = nullptr;   // 64 slots
-    unsigned long long h_scalars[64] = {};     // host copies of small results
-    uint32_t* d_queue = nullptr;               // 8 work-queue counters
+    unsigned long long* h_scalars = nullptr;   // their page-locked host side (64 slots; host_slot_acquire)
+    ga_sync* sync = nullptr;                   // counters of the triangle passes
 
     // options (ga_option)
     int64_t opt_tc_kernel = 0, opt_loop_mode = 0, opt_max_rounds = 0, opt_update_mode = 0, opt_count_bitmap = 0;
@@ -168,6 +176,11 @@ namespace ga {
 // that graphs created and destroyed repeatedly reuse memory instead of returning it to the driver. A pool of its own
 // leaves the device's default pool (which other code in the process may use) as it was.
 ga_status init_pool(int device);
+
+// 512 page-locked bytes every device can write, for the small results of one handle: from slabs the process keeps (at
+// most 64 KB of them: 128 handles; further handles allocate their own), handed back at destroy. nullptr: out of memory.
+unsigned long long* host_slot_acquire();
+void host_slot_release(unsigned long long* slot);
 
 // The pool of the current device (init_pool must have run for it; every entry point that allocates calls it).
 cudaMemPool_t pool_of_current();

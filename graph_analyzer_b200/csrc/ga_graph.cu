@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "ga_device.cuh"
 
@@ -628,6 +629,43 @@ void pool_keep_release(int device) {
     cudaMemPoolTrimTo(g_pools[device], keep);
 }
 
+// Slots of one 64 KB slab (allocated with the first handle) in a free list; beyond it every handle has its own block.
+static std::mutex g_slot_mu;
+static std::vector<unsigned long long*> g_slots_free;
+static unsigned long long* g_slab = nullptr;
+constexpr size_t kSlotWords = 64, kSlabSlots = 128;
+
+unsigned long long* host_slot_acquire() {
+    std::lock_guard<std::mutex> lock(g_slot_mu);
+    if (!g_slab) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kSlabSlots * kSlotWords * 8, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            g_slab = (unsigned long long*)p;
+            for (size_t i = kSlabSlots; i > 0; i--) g_slots_free.push_back(g_slab + (i - 1) * kSlotWords);
+        } else {
+            (void)cudaGetLastError();
+        }
+    }
+    if (!g_slots_free.empty()) {
+        unsigned long long* s = g_slots_free.back();
+        g_slots_free.pop_back();
+        return s;
+    }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kSlotWords * 8, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return (unsigned long long*)p;
+}
+
+void host_slot_release(unsigned long long* s) {
+    if (!s) return;
+    std::lock_guard<std::mutex> lock(g_slot_mu);
+    if (g_slab && s >= g_slab && s < g_slab + kSlabSlots * kSlotWords) g_slots_free.push_back(s);
+    else cudaFreeHost(s);
+}
+
 cudaMemPool_t pool_of_current() {
     int device = 0;
     cudaGetDevice(&device);
@@ -808,7 +846,9 @@ static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint
     if (cudaMemsetAsync(g->col + m, 0, 16, g->stream) != cudaSuccess)
         return bail(fail(GA_ERR_CUDA, "cudaMemsetAsync failed"));
     if ((s = dalloc(g, &g->d_scalars, 64)) != GA_OK) return bail(s);
-    if ((s = dalloc(g, &g->d_queue, 16)) != GA_OK) return bail(s);
+    if ((s = dalloc(g, &g->sync, 1)) != GA_OK) return bail(s);
+    if (!(g->h_scalars = host_slot_acquire())) return bail(fail(GA_ERR_OUT_OF_MEMORY, "page-locked slot failed"));
+    cudaMemsetAsync(g->sync, 0, sizeof(ga_sync), g->stream);
     const cudaMemcpyKind kind = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (cudaMemcpyAsync(g->rowptr, rowptr, ((size_t)n + 1) * 4, kind, g->stream) != cudaSuccess ||
         (m && cudaMemcpyAsync(g->col, col, (size_t)m * 4, kind, g->stream) != cudaSuccess))
@@ -904,6 +944,7 @@ ga_status ga_graph_destroy(ga_graph* g) {
     for (auto& a : g->allocations) cudaFreeAsync(a.first, g->stream);
     if (g->stream) cudaStreamSynchronize(g->stream);
     if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
+    host_slot_release(g->h_scalars);
     delete g;
     return GA_OK;
 }

@@ -107,7 +107,7 @@ struct ga_loops {
     uint32_t* item_c = nullptr;
     uint64_t item_cap = 0;
     ga::LoopScalars* sc = nullptr;    // device
-    ga::LoopScalars h_sc = {};         // host copy of the round state
+    uint64_t list_T = 0;              // triangles in the incidence lists, once built
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     cudaGraph_t graph[2] = {nullptr, nullptr};
     unsigned grid_scan = 1, grid_update = 1, grid_list = 1;
@@ -125,28 +125,33 @@ struct ga_loops {
 
 namespace ga {
 
-__global__ void k_loop_init(uint8_t* __restrict__ state, uint32_t* __restrict__ out, uint32_t* __restrict__ alive0,
-                            uint32_t* __restrict__ loc, uint32_t n) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+// The state a loop starts from, in one pass: every vertex alive, its triangle count (the length of its incidence list
+// when the lists exist), and the scalars (total: T, or null for the ends of the lists).
+__global__ void __launch_bounds__(256) k_loop_init(uint8_t* __restrict__ state, uint32_t* __restrict__ out,
+                                                   uint32_t* __restrict__ alive0, uint32_t* __restrict__ loc,
+                                                   const unsigned long long* __restrict__ inc_ptr,
+                                                   uint32_t* __restrict__ tri, const unsigned long long* total,
+                                                   LoopScalars* sc, uint32_t n, unsigned long long num,
+                                                   unsigned long long den, uint32_t max_rounds) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
         state[v] = 1;
         out[v] = 0xFFFFFFFFu;
-        alive0[v] = v;
+        alive0[v] = (uint32_t)v;
         if (loc) loc[v] = GA_EMPTY;
+        if (inc_ptr) tri[v] = (uint32_t)(inc_ptr[v + 1] - inc_ptr[v]);
     }
-}
-
-__global__ void k_loop_scalars(LoopScalars* sc, const unsigned long long* total, uint32_t n, unsigned long long num,
-                               unsigned long long den, uint32_t max_rounds) {
-    LoopScalars s = {};
-    s.T = *total;
-    s.nalive = n;
-    s.num = num;
-    s.den = den;
-    s.max_rounds = max_rounds;
-    s.alive_count[0] = n;
-    s.min_tri = 0xFFFFFFFFu;
-    s.cont = n > 0;
-    *sc = s;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        LoopScalars s = {};
+        s.T = inc_ptr ? inc_ptr[n] / 3 : *total;
+        s.nalive = n;
+        s.num = num;
+        s.den = den;
+        s.max_rounds = max_rounds;
+        s.alive_count[0] = n;
+        s.min_tri = 0xFFFFFFFFu;
+        s.cont = n > 0;
+        *sc = s;
+    }
 }
 
 constexpr int kMarkThreads = 256;
@@ -1160,13 +1165,6 @@ __global__ void k_widen_counts(const uint32_t* __restrict__ tri, unsigned long l
         out[v] = v < n ? tri[v] : 0ull;
 }
 
-__global__ void k_list_lengths(const unsigned long long* __restrict__ inc_ptr, uint32_t* __restrict__ tri,
-                               uint32_t n, unsigned long long* total) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        tri[v] = (uint32_t)(inc_ptr[v + 1] - inc_ptr[v]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *total = inc_ptr[n] / 3;
-}
-
 // T0 of every graph of a batch (tri[] holds the per-vertex counts).
 static ga_status segment_counts(ga_graph* g) {
     ga_loops* L = g->loops;
@@ -1241,6 +1239,7 @@ static ga_status build_lists(ga_graph* g, uint64_t T0) {
     GA_CUDA(cudaStreamSynchronize(st));
     if (overflow) return fail(GA_ERR_DEVICE_CHECK, "triangle listing disagreed with the count (%u entries)", overflow);
     L->lists = 1;
+    L->list_T = T0;
     return GA_OK;
 }
 
@@ -1342,24 +1341,17 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     const uint32_t n = g->n;
     if (KIND == LOOP_CORE && !L->loc) GA_TRY(dalloc(g, &L->loc, n));
     // tri[] = triangles per vertex on the whole graph (uint32 counters; T < 2^32 is checked below): the list lengths
-    // when the incidence lists exist, else one per-vertex triangle pass
-    if (L->lists == 1) {
-        if (n) k_list_lengths<<<grid_for(n, 256), 256, 0, st>>>(L->inc_ptr, L->tri, n, g->d_scalars);
-        GA_CUDA(cudaGetLastError());
-    } else {
+    // when the incidence lists exist (whose size is T's), else one per-vertex triangle pass
+    uint64_t T0 = L->list_T;
+    if (L->lists != 1) {
         TcArgs<unsigned int> a{};
         a.total = g->d_scalars;
+        a.host_total = g->h_scalars;
         a.vsup = L->tri;
         GA_TRY((run_tc<TC_VSUP, false, unsigned int>(g, a, true)));
+        GA_CUDA(cudaStreamSynchronize(st));
+        T0 = g->h_scalars[0];
     }
-    if (n) {
-        k_loop_init<<<grid_for(n, 256), 256, 0, st>>>(L->state, L->out, L->alive[0],
-                                                      KIND == LOOP_CORE ? L->loc : nullptr, n);
-        GA_CUDA(cudaGetLastError());
-    }
-    GA_CUDA(cudaMemcpyAsync(g->h_scalars, g->d_scalars, 8, cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaStreamSynchronize(st));
-    const uint64_t T0 = g->h_scalars[0];
     const bool seg = KIND == LOOP_PEEL && L->segs.count > 0;
     if (seg) {
         // a batch: every graph is checked on its own (peel_arith_ok with its own n and T0)
@@ -1379,8 +1371,13 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     GA_TRY(build_lists(g, T0));
     const uint64_t cap = g->opt_max_rounds ? (uint64_t)g->opt_max_rounds : (uint64_t)n + 1;
     const uint32_t max_rounds = (uint32_t)std::min<uint64_t>(cap, UINT32_MAX);
-    k_loop_scalars<<<1, 1, 0, st>>>(L->sc, g->d_scalars, n, num, den, max_rounds);
+    k_loop_init<<<grid_for(n, 256), 256, 0, st>>>(L->state, L->out, L->alive[0],
+                                                  KIND == LOOP_CORE ? L->loc : nullptr,
+                                                  L->lists == 1 ? L->inc_ptr : nullptr, L->tri, g->d_scalars, L->sc, n,
+                                                  num, den, max_rounds);
     GA_CUDA(cudaGetLastError());
+    LoopScalars* h_sc = reinterpret_cast<LoopScalars*>(g->h_scalars + 32);   // page-locked
+    static_assert(sizeof(LoopScalars) <= 32 * 8, "fits the second half of the handle's slot");
     if (n > 0) {
         const bool graph_mode = g->opt_loop_mode != 1;
         if (graph_mode) {
@@ -1389,16 +1386,16 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
         } else {
             for (uint64_t r = 0;; r++) {
                 GA_TRY(enqueue_round<KIND>(g, st, 0, 0));
-                GA_CUDA(cudaMemcpyAsync(&L->h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
+                GA_CUDA(cudaMemcpyAsync(h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
                 GA_CUDA(cudaStreamSynchronize(st));
-                if (!L->h_sc.cont) break;
+                if (!h_sc->cont) break;
                 if (r > (uint64_t)max_rounds + 1) return fail(GA_ERR_ROUND_LIMIT, "host loop bound reached");
             }
         }
     }
-    GA_CUDA(cudaMemcpyAsync(&L->h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
+    GA_CUDA(cudaMemcpyAsync(h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
     GA_CUDA(cudaStreamSynchronize(st));
-    *result = L->h_sc;
+    *result = *h_sc;
     switch (result->status) {
         case LS_OK: break;
         case LS_ROUND_LIMIT: return fail(GA_ERR_ROUND_LIMIT, "round cap %u reached", result->max_rounds);
@@ -1430,9 +1427,9 @@ ga_status incidence_lists(ga_graph* g, const uint2** inc, const unsigned long lo
         // per-vertex counts size the lists (the list build's input)
         TcArgs<unsigned int> a{};
         a.total = g->d_scalars;
+        a.host_total = g->h_scalars;
         a.vsup = L->tri;
         GA_TRY((run_tc<TC_VSUP, false, unsigned int>(g, a, true)));
-        GA_CUDA(cudaMemcpyAsync(g->h_scalars, g->d_scalars, 8, cudaMemcpyDeviceToHost, st));
         GA_CUDA(cudaStreamSynchronize(st));
         const uint64_t T0 = g->h_scalars[0];
         if (T0 >= (1ull << 32))

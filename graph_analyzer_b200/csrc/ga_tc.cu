@@ -39,6 +39,7 @@
 //          to col order after the pass.
 //   ALIVE: restricts everything to the subgraph induced by alive[] (tc_per_vertex_alive, kernels.cuh:399-425).
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -170,6 +171,29 @@ __device__ __forceinline__ uint32_t find_member(const TcArgs<CT>& a, const Ancho
     const uint32_t* row = a.ix.colr + (size_t)an.row * 8;
     const uint32_t j = lower_bound_u32(row, 0, an.dv, x);
     return j < an.dv && row[j] == x && (!ALIVE || a.alive[x]) ? j : GA_EMPTY;
+}
+
+// The end of a pass, called by all 256 threads of every block: the blocks' triangles meet in sync->acc, and the last
+// block writes the total where the caller wants it (device, and the handle's page-locked slot when the host waits for
+// it) and leaves the counters zero for the next pass - so a count is one launch, with nothing to clear before it and
+// nothing to copy after it (901 vertices: 20 us a call with two clears and a copy around the kernel).
+template <class CT>
+__device__ __forceinline__ void finish_pass(unsigned long long local, const TcArgs<CT>& a) {
+    __shared__ unsigned long long s_red[8];
+    local = warp_sum_u64(local);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    unsigned long long t = 0;
+    for (int w = 0; w < 8; w++) t += s_red[w];
+    if (t) atomicAdd(&a.sync->acc, t);
+    __threadfence();
+    if (atomicInc(&a.sync->ticket, gridDim.x - 1) != gridDim.x - 1) return;   // wraps to zero with the last block
+    __threadfence();
+    t = atomicExch(&a.sync->acc, 0ull);
+    for (int q = 0; q < 4; q++) a.sync->queue[q] = 0;   // every block is done with the queues
+    *a.total = t;
+    if (a.host_total) *a.host_total = t;
 }
 
 // The probe lists of a batch of up to 32 in-edges [kb, kend) (one warp): lane l takes the l-th in-edge's suffix of its
@@ -639,12 +663,11 @@ __global__ void k_alive_places(const uint8_t* __restrict__ alive, const uint32_t
 // places from tiny_first on; otherwise its items are run like light ones.
 template <int MODE, bool ALIVE, class CT>
 __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds,
-                                                      uint32_t heavy_bits_max, uint32_t* __restrict__ queue,
+                                                      uint32_t heavy_bits_max,
                                                       uint32_t tiny_first, uint32_t tiny_end, uint32_t light_max_deg,
                                                       TcArgs<CT> a) {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t s_item, s_next;
-    __shared__ unsigned long long s_red[kWarps];
     constexpr int W = SlotLayout<MODE>::words;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long hits = 0;
@@ -665,7 +688,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
         uint32_t *s_incl = wbase, *s_base = wbase + 32;
         wbase[64 + lane] = 0;   // ecnt
         for (;;) {
-            if (threadIdx.x == 0) s_item = h0 + atomicAdd(&queue[0], 1u);
+            if (threadIdx.x == 0) s_item = h0 + atomicAdd(&a.sync->queue[0], 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= h1) break;
@@ -730,7 +753,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
     const uint32_t nl = l1 - l0, total = nl + (groups ? 0u : t1 - t0);
     for (;;) {
         uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(&queue[1], 1u);
+        if (lane == 0) i = atomicAdd(&a.sync->queue[1], 1u);
         i = __shfl_sync(GA_FULL_MASK, i, 0);
         if (i >= total) break;
         const uint32_t item = i < nl ? l0 + i : t0 + (i - nl);
@@ -768,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
             const uint32_t ngroups = (uint32_t)(((uint64_t)tiny_end - tiny_first + 31) / 32);
             for (;;) {
                 uint32_t g0 = 0;
-                if (lane == 0) g0 = atomicAdd(&queue[2], kTinyGroups);
+                if (lane == 0) g0 = atomicAdd(&a.sync->queue[2], kTinyGroups);
                 g0 = __shfl_sync(GA_FULL_MASK, g0, 0);
                 if (g0 >= ngroups) break;
                 const uint32_t g1 = min(g0 + kTinyGroups, ngroups);
@@ -778,28 +801,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
             }
         }
     }
-    // ---- one 64-bit atomic per block ----
-    hits = warp_sum_u64(hits);
-    if (lane == 0) s_red[warp] = hits;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int w = 0; w < kWarps; w++) t += s_red[w];
-        if (t) atomicAdd(a.total, t);
-    }
-}
-
-// One atomic per block of 256 threads (all of them call it).
-__device__ __forceinline__ void add_total(unsigned long long local, unsigned long long* total) {
-    __shared__ unsigned long long s_red[8];
-    local = warp_sum_u64(local);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int w = 0; w < 8; w++) t += s_red[w];
-        if (t) atomicAdd(total, t);
-    }
+    finish_pass(hits, a);
 }
 
 // The one-thread-per-edge form on the index: thread k takes in-edge k, whose record names its suffix and, one entry
@@ -840,7 +842,7 @@ __global__ void __launch_bounds__(256) k_tc_octs(uint32_t m, TcArgs<CT> a) {
             if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[a.ix.order[v]], (CT)sum);
         }
     }
-    add_total(local, a.total);
+    finish_pass(local, a);
 }
 
 // Plain form (GA_OPT_TC_KERNEL = 1): one thread per oriented edge, two-pointer merge of N+(u) and N+(v), one
@@ -880,7 +882,7 @@ __global__ void __launch_bounds__(256) k_tc_plain(const uint32_t* __restrict__ r
             }
         }
     }
-    add_total(local, a.total);
+    finish_pass(local, a);
 }
 
 // ---- host launchers ---------------------------------------------------------------------------------------------
@@ -940,21 +942,38 @@ __global__ void k_shard_bounds(const unsigned long long* __restrict__ anchor_wor
     out[t] = lo;
 }
 
+// Blocks of a kernel resident per SM. The driver's answer for a shared-memory size does not change, so the last one is
+// kept per kernel and device (`memo`: size << 8 | blocks) instead of asking before every launch; the kernel's limit is
+// raised once to all it may use, never to one launch's size, which another thread's launch could exceed.
+static ga_status resident_blocks(const void* kern, int threads, size_t smem, std::atomic<uint64_t>& memo, int* occ) {
+    const uint64_t seen = memo.load(std::memory_order_relaxed);
+    if (seen && seen >> 8 == smem) {
+        *occ = (int)(seen & 0xFF);
+        return GA_OK;
+    }
+    if (smem > 40 * 1024)
+        GA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+    int o = 0;
+    GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, threads, smem));
+    *occ = std::max(o, 1);
+    memo.store((uint64_t)smem << 8 | (uint64_t)*occ, std::memory_order_relaxed);
+    return GA_OK;
+}
+
 template <int MODE, bool ALIVE, class CT>
 static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
     cudaStream_t st = g->stream;
     const uint32_t hb = heavy_bits_for(g, MODE);
     const size_t smem = hash_smem_bytes<MODE>(hb);
     auto kern = k_tc_hash<MODE, ALIVE, CT>;
-    GA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0;
-    GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
-    occ = std::max(occ, 1);
+    static std::atomic<uint64_t> memo[64];
+    int occ = 1;
+    GA_TRY(resident_blocks((const void*)kern, kThreads, smem, memo[g->device], &occ));
     const uint32_t* bounds = nullptr;
     uint64_t want = (g->items.bound + kWarps - 1) / kWarps;
     uint32_t tiny_first = g->isolated, tiny_end = g->n;
-    if (a.nshards > 1) {   // this shard's anchors (cut on the device; the queue counters sit in d_queue[0..3])
-        uint32_t* b = g->d_queue + 8;
+    if (a.nshards > 1) {   // this shard's anchors (cut on the device)
+        uint32_t* b = g->sync->bounds;
         k_shard_bounds<<<1, 32, 0, st>>>(g->anchor_work, g->n, g->items, a.shard, a.nshards, b);
         GA_CUDA(cudaGetLastError());
         bounds = b;
@@ -963,8 +982,7 @@ static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
     }
     want = std::max<uint64_t>(want, (uint64_t)g->max_out_degree > g->light_max_deg ? (uint64_t)g->sm_count * occ : 1);
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g->sm_count * occ, want));
-    GA_CUDA(cudaMemsetAsync(g->d_queue, 0, 4 * sizeof(uint32_t), st));
-    kern<<<grid, kThreads, smem, st>>>(g->items, bounds, hb, g->d_queue, tiny_first, tiny_end, g->light_max_deg, a);
+    kern<<<grid, kThreads, smem, st>>>(g->items, bounds, hb, tiny_first, tiny_end, g->light_max_deg, a);
     GA_CUDA(cudaGetLastError());
     return GA_OK;
 }
@@ -1009,23 +1027,23 @@ static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
 
 template <int MODE, bool ALIVE, class CT>
 static ga_status launch_plain(ga_graph* g, const TcArgs<CT>& a) {
-    if (!g->m) return GA_OK;
-    int occ = 0;
-    GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tc_plain<MODE, ALIVE, CT>, 256, 0));
+    static std::atomic<uint64_t> memo[64];
+    int occ = 1;
+    GA_TRY(resident_blocks((const void*)k_tc_plain<MODE, ALIVE, CT>, 256, 0, memo[g->device], &occ));
     uint32_t e0 = 0, e1 = g->m;
     if (a.nshards > 1) {   // this shard's equal part of the edges
         e0 = (uint32_t)((uint64_t)g->m * a.shard / a.nshards);
         e1 = (uint32_t)((uint64_t)g->m * (a.shard + 1) / a.nshards);
     }
-    if (e1 <= e0) return GA_OK;
-    const unsigned grid = grid_for(e1 - e0, 256, (unsigned)g->sm_count * std::max(occ, 1) * 4);
+    // an empty shard still runs one block, which writes the total
+    const unsigned grid = grid_for(e1 > e0 ? e1 - e0 : 1, 256, (unsigned)g->sm_count * occ * 4);
     k_tc_plain<MODE, ALIVE, CT><<<grid, 256, 0, g->stream>>>(g->rowptr, g->col, g->src, e0, e1, a);
     GA_CUDA(cudaGetLastError());
     return GA_OK;
 }
 
 template <int MODE, bool ALIVE, class CT>
-ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
+ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
     // Automatic choice: the autotuned kernel for counts. Supports take the one-thread-per-edge form too when it counts
     // faster and rows are short (row_work / m, the octs of an edge's row on average, at most 2.5: Holme-Kim graphs have
     // 1 to 2.1; edge supports of the 1.7M one take 400 us against 2,010 us, vertex supports of a 200,003-vertex one 380
@@ -1034,6 +1052,8 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
     // kernel (Holme-Kim 1.7M: 154 ms plain vs 4 ms hash).
     // A sharded count always uses the hash kernel unless one is forced: every GPU must cut the same partition, and
     // an autotuned choice could differ between GPUs.
+    TcArgs<CT> a = a0;
+    a.sync = g->sync;
     GA_TRY(a.nshards > 1 ? prepare_shards(g) : prepare(g));
     int64_t kernel = g->opt_tc_kernel ? g->opt_tc_kernel
                                       : (MODE == TC_COUNT || (MODE != TC_LIST && g->row_work * 2 <= 5ull * g->m)) &&
@@ -1047,11 +1067,14 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs) {
     const bool index = (kernel != 1 || octs) && g->m;
     cudaStream_t st = g->stream;
     if (zero_outputs) {   // on the index, edge supports are written whole from the kernels' own array
-        GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
         if (MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
         if (!index && MODE == TC_ESUP && g->m) GA_CUDA(cudaMemsetAsync(a.esup, 0, (size_t)g->m * sizeof(uint32_t), st));
     }
-    if (!g->m) return GA_OK;
+    if (!g->m) {   // no kernel: the total is zero
+        GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
+        if (a.host_total) *a.host_total = 0;
+        return GA_OK;
+    }
     return index ? launch_index<MODE, ALIVE, CT>(g, a, octs) : launch_plain<MODE, ALIVE, CT>(g, a);
 }
 
@@ -1263,8 +1286,8 @@ __global__ void k_core_mask(const uint32_t* __restrict__ core, uint32_t n, uint3
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(cnt, (unsigned long long)c);
 }
 
-ga_status read_total(ga_graph* g, const unsigned long long* d_total, uint64_t* out) {
-    GA_CUDA(cudaMemcpyAsync(g->h_scalars, d_total, 8, cudaMemcpyDeviceToHost, g->stream));
+// Waits for the stream; the pass (whose host_total is the handle's slot) has left its total there.
+ga_status read_total(ga_graph* g, uint64_t* out) {
     GA_CUDA(cudaStreamSynchronize(g->stream));
     if (out) *out = g->h_scalars[0];
     return GA_OK;
@@ -1281,8 +1304,9 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles) {
     GA_TRY(ready(g));
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     GA_TRY((run_tc<TC_COUNT, false, unsigned int>(g, a, true)));
-    return read_total(g, a.total, triangles);
+    return read_total(g, triangles);
 }
 
 ga_status ga_tc_count_shard(ga_graph* g, uint32_t shard, uint32_t nshards, uint64_t* partial) {
@@ -1293,10 +1317,11 @@ ga_status ga_tc_count_shard(ga_graph* g, uint32_t shard, uint32_t nshards, uint6
     GA_TRY(ready(g));
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     a.shard = shard;
     a.nshards = nshards;
     GA_TRY((run_tc<TC_COUNT, false, unsigned int>(g, a, true)));
-    return read_total(g, a.total, partial);
+    return read_total(g, partial);
 }
 
 ga_status ga_tc_count_shard_async(ga_graph* g, uint32_t shard, uint32_t nshards, uint64_t* d_partial) {
@@ -1327,9 +1352,10 @@ ga_status ga_tc_support_edges_device(ga_graph* g, uint32_t* d_sup, uint64_t* tri
     GA_TRY(ready(g));
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     a.esup = d_sup;
     GA_TRY((run_tc<TC_ESUP, false, unsigned int>(g, a, true)));
-    return read_total(g, a.total, triangles);
+    return read_total(g, triangles);
 }
 
 ga_status ga_tc_support_edges(ga_graph* g, uint32_t* sup, uint64_t* triangles) {
@@ -1355,21 +1381,26 @@ ga_status ga_tc_support_vertices(ga_graph* g, uint64_t* deg, uint64_t* triangles
     GA_CUDA(pool_malloc(&s.p, ((size_t)g->n + 1) * 8, g->stream));
     TcArgs<unsigned long long> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     a.vsup = (unsigned long long*)s.p;
     GA_TRY((run_tc<TC_VSUP, false, unsigned long long>(g, a, true)));
     if (g->n) GA_CUDA(cudaMemcpyAsync(deg, s.p, (size_t)g->n * 8, cudaMemcpyDeviceToHost, g->stream));
-    return read_total(g, a.total, triangles);
+    return read_total(g, triangles);
 }
 
 ga_status ga_tc_participation(ga_graph* g, const uint8_t* alive, uint32_t* tri, uint64_t* triangles) {
     if (!g || ((!alive || !tri) && g->n)) return fail(GA_ERR_INVALID_ARGUMENT, "null argument");
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
-    // T of the alive subgraph is at most T of the graph; refuse when uint32 counters could overflow (densest.h:68)
-    uint64_t T_full = 0;
-    GA_TRY(ga_tc_count(g, &T_full));
-    if (T_full >= (1ull << 32))
-        return fail(GA_ERR_ARITH, "triangle count >= 2^32: uint32 tri[] counters could overflow");
+    GA_TRY(ready(g));
+    // T of the alive subgraph is at most T of the graph; refuse when uint32 counters could overflow (densest.h:68). T is
+    // at most sum over u of C(d+(u), 2), and that at most 4 * row_work: only above 2^32 does it take a count to know
+    if (g->row_work >= (1ull << 30)) {
+        uint64_t T_full = 0;
+        GA_TRY(ga_tc_count(g, &T_full));
+        if (T_full >= (1ull << 32))
+            return fail(GA_ERR_ARITH, "triangle count >= 2^32: uint32 tri[] counters could overflow");
+    }
     Scratch s;
     s.st = g->stream;
     GA_CUDA(pool_malloc(&s.p, ((size_t)g->n + 1) * 5, g->stream));
@@ -1378,11 +1409,12 @@ ga_status ga_tc_participation(ga_graph* g, const uint8_t* alive, uint32_t* tri, 
     if (g->n) GA_CUDA(cudaMemcpyAsync(d_alive, alive, g->n, cudaMemcpyHostToDevice, g->stream));
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     a.vsup = d_tri;
     a.alive = d_alive;
     GA_TRY((run_tc<TC_VSUP, true, unsigned int>(g, a, true)));
     if (g->n) GA_CUDA(cudaMemcpyAsync(tri, d_tri, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
-    return read_total(g, a.total, triangles);
+    return read_total(g, triangles);
 }
 
 ga_status ga_graph_tuning(ga_graph* g, ga_tuning* out) {
@@ -1427,9 +1459,10 @@ ga_status ga_core_level_density(ga_graph* g, const uint32_t* core, uint32_t k, u
     }
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
+    a.host_total = g->h_scalars;
     a.alive = d_alive;
     GA_TRY((run_tc<TC_COUNT, true, unsigned int>(g, a, true)));
-    GA_CUDA(cudaMemcpyAsync(g->h_scalars, g->d_scalars, 16, cudaMemcpyDeviceToHost, g->stream));
+    GA_CUDA(cudaMemcpyAsync(g->h_scalars + 1, g->d_scalars + 1, 8, cudaMemcpyDeviceToHost, g->stream));
     GA_CUDA(cudaStreamSynchronize(g->stream));
     *triangles = g->h_scalars[0];
     *vertices = g->h_scalars[1];

@@ -26,6 +26,7 @@ inline TcIndex tc_index(const ga_graph* g) {
 template <class CT>
 struct TcArgs {
     unsigned long long* total = nullptr;
+    unsigned long long* host_total = nullptr;   // page-locked slot that receives T as well (optional)
     CT* vsup = nullptr;
     uint32_t* esup = nullptr;
     const uint8_t* alive = nullptr;
@@ -33,8 +34,9 @@ struct TcArgs {
     const unsigned long long* inc_ptr = nullptr;
     uint32_t* fill = nullptr;
     uint32_t* overflow = nullptr;   // TC_LIST: entries that found their list full (must stay 0)
-    // set by the launcher of the kernels on the index (whose alive is by place)
+    // set by the launchers (alive is by place for the kernels on the index)
     TcIndex ix = {};
+    ga_sync* sync = nullptr;        // the handle's counters
     uint32_t* esupk = nullptr;      // ESUP: supports by padded position in colr, zeroed
     bool bitmaps = false;           // heavy anchors may use bitmaps
     // shard `shard` of `nshards` (0 = the whole graph): equal parts of the probe work (hash kernel) or of the edges
@@ -42,7 +44,7 @@ struct TcArgs {
     uint32_t shard = 0, nshards = 0;
 };
 
-// One triangle pass on g's stream (asynchronous). zero_outputs: clear total/vsup/esup first.
+// One triangle pass on g's stream (asynchronous). total is written whole; zero_outputs: clear vsup/esup first.
 template <int MODE, bool ALIVE, class CT>
 ga_status run_tc(ga_graph* g, const TcArgs<CT>& a, bool zero_outputs);
 
