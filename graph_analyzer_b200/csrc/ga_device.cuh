@@ -142,6 +142,7 @@ struct ga_graph {
     ga_items items;               // work lists of the triangle kernels
     bool index_ready = false;     // vrank .. in_rng built
     bool prepared = false;        // ... and the work items for the current light_max_deg / item_work
+    bool counted_bare = false;    // counted once without the index (ga_tc_count)
     ga_loops* loops = nullptr;    // peeling / core loop state, allocated on first use
     // a batch: the graph is the disjoint union of seg_count graphs, graph s owning vertices [seg_off[s], seg_off[s+1])
     const unsigned long long* seg_off = nullptr;

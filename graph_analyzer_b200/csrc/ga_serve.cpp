@@ -136,10 +136,9 @@ void plan(const ga_server* s, const Request& r, const GraphEntry& e, uint64_t* n
     // lists (run_single grows the reservation or puts the request back at the head of the queue).
     const bool staged = r.kind != GA_REQ_TC && e.triangles == UINT64_MAX && !*small;
     *full = estimate_bytes(e, staged ? GA_REQ_TC : r.kind);
-    // bytes to reserve: the whole estimate for an upload; for a resident graph only what a loop may still add
-    *need = 0;
-    if (!e.dev) *need = *full;
-    else if (r.kind != GA_REQ_TC) *need = *full > e.dev_bytes ? *full - e.dev_bytes : 0;
+    // bytes to reserve: the whole estimate for an upload; for a resident graph what it may still add (a loop its state
+    // and lists, a second count the index that the first did without)
+    *need = e.dev ? (*full > e.dev_bytes ? *full - e.dev_bytes : 0) : *full;
 }
 
 // Rough device work of a request, for ordering the general lane: edges times a factor per kind, plus the upload.

@@ -278,3 +278,51 @@ def test_autotuner_choices(ga, oracle, cuda_ok):
             assert d.tc_count() == want
             t3 = d.tuning()
             assert (t3["light_max_deg"], t3["item_work"]) == (64, 2048)
+
+
+def test_first_count_without_index(ga, oracle, cuda_ok):
+    """The first count of an unprepared graph in the one-thread-per-edge form needs no index, the next ones build it:
+    the same count either way, and a misoriented CSR is refused by both."""
+    for n in (1, 2, 33, 900, 20_000):
+        g = ga.graph_from_pairs(n, ga.gen_holme_kim(n, 3, 5, 0.5, 0.6, seed=n) if n > 5 else np.zeros((0, 2), np.uint32))
+        T = oracle.triangles_serial(g)
+        with ga.DeviceGraph(g) as d:
+            d.set_option(ga.OPT_TC_KERNEL, 1)
+            b0 = d.device_bytes()
+            assert d.tc_count() == T
+            assert g.m == 0 or d.device_bytes() == b0              # (without edges nothing is saved: the general path)
+            assert d.tc_count() == T and d.tc_count() == T
+            assert g.m == 0 or d.device_bytes() > b0
+    bad = ga.Graph(3, 3, np.array([0, 1, 2, 3], np.uint32), np.array([1, 2, 0], np.uint32),
+                   np.array([0, 1, 2], np.uint32), 1)              # a directed cycle
+    with ga.DeviceGraph(bad) as d:
+        d.set_option(ga.OPT_TC_KERNEL, 1)
+        for _ in range(2):
+            with pytest.raises(ga.GAError) as e:
+                d.tc_count()
+            assert e.value.name == "GA_ERR_INVALID_GRAPH"
+
+
+@pytest.mark.parametrize("rows", [7, 8, 9, 16, 31, 33, 64, 65, 127, 129, 255, 257, 511, 513, 700])
+def test_index_row_lengths(ga, oracle, cuda_ok, rows):
+    """Rows at the edges of the sort's classes and of octs: one vertex with `rows` later neighbours that form a ring
+    among themselves (every anchor a short row, every suffix length from `rows` - 1 down), plus its mirror of pendant
+    edges that raises the ring's degrees above it."""
+    ring = np.arange(1, rows + 1)
+    e = [(0, int(v)) for v in ring] + [(int(ring[i]), int(ring[(i + 1) % rows])) for i in range(rows)]
+    nxt = rows + 1
+    for v in ring:                      # pendants: the ring outranks vertex 0, so its row is the long one
+        for _ in range(rows):
+            e.append((int(v), nxt))
+            nxt += 1
+    g = ga.build_graph_from_edges(nxt, ga.canonical_edges(np.array(e, np.uint32)))
+    assert g.max_out_degree >= rows
+    T, sup = oracle.edge_support(g)
+    deg = oracle.triangle_degrees(g)[1]
+    for kernel in (1, 2):
+        with ga.DeviceGraph(g) as d:
+            d.set_option(ga.OPT_TC_KERNEL, kernel)
+            d.prepare()
+            assert d.tc_count() == T and sum(d.tc_count_shard(i, 3) for i in range(3)) == T
+            assert np.array_equal(d.support_edges()[1], sup)
+            assert np.array_equal(d.support_vertices()[1], deg)
