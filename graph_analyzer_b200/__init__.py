@@ -79,6 +79,10 @@ class _PeelRes(C.Structure):
                 ("rounds", C.c_uint32)]
 
 
+_PEEL_DTYPE = np.dtype([("best_num", np.uint64), ("best_den", np.uint64), ("best_round", np.uint32),
+                        ("rounds", np.uint32)])     # _PeelRes as an array element
+
+
 class _CoreRes(C.Structure):
     _fields_ = [("kmax", C.c_uint32), ("rounds", C.c_uint32)]
 
@@ -608,7 +612,7 @@ class DeviceGraph:
 
     def batch_peel(self, num: int = 1, den: int = 10, want_removed: bool = True) -> PeelResult:
         r = _PeelRes()
-        rr = np.full(max(self.n, 1), 0xFFFFFFFF, np.uint32) if want_removed else None
+        rr = np.empty(max(self.n, 1), np.uint32) if want_removed else None
         _check(lib().ga_batch_peel(self._h, num, den, C.byref(r), _ptr(rr)))
         return PeelResult(r.best_num, r.best_den, r.best_round, r.rounds,
                           rr[: self.n] if rr is not None else np.zeros(0, np.uint32))
@@ -786,14 +790,11 @@ class DeviceBatch:
     def tc_peel(self, num: int = 1, den: int = 10, want_removed: bool = True) -> BatchPeel:
         G = self.G
         t = np.zeros(G, np.uint64)
-        res = (_PeelRes * G)()
+        res = np.zeros(G, _PEEL_DTYPE)
         st = np.zeros(G, np.uint32)
-        rr = np.zeros(max(self.N, 1), np.uint32) if want_removed else None
-        _check(lib().ga_batch_tc_peel(self._h, num, den, _ptr(t), C.addressof(res), _ptr(st), _ptr(rr)))
-        return BatchPeel(t, np.array([r.best_num for r in res], np.uint64),
-                         np.array([r.best_den for r in res], np.uint64),
-                         np.array([r.best_round for r in res], np.uint32),
-                         np.array([r.rounds for r in res], np.uint32), st,
+        rr = np.empty(max(self.N, 1), np.uint32) if want_removed else None
+        _check(lib().ga_batch_tc_peel(self._h, num, den, _ptr(t), _ptr(res), _ptr(st), _ptr(rr)))
+        return BatchPeel(t, *(res[f].copy() for f in _PEEL_DTYPE.names), st,
                          rr[: self.N] if rr is not None else np.zeros(0, np.uint32))
 
 

@@ -75,7 +75,7 @@ ga_status ga_batch_create(uint32_t num_graphs, const uint64_t* vtx_off, const ui
     cudaStream_t st = (cudaStream_t)stream;
     bool own = false;
     if (!st) {
-        GA_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        GA_CUDA(stream_acquire(device, &st));
         own = true;
     }
     // temporaries: the packed arrays and the union CSR being built
@@ -138,7 +138,7 @@ ga_status ga_batch_create(uint32_t num_graphs, const uint64_t* vtx_off, const ui
     }
     if (own) {
         cudaStreamSynchronize(st);
-        cudaStreamDestroy(st);
+        stream_release(device, st);
     }
     return s;
 }

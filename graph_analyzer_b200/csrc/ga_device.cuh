@@ -183,6 +183,13 @@ ga_status init_pool(int device);
 unsigned long long* host_slot_acquire();
 void host_slot_release(unsigned long long* slot);
 
+// A non-blocking stream of the device, and its return (idle) when the handle ends. device < 64 (init_pool checks).
+cudaError_t stream_acquire(int device, cudaStream_t* st);
+void stream_release(int device, cudaStream_t st);
+
+// Copies a result to host memory of the caller on g's stream and waits for it.
+ga_status download(ga_graph* g, void* dst, const void* src, size_t bytes);
+
 // The pool of the current device (init_pool must have run for it; every entry point that allocates calls it).
 cudaMemPool_t pool_of_current();
 

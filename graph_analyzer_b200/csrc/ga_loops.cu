@@ -1078,6 +1078,9 @@ __global__ void k_seg_init(Segs sg, unsigned long long num, unsigned long long d
 
 // ---- host side --------------------------------------------------------------------------------------------------
 
+// 64-bit words of a batch's results: T0, best_num, best_den, then best_round, rounds, status.
+static size_t seg_result_words(size_t graphs) { return 3 * graphs + (3 * graphs + 1) / 2; }
+
 static ga_status ensure_loops(ga_graph* g) {
     if (g->loops) return GA_OK;
     ga_loops* L = new ga_loops();
@@ -1104,12 +1107,12 @@ static ga_status ensure_loops(ga_graph* g) {
         GA_TRY(dalloc(g, &sg.nalive, c));
         GA_TRY(dalloc(g, &sg.removed, c));
         GA_TRY(dalloc(g, &sg.destroyed, c));
-        GA_TRY(dalloc(g, &sg.best_num, c));
-        GA_TRY(dalloc(g, &sg.best_den, c));
-        GA_TRY(dalloc(g, &sg.T0, c));
-        GA_TRY(dalloc(g, &sg.best_round, c));
-        GA_TRY(dalloc(g, &sg.rounds, c));
-        GA_TRY(dalloc(g, &sg.status, c));
+        GA_TRY(dalloc(g, &sg.T0, seg_result_words(c)));   // what a call returns is one block
+        sg.best_num = sg.T0 + c;
+        sg.best_den = sg.best_num + c;
+        sg.best_round = (uint32_t*)(sg.best_den + c);
+        sg.rounds = sg.best_round + c;
+        sg.status = sg.rounds + c;
     }
     // fixed launch shapes (the graph body is captured once): grid-stride scans, persistent update grid
     int occ = 0;
@@ -1152,8 +1155,7 @@ void reset_loops(ga_graph* g) {
     void* bufs[] = {L->tri, L->state, L->out, L->alive[0], L->alive[1], L->frontier[0], L->frontier[1], L->loc,
                     L->item_x, L->item_c, L->sc,
                     L->inc, L->inc_ptr, L->segs.T, L->segs.nalive, L->segs.removed, L->segs.destroyed,
-                    L->segs.best_num, L->segs.best_den, L->segs.T0, L->segs.best_round, L->segs.rounds,
-                    L->segs.status};
+                    L->segs.T0};
     for (void* b : bufs) dfree(g, b);
     destroy_loops(g);
 }
@@ -1490,18 +1492,12 @@ ga_status peel_segments(ga_graph* g, uint64_t num, uint64_t den, uint64_t* trian
     GA_TRY(run_loop<LOOP_PEEL>(g, num, den, &s));
     const Segs& sg = g->loops->segs;
     const uint32_t G = sg.count;
-    std::vector<unsigned long long> T0(G), bn(G), bd(G);
-    std::vector<uint32_t> br(G), rounds(G), st(G);
-    cudaStream_t stream = g->stream;
-    GA_CUDA(cudaMemcpyAsync(T0.data(), sg.T0, (size_t)G * 8, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaMemcpyAsync(bn.data(), sg.best_num, (size_t)G * 8, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaMemcpyAsync(bd.data(), sg.best_den, (size_t)G * 8, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaMemcpyAsync(br.data(), sg.best_round, (size_t)G * 4, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaMemcpyAsync(rounds.data(), sg.rounds, (size_t)G * 4, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaMemcpyAsync(st.data(), sg.status, (size_t)G * 4, cudaMemcpyDeviceToHost, stream));
-    if (removed_round && g->n)
-        GA_CUDA(cudaMemcpyAsync(removed_round, g->loops->out, (size_t)g->n * 4, cudaMemcpyDeviceToHost, stream));
-    GA_CUDA(cudaStreamSynchronize(stream));
+    // T0 and the results are one block on the device (ensure_loops)
+    std::vector<unsigned long long> block(seg_result_words(G));
+    GA_TRY(download(g, block.data(), sg.T0, block.size() * 8));
+    const unsigned long long *T0 = block.data(), *bn = T0 + G, *bd = bn + G;
+    const uint32_t *br = (const uint32_t*)(bd + G), *rounds = br + G, *st = rounds + G;
+    if (removed_round && g->n) GA_TRY(download(g, removed_round, g->loops->out, (size_t)g->n * 4));
     for (uint32_t i = 0; i < G; i++) {
         if (triangles) triangles[i] = T0[i];
         if (res) res[i] = ga_peel_result{bn[i], bd[i], br[i], rounds[i]};
@@ -1533,8 +1529,7 @@ ga_status ga_batch_peel(ga_graph* g, uint64_t num, uint64_t den, ga_peel_result*
     res->best_round = s.best_round;
     res->rounds = s.round;
     if (removed_round && g->n) {
-        GA_CUDA(cudaMemcpyAsync(removed_round, g->loops->out, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
-        GA_CUDA(cudaStreamSynchronize(g->stream));
+        GA_TRY(download(g, removed_round, g->loops->out, (size_t)g->n * 4));
     }
     return GA_OK;
 }
@@ -1550,8 +1545,7 @@ ga_status ga_core_decomposition(ga_graph* g, uint32_t* core, ga_core_result* res
     res->kmax = s.kcur;
     res->rounds = s.round;
     if (core && g->n) {
-        GA_CUDA(cudaMemcpyAsync(core, g->loops->out, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
-        GA_CUDA(cudaStreamSynchronize(g->stream));
+        GA_TRY(download(g, core, g->loops->out, (size_t)g->n * 4));
     }
     return GA_OK;
 }

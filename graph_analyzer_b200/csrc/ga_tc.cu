@@ -1388,9 +1388,7 @@ ga_status ga_tc_support_edges(ga_graph* g, uint32_t* sup, uint64_t* triangles) {
     s.st = g->stream;
     GA_CUDA(pool_malloc(&s.p, ((size_t)g->m + 1) * 4, g->stream));
     GA_TRY(ga_tc_support_edges_device(g, (uint32_t*)s.p, triangles));
-    if (g->m) GA_CUDA(cudaMemcpyAsync(sup, s.p, (size_t)g->m * 4, cudaMemcpyDeviceToHost, g->stream));
-    GA_CUDA(cudaStreamSynchronize(g->stream));
-    return GA_OK;
+    return download(g, sup, s.p, (size_t)g->m * 4);
 }
 
 ga_status ga_tc_support_vertices(ga_graph* g, uint64_t* deg, uint64_t* triangles) {
@@ -1406,7 +1404,7 @@ ga_status ga_tc_support_vertices(ga_graph* g, uint64_t* deg, uint64_t* triangles
     a.host_total = g->h_scalars;
     a.vsup = (unsigned long long*)s.p;
     GA_TRY((run_tc<TC_VSUP, false, unsigned long long>(g, a, true)));
-    if (g->n) GA_CUDA(cudaMemcpyAsync(deg, s.p, (size_t)g->n * 8, cudaMemcpyDeviceToHost, g->stream));
+    GA_TRY(download(g, deg, s.p, (size_t)g->n * 8));
     return read_total(g, triangles);
 }
 
@@ -1435,7 +1433,7 @@ ga_status ga_tc_participation(ga_graph* g, const uint8_t* alive, uint32_t* tri, 
     a.vsup = d_tri;
     a.alive = d_alive;
     GA_TRY((run_tc<TC_VSUP, true, unsigned int>(g, a, true)));
-    if (g->n) GA_CUDA(cudaMemcpyAsync(tri, d_tri, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
+    GA_TRY(download(g, tri, d_tri, (size_t)g->n * 4));
     return read_total(g, triangles);
 }
 
