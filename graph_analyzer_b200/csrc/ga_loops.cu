@@ -654,10 +654,9 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
 // R-MAT 22 cores: 147 ms with every decrement sent on its own, 235 ms with the round's state in global memory.
 constexpr uint32_t kSmallThreads = 1024;     // threads per CTA of the cluster
 constexpr uint32_t kSmallSlots = 8192;       // local vertices per CTA (8 per thread): 131,072 with 16 CTAs
-constexpr uint32_t kSmallInbox = 128;        // candidates a CTA can publish per round
 constexpr uint32_t kSmallWork = 1u << 20;    // incidence entries a round may read in the cluster
 constexpr uint32_t kSmallMaxCtas = 16;
-constexpr uint32_t kSmallFront = kSmallMaxCtas * kSmallInbox;
+constexpr uint32_t kSmallFront = 2048;       // candidates a round can have: each CTA publishes up to kSmallFront / C
 constexpr uint32_t kSmallSums = 4096;        // slots of a CTA's table of decrements (4 per thread at the flush)
 constexpr uint32_t kSmallSumsBits = 12, kSmallSumsTries = 8;
 constexpr uint32_t kSmallDead = 0xFFFFFFFFu; // count of a removed (or unused) slot
@@ -679,8 +678,7 @@ struct SmallShared {
     uint32_t st[kSmallSlots * kSmallMaxCtas / 16];   // 2 bits per local vertex: 1 alive, 2 frontier, 0 removed
     uint32_t sum_key[kSmallSums];                    // local id (GA_EMPTY: free) ...
     uint32_t sum_cnt[kSmallSums];                    // ... and its decrements in this round
-    SmallEntry own[kSmallInbox];                     // this CTA's candidates
-    SmallEntry inbox[kSmallFront];                   // every CTA's
+    SmallEntry inbox[kSmallFront];                   // every CTA's candidates, this CTA's own among them
     SmallHead head[kSmallMaxCtas];
     uint16_t front[kSmallFront];                     // inbox positions of the round's frontier
     uint32_t flid[2][kSmallFront];                   // its local ids, by round parity (retired in the next round)
@@ -717,7 +715,7 @@ __device__ __forceinline__ void small_dec(SmallShared& s, uint32_t tri0, uint32_
 
 // Runs consecutive core rounds (the work of k_core_min, k_core_mark, k_frontier_update_list and close_round_if_last
 // for LOOP_CORE) inside one cluster of C CTAs while the alive list fits the CTAs' slots, a round reads at most
-// kSmallWork incidence entries and no CTA has more than kSmallInbox candidates; returns at the first round that is
+// kSmallWork incidence entries and no CTA has more than kSmallFront / C candidates; returns at the first round that is
 // larger (untouched, for the grid kernels, which find tri[], state[] and the alive list as if they had run the rounds
 // before), when the loop ends (the WHILE condition is set to 0) or at a status other than LS_OK. Every decision is
 // computed by every thread from values all CTAs hold identically, so all CTAs leave in the same round.
@@ -725,7 +723,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
     LoopScalars* sc, uint32_t* __restrict__ tri, uint8_t* __restrict__ state, uint32_t* __restrict__ core,
     uint32_t* alive0, uint32_t* alive1, const uint32_t* fr0, const uint32_t* fr1, uint32_t* loc,
     const uint2* __restrict__ inc, const unsigned long long* __restrict__ inc_ptr,
-    cudaGraphConditionalHandle handle) {
+    cudaGraphConditionalHandle handle, int use_handle) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char small_raw[];
@@ -735,13 +733,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
     const uint32_t tid = rank * kSmallThreads + threadIdx.x, nthr = C * kSmallThreads;
     const uint32_t gwarp = warp * C + rank, nwarps = nthr >> 5;   // consecutive slices go to different CTAs
     const bool writer = tid == 0;
+    const uint32_t room = kSmallFront >> cbits;   // candidates per CTA
     // the state the grid kernels (or the loop's set-up) left; nothing writes it until the cluster leaves
     const uint32_t p = sc->parity, na0 = sc->alive_count[p];
     const uint32_t max_rounds = sc->max_rounds;
     uint32_t cont = sc->cont, round = sc->round, kcur = sc->kcur, status = sc->status, iters = sc->iters;
     unsigned long long nalive = sc->nalive;
     if (!cont) {   // the loop is over: the WHILE node must stop whoever cleared `cont`
-        if (writer) cudaGraphSetConditional(handle, 0);
+        if (writer && use_handle) cudaGraphSetConditional(handle, 0);
         return;
     }
     if (na0 > kSmallSlots * C) return;
@@ -784,13 +783,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
     cluster.sync();   // loc[] is complete, and every CTA runs before its shared memory is written from others
     const uint32_t tri0 = smem_addr(s.tri);
     uint32_t done = 0, fprev = 0;   // rounds run here, the last one's frontier
+    uint32_t fv = 0;   // the vertex of this thread's frontier entry, when this CTA holds it
     // the last round's frontier (F vertices at level k): out of the states, core numbers written by the owners
     auto retire = [&](uint32_t F, uint32_t k) {
         for (uint32_t f = threadIdx.x; f < F; f += kSmallThreads) {
             const uint32_t lid = s.flid[(done & 1) ^ 1][f];
             atomicAnd(&s.st[lid >> 4], ~(3u << (2 * (lid & 15))));
             if ((lid & (C - 1)) == rank) {
-                const uint32_t v = in[lid];
+                const uint32_t v = f < kSmallThreads ? fv : in[lid];   // read when the frontier was marked
                 core[v] = k;
                 state[v] = 0;
             }
@@ -813,9 +813,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
                 if (ts[j] > thr) continue;
                 const uint32_t slot = 4 * threadIdx.x + (j & 3) + (j >> 2) * 4 * kSmallThreads;
                 const uint32_t at = atomicAdd(&s.count, 1u);
-                if (at >= kSmallInbox) continue;   // counted: the round goes to the grid kernels
+                if (at >= room) continue;   // counted: the round goes to the grid kernels
                 const uint32_t lh = s.len_hi[slot], bl = s.beg_lo[slot];
-                s.own[at] = SmallEntry{slot * C + rank, lh, bl, 0};
+                s.inbox[rank * room + at] = SmallEntry{slot * C + rank, lh, bl, 0};
                 // its list is wanted in this round or in one soon after: from DRAM to L2 while the level is agreed on
                 const uint32_t bytes = min(lh & kSmallLenMask, kSmallPrefetch) * 8u & ~15u;
                 const char* list = (const char*)(inc + ((unsigned long long)(lh >> 30) << 32 | bl));
@@ -826,11 +826,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         }
         __syncthreads();
         const uint32_t mycount = s.count;
-        for (uint32_t i = threadIdx.x; i < min(mycount, kSmallInbox) * C; i += kSmallThreads) {   // (candidate, CTA)
-            const uint32_t at = i >> cbits;
-            const SmallEntry e = s.own[at];
+        for (uint32_t i = threadIdx.x; i < min(mycount, room) * C; i += kSmallThreads) {   // (candidate, CTA)
+            if ((i & (C - 1)) == rank) continue;
+            const SmallEntry* at = &s.inbox[rank * room + (i >> cbits)];
+            const SmallEntry e = *at;
             asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
-                             remote_addr(smem_addr(&s.inbox[rank * kSmallInbox + at]), i & (C - 1))),
+                             remote_addr(smem_addr(at), i & (C - 1))),
                          "r"(e.lid), "r"(e.len_hi), "r"(e.beg_lo), "r"(0u)
                          : "memory");
         }
@@ -850,7 +851,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         const uint32_t k = max(kcur, gmin);
         // every count <= k is a candidate of its CTA exactly when the CTA's minimum is <= k
         const uint32_t cnt = h.mn <= k && h.mn != kSmallDead ? h.count : 0u;
-        if (__any_sync(GA_FULL_MASK, cnt > kSmallInbox)) break;   // the grid kernels take this round
+        if (__any_sync(GA_FULL_MASK, cnt > room)) break;   // the grid kernels take this round
         const uint32_t incl = warp_incl_scan(cnt, lane);
         const uint32_t F = __shfl_sync(GA_FULL_MASK, incl, 31);
         const uint32_t taking = __ballot_sync(GA_FULL_MASK, cnt != 0);
@@ -868,7 +869,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
                 if (start <= f) { c = q; before = start; }
             }
             if (f < F) {
-                const uint32_t at = c * kSmallInbox + (f - before);
+                const uint32_t at = c * room + (f - before);
                 e = s.inbox[at];
                 work += min(e.len_hi & kSmallLenMask, kSmallWork + 1);
                 if (wide || warp == 0) {
@@ -889,7 +890,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         for (uint32_t f = threadIdx.x; f < F; f += kSmallThreads) {
             const uint32_t lid = wide ? flid[f] : e.lid;
             atomicXor(&s.st[lid >> 4], 3u << (2 * (lid & 15)));   // 1 -> 2
-            if ((lid & (C - 1)) == rank) s.tri[lid >> cbits] = kSmallDead;
+            if ((lid & (C - 1)) == rank) {
+                s.tri[lid >> cbits] = kSmallDead;
+                if (f < kSmallThreads) fv = in[lid];   // in flight during the update
+            }
         }
         __syncthreads();
         // update (k_frontier_update_list): each destroyed triangle once, by its smallest frontier corner
@@ -1014,7 +1018,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         sc->iters = iters;
         sc->status = status;
         sc->cont = cont;
-        if (!cont) cudaGraphSetConditional(handle, 0);
+        if (!cont && use_handle) cudaGraphSetConditional(handle, 0);
     }
 }
 
@@ -1049,6 +1053,27 @@ static int small_round_cluster(int device) {
     (void)cudaGetLastError();
     cached[device] = best;
     return best > 0 ? best : 0;
+}
+
+static ga_status launch_small_rounds(ga_graph* g, cudaStream_t st, uint32_t ctas, cudaGraphConditionalHandle h,
+                                     int use_h) {
+    ga_loops* L = g->loops;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = sizeof(SmallShared);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GA_CUDA(cudaLaunchKernelEx(&cfg, k_core_small_rounds, L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
+                               (const uint32_t*)L->frontier[0], (const uint32_t*)L->frontier[1], L->loc,
+                               (const uint2*)L->inc, (const unsigned long long*)L->inc_ptr, h, use_h));
+    return GA_OK;
 }
 
 // Per graph: T0 = (sum of its vertices' triangle counts) / 3, from the ends of its incidence lists when they exist
@@ -1256,25 +1281,9 @@ static ga_status enqueue_round(ga_graph* g, cudaStream_t st, cudaGraphConditiona
                                                   L->frontier[0], L->frontier[1], L->item_x, L->item_c, g->deg,
                                                   inc_ptr, sg);
     } else {
-        const int csize = use_h && L->lists == 1 ? small_round_cluster(g->device) : 0;
-        if (csize) {   // the small rounds first, in one cluster; the grid kernels below take the first large one
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = csize;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.gridDim = dim3(csize);
-            cfg.blockDim = dim3(kSmallThreads);
-            cfg.dynamicSmemBytes = sizeof(SmallShared);
-            cfg.stream = st;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            GA_CUDA(cudaLaunchKernelEx(&cfg, k_core_small_rounds, L->sc, L->tri, L->state, L->out, L->alive[0],
-                                       L->alive[1], (const uint32_t*)L->frontier[0],
-                                       (const uint32_t*)L->frontier[1], L->loc, (const uint2*)L->inc,
-                                       (const unsigned long long*)L->inc_ptr, h));
-        }
+        // the small rounds first, in one cluster; the grid kernels below take the first large one
+        const uint32_t ctas = use_h && L->lists == 1 ? (uint32_t)small_round_cluster(g->device) : 0;
+        if (ctas) GA_TRY(launch_small_rounds(g, st, ctas, h, 1));
         k_core_min<<<L->grid_scan, 256, 0, st>>>(L->sc, L->tri, L->alive[0], L->alive[1], L->state, L->frontier[0],
                                                  L->frontier[1], h, use_h);
         k_core_mark<<<L->grid_scan, kMarkThreads, 0, st>>>(L->sc, L->tri, L->state, L->out, L->alive[0], L->alive[1],
@@ -1380,9 +1389,24 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     GA_CUDA(cudaGetLastError());
     LoopScalars* h_sc = reinterpret_cast<LoopScalars*>(g->h_scalars + 32);   // page-locked
     static_assert(sizeof(LoopScalars) <= 32 * 8, "fits the second half of the handle's slot");
+    bool more = true;   // the final state is still to be read
     if (n > 0) {
         const bool graph_mode = g->opt_loop_mode != 1;
-        if (graph_mode) {
+        // A core loop whose vertices fit the cluster from the start is mostly one launch of it: the launches are made
+        // here, with a grid round between them where a round is too large, and only a loop that keeps alternating is
+        // captured as a graph, which costs more to make and release than such a loop takes
+        const uint32_t ctas = KIND == LOOP_CORE && graph_mode && L->lists == 1 ? (uint32_t)small_round_cluster(g->device) : 0;
+        if (ctas && (uint64_t)kSmallSlots * ctas >= n && !L->exec[LOOP_CORE]) {
+            for (int i = 0; i < 4 && more; i++) {
+                if (i) GA_TRY(enqueue_round<KIND>(g, st, 0, 0));
+                GA_TRY(launch_small_rounds(g, st, ctas, 0, 0));
+                GA_CUDA(cudaMemcpyAsync(h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
+                GA_CUDA(cudaStreamSynchronize(st));
+                more = h_sc->cont != 0;
+            }
+        }
+        if (!more) {
+        } else if (graph_mode) {
             GA_TRY(ensure_graph<KIND>(g));
             GA_CUDA(cudaGraphLaunch(seg ? L->exec_seg : L->exec[KIND], st));
         } else {
@@ -1395,8 +1419,10 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
             }
         }
     }
-    GA_CUDA(cudaMemcpyAsync(h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
-    GA_CUDA(cudaStreamSynchronize(st));
+    if (more) {
+        GA_CUDA(cudaMemcpyAsync(h_sc, L->sc, sizeof(LoopScalars), cudaMemcpyDeviceToHost, st));
+        GA_CUDA(cudaStreamSynchronize(st));
+    }
     *result = *h_sc;
     switch (result->status) {
         case LS_OK: break;
