@@ -46,6 +46,16 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x)
     return x;
 }
 
+// Additions to global counters whose old value nobody wants, as the reduction they are: in a kernel that also has a
+// __threadfence (the last block's turn), an atomicAdd without a use of its result is compiled to an atomic that returns
+// one, and a warp then waits for it (R-MAT 22 edge supports 7.2 ms against 6.3).
+__device__ __forceinline__ void red_add(uint32_t* p, uint32_t v) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v) {
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 // Multiplicative hash onto `bits` bits (Knuth): the high bits of x * 2654435761 mod 2^32.
 __device__ __forceinline__ uint32_t hash_slot(uint32_t x, uint32_t bits) {
     return (x * 2654435761u) >> (32 - bits);

@@ -532,8 +532,8 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
                     const bool owned = !((syv == 2 && yv < x) || (sw == 2 && wv < x));
                     if (owned) {
                         destroyed++;
-                        if (syv == 1) atomicSub(&tri[yv], 1u);
-                        if (sw == 1) atomicSub(&tri[wv], 1u);
+                        if (syv == 1) red_add(&tri[yv], 0xFFFFFFFFu);
+                        if (sw == 1) red_add(&tri[wv], 0xFFFFFFFFu);
                     }
                 }
             }
@@ -610,8 +610,8 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
             if (!sy || !sw) continue;                               // destroyed in an earlier round
             if ((sy == 2 && yw.x < xv) || (sw == 2 && yw.y < xv)) continue;   // a smaller frontier corner owns it
             mine++;
-            if (sy == 1) atomicSub(&tri[yw.x], 1u);
-            if (sw == 1) atomicSub(&tri[yw.y], 1u);
+            if (sy == 1) red_add(&tri[yw.x], 0xFFFFFFFFu);
+            if (sw == 1) red_add(&tri[yw.y], 0xFFFFFFFFu);
         }
         destroyed += mine;
         if (sg.count) {   // per-graph count of destroyed triangles, lanes of one graph combined

@@ -51,10 +51,11 @@
 namespace ga {
 
 #ifndef GA_TC_MIN_BLOCKS
-#define GA_TC_MIN_BLOCKS 6                // resident blocks per SM the hash kernel is compiled for (8, 7, 6: R-MAT 22
-                                          // count 2.28, 2.28, 2.28 ms, R-MAT 16 edge supports 174, 136, 130 us; 5: 2.36 ms)
+#define GA_TC_MIN_BLOCKS 6                // resident blocks per SM the support and list passes are compiled for (8:
+                                          // R-MAT 16 vertex supports 186 us, 6: 177)
 #endif
 
+constexpr int kCountBlocks = 8;           // ... and counts (R-MAT 22: 1.99 ms; 6: 2.12, 5: 2.31)
 constexpr int kWarps = 8;                 // warps per block of the hash kernel
 constexpr int kThreads = kWarps * 32;
 // Per-warp hash set of the light bin: 512 slots for counts and lists; 256 in the support modes, whose slots carry
@@ -196,6 +197,13 @@ __device__ __forceinline__ void finish_pass(unsigned long long local, const TcAr
     if (a.host_total) *a.host_total = t;
 }
 
+// Oct q of colr, in one 256-bit load (a scattered request costs the load unit the same for 4 bytes as for 32).
+__device__ __forceinline__ void load_oct(const uint32_t* __restrict__ colr, size_t q, uint32_t (&x)[8]) {
+    asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
+        : "l"(colr + 8 * q));
+}
+
 // The probe lists of a batch of up to 32 in-edges [kb, kend) (one warp): lane l takes the l-th in-edge's suffix of its
 // source's row, a run of whole octs, from in_rng. A warp scan of the oct counts flattens the lists into one sequence:
 // oct p of it is oct s_base[owner] + p of colr, owner the first with s_incl[owner] > p. Entries of the first oct before
@@ -223,9 +231,8 @@ __device__ __forceinline__ uint32_t open_batch(const IX& ix, const uint8_t* aliv
 template <int MODE, bool ALIVE, class CT>
 __device__ __forceinline__ uint32_t oct_members(const TcArgs<CT>& a, const Anchor& an, uint32_t q, const uint32_t* key,
                                                 uint32_t* list) {
-    const uint4* p = reinterpret_cast<const uint4*>(a.ix.colr) + 2 * (size_t)q;
-    const uint4 v0 = __ldg(p), v1 = __ldg(p + 1);
-    const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    uint32_t xs[8];
+    load_oct(a.ix.colr, q, xs);
     uint32_t l = 0, c3 = 0;   // c3: three times the number found
     if (an.span) {
         const uint32_t base = an.v + 1;
@@ -334,9 +341,9 @@ __device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb
             } else {
                 const uint32_t slot = find_member<MODE, ALIVE, CT>(a, an, x, key, pre);
                 if (an.span || an.bits) atomicAdd(&cnt[slot], 1u);
-                else if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)1);
-                else atomicAdd(&a.esupk[(size_t)an.row * 8 + slot], 1u);
-                if (MODE == TC_ESUP) atomicAdd(&a.esupk[e], 1u);   // u->x at its place in u's row
+                else if (MODE == TC_VSUP) red_add(&a.vsup[a.ix.order[x]], (CT)1);
+                else red_add(&a.esupk[(size_t)an.row * 8 + slot], 1u);
+                if (MODE == TC_ESUP) red_add(&a.esupk[e], 1u);   // u->x at its place in u's row
             }
         }
         __syncwarp();
@@ -345,8 +352,8 @@ __device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb
     if (counters(MODE)) {
         const uint32_t c = s_ecnt[lane];
         if (c) {
-            if (MODE == TC_VSUP) atomicAdd(&a.vsup[u], (CT)c);
-            else atomicAdd(&a.esupk[rng_at(rec)], c);
+            if (MODE == TC_VSUP) red_add(&a.vsup[u], (CT)c);
+            else red_add(&a.esupk[rng_at(rec)], c);
             s_ecnt[lane] = 0;
         }
     }
@@ -376,15 +383,14 @@ __device__ __forceinline__ uint32_t count_batch(const TcArgs<CT>& a, uint32_t kb
         __syncwarp();
         return hits;
     }
-    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
     // the eight lookups of an oct are issued without branches, so they overlap; a bucket that is full without a match
     // (rare) continues in the next buckets afterwards
     const uint32_t nb = an.bits + bucket_shift<TC_COUNT>(), bmask = (1u << nb) - 1;
     for (uint32_t p = lane; p < tot; p += 32) {
         while (end <= p) end = s_incl[++owner];
         const size_t q = s_base[owner] + p;
-        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
-        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        uint32_t xs[8];
+        load_oct(a.ix.colr, q, xs);
         uint32_t more = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -503,13 +509,12 @@ __device__ __forceinline__ uint32_t count_batch_bitmap(const TcArgs<CT>& a, uint
                                                        uint32_t* s_incl, uint32_t* s_base, uint32_t lane) {
     unsigned long long rec;
     const uint32_t tot = open_batch<ALIVE>(a.ix, a.alive, kb, kend, lane, s_incl, s_base, &rec);
-    const uint4* __restrict__ col4 = reinterpret_cast<const uint4*>(a.ix.colr);
     uint32_t owner = 0, end = s_incl[0], hits = 0;
     for (uint32_t p = lane; p < tot; p += 32) {
         while (end <= p) end = s_incl[++owner];
         const size_t q = s_base[owner] + p;
-        const uint4 v0 = __ldg(col4 + 2 * q), v1 = __ldg(col4 + 2 * q + 1);
-        const uint32_t xs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        uint32_t xs[8];
+        load_oct(a.ix.colr, q, xs);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const uint32_t o = xs[i] - base;
@@ -519,13 +524,6 @@ __device__ __forceinline__ uint32_t count_batch_bitmap(const TcArgs<CT>& a, uint
     }
     __syncwarp();
     return hits;
-}
-
-__device__ __forceinline__ void load_oct(const uint32_t* __restrict__ colr, size_t q, uint32_t (&x)[8]) {
-    const uint4* p = reinterpret_cast<const uint4*>(colr) + 2 * q;
-    const uint4 a = __ldg(p), b = __ldg(p + 1);
-    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
 }
 
 // Common entries of octs x and y of ascending rows, calling hit(place) for each when the caller books them.
@@ -546,14 +544,13 @@ __device__ __forceinline__ uint32_t oct_common(const uint32_t (&x)[8], const uin
     return c;
 }
 
-// Common places of an in-edge's suffix (octs q.. of colr, `octs` of them) and its anchor's row (octs r.. up to rend):
-// both ascend, so the oct with the smaller last entry is done after one comparison of all pairs.
+// Common places of an in-edge's suffix (x: its first oct, q, of `octs`) and its anchor's row (octs r.. up to rend): both
+// ascend, so the oct with the smaller last entry is done after one comparison of all pairs. hit(place) as above.
 template <bool BOOK, class F>
-__device__ __forceinline__ uint32_t suffix_common(const uint32_t* __restrict__ colr, size_t q, uint32_t octs, size_t r,
-                                                  size_t rend, F hit) {
+__device__ __forceinline__ uint32_t suffix_common(const uint32_t* __restrict__ colr, uint32_t (&x)[8], size_t q,
+                                                  uint32_t octs, size_t r, size_t rend, F hit) {
     const size_t qend = q + octs;
-    uint32_t x[8], y[8], c = 0;
-    load_oct(colr, q, x);
+    uint32_t y[8], c = 0;
     load_oct(colr, r, y);
     for (;;) {
         if (x[7] >= y[0])   // else the whole oct is below the row (padding counts as above)
@@ -602,9 +599,11 @@ __device__ __forceinline__ uint32_t tiny_group(const TcArgs<CT>& a, uint32_t p0,
     for (uint32_t p = lane; p < tot; p += 32) {
         while (end <= p) end = s_incl[++owner];
         const unsigned long long r = a.ix.in_rng[s_base[owner] + p];
-        if (rng_octs(r))
-            hits += suffix_common<false>(a.ix.colr, rng_oct(r), rng_octs(r), s_row[owner],
-                                         s_row[owner] + ((s_deg[owner] + 7) >> 3), [](uint32_t) {});
+        if (!rng_octs(r)) continue;
+        uint32_t x[8];
+        load_oct(a.ix.colr, rng_oct(r), x);
+        hits += suffix_common<false>(a.ix.colr, x, rng_oct(r), rng_octs(r), s_row[owner],
+                                     s_row[owner] + ((s_deg[owner] + 7) >> 3), [](uint32_t) {});
     }
     __syncwarp();
     return hits;
@@ -625,8 +624,8 @@ __device__ __forceinline__ void flush_counts(const TcArgs<CT>& a, const Anchor& 
             const uint32_t o = x - an.v - 1;
             const uint32_t c = cnt[ALIVE ? pre[o >> 5] + __popc(key[o >> 5] & ((1u << (o & 31)) - 1)) : j];
             if (!c) continue;
-            if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)c);
-            else atomicAdd(&a.esupk[(size_t)an.row * 8 + j], c);
+            if (MODE == TC_VSUP) red_add(&a.vsup[a.ix.order[x]], (CT)c);
+            else red_add(&a.esupk[(size_t)an.row * 8 + j], c);
         }
         return;
     }
@@ -634,8 +633,8 @@ __device__ __forceinline__ void flush_counts(const TcArgs<CT>& a, const Anchor& 
     for (uint32_t s = tid; s < S; s += nthr) {
         const uint32_t c = cnt[s];
         if (c) {
-            if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[key[s]]], (CT)c);   // 4-slot buckets: no spill flags
-            else atomicAdd(&a.esupk[(size_t)an.row * 8 + pos[s]], c);
+            if (MODE == TC_VSUP) red_add(&a.vsup[a.ix.order[key[s]]], (CT)c);   // 4-slot buckets: no spill flags
+            else red_add(&a.esupk[(size_t)an.row * 8 + pos[s]], c);
         }
     }
 }
@@ -662,7 +661,7 @@ __global__ void k_alive_places(const uint8_t* __restrict__ alive, const uint32_t
 // (heavy, light, tiny); null means every item. tiny_groups: counts of the whole graph take the tiny bin in groups of 32
 // places from tiny_first on; otherwise its items are run like light ones.
 template <int MODE, bool ALIVE, class CT>
-__global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds,
+__global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA_TC_MIN_BLOCKS) k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds,
                                                       uint32_t heavy_bits_max,
                                                       uint32_t tiny_first, uint32_t tiny_end, uint32_t light_max_deg,
                                                       TcArgs<CT> a) {
@@ -732,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
             hits += h;
             if (MODE == TC_VSUP) {
                 const unsigned long long t = warp_sum_u64(h);
-                if (lane == 0 && t) atomicAdd(&a.vsup[an.id], (CT)t);
+                if (lane == 0 && t) red_add(&a.vsup[an.id], (CT)t);
             }
             __syncthreads();
             if (an.span || an.bits) flush_counts<MODE, ALIVE, CT>(a, an, key, pre, cn, pos, threadIdx.x, kThreads);
@@ -779,7 +778,7 @@ __global__ void __launch_bounds__(kThreads, GA_TC_MIN_BLOCKS) k_tc_hash(ga_items
         hits += h;
         if (MODE == TC_VSUP) {
             const unsigned long long t = warp_sum_u64(h);
-            if (lane == 0 && t) atomicAdd(&a.vsup[an.id], (CT)t);
+            if (lane == 0 && t) red_add(&a.vsup[an.id], (CT)t);
         }
         __syncwarp();
         if (an.bits) flush_counts<MODE, ALIVE, CT>(a, an, key, nullptr, cnt, pos, lane, 32);
@@ -821,25 +820,32 @@ __global__ void __launch_bounds__(256) k_tc_octs(uint32_t m, TcArgs<CT> a) {
         uint32_t c = 0, v = 0, u = 0;
         if (octs) {
             const size_t at = rng_at(r);
-            v = __ldg(a.ix.colr + at);
+            uint32_t x[8];
+            load_oct(a.ix.colr, rng_oct(r), x);
+            // the anchor is the entry before the suffix: in its first oct, unless that starts one
+            const uint32_t j = at & 7;
+            v = x[0];
+#pragma unroll
+            for (int i = 1; i < 7; i++) v = j == i ? x[i] : v;
+            if (j == 7) v = __ldg(a.ix.colr + at);
             const uint32_t row = a.ix.pos[v].y, rend = a.ix.pos[v + 1].y;
             if (ALIVE || MODE == TC_VSUP) u = a.ix.osrc[at >> 3];
             if (row != rend && (!ALIVE || (a.alive[u] && a.alive[v]))) {
                 const uint32_t all = suffix_common<(ALIVE || MODE != TC_COUNT)>(
-                    a.ix.colr, rng_oct(r), octs, row, rend, [&](uint32_t x) {
-                        if (ALIVE && !a.alive[x]) return;
+                    a.ix.colr, x, rng_oct(r), octs, row, rend, [&](uint32_t w) {
+                        if (ALIVE && !a.alive[w]) return;
                         c++;
-                        if (MODE == TC_VSUP) atomicAdd(&a.vsup[a.ix.order[x]], (CT)1);
+                        if (MODE == TC_VSUP) red_add(&a.vsup[a.ix.order[w]], (CT)1);
                     });
                 if (MODE == TC_COUNT && !ALIVE) c = all;
             }
         }
         local += c;
         if (MODE == TC_VSUP && __any_sync(GA_FULL_MASK, c != 0)) {
-            if (c) atomicAdd(&a.vsup[a.ix.order[u]], (CT)c);
+            if (c) red_add(&a.vsup[a.ix.order[u]], (CT)c);
             const uint32_t peers = __match_any_sync(GA_FULL_MASK, c ? v : kPad);
             const uint32_t sum = __reduce_add_sync(peers, c);
-            if (c && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&a.vsup[a.ix.order[v]], (CT)sum);
+            if (c && lane == (uint32_t)__ffs(peers) - 1) red_add(&a.vsup[a.ix.order[v]], (CT)sum);
         }
     }
     finish_pass(local, a);
@@ -866,14 +872,14 @@ __global__ void __launch_bounds__(256) k_tc_plain(const uint32_t* __restrict__ r
                 if (!ALIVE || a.alive[x]) {
                     local++;
                     if (MODE == TC_VSUP) {
-                        atomicAdd(&a.vsup[u], (CT)1);
-                        atomicAdd(&a.vsup[v], (CT)1);
-                        atomicAdd(&a.vsup[x], (CT)1);
+                        red_add(&a.vsup[u], (CT)1);
+                        red_add(&a.vsup[v], (CT)1);
+                        red_add(&a.vsup[x], (CT)1);
                     }
                     if (MODE == TC_ESUP) {
-                        atomicAdd(&a.esup[e], 1u);
-                        atomicAdd(&a.esup[i], 1u);
-                        atomicAdd(&a.esup[j], 1u);
+                        red_add(&a.esup[e], 1u);
+                        red_add(&a.esup[i], 1u);
+                        red_add(&a.esup[j], 1u);
                     }
                     if (MODE == TC_LIST) list_triangle(a, u, v, x);
                 }
