@@ -656,9 +656,13 @@ constexpr uint32_t kSmallThreads = 1024;     // threads per CTA of the cluster
 constexpr uint32_t kSmallSlots = 8192;       // local vertices per CTA (8 per thread): 131,072 with 16 CTAs
 constexpr uint32_t kSmallWork = 1u << 20;    // incidence entries a round may read in the cluster
 constexpr uint32_t kSmallMaxCtas = 16;
-constexpr uint32_t kSmallFront = 2048;       // candidates a round can have: each CTA publishes up to kSmallFront / C
-constexpr uint32_t kSmallSums = 4096;        // slots of a CTA's table of decrements (4 per thread at the flush)
-constexpr uint32_t kSmallSumsBits = 12, kSmallSumsTries = 8;
+// The candidates a round can have (each CTA publishes up to kSmallFront / C) and the slots of a CTA's table of decrements:
+// with 2,048 and 4,096 the CTA left 28 KB of L1, a fraction of the lines a round's local ids lie in, with these 60 KB
+// (R-MAT 22 cores 105.5 -> 98.9 ms; 640 candidates send rounds of the 8,298-vertex graph to the grid, 1,024 slots are
+// too few for the thousand vertices a round touches: 103.2 ms).
+constexpr uint32_t kSmallFront = 1024;
+constexpr uint32_t kSmallSums = 2048;
+constexpr uint32_t kSmallSumsBits = 11, kSmallSumsTries = 8;
 constexpr uint32_t kSmallDead = 0xFFFFFFFFu; // count of a removed (or unused) slot
 
 // A frontier candidate: local id, incidence list (start: 34 bits, the upper two beside the length, which is capped -
@@ -951,18 +955,20 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
             if (lane == 0 && destroyed) atomicAdd(&s.destroyed, (unsigned long long)destroyed);
             __syncthreads();
             // send the sums and clear the table
-            uint4* keys = reinterpret_cast<uint4*>(s.sum_key) + threadIdx.x;
-            const uint4 kq = *keys;
-            if ((kq.x & kq.y & kq.z & kq.w) != GA_EMPTY) {
-                uint4* cnts = reinterpret_cast<uint4*>(s.sum_cnt) + threadIdx.x;
-                const uint4 cq = *cnts;
-                const uint32_t ks[4] = {kq.x, kq.y, kq.z, kq.w}, cs[4] = {cq.x, cq.y, cq.z, cq.w};
+            if (threadIdx.x < kSmallSums / 4) {
+                uint4* keys = reinterpret_cast<uint4*>(s.sum_key) + threadIdx.x;
+                const uint4 kq = *keys;
+                if ((kq.x & kq.y & kq.z & kq.w) != GA_EMPTY) {
+                    uint4* cnts = reinterpret_cast<uint4*>(s.sum_cnt) + threadIdx.x;
+                    const uint4 cq = *cnts;
+                    const uint32_t ks[4] = {kq.x, kq.y, kq.z, kq.w}, cs[4] = {cq.x, cq.y, cq.z, cq.w};
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (ks[q] != GA_EMPTY)
-                        remote_sub(remote_addr(tri0 + 4 * (ks[q] >> cbits), ks[q] & (C - 1)), cs[q]);
-                *keys = make_uint4(GA_EMPTY, GA_EMPTY, GA_EMPTY, GA_EMPTY);
-                *cnts = make_uint4(0, 0, 0, 0);
+                    for (int q = 0; q < 4; q++)
+                        if (ks[q] != GA_EMPTY)
+                            remote_sub(remote_addr(tri0 + 4 * (ks[q] >> cbits), ks[q] & (C - 1)), cs[q]);
+                    *keys = make_uint4(GA_EMPTY, GA_EMPTY, GA_EMPTY, GA_EMPTY);
+                    *cnts = make_uint4(0, 0, 0, 0);
+                }
             }
         }
         cluster.sync();

@@ -233,11 +233,11 @@ def test_core_level_density_every_level(ga, oracle, golden, cuda_ok, kernel):
                 assert d.core_level_density(core, k) == oracle.core_level_density(g, core, k), k
 
 
-@pytest.mark.parametrize("shape", ["hk-131060", "hk-131072", "hk-131090", "rmat-15", "cliques-2046", "cliques-2049",
-                                   "cliques-40000"])
+@pytest.mark.parametrize("shape", ["hk-131060", "hk-131072", "hk-131090", "rmat-15", "cliques-1023", "cliques-1026",
+                                   "cliques-2046", "cliques-2049", "cliques-40000"])
 def test_core_rounds_at_cluster_limits(ga, oracle, cuda_ok, shape):
     """Core rounds around the limits of the cluster kernel: alive lists at its 131,072 slots, rounds whose frontier
-    is at and just above the 2,048 candidates its CTAs can publish, rounds that alternate with grid rounds."""
+    is at and above the 1,024 candidates its CTAs can publish, rounds that alternate with grid rounds."""
     kind, k = shape.split("-")
     k = int(k)
     if kind == "hk":
