@@ -70,3 +70,17 @@ def test_batch_rejects_bad_input(ga, cuda_ok):
     with pytest.raises(ga.GAError) as e:
         ga.DeviceBatch(b)
     assert e.value.name == "GA_ERR_INVALID_GRAPH"
+
+
+@pytest.mark.parametrize("sizes", [(2047, 1, 0), (2048, 0, 0, 1), (0, 2049, 0), (1, 2046, 2, 4095, 0, 4097), (1,) * 300])
+def test_union_at_tile_edges(ga, oracle, cuda_ok, sizes):
+    """Graphs that begin and end on, before and after the 2,048-entry tiles in which the union is built, graphs without
+    vertices and edges among them: every graph's count is the oracle's."""
+    rng = np.random.default_rng(len(sizes))
+    graphs = []
+    for n in sizes:
+        pairs = rng.integers(0, max(n, 1), (n + n % 3, 2), dtype=np.uint32) if n > 1 else np.zeros((0, 2), np.uint32)
+        extra = np.stack(np.triu_indices(min(n, 24), 1), 1).astype(np.uint32)
+        graphs.append(ga.build_graph_from_edges(n, ga.canonical_edges(np.concatenate([pairs, extra]))))
+    with ga.DeviceBatch(ga.pack_batch(graphs)) as d:
+        assert list(d.tc()) == [oracle.triangles_serial(g) if g.m else 0 for g in graphs]
