@@ -227,7 +227,13 @@ def run_reference_arm(args):
             dist.destroy_process_group()
         return 0
     from oracle import Reference
-    ref = Reference()
+    try:
+        ref = Reference()
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        if dist:
+            dist.destroy_process_group()
+        return 0
     g = reference_graph(args.scale)
     b_alg = algorithmic_bytes(g)
     rg = ref.resident(g)
@@ -369,7 +375,12 @@ def run_ours(args):
         return 0
     peaks = read_peaks()
     achieved = b_alg / (ms / 1e3) / 1e9
-    cpu = cpu_reference_baseline(g, b_alg) if world == 1 and not args.no_cpu else None
+    cpu = None
+    if world == 1 and not args.no_cpu:
+        try:
+            cpu = cpu_reference_baseline(g, b_alg)
+        except FileNotFoundError as e:   # built from the reference's sources, where they are present
+            log(f"no CPU baseline: {e}")
     if cpu and cpu["triangles"] != T:
         raise RuntimeError(f"GPU count {T} differs from the reference CPU count {cpu['triangles']}")
     line = {
