@@ -45,6 +45,7 @@ struct GraphEntry {
     uint64_t dev_bytes = 0;              // its device bytes (accounted in `reserved`)
     uint64_t triangles = UINT64_MAX;     // known after the first request (sizes the incidence lists)
     uint64_t tri_bound = 0;              // sum over v of C(d+(v), 2): at least the triangle count
+    uint64_t octs = 0, row_work = 0;     // sums of ceil(d+ / 8) and d+ * ceil(d+ / 8): size the index
     bool busy = false;
     uint64_t last_use = 0;
 };
@@ -64,9 +65,10 @@ struct Request {
 uint64_t estimate_bytes(const GraphEntry& e, ga_request_kind kind) {
     const uint64_t n = e.n, m = e.m;
     // CSR, src, degrees; the index: four arrays by place, positions, rows in octs with their sources, in-edges; items
-    const uint64_t octs = (m + 7 * std::min(n, m)) / 8;
+    const uint64_t octs = std::min(e.octs, (m + 7 * std::min(n, m)) / 8);   // at most that in any valid CSR
+    const uint64_t items = std::min(m, std::min(n, m) + e.row_work / 128 + 1);   // at the smallest item work, 1,024
     uint64_t b = 4 * (n + 1) + 4 * (m + 4) + 4 * m + 4 * n;
-    b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (n + (2 * e.tri_bound + 8 * m) / 1024 + 1) + 1024;
+    b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (items + 1) + 1024;
     if (kind != GA_REQ_TC) {
         const uint64_t T = e.triangles != UINT64_MAX ? e.triangles : e.tri_bound;
         b += 29 * n + 8 * (n + 3 * T / 512 + 1) + 24 * T + 8 * (n + 1);
@@ -489,6 +491,8 @@ ga_status ga_server_add_graph(ga_server* s, const uint32_t* rowptr, const uint32
     for (uint32_t v = 0; v < n; v++) {
         const uint64_t d = rowptr[v + 1] - rowptr[v];
         e.tri_bound += d * (d - 1) / 2;
+        e.octs += (d + 7) / 8;
+        e.row_work += d * ((d + 7) / 8);
     }
     if (estimate_bytes(e, GA_REQ_TC) > s->cfg.hbm_budget_bytes) {
         if (e.pinned) cudaFreeHost(e.pinned);
