@@ -15,7 +15,8 @@
 // or a binary search in global memory. Rows are padded to octs (8 places, one 32-byte sector) with a value that is in
 // no set: a lane reads one oct and does eight probes without testing where the list starts or ends, so the search for
 // the list an oct belongs to and the loop around it are paid once per eight probes (once per four, with two range tests
-// a probe, when rows were unpadded ids: R-MAT 22 count 2.56 ms against 2.23, R-MAT 20 0.79 against 0.49).
+// a probe, when rows were unpadded ids: R-MAT 22 count 2.56 ms against 2.23, R-MAT 20 0.79 against 0.49; 2.00 ms since
+// an oct is one 256-bit load).
 //
 // Scheduler (degree-binned, one persistent launch):
 //   * work items = slices of an anchor's in-edge list with bounded probe work (built in ga_graph.cu);
@@ -788,12 +789,15 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
     if constexpr (MODE == TC_COUNT && !ALIVE) {
         if (groups) {
             const uint32_t ngroups = (uint32_t)(((uint64_t)tiny_end - tiny_first + 31) / 32);
+            // four groups a fetch, but no more than a warp's share: a group is a chain of up to 32 rounds of loads, and on
+            // small graphs four of them were the kernel (R-MAT 16 count 61.7 -> 49.7 us, R-MAT 18 127.7 -> 122.1)
+            const uint32_t take = min(kTinyGroups, max(1u, ngroups / (gridDim.x * kWarps)));
             for (;;) {
                 uint32_t g0 = 0;
-                if (lane == 0) g0 = atomicAdd(&a.sync->queue[2], kTinyGroups);
+                if (lane == 0) g0 = atomicAdd(&a.sync->queue[2], take);
                 g0 = __shfl_sync(GA_FULL_MASK, g0, 0);
                 if (g0 >= ngroups) break;
-                const uint32_t g1 = min(g0 + kTinyGroups, ngroups);
+                const uint32_t g1 = min(g0 + take, ngroups);
                 for (uint32_t g = g0; g < g1; g++)
                     hits += tiny_group<CT>(a, tiny_first + 32 * g, tiny_end, light_max_deg, s_incl, s_base, s_incl + 64,
                                            s_incl + 96, lane);
@@ -1261,7 +1265,7 @@ ga_status autotune(ga_graph* g) {
 // The first count of a graph that nothing has prepared, when the one-thread-per-edge form is known to be its choice (by
 // option or from the signature cache): counted straight from the CSR, since that form's plain version needs no index
 // and building one costs more than a single count saves (8,298 vertices: one-shot count 400 us with the index, 250
-// without; 1.7M vertices: 1.1 ms to build against 130 us a count). A second count shows that the graph stays in use
+// without, 111 since streams are reused; 1.7M vertices: 1.1 ms to build against 130 us a count). A second count shows that the graph stays in use
 // and builds the index. Misoriented graphs go on to ready(), which refuses them.
 static bool counts_without_index(const ga_graph* g) {
     if (g->index_ready || g->counted_bare || g->misoriented || !g->m) return false;
