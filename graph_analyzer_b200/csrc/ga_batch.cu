@@ -37,8 +37,8 @@ __device__ __forceinline__ uint32_t graph_of(const unsigned long long* __restric
 // col. Blocks take tiles of the whole batch's vertices, then of its edges, whatever graph they fall into: a thread finds
 // the graph of its first entry by binary search and steps on from there (one block per graph waited for the largest
 // graph: 256 graphs of up to 262,144 vertices, 8 M vertices and 55 M edges in all, took 28.4 ms to create with 5.4 ms of
-// it in that kernel, now 23.3 ms, the rest of it copies; one graph of 257,919 vertices 1.16 -> 0.36 ms). Flags in *err: 1 a graph's local rowptr does not start at 0
-// or end at its edge count, 2 a local id is >= its graph's vertex count.
+// it in that kernel, now 23.3 ms, the rest of it copies; one graph of 257,919 vertices 1.16 -> 0.36 ms). Flags in *err:
+// 1 a graph's local rowptr does not start at 0 or end at its edge count, 2 a local id is >= its graph's vertex count.
 constexpr uint32_t kUnionTile = 2048;
 __global__ void __launch_bounds__(256) k_union_csr(const unsigned long long* __restrict__ voff,
                                                    const unsigned long long* __restrict__ eoff,

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256) k_orient(const uint32_t* __restrict__ src
 // lane l: strides below E stay inside a thread (min / max), larger ones are one shuffle. k_in_lists then reads the
 // octs once, in order, and writes every entry's in-list record; it is a kernel of its own because it only waits (an
 // atomic with a result and a scattered write per entry) and wants all the warps an SM holds, which the sort's registers
-// do not leave (both in one kernel: 2.64 ms for R-MAT 22's rows of more than 8 entries). (64-bit (degree, id) keys
+// do not leave (both in one kernel: 2.64 ms for R-MAT 22's rows of more than 8 entries, apart 1.0 + 1.0). (64-bit (degree, id) keys
 // counted against each other in shared memory with the entries' positions carried along, then a scatter and a gather of
 // their own, took 4.0 ms of R-MAT 22's 5.4 ms of build kernels.)
 template <int E, int LANES>
@@ -694,7 +694,7 @@ void stream_release(int device, cudaStream_t st) {
     cudaStreamDestroy(st);
 }
 
-// Results of a megabyte and more go to pageable memory through two page-locked buffers: the next piece crosses the link
+// Results of half a megabyte and more go to pageable memory through two page-locked buffers: the next piece crosses the link
 // while several threads copy the last one out, whose time is mostly the page faults of a fresh array (6.8 MB: 1.1 ms by
 // one cudaMemcpy). At most four pairs of buffers exist in a process; a fifth concurrent download copies directly.
 constexpr size_t kStageBytes = 1u << 20, kStageMin = 512 * 1024;

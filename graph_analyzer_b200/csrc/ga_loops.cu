@@ -562,7 +562,11 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_frontier_update(
 // A warp takes up to 32 items at a time - one per lane, their entries flattened by a warp scan like the count's probe
 // lists - when there are that many per warp, else fewer: the first rounds of a peeling remove millions of vertices
 // whose lists hold some tens of entries, and one item at a time was a chain of four dependent loads for half-empty
-// warps (batch of 256 Holme-Kim graphs: 3.5 ms of updates a peeling).
+// warps (count and peeling of a batch of 256 Holme-Kim graphs: 9.4 ms, 3.5 of them in these updates, against 2.8).
+// A lane takes four entries at a time, so that their chains of loads (entry, then two states) overlap: that batch
+// 2.82 -> 2.52 ms, count and peeling of a 1.7M-vertex Holme-Kim graph 650 -> 585 us, R-MAT 22 cores 99.3 -> 96.1 ms
+// through their 225 grid rounds (two entries 2.60 ms and 600 us, eight like four).
+constexpr int kListUnroll = 4;
 __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, const uint2* __restrict__ inc,
                                                               const unsigned long long* __restrict__ inc_ptr,
                                                               const uint32_t* __restrict__ item_x,
@@ -596,26 +600,45 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
         s_x[w][lane] = x;
         s_des[w][lane] = 0;
         __syncwarp();
-        uint32_t owner = 0, end = s_incl[w][0], mine = 0;
-        for (uint32_t p = lane; p < tot; p += 32) {
-            if (end <= p) {
-                if (sg.count && mine) atomicAdd(&s_des[w][owner], mine);
-                destroyed += mine;
-                mine = 0;
+        uint32_t owner = 0, end = s_incl[w][0], mine = 0, mine_of = 0;   // triangles of item mine_of not booked yet
+        for (uint32_t p0 = lane; p0 < tot; p0 += 32 * kListUnroll) {
+            uint2 yw[kListUnroll];
+            uint32_t of[kListUnroll];
+            uint8_t sy[kListUnroll], sw[kListUnroll];
+#pragma unroll
+            for (int q = 0; q < kListUnroll; q++) {
+                const uint32_t p = p0 + 32 * q;
+                of[q] = GA_EMPTY;
+                if (p >= tot) continue;
                 while (end <= p) end = s_incl[w][++owner];
+                of[q] = owner;
+                yw[q] = inc[s_beg[w][owner] + p];
             }
-            const uint2 yw = inc[s_beg[w][owner] + p];
-            const uint32_t xv = s_x[w][owner];
-            const uint8_t sy = state[yw.x], sw = state[yw.y];
-            if (!sy || !sw) continue;                               // destroyed in an earlier round
-            if ((sy == 2 && yw.x < xv) || (sw == 2 && yw.y < xv)) continue;   // a smaller frontier corner owns it
-            mine++;
-            if (sy == 1) red_add(&tri[yw.x], 0xFFFFFFFFu);
-            if (sw == 1) red_add(&tri[yw.y], 0xFFFFFFFFu);
+#pragma unroll
+            for (int q = 0; q < kListUnroll; q++) {
+                sy[q] = sw[q] = 0;
+                if (of[q] != GA_EMPTY) sy[q] = state[yw[q].x], sw[q] = state[yw[q].y];
+            }
+#pragma unroll
+            for (int q = 0; q < kListUnroll; q++) {
+                if (!sy[q] || !sw[q]) continue;                     // past the end, or destroyed in an earlier round
+                const uint32_t xv = s_x[w][of[q]];
+                // a smaller frontier corner owns it
+                if ((sy[q] == 2 && yw[q].x < xv) || (sw[q] == 2 && yw[q].y < xv)) continue;
+                if (of[q] != mine_of) {
+                    if (sg.count && mine) atomicAdd(&s_des[w][mine_of], mine);
+                    destroyed += mine;
+                    mine = 0;
+                    mine_of = of[q];
+                }
+                mine++;
+                if (sy[q] == 1) red_add(&tri[yw[q].x], 0xFFFFFFFFu);
+                if (sw[q] == 1) red_add(&tri[yw[q].y], 0xFFFFFFFFu);
+            }
         }
         destroyed += mine;
         if (sg.count) {   // per-graph count of destroyed triangles, lanes of one graph combined
-            if (mine) atomicAdd(&s_des[w][owner], mine);
+            if (mine) atomicAdd(&s_des[w][mine_of], mine);
             __syncwarp();
             const uint32_t d = s_des[w][lane];
             const uint32_t peers = __match_any_sync(GA_FULL_MASK, d ? seg : GA_EMPTY);
@@ -651,7 +674,8 @@ __global__ void __launch_bounds__(256) k_frontier_update_list(LoopScalars* sc, c
 //     shared memory (1.4 for one in L2), so a CTA first sums its decrements by vertex in a small hash table and then
 //     sends each sum once (red.shared::cluster); they are complete at the second barrier. The local ids are read
 //     through L1: a round's entries name each vertex many times.
-// R-MAT 22 cores: 147 ms with every decrement sent on its own, 235 ms with the round's state in global memory.
+// R-MAT 22 cores: 235 ms with the round's state in global memory, 147 with every decrement sent on its own, 96 as it is
+// (9,318 rounds in the cluster, some 18,000 cycles each: 8,400 the update, the rest barriers, pushes and scans).
 constexpr uint32_t kSmallThreads = 1024;     // threads per CTA of the cluster
 constexpr uint32_t kSmallSlots = 8192;       // local vertices per CTA (8 per thread): 131,072 with 16 CTAs
 constexpr uint32_t kSmallWork = 1u << 20;    // incidence entries a round may read in the cluster
