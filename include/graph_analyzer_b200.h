@@ -164,8 +164,9 @@ ga_status ga_graph_prepare(ga_graph* g);
 /* Tuning knobs (the reference's compile-time macros SM_CAP / HASH_SLOTS / TASK_CHUNK, kernels.cuh:23-34, become
  * run-time options; GA_OPT_*_AUTO lets the autotuner choose). */
 typedef enum ga_option {
-    GA_OPT_TC_KERNEL = 1,     /* 0 auto (counts: the autotuned kernel; supports and incidence lists: the hash
-                                 kernel), 1 plain merge (one thread per oriented edge), 2 degree-binned hash probe */
+    GA_OPT_TC_KERNEL = 1,     /* 0 auto (counts: the autotuned kernel; supports: the same where rows are short, else
+                                 the hash kernel; incidence lists: the hash kernel), 1 plain (one thread per oriented
+                                 edge), 2 degree-binned hash probe                                                 */
     GA_OPT_LOOP_MODE = 2,     /* 0 auto, 1 host-driven rounds (one sync per round), 2 CUDA graph with a device
                                  while-node (no host sync inside the loop)                                          */
     GA_OPT_MAX_ROUNDS = 3,    /* round cap of device-resident loops (0 = n + 1)                                    */
@@ -175,7 +176,7 @@ typedef enum ga_option {
     GA_OPT_LIGHT_MAX_DEG = 6, /* anchors with out-degree <= this use per-warp tables (0 = 128, at most 256)        */
     GA_OPT_UPDATE_MODE = 7,   /* peeling/core rounds: 0 auto (triangle incidence lists when their 24*T bytes fit,
                                  else re-enumeration), 1 re-enumerate the frontier's triangles, 2 incidence lists   */
-    GA_OPT_COUNT_BITMAP = 8   /* counts in the hash kernel: 0 auto (a heavy anchor whose out-neighbours lie within
+    GA_OPT_COUNT_BITMAP = 8   /* passes of the hash kernel: 0 auto (a heavy anchor whose out-neighbours lie within
                                  32 x the table's words of places above it in the (degree, id) order is probed
                                  against a bitmap of them), 1 hash sets for every anchor                            */
 } ga_option;
