@@ -111,12 +111,19 @@ struct ga_items {
     uint64_t capacity = 0, bound = 0;   // entries allocated; at least the number of items
 };
 
-// Counters of a handle's triangle passes (device): work queues, the blocks that have finished, the triangles so far. All
-// zero between passes (the last block of a pass clears them). bounds: the item ranges of a shard.
+// Counters of a handle's triangle passes (device). Synchronous calls use the first work queues, `ticket` (blocks that have
+// finished) and `acc` (triangles so far), all zero between passes: the last block of a pass clears them. A pass that an
+// _async call enqueues shares none of these, since it may be captured and replayed beside other passes: it adds to the
+// caller's total, and its work queues, cleared before it, are the second ones, or for a captured pass the next of the
+// rest. bounds: the item ranges of a shard.
+constexpr uint32_t kCapturedWork = 64;
+struct ga_work {
+    uint32_t queue[4], bounds[6];
+};
 struct ga_sync {
-    uint32_t queue[4], ticket, pad;
+    ga_work work[2 + kCapturedWork];
+    uint32_t ticket, pad;
     unsigned long long acc;
-    uint32_t bounds[6];
 };
 
 struct ga_graph {
@@ -162,6 +169,7 @@ struct ga_graph {
     unsigned long long* d_scalars = nullptr;   // 64 slots
     unsigned long long* h_scalars = nullptr;   // their page-locked host side (64 slots; host_slot_acquire)
     ga_sync* sync = nullptr;                   // counters of the triangle passes
+    uint32_t captured = 0;                     // passes captured so far (whose work queues are next)
 
     // options (ga_option)
     int64_t opt_tc_kernel = 0, opt_loop_mode = 0, opt_max_rounds = 0, opt_update_mode = 0, opt_count_bitmap = 0;

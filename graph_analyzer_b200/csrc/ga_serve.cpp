@@ -68,7 +68,7 @@ uint64_t estimate_bytes(const GraphEntry& e, ga_request_kind kind) {
     const uint64_t octs = std::min(e.octs, (m + 7 * std::min(n, m)) / 8);   // at most that in any valid CSR
     const uint64_t items = std::min(m, std::min(n, m) + e.row_work / 128 + 1);   // at the smallest item work, 1,024
     uint64_t b = 4 * (n + 1) + 4 * (m + 4) + 4 * m + 4 * n;
-    b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (items + 1) + 1024;
+    b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (items + 1) + 4096;
     if (kind != GA_REQ_TC) {
         const uint64_t T = e.triangles != UINT64_MAX ? e.triangles : e.tri_bound;
         b += 29 * n + 8 * (n + 3 * T / 512 + 1) + 24 * T + 8 * (n + 1);

@@ -175,10 +175,12 @@ __device__ __forceinline__ uint32_t find_member(const TcArgs<CT>& a, const Ancho
     return j < an.dv && row[j] == x && (!ALIVE || a.alive[x]) ? j : GA_EMPTY;
 }
 
-// The end of a pass, called by all 256 threads of every block: the blocks' triangles meet in sync->acc, and the last
-// block writes the total where the caller wants it (device, and the handle's page-locked slot when the host waits for
-// it) and leaves the counters zero for the next pass - so a count is one launch, with nothing to clear before it and
-// nothing to copy after it (901 vertices: 20 us a call with two clears and a copy around the kernel).
+// The end of a pass, called by all 256 threads of every block. In a synchronous call the blocks' triangles meet in
+// sync->acc, and the last block writes the total where the caller wants it (device, and the handle's page-locked slot
+// when the host waits for it) and leaves the counters zero for the next pass - so a count is one launch, with nothing to
+// clear before it and nothing to copy after it (901 vertices: 20 us a call with two clears and a copy around the
+// kernel). An enqueued pass adds to the total cleared before it: replays of captured passes overlap, and would take
+// each other's blocks for their own in counters they share.
 template <class CT>
 __device__ __forceinline__ void finish_pass(unsigned long long local, const TcArgs<CT>& a) {
     __shared__ unsigned long long s_red[8];
@@ -188,12 +190,16 @@ __device__ __forceinline__ void finish_pass(unsigned long long local, const TcAr
     if (threadIdx.x != 0) return;
     unsigned long long t = 0;
     for (int w = 0; w < 8; w++) t += s_red[w];
+    if (!a.sync) {
+        if (t) atomicAdd(a.total, t);
+        return;
+    }
     if (t) atomicAdd(&a.sync->acc, t);
     __threadfence();
     if (atomicInc(&a.sync->ticket, gridDim.x - 1) != gridDim.x - 1) return;   // wraps to zero with the last block
     __threadfence();
     t = atomicExch(&a.sync->acc, 0ull);
-    for (int q = 0; q < 4; q++) a.sync->queue[q] = 0;   // every block is done with the queues
+    for (int q = 0; q < 4; q++) a.work->queue[q] = 0;   // every block is done with the queues
     *a.total = t;
     if (a.host_total) *a.host_total = t;
 }
@@ -688,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
         uint32_t *s_incl = wbase, *s_base = wbase + 32;
         wbase[64 + lane] = 0;   // ecnt
         for (;;) {
-            if (threadIdx.x == 0) s_item = h0 + atomicAdd(&a.sync->queue[0], 1u);
+            if (threadIdx.x == 0) s_item = h0 + atomicAdd(&a.work->queue[0], 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= h1) break;
@@ -753,7 +759,7 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
     const uint32_t nl = l1 - l0, total = nl + (groups ? 0u : t1 - t0);
     for (;;) {
         uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(&a.sync->queue[1], 1u);
+        if (lane == 0) i = atomicAdd(&a.work->queue[1], 1u);
         i = __shfl_sync(GA_FULL_MASK, i, 0);
         if (i >= total) break;
         const uint32_t item = i < nl ? l0 + i : t0 + (i - nl);
@@ -794,7 +800,7 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
             const uint32_t take = min(kTinyGroups, max(1u, ngroups / (gridDim.x * kWarps)));
             for (;;) {
                 uint32_t g0 = 0;
-                if (lane == 0) g0 = atomicAdd(&a.sync->queue[2], take);
+                if (lane == 0) g0 = atomicAdd(&a.work->queue[2], take);
                 g0 = __shfl_sync(GA_FULL_MASK, g0, 0);
                 if (g0 >= ngroups) break;
                 const uint32_t g1 = min(g0 + take, ngroups);
@@ -983,7 +989,7 @@ static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
     uint64_t want = (g->items.bound + kWarps - 1) / kWarps;
     uint32_t tiny_first = g->isolated, tiny_end = g->n;
     if (a.nshards > 1) {   // this shard's anchors (cut on the device)
-        uint32_t* b = g->sync->bounds;
+        uint32_t* b = a.work->bounds;
         k_shard_bounds<<<1, 32, 0, st>>>(g->anchor_work, g->n, g->items, a.shard, a.nshards, b);
         GA_CUDA(cudaGetLastError());
         bounds = b;
@@ -1063,7 +1069,6 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
     // A sharded count always uses the hash kernel unless one is forced: every GPU must cut the same partition, and
     // an autotuned choice could differ between GPUs.
     TcArgs<CT> a = a0;
-    a.sync = g->sync;
     GA_TRY(a.nshards > 1 ? prepare_shards(g) : prepare(g));
     int64_t kernel = g->opt_tc_kernel ? g->opt_tc_kernel
                                       : (MODE == TC_COUNT || (MODE != TC_LIST && g->row_work * 2 <= 5ull * g->m)) &&
@@ -1080,10 +1085,19 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
         if (MODE == TC_VSUP && g->n) GA_CUDA(cudaMemsetAsync(a.vsup, 0, (size_t)g->n * sizeof(CT), st));
         if (!index && MODE == TC_ESUP && g->m) GA_CUDA(cudaMemsetAsync(a.esup, 0, (size_t)g->m * sizeof(uint32_t), st));
     }
+    if (!g->m || a.enqueued) GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
     if (!g->m) {   // no kernel: the total is zero
-        GA_CUDA(cudaMemsetAsync(a.total, 0, sizeof(unsigned long long), st));
         if (a.host_total) *a.host_total = 0;
         return GA_OK;
+    }
+    a.work = g->sync->work;
+    if (!a.enqueued) {
+        a.sync = g->sync;
+    } else if (index && !octs) {   // the hash kernel's queues
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        GA_CUDA(cudaStreamIsCapturing(st, &capture));
+        a.work += capture == cudaStreamCaptureStatusNone ? 1 : 2 + g->captured++ % kCapturedWork;
+        GA_CUDA(cudaMemsetAsync(a.work->queue, 0, sizeof a.work->queue, st));
     }
     return index ? launch_index<MODE, ALIVE, CT>(g, a, octs) : launch_plain<MODE, ALIVE, CT>(g, a);
 }
@@ -1333,6 +1347,7 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles) {
     if (counts_without_index(g)) {
         g->counted_bare = true;
         a.sync = g->sync;
+        a.work = g->sync->work;
         GA_TRY((launch_plain<TC_COUNT, false, unsigned int>(g, a)));
     } else {
         GA_TRY(ready(g));
@@ -1363,6 +1378,7 @@ ga_status ga_tc_count_shard_async(ga_graph* g, uint32_t shard, uint32_t nshards,
     GA_TRY(use_device(g));
     TcArgs<unsigned int> a{};
     a.total = (unsigned long long*)d_partial;
+    a.enqueued = true;
     a.shard = shard;
     a.nshards = nshards;
     return run_tc<TC_COUNT, false, unsigned int>(g, a, true);
@@ -1374,6 +1390,7 @@ ga_status ga_tc_count_async(ga_graph* g, uint64_t* d_triangles) {
     GA_TRY(use_device(g));
     TcArgs<unsigned int> a{};
     a.total = (unsigned long long*)d_triangles;
+    a.enqueued = true;
     return run_tc<TC_COUNT, false, unsigned int>(g, a, true);
 }
 

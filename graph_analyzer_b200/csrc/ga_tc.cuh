@@ -36,12 +36,14 @@ struct TcArgs {
     uint32_t* overflow = nullptr;   // TC_LIST: entries that found their list full (must stay 0)
     // set by the launchers (alive is by place for the kernels on the index)
     TcIndex ix = {};
-    ga_sync* sync = nullptr;        // the handle's counters
+    ga_sync* sync = nullptr;        // where the blocks of a synchronous call meet (null: they add to *total)
+    ga_work* work = nullptr;        // this pass's work queues
     uint32_t* esupk = nullptr;      // ESUP: supports by padded position in colr, zeroed
     bool bitmaps = false;           // heavy anchors may use bitmaps
     // shard `shard` of `nshards` (0 = the whole graph): equal parts of the probe work (hash kernel) or of the edges
     // (plain kernel); the shards of a graph partition its triangles
     uint32_t shard = 0, nshards = 0;
+    bool enqueued = false;   // an _async call: the pass may run at any time, beside others of the handle
 };
 
 // One triangle pass on g's stream (asynchronous). total is written whole; zero_outputs: clear vsup/esup first.

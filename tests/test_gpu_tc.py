@@ -326,3 +326,43 @@ def test_index_row_lengths(ga, oracle, cuda_ok, rows):
             assert d.tc_count() == T and sum(d.tc_count_shard(i, 3) for i in range(3)) == T
             assert np.array_equal(d.support_edges()[1], sup)
             assert np.array_equal(d.support_vertices()[1], deg)
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+def test_overlapping_replays_of_captured_counts(ga, oracle, cuda_ok, kernel):
+    """Counts and shards of one handle, captured on different streams and replayed at the same time: every replay gives
+    its own total, and counts afterwards that overlap nothing are right too."""
+    import torch
+    g = ga.graph_from_pairs(12_000, ga.gen_holme_kim(12_000, 3, 5, 0.5, 0.6, seed=8))
+    T = oracle.triangles_serial(g)
+    with ga.DeviceGraph(g) as d:
+        d.set_option(ga.OPT_TC_KERNEL, kernel)
+        d.prepare()
+        parts = [d.tc_count_shard(i, 2) for i in range(2)]
+        out = torch.zeros(4, dtype=torch.int64, device="cuda")
+        enqueue = [lambda: d.tc_count_async(out[0:].data_ptr()), lambda: d.tc_count_async(out[1:].data_ptr()),
+                   lambda: d.tc_count_shard_async(0, 2, out[2:].data_ptr()),
+                   lambda: d.tc_count_shard_async(1, 2, out[3:].data_ptr())]
+        streams, graphs = [torch.cuda.Stream() for _ in enqueue], []
+        for st, call in zip(streams, enqueue):
+            d.set_stream(st.cuda_stream)
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1], stream=st):
+                call()
+        gate = torch.cuda.Stream()
+        for _ in range(100):
+            out.fill_(-1)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(gate):
+                torch.cuda._sleep(400_000)         # holds all replays back until the last one is enqueued
+                opened = torch.cuda.Event()
+                opened.record()
+            for st, gr in zip(streams, graphs):
+                st.wait_event(opened)
+                with torch.cuda.stream(st):
+                    gr.replay()
+            torch.cuda.synchronize()
+            assert out.tolist() == [T, T, *parts]
+        d.set_stream(None)
+        assert [d.tc_count() for _ in range(3)] == [T] * 3
+        del graphs

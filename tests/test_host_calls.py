@@ -1,0 +1,94 @@
+"""CPU tests of the library's host side against a fake CUDA runtime (tests/cpp/fake_cudart.cpp, linked with the
+library's own objects): which kernels a call launches, what it does under stream capture, and what it leaves behind when
+an allocation fails. Kernels do nothing there, so results are not looked at; the GPU tests check those."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+OPT_TC_KERNEL, OPT_LOOP_MODE = 1, 2
+GA_ERR_CUDA = 3
+
+
+class Lib:
+    """The library over the fake runtime."""
+
+    def __init__(self, path):
+        self.c = C.CDLL(path)
+        self.c.fake_log.restype = C.c_char_p
+        self.c.fake_live.restype = C.c_longlong
+        self.c.fake_fail_in.argtypes = [C.c_longlong]
+
+    def __getattr__(self, name):
+        return getattr(self.c, name)
+
+    def log(self):
+        return self.c.fake_log().decode().splitlines()
+
+    def launches(self):
+        return [line.split()[1] for line in self.log() if line.startswith("launch")]
+
+    def graph(self, n=64, stream=None):
+        """A handle of a path of n vertices (n - 1 edges)."""
+        rowptr = np.minimum(np.arange(n + 1, dtype=np.uint32), n - 1)
+        col = np.arange(1, n, dtype=np.uint32)
+        h = C.c_void_p()
+        s = self.c.ga_graph_create(rowptr.ctypes.data_as(C.c_void_p), col.ctypes.data_as(C.c_void_p), n, n - 1, 0, stream,
+                                   C.byref(h))
+        return s, h
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    from graph_analyzer_b200 import build
+    os.makedirs(build.BUILD_DIR, exist_ok=True)
+    objs = [build._compile(s, False) for s in build._sources()]
+    out = str(tmp_path_factory.mktemp("fake") / "libga_fake.so")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-fopenmp", "-Wl,-Bsymbolic", "-I", cuda,
+                           *objs, os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), "-o", out, "-lpthread"])
+    return Lib(out)
+
+
+@pytest.fixture
+def lib(fake_lib):
+    fake_lib.fake_reset()
+    yield fake_lib
+    fake_lib.fake_reset()
+
+
+@pytest.mark.parametrize("shard", [False, True])
+@pytest.mark.parametrize("kernel", [1, 2])
+def test_enqueued_counts_share_no_counters(lib, kernel, shard):
+    """An _async count clears the caller's total (and, in the hash form, work queues that are its own) before its kernel:
+    passes enqueued on one handle by several captures then share nothing they write."""
+    s, g = lib.graph()
+    assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(kernel)) == 0 and lib.ga_graph_prepare(g) == 0
+    stream = C.c_void_p(0x1000)
+    assert lib.ga_graph_set_stream(g, stream) == 0
+    totals = (C.c_uint64 * 2)(7, 7)
+    cleared = []
+    for i in range(2):
+        lib.fake_reset()
+        lib.fake_capture(stream, 1)
+        at = C.addressof(totals) + 8 * i
+        if shard:
+            assert lib.ga_tc_count_shard_async(g, 1, 3, C.c_void_p(at)) == 0
+        else:
+            assert lib.ga_tc_count_async(g, C.c_void_p(at)) == 0
+        lib.fake_capture(stream, 0)
+        log = lib.log()
+        assert all(line.endswith("captured") for line in log)
+        memsets = [line.split()[1:3] for line in log if line.startswith("memset")]
+        assert [str(at), "8"] in memsets
+        assert any(line.startswith("launch") for line in log[log.index(f"memset {at} 8 captured"):])
+        cleared.append({m[0] for m in memsets})
+        assert len(cleared[i]) == kernel          # the total, and the hash form's queues
+    assert not cleared[0] & cleared[1]
+    assert lib.ga_graph_destroy(g) == 0 and lib.fake_live() == 0
