@@ -170,6 +170,7 @@ struct ga_graph {
     unsigned long long* h_scalars = nullptr;   // their page-locked host side (64 slots; host_slot_acquire)
     ga_sync* sync = nullptr;                   // counters of the triangle passes
     uint32_t captured = 0;                     // passes captured so far (whose work queues are next)
+    bool items_captured = false;               // a captured pass reads the current work lists
 
     // options (ga_option)
     int64_t opt_tc_kernel = 0, opt_loop_mode = 0, opt_max_rounds = 0, opt_update_mode = 0, opt_count_bitmap = 0;

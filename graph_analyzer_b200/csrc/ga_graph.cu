@@ -864,6 +864,10 @@ static ga_status prepare_items(ga_graph* g) {
     const uint32_t n = g->n, m = g->m;
     if (!n || !m) return GA_OK;
     const uint64_t bound = std::min<uint64_t>(m, (uint64_t)std::min(n, m) + g->row_work * 8 / g->item_work + 1);
+    if (g->items_captured) {   // replays read those lists: they stay until the handle ends
+        g->items = ga_items{};
+        g->items_captured = false;
+    }
     if (bound > g->items.capacity) {
         dfree(g, g->items.v); dfree(g, g->items.k0); dfree(g, g->items.k1);
         g->items.v = g->items.k0 = g->items.k1 = nullptr;

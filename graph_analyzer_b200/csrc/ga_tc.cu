@@ -1096,6 +1096,7 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
     } else if (index && !octs) {   // the hash kernel's queues
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         GA_CUDA(cudaStreamIsCapturing(st, &capture));
+        g->items_captured |= capture != cudaStreamCaptureStatusNone;
         a.work += capture == cudaStreamCaptureStatusNone ? 1 : 2 + g->captured++ % kCapturedWork;
         GA_CUDA(cudaMemsetAsync(a.work->queue, 0, sizeof a.work->queue, st));
     }

@@ -12,7 +12,7 @@ import pytest
 
 from conftest import ROOT
 
-OPT_TC_KERNEL, OPT_LOOP_MODE = 1, 2
+OPT_TC_KERNEL, OPT_LOOP_MODE, OPT_ITEM_WORK = 1, 2, 4
 GA_ERR_CUDA = 3
 
 
@@ -27,6 +27,9 @@ class Lib:
 
     def __getattr__(self, name):
         return getattr(self.c, name)
+
+    def leaked(self):
+        return self.c.fake_live() - self.before
 
     def log(self):
         return self.c.fake_log().decode().splitlines()
@@ -59,6 +62,7 @@ def fake_lib(tmp_path_factory):
 @pytest.fixture
 def lib(fake_lib):
     fake_lib.fake_reset()
+    fake_lib.before = fake_lib.fake_live()
     yield fake_lib
     fake_lib.fake_reset()
 
@@ -91,4 +95,34 @@ def test_enqueued_counts_share_no_counters(lib, kernel, shard):
         cleared.append({m[0] for m in memsets})
         assert len(cleared[i]) == kernel          # the total, and the hash form's queues
     assert not cleared[0] & cleared[1]
-    assert lib.ga_graph_destroy(g) == 0 and lib.fake_live() == 0
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+def captured_call(lib, g, call):
+    """(status, log) of call(handle) on a handle whose stream is being captured."""
+    stream = C.c_void_p(0x2000)
+    assert lib.ga_graph_set_stream(g, stream) == 0
+    lib.fake_reset()
+    lib.fake_capture(stream, 1)
+    s = call(g)
+    log = lib.log()
+    lib.fake_capture(stream, 0)
+    return s, log
+
+
+TOTAL = C.c_uint64(0)
+CALLS = {"async": lambda lib, g: lib.ga_tc_count_async(g, C.byref(TOTAL))}
+
+
+def test_captured_passes_keep_their_work_lists(lib):
+    """Work lists that a captured pass reads stay as they are when other options, or the autotuner, make new ones."""
+    s, g = lib.graph()
+    assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(2)) == 0 and lib.ga_graph_prepare(g) == 0
+    for captured in (False, True, False):
+        if captured:
+            assert captured_call(lib, g, lambda g: CALLS["async"](lib, g))[0] == 0
+        held = lib.leaked()
+        assert lib.ga_graph_set_option(g, OPT_ITEM_WORK, C.c_int64(16 + 16 * captured + held)) == 0
+        assert lib.ga_graph_prepare(g) == 0
+        assert lib.leaked() == held + (4 if captured else 0)    # anchors, first and last in-edges, the bins' sizes
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
