@@ -160,6 +160,7 @@ struct ga_graph {
     bool index_ready = false;     // vrank .. in_rng built
     bool prepared = false;        // ... and the work items for the current light_max_deg / item_work
     bool counted_bare = false;    // counted once without the index (ga_tc_count)
+    cudaEvent_t built = nullptr;  // recorded behind the latest build of the index or the items
     ga_loops* loops = nullptr;    // peeling / core loop state, allocated on first use
     // a batch: the graph is the disjoint union of seg_count graphs, graph s owning vertices [seg_off[s], seg_off[s+1])
     const unsigned long long* seg_off = nullptr;
@@ -243,10 +244,16 @@ ga_status use_device(const ga_graph* g);
 // Frees the loop state (CUDA graphs, pinned buffers) of g.
 void destroy_loops(ga_graph* g);
 
-// Builds the index (once) and the work lists for the current options (idempotent).
+// Refuses (GA_ERR_CUDA) while g's stream is being captured: what a handle builds and keeps must not become part of a
+// graph, where it would not exist until the graph runs.
+ga_status not_captured(const ga_graph* g);
+// Builds the index (once) and the work lists for the current options (idempotent; refuses under capture).
 ga_status prepare(ga_graph* g);
 // prepare, and the work prefix that cuts shards.
 ga_status prepare_shards(ga_graph* g);
+// What the pass of an _async call needs. The call may be captured on a handle that is prepared, or that has been counted
+// without the index: what is missing then is built beside the capture.
+ga_status prepare_enqueued(ga_graph* g, bool shards);
 
 // Picks the count kernel for GA_OPT_TC_KERNEL = 0 from the graph's degree-distribution signature (cached per
 // signature; times both kernels once for a new one). Called by ga_graph_prepare.

@@ -896,11 +896,23 @@ static ga_status prepare_items(ga_graph* g) {
     return GA_OK;
 }
 
+ga_status not_captured(const ga_graph* g) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    GA_CUDA(cudaStreamIsCapturing(g->stream, &capture));
+    return capture == cudaStreamCaptureStatusNone
+               ? GA_OK
+               : fail(GA_ERR_CUDA, "the graph's stream is being captured and the call would build structures it keeps: "
+                                   "call ga_graph_prepare before the capture");
+}
+
 ga_status prepare(ga_graph* g) {
     if (g->prepared) return GA_OK;
     GA_TRY(use_device(g));
+    GA_TRY(not_captured(g));
     GA_TRY(prepare_index(g));
     GA_TRY(prepare_items(g));
+    if (!g->built) GA_CUDA(cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming));
+    GA_CUDA(cudaEventRecord(g->built, g->stream));
     g->prepared = true;
     return GA_OK;
 }
@@ -908,12 +920,38 @@ ga_status prepare(ga_graph* g) {
 ga_status prepare_shards(ga_graph* g) {
     GA_TRY(prepare(g));
     if (g->anchor_work) return GA_OK;
+    GA_TRY(not_captured(g));
     unsigned long long* w = nullptr;
     GA_TRY(dalloc(g, &w, (size_t)g->n + 1));
     g->anchor_work = w;
     k_widen<<<grid_for((uint64_t)g->n + 1, 256), 256, 0, g->stream>>>(g->work, g->n, w);
     GA_CUDA(cudaGetLastError());
     return scan_u64(g, w, (uint64_t)g->n + 1);
+}
+
+ga_status prepare_enqueued(ga_graph* g, bool shards) {
+    if (g->prepared && (!shards || g->anchor_work)) return GA_OK;
+    const bool counted = g->counted_bare && !g->index_ready;   // nothing of the handle is pending on its stream
+    if ((!g->prepared && !counted) || not_captured(g) == GA_OK) return shards ? prepare_shards(g) : prepare(g);
+    clear_error();
+    // on another stream, behind the last build, and complete before the pass is recorded
+    cudaStream_t own = g->stream, side = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    GA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    ga_status s = GA_OK;
+    if (stream_acquire(g->device, &side) != cudaSuccess) s = fail(GA_ERR_CUDA, "cudaStreamCreate failed");
+    if (s == GA_OK && g->built && cudaStreamWaitEvent(side, g->built, 0) != cudaSuccess)
+        s = fail(GA_ERR_CUDA, "cudaStreamWaitEvent failed");
+    if (s == GA_OK) {
+        g->stream = side;
+        s = shards ? prepare_shards(g) : prepare(g);
+        g->stream = own;
+    }
+    if (side && cudaStreamSynchronize(side) != cudaSuccess && s == GA_OK)
+        s = fail(GA_ERR_CUDA, "building beside a capture failed");
+    if (side) stream_release(g->device, side);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return s;
 }
 
 static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint32_t n, uint32_t m, int device,
@@ -1051,6 +1089,7 @@ ga_status ga_graph_destroy(ga_graph* g) {
     if (g->stream) cudaStreamSynchronize(g->stream);
     if (g->own_stream && g->stream) stream_release(g->device, g->stream);
     host_slot_release(g->h_scalars);
+    if (g->built) cudaEventDestroy(g->built);
     delete g;
     return GA_OK;
 }

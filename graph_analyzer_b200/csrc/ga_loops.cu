@@ -1374,6 +1374,7 @@ static ga_status ensure_graph(ga_graph* g) {
 // Common driver: init (full per-vertex count, state), then the round loop in the selected mode.
 template <int KIND>
 static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* result) {
+    GA_TRY(not_captured(g));
     GA_TRY(ready(g));
     GA_TRY(ensure_loops(g));
     ga_loops* L = g->loops;
@@ -1477,6 +1478,7 @@ ga_status core_numbers(ga_graph* g, const uint32_t** d_core, uint32_t* kmax) {
 }
 
 ga_status incidence_lists(ga_graph* g, const uint2** inc, const unsigned long long** inc_ptr, uint64_t* T) {
+    GA_TRY(not_captured(g));
     GA_TRY(ready(g));
     GA_TRY(ensure_loops(g));
     ga_loops* L = g->loops;

@@ -1159,21 +1159,23 @@ static uint64_t tune_key(const ga_graph* g) {
     return key;
 }
 
+// Takes the choice of a signature seen before, if there is one, for a handle without work items.
+static void choice_from_cache(ga_graph* g) {
+    if (g->opt_tc_kernel || g->tuned_kernel || g->prepared || !g->m) return;
+    const uint64_t key = tune_key(g);
+    std::lock_guard<std::mutex> lock(g_tune_mu);
+    tune_cache_load_locked();
+    auto it = g_tune_cache.find(key);
+    if (it == g_tune_cache.end()) return;
+    if (!g->light_max_deg_set) g->light_max_deg = it->second.light_max_deg;
+    if (!g->item_work_set) g->item_work = it->second.item_work;
+    g->tuned_kernel = it->second.kernel;
+    g->tune_key = key;
+    g->tune_ms = 0;
+}
+
 ga_status ready(ga_graph* g) {
-    // a signature seen before sets the options before the work items are built, so they are built once
-    if (g->opt_tc_kernel == 0 && !g->tuned_kernel && !g->prepared && g->m) {
-        const uint64_t key = tune_key(g);
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        tune_cache_load_locked();
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) {
-            if (!g->light_max_deg_set) g->light_max_deg = it->second.light_max_deg;
-            if (!g->item_work_set) g->item_work = it->second.item_work;
-            g->tuned_kernel = it->second.kernel;
-            g->tune_key = key;
-            g->tune_ms = 0;
-        }
-    }
+    choice_from_cache(g);   // before the work items are built, so they are built once
     GA_TRY(prepare(g));
     if (g->opt_tc_kernel == 0) GA_TRY(autotune(g));
     return GA_OK;
@@ -1282,15 +1284,10 @@ ga_status autotune(ga_graph* g) {
 // and building one costs more than a single count saves (8,298 vertices: one-shot count 400 us with the index, 250
 // without, 111 since streams are reused; 1.7M vertices: 1.1 ms to build against 130 us a count). A second count shows that the graph stays in use
 // and builds the index. Misoriented graphs go on to ready(), which refuses them.
-static bool counts_without_index(const ga_graph* g) {
+static bool counts_without_index(ga_graph* g) {
     if (g->index_ready || g->counted_bare || g->misoriented || !g->m) return false;
-    if (g->opt_tc_kernel) return g->opt_tc_kernel == 1;
-    if (g->tuned_kernel) return g->tuned_kernel == 1;
-    const uint64_t key = tune_key(g);
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    tune_cache_load_locked();
-    auto it = g_tune_cache.find(key);
-    return it != g_tune_cache.end() && it->second.kernel == 1;
+    choice_from_cache(g);   // kept: a later _async call counts with the same kernel
+    return (g->opt_tc_kernel ? g->opt_tc_kernel : g->tuned_kernel) == 1;
 }
 
 template ga_status run_tc<TC_COUNT, false, unsigned int>(ga_graph*, const TcArgs<unsigned int>&, bool);
@@ -1345,16 +1342,18 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles) {
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
     a.host_total = g->h_scalars;
-    if (counts_without_index(g)) {
-        g->counted_bare = true;
-        a.sync = g->sync;
-        a.work = g->sync->work;
-        GA_TRY((launch_plain<TC_COUNT, false, unsigned int>(g, a)));
-    } else {
+    if (!counts_without_index(g)) {
         GA_TRY(ready(g));
         GA_TRY((run_tc<TC_COUNT, false, unsigned int>(g, a, true)));
+        return read_total(g, triangles);
     }
-    return read_total(g, triangles);
+    GA_TRY(not_captured(g));
+    a.sync = g->sync;
+    a.work = g->sync->work;
+    GA_TRY((launch_plain<TC_COUNT, false, unsigned int>(g, a)));
+    GA_TRY(read_total(g, triangles));
+    g->counted_bare = true;
+    return GA_OK;
 }
 
 ga_status ga_tc_count_shard(ga_graph* g, uint32_t shard, uint32_t nshards, uint64_t* partial) {
@@ -1382,6 +1381,7 @@ ga_status ga_tc_count_shard_async(ga_graph* g, uint32_t shard, uint32_t nshards,
     a.enqueued = true;
     a.shard = shard;
     a.nshards = nshards;
+    GA_TRY(prepare_enqueued(g, nshards > 1));
     return run_tc<TC_COUNT, false, unsigned int>(g, a, true);
 }
 
@@ -1392,6 +1392,7 @@ ga_status ga_tc_count_async(ga_graph* g, uint64_t* d_triangles) {
     TcArgs<unsigned int> a{};
     a.total = (unsigned long long*)d_triangles;
     a.enqueued = true;
+    GA_TRY(prepare_enqueued(g, false));
     return run_tc<TC_COUNT, false, unsigned int>(g, a, true);
 }
 

@@ -366,3 +366,49 @@ def test_overlapping_replays_of_captured_counts(ga, oracle, cuda_ok, kernel):
         d.set_stream(None)
         assert [d.tc_count() for _ in range(3)] == [T] * 3
         del graphs
+
+
+@pytest.mark.parametrize("before", ["count", "prepare", "async"])
+def test_captured_counts_after_a_first_call(ga, oracle, cuda_ok, before):
+    """Counts and shards captured right after a first call - a synchronous count that did without the index, a prepare or an
+    enqueued count - give the count on every replay, as do the handle's other calls afterwards. Without such a call the
+    capture is refused and the handle stays usable."""
+    import torch
+    g = ga.graph_from_pairs(5000, ga.gen_holme_kim(5000, 3, 5, 0.5, 0.6, seed=21))
+    T = oracle.triangles_serial(g)
+    st, out = torch.cuda.Stream(), torch.zeros(4, dtype=torch.int64, device="cuda")
+
+    def capture(call):
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr, stream=st):
+            call()
+        return gr
+
+    with ga.DeviceGraph(g, stream=st.cuda_stream) as d:
+        d.set_option(ga.OPT_TC_KERNEL, 1)
+
+        def refused():
+            with pytest.raises(ga.GAError):
+                d.tc_count_async(out.data_ptr())
+            out[3:].zero_()                      # (so that the captured graph is not empty)
+        capture(refused)
+        if before == "count":
+            assert d.tc_count() == T
+        elif before == "prepare":
+            d.prepare()
+        else:
+            d.tc_count_async(out.data_ptr())
+        d.set_option(ga.OPT_TC_KERNEL, 0)
+        graphs = [capture(lambda: d.tc_count_shard_async(0, 2, out[1:].data_ptr())),
+                  capture(lambda: d.tc_count_shard_async(1, 2, out[2:].data_ptr())),
+                  capture(lambda: d.tc_count_async(out.data_ptr()))]
+        for _ in range(3):
+            out.fill_(-1)
+            torch.cuda.synchronize()
+            for gr in graphs:
+                gr.replay()
+            torch.cuda.synchronize()
+            assert out[0] == T and out[1] + out[2] == T
+            assert d.tc_count() == T and sum(d.tc_count_shard(i, 3) for i in range(3)) == T
+        assert np.array_equal(d.support_vertices()[1], oracle.triangle_degrees(g)[1])
+        del graphs

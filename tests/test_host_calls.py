@@ -87,8 +87,7 @@ def test_enqueued_counts_share_no_counters(lib, kernel, shard):
         else:
             assert lib.ga_tc_count_async(g, C.c_void_p(at)) == 0
         lib.fake_capture(stream, 0)
-        log = lib.log()
-        assert all(line.endswith("captured") for line in log)
+        log = [line for line in lib.log() if line.endswith("captured")]
         memsets = [line.split()[1:3] for line in log if line.startswith("memset")]
         assert [str(at), "8"] in memsets
         assert any(line.startswith("launch") for line in log[log.index(f"memset {at} 8 captured"):])
@@ -111,7 +110,68 @@ def captured_call(lib, g, call):
 
 
 TOTAL = C.c_uint64(0)
-CALLS = {"async": lambda lib, g: lib.ga_tc_count_async(g, C.byref(TOTAL))}
+CALLS = {
+    "async": lambda lib, g: lib.ga_tc_count_async(g, C.byref(TOTAL)),
+    "shard_async": lambda lib, g: lib.ga_tc_count_shard_async(g, 0, 2, C.byref(TOTAL)),
+    "count": lambda lib, g: lib.ga_tc_count(g, C.byref(TOTAL)),
+    "shard": lambda lib, g: lib.ga_tc_count_shard(g, 0, 2, C.byref(TOTAL)),
+    "prepare": lambda lib, g: lib.ga_graph_prepare(g),
+    "cores": lambda lib, g: lib.ga_core_decomposition(g, None, C.byref((C.c_uint32 * 2)())),
+    "peel": lambda lib, g: lib.ga_batch_peel(g, C.c_uint64(1), C.c_uint64(10), C.byref((C.c_uint64 * 3)()), None),
+}
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_nothing_is_built_inside_a_capture(lib, call):
+    """On a handle that nothing has prepared, a call under stream capture is refused and leaves nothing in the capture:
+    an index recorded there would not exist until the graph runs. The same call afterwards builds what it needs."""
+    s, g = lib.graph(n=200)
+    assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(2)) == 0
+    s, log = captured_call(lib, g, lambda g: CALLS[call](lib, g))
+    assert s == GA_ERR_CUDA and not [line for line in log if line.endswith("captured")]
+    lib.fake_reset()
+    assert CALLS[call](lib, g) == 0 and any("k_in_lists" in k for k in lib.launches())
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+@pytest.mark.parametrize("call", ["cores", "peel"])
+def test_no_loop_state_is_built_inside_a_capture(lib, call):
+    s, g = lib.graph(n=200)
+    assert s == 0 and lib.ga_graph_prepare(g) == 0
+    for run_other_first in (False, True):
+        if run_other_first:   # the other loop's state stands, this one's may not
+            assert CALLS["peel" if call == "cores" else "cores"](lib, g) == 0
+        s, log = captured_call(lib, g, lambda g: CALLS[call](lib, g))
+        assert s == GA_ERR_CUDA and not [line for line in log if line.startswith("alloc") and line.endswith("captured")]
+    assert CALLS[call](lib, g) == 0
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+@pytest.mark.parametrize("call,kernel", [("async", "k_tc_octs"), ("shard_async", "k_tc_hash")])
+@pytest.mark.parametrize("before", ["prepare", "count", "async"])
+def test_capture_after_a_first_call(lib, before, call, kernel):
+    """After ga_graph_prepare, a synchronous count (which may have done without the index) or an enqueued one, counts and
+    shards can be captured: what they still need is built outside the capture, and the kernel is the handle's choice."""
+    n = 300                                      # one signature: the first handle tunes (one-thread form), later ones know
+    s, first = lib.graph(n=n)
+    assert s == 0 and lib.ga_graph_prepare(first) == 0
+    s, g = lib.graph(n=n)
+    assert s == 0
+    lib.fake_reset()
+    assert CALLS[before](lib, g) == 0
+    if before == "count":
+        assert [k for k in lib.launches() if "k_tc_" in k] and not any("k_in_lists" in k for k in lib.launches())
+    if before == "async":                        # (enqueued on a handle whose choice nothing has looked up: the hash form)
+        kernel = "k_tc_hash"
+    s, log = captured_call(lib, g, lambda g: CALLS[call](lib, g))
+    assert s == 0
+    inside = [line for line in log if line.endswith("captured")]
+    assert not [line for line in inside if line.startswith(("alloc", "sync", "record", "wait"))]
+    ran = [line for line in inside if line.startswith("launch")]
+    assert kernel in ran[-1] and all("k_tc_" in k or "k_shard_bounds" in k for k in ran)
+    for h in (first, g):
+        assert lib.ga_graph_destroy(h) == 0
+    assert lib.leaked() == 0
 
 
 def test_captured_passes_keep_their_work_lists(lib):
