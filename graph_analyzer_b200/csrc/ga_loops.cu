@@ -23,7 +23,8 @@
 // (double-buffered by round parity) is retired by the next round's first kernel. In GA_OPT_LOOP_MODE 2
 // the round is the body of a CUDA graph conditional WHILE node (cudaGraphSetConditional from the tail), so the
 // whole loop is one graph launch; mode 1 launches the same kernels round by round and reads the 100-byte round state
-// back after each (the reference's host loop with its one sync per round).
+// back after each (the reference's host loop with its one sync per round). Mode 0 is mode 2, except for core loops that
+// one cluster can hold from the start (run_loop).
 //
 // Small core rounds: most of the thousands of core rounds of a power-law graph are small (R-MAT scale 22: 9,543
 // rounds, nine in ten with at most 131,072 alive vertices, the median removing three), and a grid round of three
@@ -1423,10 +1424,13 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     bool more = true;   // the final state is still to be read
     if (n > 0) {
         const bool graph_mode = g->opt_loop_mode != 1;
-        // A core loop whose vertices fit the cluster from the start is mostly one launch of it: the launches are made
-        // here, with a grid round between them where a round is too large, and only a loop that keeps alternating is
-        // captured as a graph, which costs more to make and release than such a loop takes
-        const uint32_t ctas = KIND == LOOP_CORE && graph_mode && L->lists == 1 ? (uint32_t)small_round_cluster(g->device) : 0;
+        // A core loop whose vertices fit the cluster from the start is mostly one launch of it: where the mode is left to
+        // the library, the launches are made here, with a grid round between them where a round is too large, and only a
+        // loop that keeps alternating is captured as a graph, which costs more to make and release (about 0.3 ms) than
+        // such a loop takes
+        const uint32_t ctas = KIND == LOOP_CORE && g->opt_loop_mode == 0 && L->lists == 1
+                                  ? (uint32_t)small_round_cluster(g->device)
+                                  : 0;
         if (ctas && (uint64_t)kSmallSlots * ctas >= n && !L->exec[LOOP_CORE]) {
             for (int i = 0; i < 4 && more; i++) {
                 if (i) GA_TRY(enqueue_round<KIND>(g, st, 0, 0));

@@ -167,8 +167,9 @@ typedef enum ga_option {
     GA_OPT_TC_KERNEL = 1,     /* 0 auto (counts: the autotuned kernel; supports: the same where rows are short, else
                                  the hash kernel; incidence lists: the hash kernel), 1 plain (one thread per oriented
                                  edge), 2 degree-binned hash probe                                                 */
-    GA_OPT_LOOP_MODE = 2,     /* 0 auto, 1 host-driven rounds (one sync per round), 2 CUDA graph with a device
-                                 while-node (no host sync inside the loop)                                          */
+    GA_OPT_LOOP_MODE = 2,     /* 0 auto (2; a core loop of at most 131,072 vertices is a few direct launches, each
+                                 with a sync, instead), 1 host-driven rounds (one sync per round), 2 CUDA graph with
+                                 a device while-node (no host sync inside the loop)                                */
     GA_OPT_MAX_ROUNDS = 3,    /* round cap of device-resident loops (0 = n + 1)                                    */
     GA_OPT_ITEM_WORK = 4,     /* probe work (list elements) per work item of the hash kernel (0 = 4096)            */
     GA_OPT_HEAVY_TABLE_BITS = 5, /* log2 buckets (4 slots each) of the block-wide hash set; anchors that need more

@@ -256,3 +256,25 @@ def test_core_rounds_at_cluster_limits(ga, oracle, cuda_ok, shape):
         for _ in range(2):       # again, on the state the first run left
             r = d.core_decomposition()
             assert (r.kmax, r.rounds) == (kmax, rounds) and np.array_equal(r.core, core)
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("low", [63, 64, 65, 200])
+def test_core_round_with_candidates_on_one_block(ga, oracle, cuda_ok, low, mode):
+    """Rounds whose candidates all belong to one block of the cluster (ids with one remainder modulo 16): up to 64 of them,
+    a block's share, run in the cluster, more go to a grid round between cluster launches (mode 0) or in the captured loop's
+    body (mode 2)."""
+    n = 16 * (low + 4)
+    pend = [16 * i + 3 for i in range(low)]                        # one triangle each, on an edge of the clique
+    clique = [v for v in range(n) if v % 16 != 3][:30]
+    e = [(a, b) for i, a in enumerate(clique) for b in clique[i + 1:]]
+    for i, p in enumerate(pend):
+        a, b = clique[i % 29], clique[i % 29 + 1]
+        e += [(p, a), (p, b)]
+    g = ga.build_graph_from_edges(n, ga.canonical_edges(np.array(e, np.uint32)))
+    core, kmax, rounds = oracle.core_levels_inc(g)
+    with ga.DeviceGraph(g) as d:
+        d.set_option(ga.OPT_LOOP_MODE, mode)
+        for _ in range(2):
+            r = d.core_decomposition()
+            assert (r.kmax, r.rounds) == (kmax, rounds) and np.array_equal(r.core, core)

@@ -186,3 +186,18 @@ def test_captured_passes_keep_their_work_lists(lib):
         assert lib.ga_graph_prepare(g) == 0
         assert lib.leaked() == held + (4 if captured else 0)    # anchors, first and last in-edges, the bins' sizes
     assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+@pytest.mark.parametrize("mode,graph", [(0, False), (2, True)])
+def test_core_loop_honours_the_loop_mode(lib, mode, graph):
+    """A core loop that fits one cluster is launched round by round only when the mode is automatic; mode 2 is one launch of
+    a captured graph, without a synchronisation inside the loop."""
+    s, g = lib.graph(n=200)
+    assert s == 0 and lib.ga_graph_set_option(g, OPT_LOOP_MODE, C.c_int64(mode)) == 0 and lib.ga_graph_prepare(g) == 0
+    for _ in range(2):
+        lib.fake_reset()
+        assert CALLS["cores"](lib, g) == 0
+        log = lib.log()
+        direct = [line for line in log if "k_core_small_rounds" in line and not line.endswith("captured")]
+        assert (log.count("graph launch"), len(direct)) == ((1, 0) if graph else (0, 1))
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
