@@ -1120,7 +1120,10 @@ ga_status ga_graph_prepare(ga_graph* g) {
     if (!g) return fail(GA_ERR_INVALID_ARGUMENT, "null graph");
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
-    return ready(g);
+    const bool builds = !g->prepared || (g->opt_tc_kernel == 0 && !g->tuned_kernel);
+    GA_TRY(ready(g));
+    if (builds) GA_CUDA(cudaStreamSynchronize(g->stream));   // the call ends with the structures built, not enqueued
+    return GA_OK;
 }
 
 ga_status ga_graph_set_option(ga_graph* g, ga_option opt, int64_t value) {

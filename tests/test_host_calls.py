@@ -201,3 +201,22 @@ def test_core_loop_honours_the_loop_mode(lib, mode, graph):
         direct = [line for line in log if "k_core_small_rounds" in line and not line.endswith("captured")]
         assert (log.count("graph launch"), len(direct)) == ((1, 0) if graph else (0, 1))
     assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+def test_prepare_returns_when_the_index_stands(lib):
+    """ga_graph_prepare waits for what it built - also where it need not time candidates, because the signature is known -
+    and for nothing when nothing was missing (it may then be called under capture)."""
+    n = 400
+    handles = [lib.graph(n=n) for _ in range(2)]
+    assert all(s == 0 for s, _ in handles)
+    for _, g in handles:
+        lib.fake_reset()
+        assert lib.ga_graph_prepare(g) == 0
+        log = lib.log()
+        launches = [i for i, line in enumerate(log) if line.startswith("launch")]
+        assert launches and "sync" in log[launches[-1]:]
+        s, log = captured_call(lib, g, lambda g: CALLS["prepare"](lib, g))
+        assert s == 0 and not log
+    for _, g in handles:
+        assert lib.ga_graph_destroy(g) == 0
+    assert lib.leaked() == 0
