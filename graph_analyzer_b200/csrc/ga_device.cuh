@@ -11,11 +11,13 @@
 #define GA_FULL_MASK 0xFFFFFFFFu
 #define GA_EMPTY 0xFFFFFFFFu
 
-// Returns GA_ERR_CUDA / GA_ERR_OUT_OF_MEMORY with the failing call's text when a CUDA call fails.
+// Returns GA_ERR_CUDA / GA_ERR_OUT_OF_MEMORY with the failing call's text when a CUDA call fails (and takes the error off
+// the runtime's record, where the next call's launch check would find it).
 #define GA_CUDA(call)                                                                                          \
     do {                                                                                                       \
         cudaError_t e_ = (call);                                                                               \
         if (e_ != cudaSuccess) {                                                                               \
+            (void)cudaGetLastError();                                                                          \
             return ::ga::fail(e_ == cudaErrorMemoryAllocation ? GA_ERR_OUT_OF_MEMORY : GA_ERR_CUDA,            \
                               "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);     \
         }                                                                                                      \

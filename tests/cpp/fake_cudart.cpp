@@ -24,6 +24,7 @@ std::set<void*> live;                         // pool allocations not freed yet
 std::set<const void*> capturing;              // streams being captured
 std::string text, last_kernel;
 long long fail_in = -1;                       // pool allocations until one fails (-1: none does)
+bool failed = false;                          // ... and whether one has
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct { dim3 grid, block; size_t smem; cudaStream_t st; } config;
 
@@ -40,7 +41,8 @@ extern "C" {
 
 // ---- what the tests use ----
 void fake_reset() { std::lock_guard<std::mutex> l(mu); text.clear(); fail_in = -1; capturing.clear(); last = cudaSuccess; }
-void fake_fail_in(long long k) { std::lock_guard<std::mutex> l(mu); fail_in = k; }
+void fake_fail_in(long long k) { std::lock_guard<std::mutex> l(mu); fail_in = k; failed = false; }
+int fake_failed() { std::lock_guard<std::mutex> l(mu); return failed; }
 long long fake_live() { std::lock_guard<std::mutex> l(mu); return (long long)live.size(); }
 void fake_capture(void* st, int on) {
     std::lock_guard<std::mutex> l(mu);
@@ -77,7 +79,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 // ---- memory ----
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t st) {
     std::lock_guard<std::mutex> l(mu);
-    if (fail_in >= 0 && fail_in-- == 0) return err(cudaErrorMemoryAllocation);
+    if (fail_in >= 0 && fail_in-- == 0) {
+        failed = true;
+        return err(cudaErrorMemoryAllocation);
+    }
     note("alloc", st);
     *p = std::calloc(n ? n : 1, 1);
     live.insert(*p);

@@ -13,7 +13,7 @@ import pytest
 from conftest import ROOT
 
 OPT_TC_KERNEL, OPT_LOOP_MODE, OPT_ITEM_WORK = 1, 2, 4
-GA_ERR_CUDA = 3
+GA_ERR_CUDA, GA_ERR_OUT_OF_MEMORY = 3, 4
 
 
 class Lib:
@@ -220,3 +220,38 @@ def test_prepare_returns_when_the_index_stands(lib):
     for _, g in handles:
         assert lib.ga_graph_destroy(g) == 0
     assert lib.leaked() == 0
+
+
+WORDS = (C.c_uint64 * 5000)()
+CALLS.update({
+    "supports": lambda lib, g: lib.ga_tc_support_edges(g, WORDS, None),
+    "vertex_supports": lambda lib, g: lib.ga_tc_support_vertices(g, WORDS, None),
+    "participation": lambda lib, g: lib.ga_tc_participation(g, WORDS, WORDS, None),
+    "density": lambda lib, g: lib.ga_core_level_density(g, WORDS, 0, C.byref(TOTAL), C.byref(TOTAL)),
+})
+
+
+def check_after_failed_allocations(lib, call, setup=()):
+    """Lets the k-th allocation of `call` fail, for every k: the call reports it or does without, and a repeat succeeds."""
+    for k in range(200):
+        s, g = lib.graph(n=5000)                  # (scans of more than one tile allocate too)
+        assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(2)) == 0
+        for c in setup:
+            assert CALLS[c](lib, g) == 0
+        lib.fake_fail_in(C.c_longlong(k))
+        s = CALLS[call](lib, g)
+        failed = lib.fake_failed()
+        lib.fake_fail_in(C.c_longlong(-1))
+        assert s in (0, GA_ERR_OUT_OF_MEMORY) and (failed or s == 0), (k, s)
+        if s:
+            assert CALLS[call](lib, g) == 0, k
+        assert lib.ga_graph_destroy(g) == 0, k
+        if not failed:
+            return k
+    raise AssertionError("still allocating")
+
+
+@pytest.mark.parametrize("call,setup", [("prepare", ()), ("count", ()), ("supports", ()), ("vertex_supports", ()),
+                                        ("participation", ()), ("density", ()), ("shard", ("prepare",)), ("shard", ())])
+def test_calls_after_failed_allocations(lib, call, setup):
+    assert check_after_failed_allocations(lib, call, setup) > 0
