@@ -221,6 +221,26 @@ inline cudaError_t pool_malloc(T** p, size_t bytes, cudaStream_t st) {
     return cudaMallocFromPoolAsync((void**)p, bytes, pool_of_current(), st);
 }
 
+// A temporary of a call, given back (stream-ordered) when it goes out of scope, whatever ends the scope.
+struct Scratch {
+    void* p = nullptr;
+    cudaStream_t st = nullptr;
+    explicit Scratch(cudaStream_t s) : st(s) {}
+    Scratch(const Scratch&) = delete;
+    ~Scratch() { if (p) cudaFreeAsync(p, st); }
+    template <class T>
+    ga_status alloc(T** out, size_t count) {
+        const size_t bytes = (count ? count : 1) * sizeof(T);
+        if (pool_malloc(&p, bytes, st) != cudaSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+            return fail(GA_ERR_OUT_OF_MEMORY, "device scratch of %zu bytes failed", bytes);
+        }
+        *out = (T*)p;
+        return GA_OK;
+    }
+};
+
 // Device allocation owned by g (stream-ordered from the pool on g's stream, freed at destroy), counted in g->bytes.
 template <class T>
 inline ga_status dalloc(ga_graph* g, T** p, size_t count) {

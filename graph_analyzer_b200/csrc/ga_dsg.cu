@@ -82,24 +82,6 @@ __global__ void k_list_triangles(const uint2* __restrict__ inc, const unsigned l
 
 namespace {
 
-// A stream-ordered scratch allocation from the library's pool, returned when it goes out of scope.
-struct Scratch {
-    void* p = nullptr;
-    cudaStream_t st = nullptr;
-    explicit Scratch(cudaStream_t s) : st(s) {}
-    ~Scratch() { if (p) cudaFreeAsync(p, st); }
-    template <class T>
-    ga_status alloc(T** out, size_t count) {
-        if (pool_malloc(&p, (count ? count : 1) * sizeof(T), st) != cudaSuccess) {
-            (void)cudaGetLastError();
-            p = nullptr;
-            return fail(GA_ERR_OUT_OF_MEMORY, "device scratch of %zu bytes failed", (count ? count : 1) * sizeof(T));
-        }
-        *out = (T*)p;
-        return GA_OK;
-    }
-};
-
 ga_status download(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     if (bytes) GA_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     return GA_OK;

@@ -103,19 +103,16 @@ static ga_status scan_impl(cudaStream_t st, const T* in, T* out, uint64_t n) {
         GA_CUDA(cudaGetLastError());
         return GA_OK;
     }
-    T* sums = nullptr;
-    GA_CUDA(pool_malloc((void**)&sums, nb * sizeof(T), st));
+    Scratch tmp(st);
+    T* sums;
+    GA_TRY(tmp.alloc(&sums, nb));
     k_scan_sums<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, sums);
-    ga_status s = GA_OK;
-    if (cudaGetLastError() != cudaSuccess) s = fail(GA_ERR_CUDA, "scan sums launch failed");
+    GA_CUDA(cudaGetLastError());
     const bool scanned = nb > kScanDirect;
-    if (s == GA_OK && scanned) s = scan_impl<T>(st, sums, sums, nb);
-    if (s == GA_OK) {
-        k_scan_tiles<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, sums, scanned);
-        if (cudaGetLastError() != cudaSuccess) s = fail(GA_ERR_CUDA, "scan launch failed");
-    }
-    cudaFreeAsync(sums, st);
-    return s;
+    if (scanned) GA_TRY(scan_impl<T>(st, sums, sums, nb));
+    k_scan_tiles<T><<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, sums, scanned);
+    GA_CUDA(cudaGetLastError());
+    return GA_OK;
 }
 
 ga_status scan_u64(ga_graph* g, unsigned long long* data, uint64_t n) {
@@ -806,9 +803,10 @@ static ga_status prepare_index(ga_graph* g) {
         const uint64_t ncounts = (uint64_t)kRankDigits * nchunks;
         uint32_t passes = 1;
         while (passes * kRankBits < 32 && (g->max_degree >> (passes * kRankBits)) != 0) passes++;
-        uint32_t *other = nullptr, *counts = nullptr;
-        GA_CUDA(pool_malloc((void**)&other, (size_t)n * 4, st));
-        GA_CUDA(pool_malloc((void**)&counts, ncounts * 4, st));
+        Scratch s_other(st), s_counts(st);
+        uint32_t *other, *counts;
+        GA_TRY(s_other.alloc(&other, n));
+        GA_TRY(s_counts.alloc(&counts, ncounts));
         const unsigned gr = (nchunks + kRankWarps - 1) / kRankWarps;
         const uint32_t* cur = nullptr;   // the identity (id order) before the first pass
         for (uint32_t ps = 0; ps < passes; ps++) {
@@ -825,10 +823,11 @@ static ga_status prepare_index(ga_graph* g) {
         GA_TRY(scan_impl<unsigned long long>(st, (unsigned long long*)g->pos, (unsigned long long*)g->pos,
                                              (uint64_t)n + 1));
         if (m) {
-            unsigned long long* cur = nullptr;
-            uint32_t* listed = nullptr;   // rows longer than 8, then their count
-            GA_CUDA(pool_malloc((void**)&cur, (size_t)n * 8, st));
-            GA_CUDA(pool_malloc((void**)&listed, ((size_t)n + 1) * 4, st));
+            Scratch s_cur(st), s_listed(st);
+            unsigned long long* cur;
+            uint32_t* listed;   // rows longer than 8, then their count
+            GA_TRY(s_cur.alloc(&cur, n));
+            GA_TRY(s_listed.alloc(&listed, (size_t)n + 1));
             GA_CUDA(cudaMemsetAsync(listed + n, 0, 4, st));
             k_in_cursors<<<gv, 256, 0, st>>>(g->pos, n, cur);
             GA_CUDA(cudaGetLastError());
@@ -844,13 +843,9 @@ static ga_status prepare_index(ga_graph* g) {
             GA_CUDA(cudaGetLastError());
             k_work<<<gv, 256, 0, st>>>(cur, n, g->work);
             GA_CUDA(cudaGetLastError());
-            cudaFreeAsync(cur, st);
-            cudaFreeAsync(listed, st);
         } else {
             GA_CUDA(cudaMemsetAsync(g->work, 0, (size_t)n * 4, st));
         }
-        cudaFreeAsync(other, st);
-        cudaFreeAsync(counts, st);
     }
     g->index_ready = true;
     return GA_OK;
@@ -879,10 +874,11 @@ static ga_status prepare_items(ga_graph* g) {
     }
     if (!g->items.info) GA_TRY(dalloc(g, &g->items.info, 3));
     g->items.bound = bound;
-    unsigned long long* cnt = nullptr;
-    uint32_t* tiny = nullptr;
-    GA_CUDA(pool_malloc((void**)&cnt, ((size_t)n + 1) * 8, st));
-    GA_CUDA(pool_malloc((void**)&tiny, ((size_t)n + 1) * 4, st));
+    Scratch s_cnt(st), s_tiny(st);
+    unsigned long long* cnt;
+    uint32_t* tiny;
+    GA_TRY(s_cnt.alloc(&cnt, (size_t)n + 1));
+    GA_TRY(s_tiny.alloc(&tiny, (size_t)n + 1));
     k_count_items<<<grid_for((uint64_t)n + 1, 256), 256, 0, st>>>(g->pos, g->dout, g->work, n, g->light_max_deg,
                                                                   g->item_work, cnt, tiny);
     GA_CUDA(cudaGetLastError());
@@ -891,8 +887,6 @@ static ga_status prepare_items(ga_graph* g) {
     k_emit_items<<<grid_for(bound, 256), 256, 0, st>>>(g->pos, cnt, tiny, n, g->items.v, g->items.k0, g->items.k1,
                                                        g->items.info);
     GA_CUDA(cudaGetLastError());
-    cudaFreeAsync(cnt, st);
-    cudaFreeAsync(tiny, st);
     return GA_OK;
 }
 

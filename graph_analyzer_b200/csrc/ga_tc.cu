@@ -1012,18 +1012,17 @@ static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
     TcArgs<CT> a = a0;
     a.ix = tc_index(g);
     a.bitmaps = !g->opt_count_bitmap;
-    void* tmp = nullptr;   // supports by position in colr, the mask by place
-    const size_t osize = MODE == TC_ESUP ? (size_t)g->octs * 8 * 4 : 0;
-    if (osize + (ALIVE ? g->n : 0)) {
-        GA_CUDA(pool_malloc(&tmp, osize + (ALIVE ? g->n : 0), st));
-        if (osize) GA_CUDA(cudaMemsetAsync(tmp, 0, osize, st));
-        if (MODE == TC_ESUP) a.esupk = (uint32_t*)tmp;
-        if (ALIVE) {
-            uint8_t* al = (uint8_t*)tmp + osize;
-            k_alive_places<<<grid_for(g->n, 256), 256, 0, st>>>(a0.alive, g->order, g->n, al);
-            GA_CUDA(cudaGetLastError());
-            a.alive = al;
-        }
+    Scratch tmp(st);   // supports by position in colr, or the mask by place
+    if (MODE == TC_ESUP) {
+        GA_TRY(tmp.alloc(&a.esupk, (size_t)g->octs * 8));
+        GA_CUDA(cudaMemsetAsync(a.esupk, 0, (size_t)g->octs * 8 * 4, st));
+    }
+    if (ALIVE) {
+        uint8_t* al;
+        GA_TRY(tmp.alloc(&al, g->n));
+        k_alive_places<<<grid_for(g->n, 256), 256, 0, st>>>(a0.alive, g->order, g->n, al);
+        GA_CUDA(cudaGetLastError());
+        a.alive = al;
     }
     if constexpr (MODE == TC_COUNT || MODE == TC_VSUP) {
         if (octs) {
@@ -1031,12 +1030,10 @@ static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
             GA_CUDA(cudaGetLastError());
         }
     }
-    ga_status s = GA_OK;
-    if (!octs) s = launch_hash<MODE, ALIVE, CT>(g, a);
-    if (s == GA_OK && MODE == TC_ESUP)
+    static_assert(MODE != TC_ESUP || !ALIVE, "one temporary");
+    if (!octs) GA_TRY((launch_hash<MODE, ALIVE, CT>(g, a)));
+    if (MODE == TC_ESUP)
         k_esup_fold<<<grid_for(g->m, 256), 256, 0, st>>>(a.ix, g->src, g->col, g->m, a.esupk, a0.esup);
-    if (tmp) cudaFreeAsync(tmp, st);
-    GA_TRY(s);
     GA_CUDA(cudaGetLastError());
     return GA_OK;
 }
@@ -1304,13 +1301,6 @@ using namespace ga;
 
 namespace {
 
-// Device buffer released at scope exit (stream-ordered).
-struct Scratch {
-    void* p = nullptr;
-    cudaStream_t st = nullptr;
-    ~Scratch() { if (p) cudaFreeAsync(p, st); }
-};
-
 // alive[v] = core[v] >= k; the number of such vertices is added to *cnt (one atomic per warp).
 __global__ void k_core_mask(const uint32_t* __restrict__ core, uint32_t n, uint32_t k, uint8_t* __restrict__ alive,
                             unsigned long long* cnt) {
@@ -1413,11 +1403,11 @@ ga_status ga_tc_support_edges(ga_graph* g, uint32_t* sup, uint64_t* triangles) {
     if (!g || (!sup && g->m)) return fail(GA_ERR_INVALID_ARGUMENT, "null argument");
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
-    Scratch s;
-    s.st = g->stream;
-    GA_CUDA(pool_malloc(&s.p, ((size_t)g->m + 1) * 4, g->stream));
-    GA_TRY(ga_tc_support_edges_device(g, (uint32_t*)s.p, triangles));
-    return download(g, sup, s.p, (size_t)g->m * 4);
+    Scratch s(g->stream);
+    uint32_t* d_sup;
+    GA_TRY(s.alloc(&d_sup, (size_t)g->m + 1));
+    GA_TRY(ga_tc_support_edges_device(g, d_sup, triangles));
+    return download(g, sup, d_sup, (size_t)g->m * 4);
 }
 
 ga_status ga_tc_support_vertices(ga_graph* g, uint64_t* deg, uint64_t* triangles) {
@@ -1425,15 +1415,13 @@ ga_status ga_tc_support_vertices(ga_graph* g, uint64_t* deg, uint64_t* triangles
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
     GA_TRY(ready(g));
-    Scratch s;
-    s.st = g->stream;
-    GA_CUDA(pool_malloc(&s.p, ((size_t)g->n + 1) * 8, g->stream));
+    Scratch s(g->stream);
     TcArgs<unsigned long long> a{};
+    GA_TRY(s.alloc(&a.vsup, (size_t)g->n + 1));
     a.total = g->d_scalars;
     a.host_total = g->h_scalars;
-    a.vsup = (unsigned long long*)s.p;
     GA_TRY((run_tc<TC_VSUP, false, unsigned long long>(g, a, true)));
-    GA_TRY(download(g, deg, s.p, (size_t)g->n * 8));
+    GA_TRY(download(g, deg, a.vsup, (size_t)g->n * 8));
     return read_total(g, triangles);
 }
 
@@ -1450,11 +1438,11 @@ ga_status ga_tc_participation(ga_graph* g, const uint8_t* alive, uint32_t* tri, 
         if (T_full >= (1ull << 32))
             return fail(GA_ERR_ARITH, "triangle count >= 2^32: uint32 tri[] counters could overflow");
     }
-    Scratch s;
-    s.st = g->stream;
-    GA_CUDA(pool_malloc(&s.p, ((size_t)g->n + 1) * 5, g->stream));
-    uint32_t* d_tri = (uint32_t*)s.p;
-    uint8_t* d_alive = (uint8_t*)(d_tri + g->n + 1);
+    Scratch s(g->stream);
+    uint8_t* d_alive;   // the mask behind the counts
+    GA_TRY(s.alloc(&d_alive, ((size_t)g->n + 1) * 5));
+    uint32_t* d_tri = (uint32_t*)d_alive;
+    d_alive += ((size_t)g->n + 1) * 4;
     if (g->n) GA_CUDA(cudaMemcpyAsync(d_alive, alive, g->n, cudaMemcpyHostToDevice, g->stream));
     TcArgs<unsigned int> a{};
     a.total = g->d_scalars;
@@ -1493,12 +1481,12 @@ ga_status ga_core_level_density(ga_graph* g, const uint32_t* core, uint32_t k, u
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
     GA_TRY(ready(g));
-    Scratch s;
-    s.st = g->stream;
+    Scratch s(g->stream);
     const size_t n = g->n;
-    GA_CUDA(pool_malloc(&s.p, (n + 1) * 5, g->stream));
-    uint32_t* d_core = (uint32_t*)s.p;
-    uint8_t* d_alive = (uint8_t*)(d_core + n + 1);
+    uint8_t* d_alive;   // the mask behind the core numbers
+    GA_TRY(s.alloc(&d_alive, (n + 1) * 5));
+    uint32_t* d_core = (uint32_t*)d_alive;
+    d_alive += (n + 1) * 4;
     unsigned long long* d_cnt = g->d_scalars + 1;
     GA_CUDA(cudaMemsetAsync(d_cnt, 0, 8, g->stream));
     if (n) {

@@ -232,12 +232,15 @@ CALLS.update({
 
 
 def check_after_failed_allocations(lib, call, setup=()):
-    """Lets the k-th allocation of `call` fail, for every k: the call reports it or does without, and a repeat succeeds."""
-    for k in range(200):
+    """Lets the k-th allocation of `call` fail, for every k: the call reports it or does without; a repeat succeeds and leaves
+    the handle with as many blocks as one that was never disturbed; destroying the handle frees everything."""
+    held = None
+    for k in range(-1, 200):
         s, g = lib.graph(n=5000)                  # (scans of more than one tile allocate too)
         assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(2)) == 0
         for c in setup:
             assert CALLS[c](lib, g) == 0
+        before = lib.leaked()
         lib.fake_fail_in(C.c_longlong(k))
         s = CALLS[call](lib, g)
         failed = lib.fake_failed()
@@ -245,8 +248,12 @@ def check_after_failed_allocations(lib, call, setup=()):
         assert s in (0, GA_ERR_OUT_OF_MEMORY) and (failed or s == 0), (k, s)
         if s:
             assert CALLS[call](lib, g) == 0, k
-        assert lib.ga_graph_destroy(g) == 0, k
-        if not failed:
+        if k < 0:
+            held = lib.leaked() - before
+        elif s:
+            assert lib.leaked() - before == held, k
+        assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0, k
+        if k >= 0 and not failed:
             return k
     raise AssertionError("still allocating")
 
