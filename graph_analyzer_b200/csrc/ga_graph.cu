@@ -917,10 +917,11 @@ ga_status prepare_shards(ga_graph* g) {
     GA_TRY(not_captured(g));
     unsigned long long* w = nullptr;
     GA_TRY(dalloc(g, &w, (size_t)g->n + 1));
-    g->anchor_work = w;
     k_widen<<<grid_for((uint64_t)g->n + 1, 256), 256, 0, g->stream>>>(g->work, g->n, w);
-    GA_CUDA(cudaGetLastError());
-    return scan_u64(g, w, (uint64_t)g->n + 1);
+    const ga_status s = scan_u64(g, w, (uint64_t)g->n + 1);
+    if (s == GA_OK) g->anchor_work = w;
+    else dfree(g, w);
+    return s;
 }
 
 ga_status prepare_enqueued(ga_graph* g, bool shards) {

@@ -262,3 +262,15 @@ def check_after_failed_allocations(lib, call, setup=()):
                                         ("participation", ()), ("density", ()), ("shard", ("prepare",)), ("shard", ())])
 def test_calls_after_failed_allocations(lib, call, setup):
     assert check_after_failed_allocations(lib, call, setup) > 0
+
+
+def test_shard_cut_after_a_failed_allocation(lib):
+    """A work prefix whose scan could not run is not kept: the next call makes it again."""
+    for k in (0, 1):                             # the prefix itself, the scan's temporary
+        s, g = lib.graph(n=5000)
+        assert s == 0 and CALLS["prepare"](lib, g) == 0
+        lib.fake_fail_in(C.c_longlong(k))
+        assert CALLS["shard"](lib, g) == GA_ERR_OUT_OF_MEMORY and lib.fake_failed()
+        lib.fake_reset()
+        assert CALLS["shard"](lib, g) == 0 and any("k_scan_tiles" in name for name in lib.launches())
+        assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
