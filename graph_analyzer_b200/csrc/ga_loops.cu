@@ -1137,8 +1137,7 @@ __global__ void k_seg_init(Segs sg, unsigned long long num, unsigned long long d
 // 64-bit words of a batch's results: T0, best_num, best_den, then best_round, rounds, status.
 static size_t seg_result_words(size_t graphs) { return 3 * graphs + (3 * graphs + 1) / 2; }
 
-static ga_status ensure_loops(ga_graph* g) {
-    if (g->loops) return GA_OK;
+static ga_status make_loops(ga_graph* g) {
     ga_loops* L = new ga_loops();
     g->loops = L;
     const uint32_t n = g->n;
@@ -1178,6 +1177,14 @@ static ga_status ensure_loops(ga_graph* g) {
     GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_frontier_update_list, 256, 0));
     L->grid_list = (unsigned)g->sm_count * (unsigned)std::max(occ, 1);
     return GA_OK;
+}
+
+// The loop state, whole or not at all.
+static ga_status ensure_loops(ga_graph* g) {
+    if (g->loops) return GA_OK;
+    const ga_status s = make_loops(g);
+    if (s != GA_OK) reset_loops(g);
+    return s;
 }
 
 // Releases the captured loop graphs. A captured round holds the addresses of the buffers it was captured with, so
@@ -1227,16 +1234,43 @@ __global__ void k_widen_counts(const uint32_t* __restrict__ tri, unsigned long l
 static ga_status segment_counts(ga_graph* g) {
     ga_loops* L = g->loops;
     cudaStream_t st = g->stream;
+    Scratch tmp(st);
     unsigned long long* sums = nullptr;
     if (L->lists != 1) {
-        GA_CUDA(pool_malloc((void**)&sums, ((size_t)g->n + 1) * 8, st));
+        GA_TRY(tmp.alloc(&sums, (size_t)g->n + 1));
         k_widen_counts<<<grid_for((uint64_t)g->n + 1, 256), 256, 0, st>>>(L->tri, sums, g->n);
         GA_CUDA(cudaGetLastError());
         GA_TRY(scan_u64(g, sums, (uint64_t)g->n + 1));
     }
     k_seg_T<<<grid_for(L->segs.count, 256), 256, 0, st>>>(sums ? sums : L->inc_ptr, L->segs);
     GA_CUDA(cudaGetLastError());
-    if (sums) cudaFreeAsync(sums, st);
+    return GA_OK;
+}
+
+// Fills the lists (inc_ptr and inc allocated, tri[] the vertices' counts).
+static ga_status fill_lists(ga_graph* g) {
+    ga_loops* L = g->loops;
+    cudaStream_t st = g->stream;
+    const uint32_t n = g->n;
+    Scratch tmp(st);
+    uint32_t* fill;   // n cursors + the overflow counter
+    GA_TRY(tmp.alloc(&fill, (size_t)n + 1));
+    k_widen_counts<<<grid_for((uint64_t)n + 1, 256), 256, 0, st>>>(L->tri, L->inc_ptr, n);
+    GA_CUDA(cudaGetLastError());
+    GA_TRY(scan_u64(g, L->inc_ptr, (uint64_t)n + 1));
+    GA_CUDA(cudaMemsetAsync(fill, 0, ((size_t)n + 1) * 4, st));
+    TcArgs<unsigned int> a{};
+    a.total = g->d_scalars + 1;
+    a.inc = L->inc;
+    a.inc_ptr = L->inc_ptr;
+    a.fill = fill;
+    a.overflow = fill + n;
+    GA_TRY((run_tc<TC_LIST, false, unsigned int>(g, a, true)));
+    uint32_t overflow = 0;
+    if (cudaMemcpyAsync(&overflow, fill + n, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+        return fail(GA_ERR_CUDA, "overflow read failed");
+    GA_CUDA(cudaStreamSynchronize(st));
+    if (overflow) return fail(GA_ERR_DEVICE_CHECK, "triangle listing disagreed with the count (%u entries)", overflow);
     return GA_OK;
 }
 
@@ -1247,7 +1281,6 @@ static ga_status build_lists(ga_graph* g, uint64_t T0) {
     ga_loops* L = g->loops;
     if (L->lists >= 0) return GA_OK;
     if (g->opt_update_mode == 1 || g->n == 0) { L->lists = 0; return GA_OK; }
-    cudaStream_t st = g->stream;
     const uint32_t n = g->n;
     const uint64_t entries = 3 * T0;
     const uint64_t need_items = (uint64_t)n + entries / kListChunk + 1;
@@ -1258,15 +1291,11 @@ static ga_status build_lists(ga_graph* g, uint64_t T0) {
         s = dalloc(g, &ix, need_items);
         if (s == GA_OK) s = dalloc(g, &ic, need_items);
     }
-    uint32_t* fill = nullptr;   // n cursors + the overflow counter
-    if (s == GA_OK && pool_malloc((void**)&fill, ((size_t)n + 1) * 4, st) != cudaSuccess) {
-        (void)cudaGetLastError();
-        s = fail(GA_ERR_OUT_OF_MEMORY, "incidence list cursors do not fit");
-    }
-    if (s != GA_OK) {
+    if (s == GA_OK) s = fill_lists(g);
+    if (s != GA_OK) {   // no half-made lists: the next call would take them for whole ones
         dfree(g, L->inc_ptr); dfree(g, L->inc); dfree(g, ix); dfree(g, ic);
         L->inc_ptr = nullptr; L->inc = nullptr;
-        if (g->opt_update_mode == 2) return s;
+        if (g->opt_update_mode == 2 || s != GA_ERR_OUT_OF_MEMORY) return s;
         clear_error();
         L->lists = 0;
         return GA_OK;
@@ -1278,24 +1307,6 @@ static ga_status build_lists(ga_graph* g, uint64_t T0) {
         dfree(g, L->item_x); dfree(g, L->item_c);
         L->item_x = ix; L->item_c = ic; L->item_cap = need_items;
     }
-    k_widen_counts<<<grid_for((uint64_t)n + 1, 256), 256, 0, st>>>(L->tri, L->inc_ptr, n);
-    GA_CUDA(cudaGetLastError());
-    GA_TRY(scan_u64(g, L->inc_ptr, (uint64_t)n + 1));
-    GA_CUDA(cudaMemsetAsync(fill, 0, ((size_t)n + 1) * 4, st));
-    TcArgs<unsigned int> a{};
-    a.total = g->d_scalars + 1;
-    a.inc = L->inc;
-    a.inc_ptr = L->inc_ptr;
-    a.fill = fill;
-    a.overflow = fill + n;
-    s = run_tc<TC_LIST, false, unsigned int>(g, a, true);
-    uint32_t overflow = 0;
-    if (s == GA_OK && cudaMemcpyAsync(&overflow, fill + n, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        s = fail(GA_ERR_CUDA, "overflow read failed");
-    cudaFreeAsync(fill, st);
-    GA_TRY(s);
-    GA_CUDA(cudaStreamSynchronize(st));
-    if (overflow) return fail(GA_ERR_DEVICE_CHECK, "triangle listing disagreed with the count (%u entries)", overflow);
     L->lists = 1;
     L->list_T = T0;
     return GA_OK;

@@ -228,6 +228,8 @@ CALLS.update({
     "vertex_supports": lambda lib, g: lib.ga_tc_support_vertices(g, WORDS, None),
     "participation": lambda lib, g: lib.ga_tc_participation(g, WORDS, WORDS, None),
     "density": lambda lib, g: lib.ga_core_level_density(g, WORDS, 0, C.byref(TOTAL), C.byref(TOTAL)),
+    "exact": lambda lib, g: lib.ga_exact_densest(g, C.byref((C.c_uint64 * 4)()), None),
+    "lists_then_peel": lambda lib, g: CALLS["exact"](lib, g) or CALLS["peel"](lib, g),
 })
 
 
@@ -274,3 +276,9 @@ def test_shard_cut_after_a_failed_allocation(lib):
         lib.fake_reset()
         assert CALLS["shard"](lib, g) == 0 and any("k_scan_tiles" in name for name in lib.launches())
         assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
+
+
+@pytest.mark.parametrize("call", ["peel", "cores", "exact", "lists_then_peel"])
+def test_loops_after_failed_allocations(lib, call):
+    """Loop state and incidence lists of which an allocation failed are not taken for complete ones by the next call."""
+    assert check_after_failed_allocations(lib, call, ("prepare",)) > 0
