@@ -98,13 +98,14 @@ namespace {
 
 using namespace ga;
 
-// Evicts idle resident graphs (least recently used first) until `need` more bytes fit. Caller holds the lock.
-bool make_room(ga_server* s, uint64_t need) {
+// Evicts idle resident graphs (least recently used first) until `need` more bytes fit. `keep`: the graph they are needed
+// for, whose resident part `need` does not count. Caller holds the lock.
+bool make_room(ga_server* s, uint64_t need, const GraphEntry* keep) {
     while (s->reserved + need > s->cfg.hbm_budget_bytes) {
         GraphEntry* victim = nullptr;
         for (auto& kv : s->graphs) {
             GraphEntry& e = kv.second;
-            if (e.dev && !e.busy && (!victim || e.last_use < victim->last_use)) victim = &e;
+            if (e.dev && !e.busy && &e != keep && (!victim || e.last_use < victim->last_use)) victim = &e;
         }
         if (!victim) return false;
         // the victim's work is complete, but the worker stream it last ran on may be busy with another request:
@@ -223,7 +224,7 @@ bool take_work(ga_server* s, Work* w, bool small_only) {
             s->cv_done.notify_all();
             return take_work(s, w, small_only);
         }
-        if (s->reserved + need > s->cfg.hbm_budget_bytes && !make_room(s, need)) continue;
+        if (s->reserved + need > s->cfg.hbm_budget_bytes && !make_room(s, need, &e)) continue;
         return admit(it, need, small);
     }
     return false;
@@ -238,7 +239,7 @@ bool grow_reservation(ga_server* s, Work* w, const GraphEntry& e, ga_request_kin
     if (full <= have) return true;
     const uint64_t extra = full - have;
     if (full > s->cfg.hbm_budget_bytes) return true;  // the loop runs and reports its own allocation failure
-    if (s->reserved + extra > s->cfg.hbm_budget_bytes && !make_room(s, extra)) return false;
+    if (s->reserved + extra > s->cfg.hbm_budget_bytes && !make_room(s, extra, &e)) return false;
     s->reserved += extra;
     w->reserve += extra;
     s->peak_reserved = std::max(s->peak_reserved, s->reserved);
@@ -396,7 +397,7 @@ void worker_main(ga_server* s, bool small_only) {
             }
             s->running--;
             // a resident graph above budget (its lists grew beyond the estimate) gives back idle memory
-            make_room(s, 0);
+            make_room(s, 0, nullptr);
         }
         s->cv_done.notify_all();
         s->cv_work.notify_all();

@@ -282,3 +282,55 @@ def test_shard_cut_after_a_failed_allocation(lib):
 def test_loops_after_failed_allocations(lib, call):
     """Loop state and incidence lists of which an allocation failed are not taken for complete ones by the next call."""
     assert check_after_failed_allocations(lib, call, ("prepare",)) > 0
+
+
+class ServerConfig(C.Structure):
+    _fields_ = [("device", C.c_int), ("budget", C.c_uint64), ("slots", C.c_uint32), ("fold_max_graphs", C.c_uint32),
+                ("fold_max_edges", C.c_uint32), ("small_slots", C.c_uint32), ("pin_min_edges", C.c_uint32)]
+
+
+class RequestResult(C.Structure):
+    _fields_ = [("status", C.c_int), ("triangles", C.c_uint64), ("peel", C.c_uint64 * 3), ("core", C.c_uint32 * 2),
+                ("queue_ms", C.c_double), ("run_ms", C.c_double), ("folded", C.c_uint32), ("resident_hit", C.c_uint32)]
+
+
+class ServerStats(C.Structure):
+    _fields_ = [(f, C.c_uint64) for f in ("submitted", "completed", "folded", "evictions", "resident", "resident_bytes",
+                                          "peak_reserved", "queued", "running", "reserved")]
+
+
+def serve_counts(lib, sizes, requests, budget):
+    """Counts, one after the other, of paths of sizes[i] vertices on a server of one worker: the results and the final
+    statistics."""
+    cfg = ServerConfig(0, budget, 1, 1, 1, 0xFFFFFFFF, 0)
+    s = C.c_void_p()
+    assert lib.ga_server_create(C.byref(cfg), C.byref(s)) == 0
+    ids, results = [], []
+    for n in sizes:
+        rowptr = np.minimum(np.arange(n + 1, dtype=np.uint32), n - 1)
+        col, gid = np.arange(1, n, dtype=np.uint32), C.c_uint64()
+        assert lib.ga_server_add_graph(s, rowptr.ctypes.data_as(C.c_void_p), col.ctypes.data_as(C.c_void_p), n, n - 1,
+                                       C.byref(gid)) == 0
+        ids.append(gid)
+    for i in requests:
+        ticket, r = C.c_uint64(), RequestResult()
+        assert lib.ga_server_submit(s, ids[i], 0, C.c_uint64(0), C.c_uint64(1), C.byref(ticket)) == 0
+        assert lib.ga_server_wait(s, ticket, C.byref(r)) == 0 and r.status == 0
+        results.append(r)
+    stats = ServerStats()
+    assert lib.ga_server_stats_get(s, C.byref(stats)) == 0 and lib.ga_server_destroy(s) == 0
+    return results, stats
+
+
+def test_a_request_does_not_evict_its_own_graph(lib):
+    """A second count, which needs the index that the first did without, makes room by evicting others, not the graph it is
+    about to run on."""
+    a, b, much = 30011, 29001, 1 << 30
+    for n in (a, b):                                                   # both signatures known: first counts without index
+        s, g = lib.graph(n=n)
+        assert s == 0 and lib.ga_graph_prepare(g) == 0 and lib.ga_graph_destroy(g) == 0
+    bare = serve_counts(lib, [a], [0], much)[1].resident_bytes
+    upload = serve_counts(lib, [b], [0], much)[1].peak_reserved
+    results, stats = serve_counts(lib, [a, b], [0, 1, 0], bare + upload)
+    assert [r.resident_hit for r in results] == [0, 0, 1] and stats.evictions == 1
+    assert stats.peak_reserved <= bare + upload
