@@ -911,6 +911,11 @@ ga_status prepare(ga_graph* g) {
     return GA_OK;
 }
 
+bool index_stands(const ga_graph* g) {
+    GA_GRAPH_LOCK(g);
+    return g->prepared;
+}
+
 ga_status prepare_shards(ga_graph* g) {
     GA_TRY(prepare(g));
     if (g->anchor_work) return GA_OK;

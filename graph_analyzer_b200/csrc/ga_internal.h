@@ -26,6 +26,9 @@ ga_status pool_keep_at_least(int device, uint64_t bytes);
 // Ends one pool_keep_at_least; when the last one ends the pool returns to its default and trims its cache.
 void pool_keep_release(int device);
 
+// Whether everything a count of g reads has been built.
+bool index_stands(const ga_graph* g);
+
 // 64-bit mixer (splitmix64 finaliser) and a small counter-based stream built on it: every (seed, stream, index)
 // gives an independent value, so generators are deterministic for any thread count.
 inline uint64_t mix64(uint64_t z) {

@@ -43,6 +43,7 @@ struct GraphEntry {
     const uint32_t* col() const { return pinned ? pinned + n + 1 : col_v.data(); }
     ga_graph* dev = nullptr;             // resident device graph
     uint64_t dev_bytes = 0;              // its device bytes (accounted in `reserved`)
+    bool indexed = false;                // its index stands: another count allocates nothing that stays
     uint64_t triangles = UINT64_MAX;     // known after the first request (sizes the incidence lists)
     uint64_t tri_bound = 0;              // sum over v of C(d+(v), 2): at least the triangle count
     uint64_t octs = 0, row_work = 0;     // sums of ceil(d+ / 8) and d+ * ceil(d+ / 8): size the index
@@ -140,8 +141,10 @@ void plan(const ga_server* s, const Request& r, const GraphEntry& e, uint64_t* n
     const bool staged = r.kind != GA_REQ_TC && e.triangles == UINT64_MAX && !*small;
     *full = estimate_bytes(e, staged ? GA_REQ_TC : r.kind);
     // bytes to reserve: the whole estimate for an upload; for a resident graph what it may still add (a loop its state
-    // and lists, a second count the index that the first did without)
-    *need = e.dev ? (*full > e.dev_bytes ? *full - e.dev_bytes : 0) : *full;
+    // and lists, a second count the index that the first did without - and nothing once that stands: the estimate is for
+    // the smallest item work, so what is left of it never comes down to zero)
+    const bool nothing = e.dev && e.indexed && (r.kind == GA_REQ_TC || staged);
+    *need = nothing ? 0 : e.dev ? (*full > e.dev_bytes ? *full - e.dev_bytes : 0) : *full;
 }
 
 // Rough device work of a request, for ordering the general lane: edges times a factor per kind, plus the upload.
@@ -373,6 +376,7 @@ void worker_main(ga_server* s, bool small_only) {
                     ga_graph_device_bytes(e.dev, &bytes);
                     s->reserved -= std::min(s->reserved, was_resident ? e.dev_bytes : 0);
                     e.dev_bytes = bytes;
+                    e.indexed = index_stands(e.dev);
                     s->reserved += bytes;
                     s->peak_reserved = std::max(s->peak_reserved, s->reserved);
                 }

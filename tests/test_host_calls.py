@@ -322,6 +322,17 @@ def serve_counts(lib, sizes, requests, budget):
     return results, stats
 
 
+def test_recount_of_an_indexed_graph_reserves_nothing(lib):
+    """A count on a resident graph whose index stands needs no more memory, whatever the estimate of an upload says: it
+    evicts nothing."""
+    a, b, much = 20011, 19001, 1 << 30
+    used = serve_counts(lib, [a], [0, 0], much)[1].resident_bytes      # with the index
+    upload = serve_counts(lib, [b], [0], much)[1].peak_reserved
+    results, stats = serve_counts(lib, [a, b], [0, 0, 1, 1, 0, 0], used + upload)
+    assert stats.evictions == 0 and [r.resident_hit for r in results] == [0, 1, 0, 1, 1, 1]
+    assert stats.peak_reserved <= used + upload
+
+
 def test_a_request_does_not_evict_its_own_graph(lib):
     """A second count, which needs the index that the first did without, makes room by evicting others, not the graph it is
     about to run on."""
