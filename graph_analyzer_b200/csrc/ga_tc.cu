@@ -1102,13 +1102,13 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
 
 // ---- autotuner ----------------------------------------------------------------------------------------------------
 // What runs fastest depends on the degree distribution: on graphs whose out-lists are all short (Holme-Kim with a
-// handful of edges per vertex) the plain merge can win, on skewed graphs with long lists (R-MAT) the degree-binned
-// hash kernel wins by several times, and within the hash kernel the bin cutoff between per-warp and block-wide sets
+// handful of edges per vertex) the one-thread-per-in-edge form (k_tc_octs, choice 1) can win, on skewed graphs with long
+// lists (R-MAT) the degree-binned hash kernel wins by several times, and within the hash kernel the bin cutoff between per-warp and block-wide sets
 // (light_max_deg) and the probe work per item (item_work, which sets how many warps share an anchor) move the time
 // by some percent. The choice - kernel, cutoff, item work - is cached per degree-distribution signature: log2 of n
 // and m and the fraction of edges whose source has out-degree in each log2 bucket, in sixteenths. A signature seen
 // before is answered from the cache (process-wide; also kept in the file named by GA_TUNE_CACHE when that is set); a
-// new one is decided by timing candidates on the graph: the hash kernel and the plain kernel at the current options,
+// new one is decided by timing candidates on the graph: both forms at the current options,
 // then the cutoffs {32, 64, 128, 256} and the item works {1024, 4096, 16384} (coordinate-wise; options the caller
 // set explicitly stay as set). Every candidate gives the same count.
 
@@ -1218,7 +1218,7 @@ ga_status autotune(ga_graph* g) {
     a.total = g->d_scalars + 2;
     cudaFuncAttributes fa;
     cudaFuncGetAttributes(&fa, k_tc_hash<TC_COUNT, false, unsigned int>);
-    cudaFuncGetAttributes(&fa, k_tc_plain<TC_COUNT, false, unsigned int>);
+    cudaFuncGetAttributes(&fa, k_tc_octs<TC_COUNT, false, unsigned int>);
     ga_status s = GA_OK;
     // best of two launches of candidate c
     auto time_of = [&](const TuneChoice& c, float* ms) -> ga_status {
@@ -1240,7 +1240,7 @@ ga_status autotune(ga_graph* g) {
     TuneChoice hash{2, g->light_max_deg, g->item_work}, plain{1, g->light_max_deg, g->item_work};
     float hash_ms = 0, plain_ms = 0;
     s = time_of(hash, &hash_ms);
-    if (s == GA_OK) s = time_of(plain, &plain_ms);   // the plain kernel does not use the items
+    if (s == GA_OK) s = time_of(plain, &plain_ms);   // this form does not use the items
     for (uint32_t light : {32u, 64u, 128u, 256u}) {   // the bin cutoff, at the current item work
         if (s != GA_OK || g->light_max_deg_set || light == hash.light_max_deg) continue;
         TuneChoice c = hash;
@@ -1278,9 +1278,15 @@ ga_status autotune(ga_graph* g) {
 
 // The first count of a graph that nothing has prepared, when the one-thread-per-edge form is known to be its choice (by
 // option or from the signature cache): counted straight from the CSR, since that form's plain version needs no index
-// and building one costs more than a single count saves (8,298 vertices: one-shot count 400 us with the index, 250
-// without, 111 since streams are reused; 1.7M vertices: 1.1 ms to build against 130 us a count). A second count shows that the graph stays in use
-// and builds the index. Misoriented graphs go on to ready(), which refuses them.
+// and building one costs more than a single count saves. The choice was made for k_tc_octs and this runs k_tc_plain, which
+// loses more on longer rows; but where it loses to index + octs, the choice is the hash form. First calls on a new
+// handle, us, k_tc_plain / index + k_tc_octs / index + hash, with row_work / m (octs to an edge's row):
+//   chosen:     Holme-Kim 8,298 vertices 17-24 / 117-153 / 154-198 (1.0-2.5), 1.7M 155 / 600 / 782 (1.0), 381 / 946 / 1,202
+//               (1.1), 1,718 / 2,860 / 3,119 (2.5); R-MAT 10 18-25 / 85-92 / 102-117 (1.1-3.1), R-MAT 14 25-39 / 148-169 /
+//               183-211 (1.7-4.1), R-MAT 16 51 / 181 / 231 (3.4), R-MAT 18 77 / 239 / 284 (2.7)
+//   not chosen: R-MAT 18 589 / 617 / 433 (8.0), 1,874 / 1,416 / 605 (14.0); Holme-Kim 1.7M 7,755 / 6,902 / 5,579 (4.9)
+// A second count shows that the graph stays in use and builds the index. Misoriented graphs go on to ready(), which
+// refuses them.
 static bool counts_without_index(ga_graph* g) {
     if (g->index_ready || g->counted_bare || g->misoriented || !g->m) return false;
     choice_from_cache(g);   // kept: a later _async call counts with the same kernel

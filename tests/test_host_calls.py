@@ -345,3 +345,16 @@ def test_a_request_does_not_evict_its_own_graph(lib):
     results, stats = serve_counts(lib, [a, b], [0, 1, 0], bare + upload)
     assert [r.resident_hit for r in results] == [0, 0, 1] and stats.evictions == 1
     assert stats.peak_reserved <= bare + upload
+
+
+def test_autotuner_loads_what_it_times(lib):
+    """The code of every kernel the autotuner times is loaded before the first timed launch."""
+    s, g = lib.graph(n=777)
+    assert s == 0
+    lib.fake_reset()
+    assert lib.ga_graph_prepare(g) == 0
+    log = lib.log()
+    loaded = {line.split()[1] for line in log if line.startswith("load")}
+    timed = {line.split()[1] for line in log if line.startswith("launch") and "k_tc_" in line}
+    assert len(timed) == 2 and timed == loaded
+    assert lib.ga_graph_destroy(g) == 0
