@@ -4,8 +4,9 @@
 // vertex offset to its local ids, the oriented CSR of the DISJOINT UNION of its graphs: a vertex's degree inside the
 // union equals its degree inside its own graph, so the (degree, id) orientation of every graph is kept, and no
 // triangle crosses two graphs. Hence
-//   * one launch of the degree-binned hash kernel counts every graph at once (its device work queue hands out items
-//     of all graphs, largest bins first), and per-graph counts are a segmented sum of the per-vertex counts;
+//   * one pass counts the triangles of every vertex of all graphs at once (run_tc's choice of kernel, as for one graph),
+//     and a graph's count is a third of its vertices' sum: a difference of prefix sums at its offsets, or of the offsets
+//     into the incidence lists once a peeling has built those, which then runs no count at all;
 //   * one device-resident peeling loop (a CUDA graph with a conditional WHILE node) peels every graph at once, with
 //     per-graph T, alive count, threshold, best density, round count and status (ga_loops.cu, "segments"), so each
 //     graph's result is identical to peeling it alone.
@@ -34,11 +35,12 @@ __device__ __forceinline__ uint32_t graph_of(const unsigned long long* __restric
 }
 
 // Builds the union CSR: global rowptr[vtx_off[s] + v] = edge_off[s] + local rowptr, global col = vtx_off[s] + local
-// col. Blocks take tiles of the whole batch's vertices, then of its edges, whatever graph they fall into: a thread finds
-// the graph of its first entry by binary search and steps on from there (one block per graph waited for the largest
-// graph: 256 graphs of up to 262,144 vertices, 8 M vertices and 55 M edges in all, took 28.4 ms to create with 5.4 ms of
-// it in that kernel, now 23.3 ms, the rest of it copies; one graph of 257,919 vertices 1.16 -> 0.36 ms). Flags in *err:
-// 1 a graph's local rowptr does not start at 0 or end at its edge count, 2 a local id is >= its graph's vertex count.
+// col. Blocks take tiles of the whole batch's vertices, then of its edges, whatever graph they fall into: a thread
+// finds the graph of its first entry by binary search and steps on from there (one block per graph waited for the
+// largest graph: 256 graphs of up to 262,144 vertices, 8 M vertices and 55 M edges in all, took 28.4 ms to create with
+// 5.4 ms of it in that kernel, now 23.3 ms, the rest of it copies; one graph of 257,919 vertices 1.16 -> 0.36 ms).
+// Flags in *err: 1 a graph's local rowptr does not start at 0 or end at its edge count, 2 a local id is >= its graph's
+// vertex count.
 constexpr uint32_t kUnionTile = 2048;
 __global__ void __launch_bounds__(256) k_union_csr(const unsigned long long* __restrict__ voff,
                                                    const unsigned long long* __restrict__ eoff,

@@ -11,8 +11,8 @@
 #define GA_FULL_MASK 0xFFFFFFFFu
 #define GA_EMPTY 0xFFFFFFFFu
 
-// Returns GA_ERR_CUDA / GA_ERR_OUT_OF_MEMORY with the failing call's text when a CUDA call fails (and takes the error off
-// the runtime's record, where the next call's launch check would find it).
+// Returns GA_ERR_CUDA / GA_ERR_OUT_OF_MEMORY with the failing call's text when a CUDA call fails (and takes the error
+// off the runtime's record, where the next call's launch check would find it).
 #define GA_CUDA(call)                                                                                          \
     do {                                                                                                       \
         cudaError_t e_ = (call);                                                                               \
@@ -113,11 +113,11 @@ struct ga_items {
     uint64_t capacity = 0, bound = 0;   // entries allocated; at least the number of items
 };
 
-// Counters of a handle's triangle passes (device). Synchronous calls use the first work queues, `ticket` (blocks that have
-// finished) and `acc` (triangles so far), all zero between passes: the last block of a pass clears them. A pass that an
-// _async call enqueues shares none of these, since it may be captured and replayed beside other passes: it adds to the
-// caller's total, and its work queues, cleared before it, are the second ones, or for a captured pass the next of the
-// rest. bounds: the item ranges of a shard.
+// Counters of a handle's triangle passes (device). Synchronous calls use the first work queues, `ticket` (blocks that
+// have finished) and `acc` (triangles so far), all zero between passes: the last block of a pass clears them. A pass
+// that an _async call enqueues shares none of these, since it may be captured and replayed beside other passes: it adds
+// to the caller's total, and its work queues, cleared before it, are the second ones, or for a captured pass the next
+// of the rest. bounds: the item ranges of a shard.
 constexpr uint32_t kCapturedWork = 64;
 struct ga_work {
     uint32_t queue[4], bounds[6];
@@ -273,8 +273,8 @@ ga_status not_captured(const ga_graph* g);
 ga_status prepare(ga_graph* g);
 // prepare, and the work prefix that cuts shards.
 ga_status prepare_shards(ga_graph* g);
-// What the pass of an _async call needs. The call may be captured on a handle that is prepared, or that has been counted
-// without the index: what is missing then is built beside the capture.
+// What the pass of an _async call needs. The call may be captured on a handle that is prepared, or that has been
+// counted without the index: what is missing then is built beside the capture.
 ga_status prepare_enqueued(ga_graph* g, bool shards);
 
 // Picks the count kernel for GA_OPT_TC_KERNEL = 0 from the graph's degree-distribution signature (cached per

@@ -23,7 +23,7 @@
 
 namespace ga {
 
-// ---- exclusive scan: tiles of 512 threads x 8 elements, two launches -------------------------------------------------
+// ---- exclusive scan: tiles of 512 threads x 8 elements, two launches ------------------------------------------------
 // k_scan_sums writes every tile's sum; k_scan_tiles adds up the sums of the tiles before its own itself (a few KB from
 // L2 for the sizes here) and scans its tile from registers, so there is no third launch for the sums. Above
 // kScanDirect tiles the sums are scanned first.
@@ -256,9 +256,9 @@ __global__ void __launch_bounds__(256) k_orient(const uint32_t* __restrict__ src
 // lane l: strides below E stay inside a thread (min / max), larger ones are one shuffle. k_in_lists then reads the
 // octs once, in order, and writes every entry's in-list record; it is a kernel of its own because it only waits (an
 // atomic with a result and a scattered write per entry) and wants all the warps an SM holds, which the sort's registers
-// do not leave (both in one kernel: 2.64 ms for R-MAT 22's rows of more than 8 entries, apart 1.0 + 1.0). (64-bit (degree, id) keys
-// counted against each other in shared memory with the entries' positions carried along, then a scatter and a gather of
-// their own, took 4.0 ms of R-MAT 22's 5.4 ms of build kernels.)
+// do not leave (both in one kernel: 2.64 ms for R-MAT 22's rows of more than 8 entries, apart 1.0 + 1.0). (64-bit
+// (degree, id) keys counted against each other in shared memory with the entries' positions carried along, then a
+// scatter and a gather of their own, took 4.0 ms of R-MAT 22's 5.4 ms of build kernels.)
 template <int E, int LANES>
 __device__ __forceinline__ void sort_keys(uint32_t (&k)[E], uint32_t l) {
 #pragma unroll
@@ -398,9 +398,10 @@ __global__ void __launch_bounds__(128) k_place_rows_listed(const uint32_t* __res
     }
 }
 
-// One lane per entry of colr: the entry x of place a's row is the in-edge a->x, whose record goes to the next free place
-// of x's in-list. cur[x] holds that place in its low word and the octs x's in-edges have to probe in its high word, so
-// one 64-bit atomic serves both (neither reaches 2^32: an in-edge with a suffix of s octs needs a row of 8(s-1) others).
+// One lane per entry of colr: the entry x of place a's row is the in-edge a->x, whose record goes to the next free
+// place of x's in-list. cur[x] holds that place in its low word and the octs x's in-edges have to probe in its high
+// word, so one 64-bit atomic serves both (neither reaches 2^32: an in-edge with a suffix of s octs needs a row of
+// 8(s-1) others).
 __global__ void __launch_bounds__(256) k_in_lists(const uint32_t* __restrict__ colr, const uint32_t* __restrict__ osrc,
                                                   const uint2* __restrict__ pos, uint64_t entries,
                                                   unsigned long long* __restrict__ cur,
@@ -691,9 +692,9 @@ void stream_release(int device, cudaStream_t st) {
     cudaStreamDestroy(st);
 }
 
-// Results of half a megabyte and more go to pageable memory through two page-locked buffers: the next piece crosses the link
-// while several threads copy the last one out, whose time is mostly the page faults of a fresh array (6.8 MB: 1.1 ms by
-// one cudaMemcpy). At most four pairs of buffers exist in a process; a fifth concurrent download copies directly.
+// Results of half a megabyte and more go to pageable memory through two page-locked buffers: the next piece crosses the
+// link while several threads copy the last one out, whose time is mostly the page faults of a fresh array (6.8 MB: 1.1
+// ms by one cudaMemcpy). At most four pairs of buffers exist in a process; a fifth concurrent download copies directly.
 constexpr size_t kStageBytes = 1u << 20, kStageMin = 512 * 1024;
 constexpr int kStages = 4, kStageThreads = 6;
 static std::mutex g_stage_mu;
@@ -985,10 +986,7 @@ static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint
         g->own_stream = true;
     }
     if ((s = dalloc(g, &g->rowptr, (size_t)n + 1)) != GA_OK) return bail(s);
-    // col is padded by 4 zero entries so that 16-byte (quad) loads of the last row stay inside the allocation
-    if ((s = dalloc(g, &g->col, (size_t)m + 4)) != GA_OK) return bail(s);
-    if (cudaMemsetAsync(g->col + m, 0, 16, g->stream) != cudaSuccess)
-        return bail(fail(GA_ERR_CUDA, "cudaMemsetAsync failed"));
+    if ((s = dalloc(g, &g->col, m)) != GA_OK) return bail(s);
     if ((s = dalloc(g, &g->d_scalars, 64)) != GA_OK) return bail(s);
     if ((s = dalloc(g, &g->sync, 1)) != GA_OK) return bail(s);
     if (!(g->h_scalars = host_slot_acquire())) return bail(fail(GA_ERR_OUT_OF_MEMORY, "page-locked slot failed"));

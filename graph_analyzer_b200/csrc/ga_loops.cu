@@ -28,12 +28,13 @@
 //
 // Small core rounds: most of the thousands of core rounds of a power-law graph are small (R-MAT scale 22: 9,543
 // rounds, nine in ten with at most 131,072 alive vertices, the median removing three), and a grid round of three
-// dependent kernels costs tens of microseconds of launch and drain latency whatever its size. In graph mode the core
-// round's body therefore starts with k_core_small_rounds, ONE thread block cluster (16 CTAs of 1,024 threads, 8 where
-// 16 cannot be co-scheduled) that keeps the whole loop state in its shared memory and runs consecutive rounds itself
-// with cluster barriers between the phases, for as long as the alive list fits its slots and the next round reads at
-// most kSmallWork incidence entries. The first round that does not fit is left untouched for the grid kernels that
-// follow in the same body; the loop decisions and every result are the grid round's, so the output is unchanged.
+// dependent kernels costs tens of microseconds of launch and drain latency whatever its size. The body of a captured
+// core round therefore starts with k_core_small_rounds (a loop that fits from the start launches it directly), ONE
+// cluster (16 CTAs of 1,024 threads, 8 where 16 cannot be co-scheduled) that keeps the whole loop state in its shared
+// memory and runs consecutive rounds itself with cluster barriers between the phases, for as long as the alive list
+// fits its slots and the next round reads at most kSmallWork incidence entries. The first round that does not fit is
+// left untouched for the grid kernels that follow in the same body; the loop decisions and every result are the grid
+// round's, so the output is unchanged.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -162,10 +163,10 @@ struct MarkShared {
     uint32_t n[3][kMarkThreads / 32], base[3];
 };
 
-// Appends this block's vertices (one per thread, every thread calls it): frontier vertices `rem` with their update items
-// - ceil(|Tri(v)| / kListChunk) slices of v's incidence list, or ceil(deg(v) / kChunk) of its neighbours without lists -
-// and survivors `keep` to the next alive list. One atomic per block and list: with one per warp, the first round over
-// eight million vertices waited for 750,000 atomics on three addresses (0.55 ms).
+// Appends this block's vertices (one per thread, every thread calls it): frontier vertices `rem` with their update
+// items (ceil(|Tri(v)| / kListChunk) slices of v's incidence list, or ceil(deg(v) / kChunk) of its neighbours without
+// lists) and survivors `keep` to the next alive list. One atomic per block and list: with one per warp, the first round
+// over eight million vertices waited for 750,000 atomics on three addresses (0.55 ms).
 __device__ __forceinline__ void append_block(bool rem, bool keep, uint32_t v, const uint32_t* __restrict__ degree,
                                              const unsigned long long* __restrict__ inc_ptr, LoopScalars* sc,
                                              uint32_t* __restrict__ frontier, uint32_t* __restrict__ item_x,
@@ -681,10 +682,11 @@ constexpr uint32_t kSmallThreads = 1024;     // threads per CTA of the cluster
 constexpr uint32_t kSmallSlots = 8192;       // local vertices per CTA (8 per thread): 131,072 with 16 CTAs
 constexpr uint32_t kSmallWork = 1u << 20;    // incidence entries a round may read in the cluster
 constexpr uint32_t kSmallMaxCtas = 16;
-// The candidates a round can have (each CTA publishes up to kSmallFront / C) and the slots of a CTA's table of decrements:
-// with 2,048 and 4,096 the CTA left 28 KB of L1, a fraction of the lines a round's local ids lie in, with these 60 KB
-// (R-MAT 22 cores 105.5 -> 98.9 ms; 640 candidates send rounds of the 8,298-vertex graph to the grid, 1,024 slots are
-// too few for the thousand vertices a round touches: 103.2 ms).
+// The candidates a round can have - each CTA publishes up to kSmallFront / C of its own, so a round with 65 on one of
+// 16 CTAs already goes to the grid - and the slots of a CTA's table of decrements: with 2,048 and 4,096 the CTA left 28
+// KB of L1, a fraction of the lines a round's local ids lie in, with these 60 KB (R-MAT 22 cores 105.5 -> 98.9 ms; 640
+// candidates send rounds of the 8,298-vertex graph to the grid, 1,024 slots are too few for the thousand vertices a
+// round touches: 103.2 ms).
 constexpr uint32_t kSmallFront = 1024;
 constexpr uint32_t kSmallSums = 2048;
 constexpr uint32_t kSmallSumsBits = 11, kSmallSumsTries = 8;
@@ -889,7 +891,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
         // itself; more are spread over the block.
         const bool wide = F > 32;
         SmallEntry e = {0, 0, 0, 0};
-        uint32_t work = 0;   // capped lengths: a sum over at most 2,048 lists fits 32 bits
+        uint32_t work = 0;   // capped lengths: a sum over at most kSmallFront lists fits 32 bits
         for (uint32_t f0 = wide ? 32 * warp : 0; f0 < F; f0 += kSmallThreads) {   // warp-uniform
             const uint32_t f = f0 + lane;
             uint32_t c = 0, before = 0;   // the CTA of candidate f: the last taking one whose range starts at or below f
@@ -945,8 +947,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_core_small_rounds(
                     const uint32_t x = __shfl_sync(GA_FULL_MASK, e.lid, o);
                     const uint32_t xl = __shfl_sync(GA_FULL_MASK, len, o);
                     const uint32_t first = (j - __shfl_sync(GA_FULL_MASK, ci - nc, o)) * chunk;
-                    const unsigned long long b = (unsigned long long)(__shfl_sync(GA_FULL_MASK, e.len_hi, o) >> 30) << 32 |
-                                                 __shfl_sync(GA_FULL_MASK, e.beg_lo, o);
+                    const uint32_t hi = __shfl_sync(GA_FULL_MASK, e.len_hi, o) >> 30;
+                    const unsigned long long b = (unsigned long long)hi << 32 | __shfl_sync(GA_FULL_MASK, e.beg_lo, o);
                     const uint2* list = inc + b;
                     const uint32_t end = min(xl, first + chunk);
                     for (uint32_t i = first + lane; i < end; i += 128) {
@@ -1435,10 +1437,10 @@ static ga_status run_loop(ga_graph* g, uint64_t num, uint64_t den, LoopScalars* 
     bool more = true;   // the final state is still to be read
     if (n > 0) {
         const bool graph_mode = g->opt_loop_mode != 1;
-        // A core loop whose vertices fit the cluster from the start is mostly one launch of it: where the mode is left to
-        // the library, the launches are made here, with a grid round between them where a round is too large, and only a
-        // loop that keeps alternating is captured as a graph, which costs more to make and release (about 0.3 ms) than
-        // such a loop takes
+        // A core loop whose vertices fit the cluster from the start is mostly one launch of it: where the mode is left
+        // to the library, the launches are made here, with a grid round between them where a round is too large, and
+        // only a loop that keeps alternating is captured as a graph, which costs more to make and release (about 0.3
+        // ms) than such a loop takes
         const uint32_t ctas = KIND == LOOP_CORE && g->opt_loop_mode == 0 && L->lists == 1
                                   ? (uint32_t)small_round_cluster(g->device)
                                   : 0;

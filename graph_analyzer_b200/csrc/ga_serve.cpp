@@ -68,7 +68,7 @@ uint64_t estimate_bytes(const GraphEntry& e, ga_request_kind kind) {
     // CSR, src, degrees; the index: four arrays by place, positions, rows in octs with their sources, in-edges; items
     const uint64_t octs = std::min(e.octs, (m + 7 * std::min(n, m)) / 8);   // at most that in any valid CSR
     const uint64_t items = std::min(m, std::min(n, m) + e.row_work / 128 + 1);   // at the smallest item work, 1,024
-    uint64_t b = 4 * (n + 1) + 4 * (m + 4) + 4 * m + 4 * n;
+    uint64_t b = 4 * (n + 1) + 4 * (m + 1) + 4 * m + 4 * n;
     b += 16 * n + 8 * (n + 1) + 36 * octs + 8 * m + 12 * (items + 1) + 4096;
     if (kind != GA_REQ_TC) {
         const uint64_t T = e.triangles != UINT64_MAX ? e.triangles : e.tri_bound;
@@ -99,8 +99,8 @@ namespace {
 
 using namespace ga;
 
-// Evicts idle resident graphs (least recently used first) until `need` more bytes fit. `keep`: the graph they are needed
-// for, whose resident part `need` does not count. Caller holds the lock.
+// Evicts idle resident graphs (least recently used first) until `need` more bytes fit. `keep`: the graph they are
+// needed for, whose resident part `need` does not count. Caller holds the lock.
 bool make_room(ga_server* s, uint64_t need, const GraphEntry* keep) {
     while (s->reserved + need > s->cfg.hbm_budget_bytes) {
         GraphEntry* victim = nullptr;
@@ -141,8 +141,8 @@ void plan(const ga_server* s, const Request& r, const GraphEntry& e, uint64_t* n
     const bool staged = r.kind != GA_REQ_TC && e.triangles == UINT64_MAX && !*small;
     *full = estimate_bytes(e, staged ? GA_REQ_TC : r.kind);
     // bytes to reserve: the whole estimate for an upload; for a resident graph what it may still add (a loop its state
-    // and lists, a second count the index that the first did without - and nothing once that stands: the estimate is for
-    // the smallest item work, so what is left of it never comes down to zero)
+    // and lists, a second count the index that the first did without - and nothing once that stands: the estimate is
+    // for the smallest item work, so what is left of it never comes down to zero)
     const bool nothing = e.dev && e.indexed && (r.kind == GA_REQ_TC || staged);
     *need = nothing ? 0 : e.dev ? (*full > e.dev_bytes ? *full - e.dev_bytes : 0) : *full;
 }

@@ -177,8 +177,8 @@ __device__ __forceinline__ uint32_t find_member(const TcArgs<CT>& a, const Ancho
 
 // The end of a pass, called by all 256 threads of every block. In a synchronous call the blocks' triangles meet in
 // sync->acc, and the last block writes the total where the caller wants it (device, and the handle's page-locked slot
-// when the host waits for it) and leaves the counters zero for the next pass - so a count is one launch, with nothing to
-// clear before it and nothing to copy after it (901 vertices: 20 us a call with two clears and a copy around the
+// when the host waits for it) and leaves the counters zero for the next pass - so a count is one launch, with nothing
+// to clear before it and nothing to copy after it (901 vertices: 20 us a call with two clears and a copy around the
 // kernel). An enqueued pass adds to the total cleared before it: replays of captured passes overlap, and would take
 // each other's blocks for their own in counters they share.
 template <class CT>
@@ -283,10 +283,11 @@ __device__ __forceinline__ uint32_t oct_members(const TcArgs<CT>& a, const Ancho
 
 // Probes one batch of anchor `an` and books what MODE (supports, lists) asks for. A lane takes an oct and finds all its
 // members; the hits of the 32 octs, a fifth to a quarter of the entries and unevenly spread, are then dealt out to the
-// lanes 32 at a time, so the booking runs with full warps, and neighbouring lanes hold hits of one oct (their increments
-// of the edges u->x share a sector; the entries of the anchor's list are consecutive). What an oct's triangles have in
-// common (the edge u->v, u's list) is booked once per oct. Returns this lane's hits. (R-MAT 22 edge supports: booking
-// inside the probe of each entry 7.4 ms; a loop over a lane's own hits 7.8 ms, 290 instructions a hit, most lanes idle.)
+// lanes 32 at a time, so the booking runs with full warps, and neighbouring lanes hold hits of one oct (their
+// increments of the edges u->x share a sector; the entries of the anchor's list are consecutive). What an oct's
+// triangles have in common (the edge u->v, u's list) is booked once per oct. Returns this lane's hits. (R-MAT 22 edge
+// supports: booking inside the probe of each entry 7.4 ms; a loop over a lane's own hits 7.8 ms, 290 instructions a
+// hit, most lanes idle.)
 template <int MODE, bool ALIVE, class CT>
 __device__ __forceinline__ uint32_t probe_batch(const TcArgs<CT>& a, uint32_t kb, uint32_t kend, const uint32_t* key,
                                                 const uint16_t* pre, uint32_t* cnt, const Anchor& an, uint32_t* s_incl,
@@ -468,10 +469,11 @@ __device__ __forceinline__ void build_table(const TcArgs<CT>& a, const Anchor& a
 // Heavy anchors use a bitmap of N+(v) instead of a hash set when it fits the table's shared memory: every
 // out-neighbour's place is above v's own, and for the anchors of many out-neighbours (high degree) they lie in a short
 // range (R-MAT 22: under 65,536 places for every anchor of more than 128 out-neighbours, against 4.2M vertices). Bit o
-// of the bitmap is set iff place v + 1 + o is an (alive) out-neighbour of v; span = the largest out-neighbour - v bounds
-// o. A probe is then one shared 32-bit load and a bit test, with no collisions and nothing to continue; the entries
-// before the suffix and the padding fall outside [0, span). Supports also need which member it is: pre[w], the members
-// below word w, plus a population count: the rank among the row's (alive) members, which the flush goes through again.
+// of the bitmap is set iff place v + 1 + o is an (alive) out-neighbour of v; span = the largest out-neighbour - v
+// bounds o. A probe is then one shared 32-bit load and a bit test, with no collisions and nothing to continue; the
+// entries before the suffix and the padding fall outside [0, span). Supports also need which member it is: pre[w], the
+// members below word w, plus a population count: the rank among the row's (alive) members, which the flush goes through
+// again.
 template <int MODE, bool ALIVE, class CT>
 __device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& an, uint32_t* bm, uint16_t* pre,
                                              uint32_t* cnt) {
@@ -494,7 +496,8 @@ __device__ __forceinline__ void build_bitmap(const TcArgs<CT>& a, const Anchor& 
         const uint32_t words = (an.span + 31) >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t per = ((words + kWarps - 1) / kWarps + 31) & ~31u, w0 = warp * per, w1 = min(words, w0 + per);
         uint32_t run = 0;
-        for (uint32_t w = w0; w < w1; w += 32) run += __reduce_add_sync(GA_FULL_MASK, w + lane < w1 ? __popc(bm[w + lane]) : 0);
+        for (uint32_t w = w0; w < w1; w += 32)
+            run += __reduce_add_sync(GA_FULL_MASK, w + lane < w1 ? __popc(bm[w + lane]) : 0);
         if (lane == 0) s_part[warp] = run;
         __syncthreads();
         run = 0;
@@ -551,8 +554,8 @@ __device__ __forceinline__ uint32_t oct_common(const uint32_t (&x)[8], const uin
     return c;
 }
 
-// Common places of an in-edge's suffix (x: its first oct, q, of `octs`) and its anchor's row (octs r.. up to rend): both
-// ascend, so the oct with the smaller last entry is done after one comparison of all pairs. hit(place) as above.
+// Common places of an in-edge's suffix (x: its first oct, q, of `octs`) and its anchor's row (octs r.. up to rend):
+// both ascend, so the oct with the smaller last entry is done after one comparison of all pairs. hit(place) as above.
 template <bool BOOK, class F>
 __device__ __forceinline__ uint32_t suffix_common(const uint32_t* __restrict__ colr, uint32_t (&x)[8], size_t q,
                                                   uint32_t octs, size_t r, size_t rend, F hit) {
@@ -646,8 +649,8 @@ __device__ __forceinline__ void flush_counts(const TcArgs<CT>& a, const Anchor& 
     }
 }
 
-// esup[e] = esupk at the padded position of edge e's entry in its row: the place of col[e], found in the (short, sorted)
-// row. Every edge is written, so esup needs no clearing.
+// esup[e] = esupk at the padded position of edge e's entry in its row: the place of col[e], found in the (short,
+// sorted) row. Every edge is written, so esup needs no clearing.
 __global__ void k_esup_fold(TcIndex ix, const uint32_t* __restrict__ src, const uint32_t* __restrict__ col, uint32_t m,
                             const uint32_t* __restrict__ esupk, uint32_t* __restrict__ esup) {
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -668,10 +671,9 @@ __global__ void k_alive_places(const uint8_t* __restrict__ alive, const uint32_t
 // (heavy, light, tiny); null means every item. tiny_groups: counts of the whole graph take the tiny bin in groups of 32
 // places from tiny_first on; otherwise its items are run like light ones.
 template <int MODE, bool ALIVE, class CT>
-__global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA_TC_MIN_BLOCKS) k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds,
-                                                      uint32_t heavy_bits_max,
-                                                      uint32_t tiny_first, uint32_t tiny_end, uint32_t light_max_deg,
-                                                      TcArgs<CT> a) {
+__global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA_TC_MIN_BLOCKS)
+k_tc_hash(ga_items items, const uint32_t* __restrict__ bounds, uint32_t heavy_bits_max, uint32_t tiny_first,
+          uint32_t tiny_end, uint32_t light_max_deg, TcArgs<CT> a) {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t s_item, s_next;
     constexpr int W = SlotLayout<MODE>::words;
@@ -712,7 +714,8 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
             // counters of the support modes behind it
             const uint32_t span = a.ix.colr[(size_t)an.row * 8 + an.dv - 1] - an.v;
             const uint32_t words = (span + 127) >> 7 << 2, ranks = counters(MODE) ? words / 2 : 0;
-            const bool bitmap = a.bitmaps && words + ranks + (counters(MODE) ? an.dv : 0u) <= Smax * W && an.dv <= 0xFFFFu;
+            const bool bitmap =
+                a.bitmaps && words + ranks + (counters(MODE) ? an.dv : 0u) <= Smax * W && an.dv <= 0xFFFFu;
             an.span = bitmap ? span : 0u;
             an.bits = bitmap ? 0u : table_bits(an.dv, heavy_bits_max);
             uint16_t* pre = reinterpret_cast<uint16_t*>(key + words);
@@ -795,8 +798,8 @@ __global__ void __launch_bounds__(kThreads, MODE == TC_COUNT ? kCountBlocks : GA
     if constexpr (MODE == TC_COUNT && !ALIVE) {
         if (groups) {
             const uint32_t ngroups = (uint32_t)(((uint64_t)tiny_end - tiny_first + 31) / 32);
-            // four groups a fetch, but no more than a warp's share: a group is a chain of up to 32 rounds of loads, and on
-            // small graphs four of them were the kernel (R-MAT 16 count 61.7 -> 49.7 us, R-MAT 18 127.7 -> 122.1)
+            // four groups a fetch, but no more than a warp's share: a group is a chain of up to 32 rounds of loads, and
+            // on small graphs four of them were the kernel (R-MAT 16 count 61.7 -> 49.7 us, R-MAT 18 127.7 -> 122.1)
             const uint32_t take = min(kTinyGroups, max(1u, ngroups / (gridDim.x * kWarps)));
             for (;;) {
                 uint32_t g0 = 0;
@@ -1003,9 +1006,10 @@ static ga_status launch_hash(ga_graph* g, const TcArgs<CT>& a) {
     return GA_OK;
 }
 
-// One pass on the index (octs: one thread per in-edge, else the hash kernel). Per-vertex outputs are the caller's, by id:
-// by place the hubs' counters would be neighbours, and the atomics on them meet in a few L2 sectors (vertex supports of
-// R-MAT 18: 1.06 ms against 0.78). Per-edge outputs are by position in colr and moved to the caller's col order.
+// One pass on the index (octs: one thread per in-edge, else the hash kernel). Per-vertex outputs are the caller's, by
+// id: by place the hubs' counters would be neighbours, and the atomics on them meet in a few L2 sectors (vertex
+// supports of R-MAT 18: 1.06 ms against 0.78). Per-edge outputs are by position in colr and moved to the caller's col
+// order.
 template <int MODE, bool ALIVE, class CT>
 static ga_status launch_index(ga_graph* g, const TcArgs<CT>& a0, bool octs) {
     cudaStream_t st = g->stream;
@@ -1073,8 +1077,8 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
                                             ? g->tuned_kernel
                                             : 2;
     if (g->n > kTabEmpty) kernel = 1;   // ids of kTabEmpty and above do not fit the hash kernel's table slots
-    // the one-thread-per-edge form on the index for counts of any kind (per-edge supports are written in col's own order
-    // by the plain form, without a pass to move them: 400 us vs 590); shards cut the edges themselves
+    // the one-thread-per-edge form on the index for counts of any kind (per-edge supports are written in col's own
+    // order by the plain form, without a pass to move them: 400 us vs 590); shards cut the edges themselves
     const bool octs = kernel == 1 && (MODE == TC_COUNT || MODE == TC_VSUP) && a.nshards <= 1 && g->n <= kTabEmpty;
     const bool index = (kernel != 1 || octs) && g->m;
     cudaStream_t st = g->stream;
@@ -1102,15 +1106,15 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
 
 // ---- autotuner ----------------------------------------------------------------------------------------------------
 // What runs fastest depends on the degree distribution: on graphs whose out-lists are all short (Holme-Kim with a
-// handful of edges per vertex) the one-thread-per-in-edge form (k_tc_octs, choice 1) can win, on skewed graphs with long
-// lists (R-MAT) the degree-binned hash kernel wins by several times, and within the hash kernel the bin cutoff between per-warp and block-wide sets
-// (light_max_deg) and the probe work per item (item_work, which sets how many warps share an anchor) move the time
-// by some percent. The choice - kernel, cutoff, item work - is cached per degree-distribution signature: log2 of n
-// and m and the fraction of edges whose source has out-degree in each log2 bucket, in sixteenths. A signature seen
-// before is answered from the cache (process-wide; also kept in the file named by GA_TUNE_CACHE when that is set); a
-// new one is decided by timing candidates on the graph: both forms at the current options,
-// then the cutoffs {32, 64, 128, 256} and the item works {1024, 4096, 16384} (coordinate-wise; options the caller
-// set explicitly stay as set). Every candidate gives the same count.
+// handful of edges per vertex) the one-thread-per-in-edge form (k_tc_octs, choice 1) can win, on skewed graphs with
+// long lists (R-MAT) the degree-binned hash kernel wins by several times, and within the hash kernel the bin cutoff
+// between per-warp and block-wide sets (light_max_deg) and the probe work per item (item_work, which sets how many
+// warps share an anchor) move the time by some percent. The choice - kernel, cutoff, item work - is cached per
+// degree-distribution signature: log2 of n and m and the fraction of edges whose source has out-degree in each log2
+// bucket, in sixteenths. A signature seen before is answered from the cache (process-wide; also kept in the file named
+// by GA_TUNE_CACHE when that is set); a new one is decided by timing candidates on the graph: both forms at the current
+// options, then the cutoffs {32, 64, 128, 256} and the item works {1024, 4096, 16384} (coordinate-wise; options the
+// caller set explicitly stay as set). Every candidate gives the same count.
 
 struct TuneChoice {
     int kernel = 2;
@@ -1278,12 +1282,13 @@ ga_status autotune(ga_graph* g) {
 
 // The first count of a graph that nothing has prepared, when the one-thread-per-edge form is known to be its choice (by
 // option or from the signature cache): counted straight from the CSR, since that form's plain version needs no index
-// and building one costs more than a single count saves. The choice was made for k_tc_octs and this runs k_tc_plain, which
-// loses more on longer rows; but where it loses to index + octs, the choice is the hash form. First calls on a new
-// handle, us, k_tc_plain / index + k_tc_octs / index + hash, with row_work / m (octs to an edge's row):
-//   chosen:     Holme-Kim 8,298 vertices 17-24 / 117-153 / 154-198 (1.0-2.5), 1.7M 155 / 600 / 782 (1.0), 381 / 946 / 1,202
-//               (1.1), 1,718 / 2,860 / 3,119 (2.5); R-MAT 10 18-25 / 85-92 / 102-117 (1.1-3.1), R-MAT 14 25-39 / 148-169 /
-//               183-211 (1.7-4.1), R-MAT 16 51 / 181 / 231 (3.4), R-MAT 18 77 / 239 / 284 (2.7)
+// and building one costs more than a single count saves. The choice was made for k_tc_octs and this runs k_tc_plain,
+// which loses more on longer rows; but where it loses to index + octs, the choice is the hash form. First calls on a
+// new handle, us, k_tc_plain / index + k_tc_octs / index + hash, with row_work / m (octs to an edge's row):
+//   chosen:     Holme-Kim 8,298 vertices 17-24 / 117-153 / 154-198 (1.0-2.5), 1.7M vertices 155 / 600 / 782 (1.0),
+//               381 / 946 / 1,202 (1.1), 1,718 / 2,860 / 3,119 (2.5); R-MAT 10 18-25 / 85-92 / 102-117 (1.1-3.1),
+//               R-MAT 14 25-39 / 148-169 / 183-211 (1.7-4.1), R-MAT 16 51 / 181 / 231 (3.4), R-MAT 18 77 / 239 / 284
+//               (2.7)
 //   not chosen: R-MAT 18 589 / 617 / 433 (8.0), 1,874 / 1,416 / 605 (14.0); Holme-Kim 1.7M 7,755 / 6,902 / 5,579 (4.9)
 // A second count shows that the graph stays in use and builds the index. Misoriented graphs go on to ready(), which
 // refuses them.
@@ -1436,8 +1441,8 @@ ga_status ga_tc_participation(ga_graph* g, const uint8_t* alive, uint32_t* tri, 
     GA_GRAPH_LOCK(g);
     GA_TRY(use_device(g));
     GA_TRY(ready(g));
-    // T of the alive subgraph is at most T of the graph; refuse when uint32 counters could overflow (densest.h:68). T is
-    // at most sum over u of C(d+(u), 2), and that at most 4 * row_work: only above 2^32 does it take a count to know
+    // T of the alive subgraph is at most T of the graph; refuse when uint32 counters could overflow (densest.h:68). T
+    // is at most sum over u of C(d+(u), 2), and that at most 4 * row_work: only above 2^32 does it take a count to know
     if (g->row_work >= (1ull << 30)) {
         uint64_t T_full = 0;
         GA_TRY(ga_tc_count(g, &T_full));

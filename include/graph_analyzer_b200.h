@@ -177,9 +177,10 @@ typedef enum ga_option {
     GA_OPT_LIGHT_MAX_DEG = 6, /* anchors with out-degree <= this use per-warp tables (0 = 128, at most 256)        */
     GA_OPT_UPDATE_MODE = 7,   /* peeling/core rounds: 0 auto (triangle incidence lists when their 24*T bytes fit,
                                  else re-enumeration), 1 re-enumerate the frontier's triangles, 2 incidence lists   */
-    GA_OPT_COUNT_BITMAP = 8   /* passes of the hash kernel: 0 auto (a heavy anchor whose out-neighbours lie within
-                                 32 x the table's words of places above it in the (degree, id) order is probed
-                                 against a bitmap of them), 1 hash sets for every anchor                            */
+    GA_OPT_COUNT_BITMAP = 8   /* passes of the hash kernel: 0 auto (a heavy anchor is probed against a bitmap of its
+                                 out-neighbours' places in the (degree, id) order where that fits the table's words:
+                                 in counts a range of 32 places a word, in supports less, by the ranks and counters
+                                 beside it), 1 hash sets for every anchor                                           */
 } ga_option;
 ga_status ga_graph_set_option(ga_graph* g, ga_option opt, int64_t value);
 
@@ -193,8 +194,8 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles);
  * counts and shards captured from one handle may overlap each other and the handle's other calls on any streams, as
  * long as their totals are different memory (in the hash kernel up to 64 captured passes of a handle; the 65th
  * shares its work queues with the first). A captured pass keeps the options and work lists it was captured with.
- * A handle is captured after ga_graph_prepare or a first call; before, the call would build what the handle keeps inside
- * the capture, and is refused (GA_ERR_CUDA), as are its synchronous calls. */
+ * A handle is captured after ga_graph_prepare or a first call; before, the call would build what the handle keeps
+ * inside the capture, and is refused (GA_ERR_CUDA), as are the synchronous calls. */
 ga_status ga_tc_count_async(ga_graph* g, uint64_t* d_triangles);
 
 /* Sharded count, for counting one graph on several GPUs (no counterpart in the reference, which runs on one GPU):
