@@ -116,14 +116,13 @@ struct ga_items {
 // Counters of a handle's triangle passes (device). Synchronous calls use the first work queues, `ticket` (blocks that
 // have finished) and `acc` (triangles so far), all zero between passes: the last block of a pass clears them. A pass
 // that an _async call enqueues shares none of these, since it may be captured and replayed beside other passes: it adds
-// to the caller's total, and its work queues, cleared before it, are the second ones, or for a captured pass the next
-// of the rest. bounds: the item ranges of a shard.
-constexpr uint32_t kCapturedWork = 64;
+// to the caller's total, and its work queues, cleared before it, are the second ones, or for a captured pass its own
+// (captured_work). bounds: the item ranges of a shard.
 struct ga_work {
     uint32_t queue[4], bounds[6];
 };
 struct ga_sync {
-    ga_work work[2 + kCapturedWork];
+    ga_work work[2];
     uint32_t ticket, pad;
     unsigned long long acc;
 };
@@ -172,7 +171,8 @@ struct ga_graph {
     unsigned long long* d_scalars = nullptr;   // 64 slots
     unsigned long long* h_scalars = nullptr;   // their page-locked host side (64 slots; host_slot_acquire)
     ga_sync* sync = nullptr;                   // counters of the triangle passes
-    uint32_t captured = 0;                     // passes captured so far (whose work queues are next)
+    ga_work* captured = nullptr;               // work queues for the next captured passes ...
+    uint32_t captured_left = 0;                // ... and how many there are
     bool items_captured = false;               // a captured pass reads the current work lists
 
     // options (ga_option)
@@ -276,6 +276,8 @@ ga_status prepare_shards(ga_graph* g);
 // What the pass of an _async call needs. The call may be captured on a handle that is prepared, or that has been
 // counted without the index: what is missing then is built beside the capture.
 ga_status prepare_enqueued(ga_graph* g, bool shards);
+// Work queues for a pass being captured: no other pass's. Allocated 64 at a time, beside the capture.
+ga_status captured_work(ga_graph* g, ga_work** work);
 
 // Picks the count kernel for GA_OPT_TC_KERNEL = 0 from the graph's degree-distribution signature (cached per
 // signature; times both kernels once for a new one). Called by ga_graph_prepare.

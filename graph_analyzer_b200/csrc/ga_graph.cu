@@ -930,12 +930,10 @@ ga_status prepare_shards(ga_graph* g) {
     return s;
 }
 
-ga_status prepare_enqueued(ga_graph* g, bool shards) {
-    if (g->prepared && (!shards || g->anchor_work)) return GA_OK;
-    const bool counted = g->counted_bare && !g->index_ready;   // nothing of the handle is pending on its stream
-    if ((!g->prepared && !counted) || not_captured(g) == GA_OK) return shards ? prepare_shards(g) : prepare(g);
-    clear_error();
-    // on another stream, behind the last build, and complete before the pass is recorded
+// Runs `make` with g on another stream, behind the last build, and waits for it: what it builds is complete before a pass
+// that needs it is recorded in the capture of g's own stream.
+template <class F>
+static ga_status beside_capture(ga_graph* g, F make) {
     cudaStream_t own = g->stream, side = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     GA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
@@ -945,7 +943,7 @@ ga_status prepare_enqueued(ga_graph* g, bool shards) {
         s = fail(GA_ERR_CUDA, "cudaStreamWaitEvent failed");
     if (s == GA_OK) {
         g->stream = side;
-        s = shards ? prepare_shards(g) : prepare(g);
+        s = make();
         g->stream = own;
     }
     if (side && cudaStreamSynchronize(side) != cudaSuccess && s == GA_OK)
@@ -953,6 +951,25 @@ ga_status prepare_enqueued(ga_graph* g, bool shards) {
     if (side) stream_release(g->device, side);
     cudaThreadExchangeStreamCaptureMode(&mode);
     return s;
+}
+
+ga_status prepare_enqueued(ga_graph* g, bool shards) {
+    if (g->prepared && (!shards || g->anchor_work)) return GA_OK;
+    const bool counted = g->counted_bare && !g->index_ready;   // nothing of the handle is pending on its stream
+    if ((!g->prepared && !counted) || not_captured(g) == GA_OK) return shards ? prepare_shards(g) : prepare(g);
+    clear_error();
+    return beside_capture(g, [&] { return shards ? prepare_shards(g) : prepare(g); });
+}
+
+ga_status captured_work(ga_graph* g, ga_work** work) {
+    if (!g->captured_left) {
+        constexpr uint32_t kSlab = 64;
+        GA_TRY(beside_capture(g, [&] { return dalloc(g, &g->captured, kSlab); }));
+        g->captured_left = kSlab;
+    }
+    *work = g->captured++;
+    g->captured_left--;
+    return GA_OK;
 }
 
 static ga_status create_common(const uint32_t* rowptr, const uint32_t* col, uint32_t n, uint32_t m, int device,

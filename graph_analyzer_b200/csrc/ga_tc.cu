@@ -1097,8 +1097,12 @@ ga_status run_tc(ga_graph* g, const TcArgs<CT>& a0, bool zero_outputs) {
     } else if (index && !octs) {   // the hash kernel's queues
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         GA_CUDA(cudaStreamIsCapturing(st, &capture));
-        g->items_captured |= capture != cudaStreamCaptureStatusNone;
-        a.work += capture == cudaStreamCaptureStatusNone ? 1 : 2 + g->captured++ % kCapturedWork;
+        if (capture == cudaStreamCaptureStatusNone) {
+            a.work++;
+        } else {
+            GA_TRY(captured_work(g, &a.work));
+            g->items_captured = true;
+        }
         GA_CUDA(cudaMemsetAsync(a.work->queue, 0, sizeof a.work->queue, st));
     }
     return index ? launch_index<MODE, ALIVE, CT>(g, a, octs) : launch_plain<MODE, ALIVE, CT>(g, a);
@@ -1348,7 +1352,6 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles) {
         GA_TRY((run_tc<TC_COUNT, false, unsigned int>(g, a, true)));
         return read_total(g, triangles);
     }
-    GA_TRY(not_captured(g));
     a.sync = g->sync;
     a.work = g->sync->work;
     GA_TRY((launch_plain<TC_COUNT, false, unsigned int>(g, a)));

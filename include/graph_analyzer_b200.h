@@ -192,8 +192,7 @@ ga_status ga_tc_count(ga_graph* g, uint64_t* triangles);
  * (8 bytes) without a host sync (kernels.cuh's "unsigned long long* total" output). Call ga_graph_prepare first if
  * the launch must not include the one-time preparation. The _async calls can be captured into CUDA graphs; replays of
  * counts and shards captured from one handle may overlap each other and the handle's other calls on any streams, as
- * long as their totals are different memory (in the hash kernel up to 64 captured passes of a handle; the 65th
- * shares its work queues with the first). A captured pass keeps the options and work lists it was captured with.
+ * long as their totals are different memory. A captured pass keeps the options and work lists it was captured with.
  * A handle is captured after ga_graph_prepare or a first call; before, the call would build what the handle keeps
  * inside the capture, and is refused (GA_ERR_CUDA), as are the synchronous calls. */
 ga_status ga_tc_count_async(ga_graph* g, uint64_t* d_triangles);

@@ -358,3 +358,16 @@ def test_autotuner_loads_what_it_times(lib):
     timed = {line.split()[1] for line in log if line.startswith("launch") and "k_tc_" in line}
     assert len(timed) == 2 and timed == loaded
     assert lib.ga_graph_destroy(g) == 0
+
+
+def test_every_captured_pass_has_its_own_queues(lib):
+    s, g = lib.graph()
+    assert s == 0 and lib.ga_graph_set_option(g, OPT_TC_KERNEL, C.c_int64(2)) == 0 and lib.ga_graph_prepare(g) == 0
+    cleared = set()
+    for _ in range(150):
+        s, log = captured_call(lib, g, lambda g: CALLS["async"](lib, g))
+        inside = [line for line in log if line.endswith("captured")]
+        assert s == 0 and not [line for line in inside if line.startswith("alloc")]
+        cleared |= {line for line in inside if line.startswith("memset") and str(C.addressof(TOTAL)) not in line}
+    assert len(cleared) == 150
+    assert lib.ga_graph_destroy(g) == 0 and lib.leaked() == 0
